@@ -1,0 +1,507 @@
+// The tile body of the box-mass gather (FP64 form, all kernels): one CTA takes one 8 x 8 x 8 cell tile, shared
+// by the single-grid kernels and the batch's persistent kernel.
+//
+// Per particle of the tile's list, the box of its support clipped to the tile (n0 x n1 x n2 cells) has
+// n0' + n1' + n2' planes (n' = n + 1), n0' n1' + n0' n2' + n1' n2' edge lines and n0' n1' n2' lattice points.
+// A plane's record, an edge line's record and a point's box mass are formed once each (box_math.cuh); a cell
+// of the box is the alternating sum of its eight corners' masses, which is the reference's sum over the cell's
+// 6 faces x 4 edges x 2 vertex pyramids regrouped by corner (src/cartesian_grid.cpp:246-259,
+// src/kernel_integral.cpp:471-647).
+//
+// The list (ascending particle index) is walked in chunks, in phases separated by barriers:
+//   (E) edge lines; warp 0 first loads the next chunk (particles, boxes, offsets) into the other buffer;
+//   (P) points;
+//   (C1) every (particle, cell of its box) pair as one flat list: support test, counters, alternating sum;
+//   (C2) each thread adds, for the cells it owns, the chunk's pairs in particle order, so that every cell's sum
+//        runs over its particles in ascending index order with no atomics; and the next chunk's planes.
+// Within (E) and (P) a warp walks its share of the flat list and sorts what it meets by cost: the cheap items
+// (lines and points beyond the support) it finishes at once, the others it queues by kind (a line by its piece, a
+// point within the support) and evaluates 32 of a kind at a time, so that no lane waits for another kind's work
+// and no list is shared between warps.
+//
+// What bounds it: the FP64 pipe and the shared-memory loads of the records, about equally (a point within the
+// support issues about 150 FP64 instructions and 20 shared loads).
+#pragma once
+
+#include <climits>
+
+#include "box_math.cuh"
+#include "engine.hpp"
+#include "lattice.cuh"
+
+namespace kiwi_b200 {
+
+#ifndef KIWI_BOX_THREADS
+#define KIWI_BOX_THREADS 256
+#endif
+constexpr int kBoxThreads = KIWI_BOX_THREADS;
+constexpr int kBoxWarps = kBoxThreads / 32;
+constexpr int kBoxCells = (kTileCells + kBoxThreads - 1) / kBoxThreads;  // cells a thread owns
+constexpr int kBoxPMax = 32;                                            // particles per chunk
+#ifndef KIWI_BOX_PT_CAP
+#define KIWI_BOX_PT_CAP 2304
+#endif
+#ifndef KIWI_BOX_PAIR_CAP
+#define KIWI_BOX_PAIR_CAP 1024
+#endif
+#ifndef KIWI_BOX_PLANE_CAP
+#define KIWI_BOX_PLANE_CAP 296
+#endif
+constexpr int kBoxPtCap = KIWI_BOX_PT_CAP;        // lattice points per chunk (a full 8^3 box has 729)
+constexpr int kBoxPairCap = KIWI_BOX_PAIR_CAP;    // edge lines per chunk (a full box has 243)
+constexpr int kBoxPlaneCap = KIWI_BOX_PLANE_CAP;  // planes per chunk (a full box has 27)
+// The three-piece kernels' records are larger: fewer lines and planes in the same shared memory.
+constexpr int kBoxGenPtCap = 1792, kBoxGenPairCap = 640, kBoxGenPlaneCap = 256;
+static_assert(kBoxPairCap <= 1024 && kBoxPlaneCap <= 512, "packed edge entries");
+
+template <int NP>
+struct BoxCaps {
+    static constexpr int kN = NP ? NP : KIWI_BOX_PIECES;
+    static constexpr int kPt = NP ? kBoxPtCap : kBoxGenPtCap;
+    static constexpr int kPair = NP ? kBoxPairCap : kBoxGenPairCap;
+    static constexpr int kPlane = NP ? kBoxPlaneCap : kBoxGenPlaneCap;
+    static constexpr int kQueues = kN;  // edge kinds; the point phase uses the first
+    // dynamic shared memory, in doubles: the cells' sums, the octant values, the edge and plane records
+    static constexpr int kOffT = 4 * kTileCells;
+    static constexpr int kOffE = kOffT + kPt;
+    static constexpr int kOffP = kOffE + box_edge_stride(kN) * kPair;
+    static constexpr int kEnd = kOffP + box_plane_stride(kN) * kPlane;
+    static constexpr size_t kSmem = sizeof(double) * kEnd + sizeof(uint32_t) * 64 * kBoxWarps * kQueues;
+    // (C1) keeps the pairs' values in the edge records' place (with one piece the records are smaller)
+    static_assert((NP ? box_edge_stride(kN) : box_edge_stride(1)) * kPair >= kPt, "pair values fit");
+};
+
+// One chunk of a tile's particle list: the particles' data, their boxes clipped to the tile (lo, dim), their
+// first plane, edge line, point and cell, and the magic divisors of their dimensions.
+struct BoxChunk {
+    double x[kBoxPMax], y[kBoxPMax], z[kBoxPMax], H[kBoxPMax], iH[kBoxPMax], m[kBoxPMax], vx[kBoxPMax], vy[kBoxPMax],
+        vz[kBoxPMax];
+    int lo[kBoxPMax][3], dim[kBoxPMax][3];  // lo relative to the tile
+    int loff[kBoxPMax], eoff[kBoxPMax], poff[kBoxPMax], coff[kBoxPMax];
+    uint32_t mag[kBoxPMax][3];   // div_magic of n1', n2' and n1' n2'
+    uint32_t cmag[kBoxPMax][2];  // div_magic of n2 and n1 n2
+    int np, ltot, etot, ptot, ctot;
+};
+
+__device__ __forceinline__ void box_add_stat(unsigned long long* dst, unsigned long long v) {
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0 && v) atomicAdd(dst, v);
+}
+
+// x with the sign bits of a, b, c multiplied in.
+__device__ __forceinline__ double box_signed(double x, double a, double b, double c) {
+    const int s = (__double2hiint(a) ^ __double2hiint(b) ^ __double2hiint(c)) & (int)0x80000000;
+    return __hiloint2double(__double2hiint(x) ^ s, __double2loint(x));
+}
+
+// NP, DEG: the kernel's pieces and largest power, known when compiling (the cubic spline: 2, 3), or 0 for any
+// kernel of the tables.  T: the kernel's table in constant memory.
+template <bool CULL, int NP, int DEG>
+__device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& P, const uint32_t* __restrict__ list,
+                                         const int64_t* __restrict__ range, int64_t t_range, int64_t t,
+                                         const CartOutputs& out, DevStats* __restrict__ st, const KiwiBoxTable& T) {
+    using Caps = BoxCaps<NP>;
+    __shared__ BoxChunk s_cp[2];
+    __shared__ double s_pl[3][kTileX + 1], s_cc[3][kTileX];
+    __shared__ double s_C[NP ? 1 : (kBoxC + 1) * KIWI_BOX_PIECES];  // any kernel: c and C of its pieces (lanes differ in piece)
+    static_assert(kTileX == kTileY && kTileX == kTileZ, "cubic tiles");
+    extern __shared__ double s_dyn[];
+    const int n = NP ? NP : T.npiece;
+    const int kPS = box_plane_stride(n), kES = box_edge_stride(n);
+    double* const s_acc = s_dyn;
+    double* const s_T = s_dyn + Caps::kOffT;
+    double* const s_E = s_dyn + Caps::kOffE;
+    double* const s_P = s_dyn + Caps::kOffP;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1;
+    uint32_t* const s_q = reinterpret_cast<uint32_t*>(s_dyn + Caps::kEnd) + 64 * Caps::kQueues * warp;
+
+    const int tz = (int)(t % g.ntz), ty = (int)((t / g.ntz) % g.nty), tx = (int)(t / ((int64_t)g.ntz * g.nty));
+    const int bx = tx * kTileX, by = ty * kTileY, bz = tz * kTileZ;
+    // the tile's lattice planes and cell centres, formed as the reference forms them
+    if (threadIdx.x < 3 * (kTileX + 1)) {
+        const int a = threadIdx.x / (kTileX + 1), l = threadIdx.x % (kTileX + 1);
+        const double mn = a == 0 ? g.x_min : (a == 1 ? g.y_min : g.z_min), d = a == 0 ? g.dpx : (a == 1 ? g.dpy : g.dpz);
+        const int b0 = a == 0 ? bx : (a == 1 ? by : bz);
+        s_pl[a][l] = add_rn(mn, mul_rn((double)(b0 + l), d));
+        if (l < kTileX) s_cc[a][l] = cell_centre(mn, b0 + l, d);
+    }
+    if (!NP)
+        for (int i = threadIdx.x; i < (kBoxC + 1) * n; i += kBoxThreads) {
+            const int k = i / (kBoxC + 1), c = i % (kBoxC + 1);
+            s_C[i] = c < kBoxC ? T.reg[k].C[c] : T.reg[k].c;
+        }
+    for (int i = threadIdx.x; i < 4 * kTileCells; i += kBoxThreads) s_acc[i] = 0.0;
+
+    // work counters: 32-bit per thread, flushed to the 64-bit totals every 2^16 chunks and at the end
+    unsigned n_bbox = 0, n_sphere = 0, n_eval = 0, n_neg = 0, n_warn = 0, n_eo = 0, n_em = 0, n_ei = 0, n_vp = 0,
+             n_chunks = 0;
+    auto flush = [&]() {
+        box_add_stat(&st->bbox_pairs, n_bbox);
+        box_add_stat(&st->sphere_pairs, n_sphere);
+        box_add_stat(&st->evaluated_pairs, n_eval);
+        box_add_stat(&st->neg_clamped, n_neg);
+        box_add_stat(&st->neg_warned, n_warn);
+        box_add_stat(&st->edge_outer, n_eo);
+        box_add_stat(&st->edge_middle, n_em);
+        box_add_stat(&st->edge_inner, n_ei);
+        box_add_stat(&st->vertex_pyramids, n_vp);
+        n_bbox = n_sphere = n_eval = n_neg = n_warn = n_eo = n_em = n_ei = n_vp = 0;
+    };
+    const int64_t beg = range[2 * t_range], end = range[2 * t_range + 1];
+
+    // warp 0: the chunk of the particle list starting at `at` (as many particles as the capacities take)
+    auto load_chunk = [&](BoxChunk* dst, int64_t at) {
+        const int64_t idx = at + lane;
+        int nl = 0, ne = 0, npt = 0, ncl = 0, lo0 = 0, lo1 = 0, lo2 = 0, d0 = 0, d1 = 0, d2 = 0;
+        double px = 0, py = 0, pz = 0, ph = 1, pm = 0, pvx = 0, pvy = 0, pvz = 0;
+        if (idx < end) {
+            const uint32_t p = list[idx];
+            px = P.x[p]; py = P.y[p]; pz = P.z[p]; ph = P.h[p];
+            pm = P.m[p]; pvx = P.vx[p]; pvy = P.vy[p]; pvz = P.vz[p];
+            CellBox b;
+            bool outside;
+            particle_cell_box(g, px, py, pz, ph, b, &outside);
+            lo0 = max(b.x0 - bx, 0); lo1 = max(b.y0 - by, 0); lo2 = max(b.z0 - bz, 0);
+            d0 = min(b.x1 - bx, kTileX - 1) - lo0 + 1;
+            d1 = min(b.y1 - by, kTileY - 1) - lo1 + 1;
+            d2 = min(b.z1 - bz, kTileZ - 1) - lo2 + 1;
+            const int n0 = d0 + 1, n1 = d1 + 1, n2 = d2 + 1;
+            nl = n0 + n1 + n2;
+            ne = n0 * n1 + n0 * n2 + n1 * n2;
+            npt = n0 * n1 * n2;
+            ncl = d0 * d1 * d2;
+        }
+        int il = nl, ie = ne, ip = npt, ic = ncl;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int vl = __shfl_up_sync(0xffffffffu, il, o), ve = __shfl_up_sync(0xffffffffu, ie, o);
+            const int vp = __shfl_up_sync(0xffffffffu, ip, o), vc = __shfl_up_sync(0xffffffffu, ic, o);
+            if (lane >= o) {
+                il += vl;
+                ie += ve;
+                ip += vp;
+                ic += vc;
+            }
+        }
+        const bool take = idx < end && il <= Caps::kPlane && ie <= Caps::kPair && ip <= Caps::kPt;
+        const int np = __popc(__ballot_sync(0xffffffffu, take));
+        if (take) {
+            const double H = mul_rn(g.support_in_h, ph);
+            dst->x[lane] = px; dst->y[lane] = py; dst->z[lane] = pz; dst->H[lane] = H; dst->iH[lane] = 1.0 / H;
+            dst->m[lane] = pm; dst->vx[lane] = pvx; dst->vy[lane] = pvy; dst->vz[lane] = pvz;
+            dst->lo[lane][0] = lo0; dst->lo[lane][1] = lo1; dst->lo[lane][2] = lo2;
+            dst->dim[lane][0] = d0; dst->dim[lane][1] = d1; dst->dim[lane][2] = d2;
+            dst->loff[lane] = il - nl;
+            dst->eoff[lane] = ie - ne;
+            dst->poff[lane] = ip - npt;
+            dst->coff[lane] = ic - ncl;
+            dst->mag[lane][0] = div_magic(d1 + 1);
+            dst->mag[lane][1] = div_magic(d2 + 1);
+            dst->mag[lane][2] = div_magic((d1 + 1) * (d2 + 1));
+            dst->cmag[lane][0] = div_magic(d2);
+            dst->cmag[lane][1] = div_magic(d1 * d2);
+        }
+        if (lane == np - 1) {
+            dst->np = np;
+            dst->ltot = il;
+            dst->etot = ie;
+            dst->ptot = ip;
+            dst->ctot = ic;
+        }
+    };
+    // all warps: a chunk's plane records
+    auto form_planes = [&](const BoxChunk* cp) {
+        const int off_l = lane < cp->np ? cp->loff[lane] : INT_MAX, tot = cp->ltot;
+        for (int base = warp * 32; base < tot; base += kBoxThreads) {
+            const int j = warp_owner(base, off_l, lane), it = base + lane;
+            const int off = __shfl_sync(0xffffffffu, off_l, j & 31);
+            if (it < tot) {
+                int l = it - off;
+                const int n0 = cp->dim[j][0] + 1, n1 = cp->dim[j][1] + 1;
+                const int a = (l >= n0) + (l >= n0 + n1);
+                l -= a == 0 ? 0 : (a == 1 ? n0 : n0 + n1);
+                const double c = a == 0 ? cp->x[j] : (a == 1 ? cp->y[j] : cp->z[j]);
+                box_plane<NP, DEG>(T, (s_pl[a][cp->lo[j][a] + l] - c) * cp->iH[j], s_P + kPS * it);
+            }
+        }
+    };
+
+    BoxChunk* cp = &s_cp[0];
+    if (warp == 0 && beg < end) load_chunk(cp, beg);
+    __syncthreads();
+    if (beg < end) form_planes(cp);
+    __syncthreads();
+
+    for (int64_t pos = beg; pos < end;) {
+        BoxChunk* const nx = cp == &s_cp[0] ? &s_cp[1] : &s_cp[0];
+        const int np = cp->np;
+        const bool more = pos + np < end;
+        if (warp == 0 && more) load_chunk(nx, pos + np);
+
+        // (E) edge lines, block (x, y) over n0' x n1', (x, z) over n0' x n2', (y, z) over n1' x n2'
+        {
+            const int tot = cp->etot;
+            const int off_l = lane < np ? cp->eoff[lane] : INT_MAX;
+            int cnt[Caps::kQueues];
+#pragma unroll
+            for (int c = 0; c < Caps::kQueues; ++c) cnt[c] = 0;
+            for (int base = warp * 32;; base += kBoxThreads) {
+                const bool last = base >= tot;
+                if (!last) {
+                    const int j = warp_owner(base, off_l, lane), it = base + lane;
+                    const int off = __shfl_sync(0xffffffffu, off_l, j & 31);
+                    int kind = -1;
+                    uint32_t rec = 0;
+                    if (it < tot) {
+                        int e = it - off;
+                        const int n0 = cp->dim[j][0] + 1, n1 = cp->dim[j][1] + 1, n2 = cp->dim[j][2] + 1;
+                        const int nxy = n0 * n1, nxz = n0 * n2;
+                        const int blk = (e >= nxy) + (e >= nxy + nxz);
+                        e -= blk == 0 ? 0 : (blk == 1 ? nxy : nxy + nxz);
+                        const int pi = div_by(e, cp->mag[j][blk == 0 ? 0 : 1]), qi = e - pi * (blk == 0 ? n1 : n2);
+                        const int la = cp->loff[j] + (blk == 2 ? n0 : 0) + pi;
+                        const int lb = cp->loff[j] + (blk == 0 ? n0 : n0 + n1) + qi;
+                        const double p = s_P[kPS * la], q = s_P[kPS * lb];
+                        const double D = fma(p, p, q * q);
+                        if (D >= 1.0 || p == 0.0 || q == 0.0) {
+                            s_E[kES * it + 2 * n] = 0.0;
+                            n_eo += 2;
+                        } else {
+                            kind = 0;
+#pragma unroll
+                            for (int k = 0; k + 1 < n; ++k) kind += D >= T.scale[k].b * T.scale[k].b;
+                            if (kind == 0) n_ei += 2;
+                            else n_em += 2;
+                            rec = (uint32_t)it | (uint32_t)la << 10 | (uint32_t)lb << 19;
+                        }
+                    }
+#pragma unroll
+                    for (int c = 0; c < Caps::kQueues; ++c) {
+                        const unsigned m = __ballot_sync(0xffffffffu, kind == c);
+                        if (kind == c) s_q[64 * c + cnt[c] + __popc(m & below)] = rec;
+                        cnt[c] += __popc(m);
+                    }
+                    __syncwarp();
+                }
+#pragma unroll
+                for (int c = 0; c < Caps::kQueues; ++c) {
+                    // (a queue gains at most 32 entries per step, so one batch per step keeps it below 32)
+                    if (cnt[c] >= 32 || (last && cnt[c] > 0)) {
+                        const int first = max(cnt[c] - 32, 0);
+                        if (first + lane < cnt[c]) {
+                            const uint32_t rec = s_q[64 * c + first + lane];
+                            box_edge<NP, DEG>(T, c, s_P + kPS * ((rec >> 10) & 511u), s_P + kPS * (rec >> 19),
+                                              s_E + kES * (rec & 1023u));
+                        }
+                        cnt[c] = first;
+                        __syncwarp();
+                    }
+                }
+                if (last) break;
+            }
+        }
+        __syncthreads();
+
+        // (P) lattice points
+        {
+            const int tot = cp->ptot;
+            const int off_l = lane < np ? cp->poff[lane] : INT_MAX;
+            int cnt = 0;
+            const double far_c = box_centre<NP>(T, n);
+            for (int base = warp * 32;; base += kBoxThreads) {
+                const bool last = base >= tot;
+                if (!last) {
+                    const int j = warp_owner(base, off_l, lane), it = base + lane;
+                    const int off = __shfl_sync(0xffffffffu, off_l, j & 31);
+                    bool near = false;
+                    uint32_t rec = 0;
+                    if (it < tot) {
+                        const int lp = it - off;
+                        const int n0 = cp->dim[j][0] + 1, n1 = cp->dim[j][1] + 1, n2 = cp->dim[j][2] + 1;
+                        const int i = div_by(lp, cp->mag[j][2]), rem = lp - i * (n1 * n2);
+                        const int jj = div_by(rem, cp->mag[j][1]), k = rem - jj * n2;
+                        const double* const rx = s_P + kPS * (cp->loff[j] + i);
+                        const double* const ry = s_P + kPS * (cp->loff[j] + n0 + jj);
+                        const double* const rz = s_P + kPS * (cp->loff[j] + n0 + n1 + k);
+                        const double x = rx[0], y = ry[0], z = rz[0];
+                        if (x == 0.0 || y == 0.0 || z == 0.0) {
+                            s_T[it] = 0.0;
+                        } else if (fma(x, x, fma(y, y, z * z)) < 1.0) {
+                            near = true;
+                            rec = (uint32_t)j | (uint32_t)i << 5 | (uint32_t)jj << 9 | (uint32_t)k << 13;
+                        } else {
+                            const double* const E = s_E + kES * cp->eoff[j] + 2 * n;
+                            const double f = (E[kES * (i * n1 + jj)] + E[kES * (n0 * n1 + i * n2 + k)]) +
+                                             E[kES * (n0 * (n1 + n2) + jj * n2 + k)] +
+                                             ((rx[1 + 2 * n] + ry[1 + 2 * n]) + (rz[1 + 2 * n] + far_c));
+                            s_T[it] = box_signed(f, x, y, z);
+                            n_vp += 6;
+                        }
+                    }
+                    const unsigned m = __ballot_sync(0xffffffffu, near);
+                    if (near) s_q[cnt + __popc(m & below)] = rec;
+                    cnt += __popc(m);
+                    __syncwarp();
+                }
+                if (cnt >= 32 || (last && cnt > 0)) {
+                    const int first = max(cnt - 32, 0);
+                    if (first + lane < cnt) {
+                        const uint32_t rec = s_q[first + lane];
+                        const int j = (int)(rec & 31u), i = (int)((rec >> 5) & 15u), jj = (int)((rec >> 9) & 15u),
+                                  kk = (int)(rec >> 13);
+                        const int n0 = cp->dim[j][0] + 1, n1 = cp->dim[j][1] + 1, n2 = cp->dim[j][2] + 1;
+                        const double* const rx = s_P + kPS * (cp->loff[j] + i);
+                        const double* const ry = s_P + kPS * (cp->loff[j] + n0 + jj);
+                        const double* const rz = s_P + kPS * (cp->loff[j] + n0 + n1 + kk);
+                        const double x = rx[0], y = ry[0], z = rz[0];
+                        const double ax = fabs(x), ay = fabs(y), az = fabs(z);
+                        const double r2 = fma(x, x, fma(y, y, z * z));
+                        int k = 0;  // the point's piece
+#pragma unroll
+                        for (int s = 0; s + 1 < n; ++s) k += r2 >= T.scale[s].b * T.scale[s].b;
+                        const double* const E = s_E + kES * cp->eoff[j] + k;
+                        const double* const exy = E + kES * (i * n1 + jj);
+                        const double* const exz = E + kES * (n0 * n1 + i * n2 + kk);
+                        const double* const eyz = E + kES * (n0 * (n1 + n2) + jj * n2 + kk);
+                        // the smallest offset first: the other two's angles are then at most pi/4
+                        const bool mx = ax <= ay && ax <= az, my = !mx && ay <= az;
+                        const double* const r0 = mx ? rx : (my ? ry : rz);
+                        const double* const r1 = mx ? ry : rx;
+                        const double* const r2_ = mx || my ? rz : ry;
+                        double Cl[14], c0;
+                        const double* C = Cl;
+                        if (NP == 2) {  // two pieces, six coefficients each: selected constants
+#pragma unroll
+                            for (int c = 0; c < 14; ++c) Cl[c] = k ? T.reg[1].C[c] : T.reg[0].C[c];
+                            c0 = k ? T.reg[1].c : T.reg[0].c;
+                        } else {
+                            C = s_C + (kBoxC + 1) * k;
+                            c0 = C[kBoxC];
+                        }
+                        double f = box_inside<DEG>(C, c0, T.deg, ax, ay, az, r2, eyz[0], eyz[n], exz[0], exz[n], exy[0],
+                                                   exy[n], fabs(r0[0]), r0[2 + k], fabs(r1[0]), r1[1], r1[2 + k],
+                                                   fabs(r2_[0]), r2_[1], r2_[2 + k]);
+                        if (k > 0) f += ((rx[1 + n + k] + ry[1 + n + k]) + (rz[1 + n + k] + box_centre<NP>(T, k)));
+                        s_T[cp->poff[j] + (i * n1 + jj) * n2 + kk] = box_signed(f, x, y, z);
+                        n_vp += 6;
+                    }
+                    cnt = first;
+                    __syncwarp();
+                }
+                if (last) break;
+            }
+        }
+        __syncthreads();
+
+        // (C1) the chunk's (particle, cell) pairs, into the edge records' place (dead after (P))
+        double* const s_cm = s_E;
+        {
+            const int tot = cp->ctot;
+            const int off_l = lane < np ? cp->coff[lane] : INT_MAX;
+            for (int base = warp * 32; base < tot; base += kBoxThreads) {
+                const int j = warp_owner(base, off_l, lane), it = base + lane;
+                const int off = __shfl_sync(0xffffffffu, off_l, j & 31);
+                if (it < tot) {
+                    const int lc = it - off;
+                    const int d1 = cp->dim[j][1], d2 = cp->dim[j][2];
+                    const int i = div_by(lc, cp->cmag[j][1]), rem = lc - i * (d1 * d2);
+                    const int jj = div_by(rem, cp->cmag[j][0]), k = rem - jj * d2;
+                    ++n_bbox;
+                    const double radius = cp->H[j];
+                    const double ex = fmax(fabs(cp->x[j] - s_cc[0][cp->lo[j][0] + i]) - g.hpx, 0.0);
+                    const double ey = fmax(fabs(cp->y[j] - s_cc[1][cp->lo[j][1] + jj]) - g.hpy, 0.0);
+                    const double ez = fmax(fabs(cp->z[j] - s_cc[2][cp->lo[j][2] + k]) - g.hpz, 0.0);
+                    // the support test of the pair counters, rounded as the host restatement rounds it
+                    const bool in = add_rn(add_rn(mul_rn(ex, ex), mul_rn(ey, ey)), mul_rn(ez, ez)) < mul_rn(radius, radius);
+                    n_sphere += in;
+                    double msum = 0.0;
+                    if (!CULL || in) {
+                        ++n_eval;
+                        const int n2 = d2 + 1, n12 = (d1 + 1) * n2;
+                        const double* const Tp = s_T + cp->poff[j] + (i * (d1 + 1) + jj) * n2 + k;
+                        const double m1 = (Tp[n12 + n2 + 1] - Tp[n12 + n2]) - (Tp[n12 + 1] - Tp[n12]);
+                        const double m0 = (Tp[n2 + 1] - Tp[n2]) - (Tp[1] - Tp[0]);
+                        msum = m1 - m0;
+                        if (msum < 0.0) {
+                            ++n_neg;
+                            if (msum <= -0.01) ++n_warn;
+                            msum = 0.0;
+                        }
+                    }
+                    s_cm[it] = msum;
+                }
+            }
+        }
+        __syncthreads();
+
+        // (C2) the owned cells' sums: a warp's 32 cells are four z rows of one x slab; it visits the particles whose
+        // boxes reach them
+#pragma unroll
+        for (int c = 0; c < kBoxCells; ++c) {
+            const int li = threadIdx.x + c * kBoxThreads;
+            if (kTileCells % kBoxThreads && (li & ~31) >= kTileCells) break;
+            const int lx = li / (kTileZ * kTileY), ly = (li / kTileZ) % kTileY, lz = li % kTileZ;
+            const int ly0 = ly & ~3;
+            bool hit = false;
+            if (lane < np) {
+                const int i = lx - cp->lo[lane][0], j0 = cp->lo[lane][1];
+                hit = i >= 0 && i < cp->dim[lane][0] && j0 < ly0 + 4 && j0 + cp->dim[lane][1] > ly0;
+            }
+            unsigned todo = __ballot_sync(0xffffffffu, hit);
+            if (todo == 0) continue;
+            double a0 = s_acc[li], a1 = s_acc[kTileCells + li];
+            double a2 = s_acc[2 * kTileCells + li], a3 = s_acc[3 * kTileCells + li];
+            for (; todo; todo &= todo - 1) {
+                const int j = __ffs((int)todo) - 1;
+                const int i = lx - cp->lo[j][0], jj = ly - cp->lo[j][1], k = lz - cp->lo[j][2];
+                const int d1 = cp->dim[j][1], d2 = cp->dim[j][2];
+                if ((unsigned)jj >= (unsigned)d1 || (unsigned)k >= (unsigned)d2) continue;
+                const double mm = s_cm[cp->coff[j] + (i * d1 + jj) * d2 + k] * cp->m[j];
+                if (mm == 0.0) continue;
+                a0 = add_rn(a0, mm);
+                a1 = fma(mm, cp->vx[j], a1);
+                a2 = fma(mm, cp->vy[j], a2);
+                a3 = fma(mm, cp->vz[j], a3);
+            }
+            s_acc[li] = a0;
+            s_acc[kTileCells + li] = a1;
+            s_acc[2 * kTileCells + li] = a2;
+            s_acc[3 * kTileCells + li] = a3;
+        }
+        if (more) form_planes(nx);
+        __syncthreads();
+        pos += np;
+        cp = nx;
+        if (++n_chunks == (1u << 16)) {
+            flush();
+            n_chunks = 0;
+        }
+    }
+
+    const double mvx = out.meanv[0], mvy = out.meanv[1], mvz = out.meanv[2];
+    const int64_t ncell = (int64_t)g.nx * g.ny * g.nz;
+#pragma unroll
+    for (int c = 0; c < kBoxCells; ++c) {
+        const int li = threadIdx.x + c * kBoxThreads;
+        if (kTileCells % kBoxThreads && li >= kTileCells) break;
+        const int ix = bx + li / (kTileZ * kTileY), iy = by + (li / kTileZ) % kTileY, iz = bz + li % kTileZ;
+        if (ix >= g.nx || iy >= g.ny || iz >= g.nz) continue;
+        const int64_t i3 = ((int64_t)ix * g.ny + iy) * g.nz + iz;
+        const double M = s_acc[li];
+        if (out.density) out.density[i3] = M / g.cell_volume;
+        const bool has = M > 0.0;
+        const double P1 = s_acc[kTileCells + li], P2 = s_acc[2 * kTileCells + li], P3 = s_acc[3 * kTileCells + li];
+        if (out.vx) out.vx[i3] = has ? P1 / M : mvx;
+        if (out.vy) out.vy[i3] = has ? P2 / M : mvy;
+        if (out.vz) out.vz[i3] = has ? P3 / M : mvz;
+        if (out.raw4) {
+            out.raw4[i3] = M;
+            out.raw4[ncell + i3] = P1;
+            out.raw4[2 * ncell + i3] = P2;
+            out.raw4[3 * ncell + i3] = P3;
+        }
+    }
+    flush();
+}
+
+}  // namespace kiwi_b200

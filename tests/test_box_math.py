@@ -1,0 +1,76 @@
+"""The box masses of the Cartesian kernels (kiwi_b200/csrc/box_math.cuh, compiled for the host) against the
+float128 oracle: each cell of a particle's support box as the alternating sum of its corners' masses."""
+import ctypes as C
+import os
+import subprocess
+import sys
+
+import numpy as np
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+KERNELS = ["M4", "M5", "M6", "WC2", "WC4", "WC6"]
+SUPPORT = [2.0, 2.5, 3.0, 2.0, 2.0, 2.0]
+EPS = 2.0 ** -53
+
+
+@pytest.fixture(scope="module")
+def bx(tmp_path_factory):
+    out = tmp_path_factory.mktemp("bx") / "libbx.so"
+    subprocess.run(["g++", "-O2", "-fPIC", "-shared", "-std=c++17", "-ffp-contract=off", "-o", str(out),
+                    os.path.join(ROOT, "tests", "box_host_check.cpp")], check=True)
+    L = C.CDLL(str(out))
+    for f in ("bx_log", "bx_atan01"):
+        getattr(L, f).restype, getattr(L, f).argtypes = C.c_double, [C.c_double]
+    L.bx_mass.restype, L.bx_mass.argtypes = C.c_double, [C.c_int, C.c_int, C.POINTER(C.c_double)]
+    L.bx_coef_sum.restype, L.bx_coef_sum.argtypes = C.c_double, [C.c_int]
+    return L
+
+
+@pytest.fixture(scope="module")
+def quad_oracle():
+    from oracle.oracle import Oracle
+
+    return Oracle(quad=True)
+
+
+def test_tables_are_current():
+    gen = os.path.join(ROOT, "kiwi_b200", "tables", "gen_box_tables.py")
+    assert subprocess.run([sys.executable, gen, "--check"]).returncode == 0
+
+
+def test_functions(bx):
+    """Rounding level in absolute terms: the reduction's and the polynomial's few roundings of values up to |f|."""
+    x = np.concatenate([[0.0, 1e-300, 1e-17, 1.0], np.random.default_rng(1).random(2000)])
+    assert max(abs(bx.bx_atan01(v) - np.arctan(np.longdouble(v))) for v in x) <= 4 * EPS
+    v = np.concatenate([[1.0, np.sqrt(0.5), np.sqrt(2.0), 2.0, 1e-200], np.exp(np.random.default_rng(2).uniform(-40, 3, 2000))])
+    for t in v:
+        want = np.log(np.longdouble(t))
+        assert abs(bx.bx_log(t) - want) <= 4 * EPS * max(1.0, abs(want))
+
+
+@pytest.mark.parametrize("kernel", range(6), ids=KERNELS)
+def test_cells_against_float128(bx, quad_oracle, kernel):
+    """Particles at a general place, near planes (offsets of 1e-3, 1e-9 and 1e-15 of a cell) and with a support that
+    ends on planes; a wide and a narrow support.  Bound: each of a cell's eight corner masses carries at most 16
+    roundings of terms no larger than the table's coefficients allow."""
+    n = 6
+    bound = 8 * 16 * EPS * max(1.0, bx.bx_coef_sum(kernel))
+    for frac, H in (((0.31, 0.57, 0.44), 0.42), ((1e-3, 0.5, 1 - 1e-3), 0.3), ((1e-9, 1e-15, 0.7), 0.25),
+                    ((0.5, 0.5, 0.5), 0.25), ((0.2, 0.9, 1e-9), 0.06)):
+        pos = [(2 + f) / n for f in frac]
+        P = {k: np.array([v]) for k, v in zip(("x", "y", "z", "vx", "vy", "vz", "m", "h"),
+                                             (*pos, 0.0, 0.0, 0.0, 1.0, H / SUPPORT[kernel]))}
+        truth = quad_oracle.sph_to_grid(P, (0.0, 1.0) * 3, (n, n, n), kernel=-1 if kernel == 0 else kernel,
+                                        support_in_h=SUPPORT[kernel])[4][0].reshape(n, n, n)
+        H = SUPPORT[kernel] * P["h"][0]
+        d = 1.0 / n
+        off = [(np.arange(n + 1) * d - p) / H for p in pos]
+        for fixed in ((0, 1) if kernel == 0 else (0,)):
+            T = np.zeros((n + 1,) * 3)
+            for i in np.ndindex(T.shape):
+                u = [off[a][i[a]] for a in range(3)]
+                if 0.0 not in u:
+                    T[i] = np.sign(u).prod() * bx.bx_mass(kernel, fixed, (C.c_double * 3)(*np.abs(u)))
+            cells = np.diff(np.diff(np.diff(T, axis=0), axis=1), axis=2)
+            assert np.max(np.abs(np.maximum(cells, 0.0) - truth.astype(float))) <= bound
