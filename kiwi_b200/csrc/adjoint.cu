@@ -6,448 +6,453 @@
 //   dL/dm_p     = sum_c K_pc (gM_c + v_p . gP_c)
 //   dL/dv_p     = m_p sum_c K_pc gP_c
 //   dL/dtheta_p = m_p sum_c dK_pc/dtheta (gM_c + v_p . gP_c),   theta = x, y, z, h.
-// The per-pair cell integrals are recomputed, not stored: the forward kernel's lattice tiers
-// (lattice_edge_pair, lattice_point) are instantiated with the Dual3 type, which carries d/dx, d/dy, d/dz of
-// every intermediate through the same operations (d/dh follows from them, see k_cart_adjoint_lattice), so the
-// derivative part is the exact derivative of the evaluated formula (branch choices are taken on values).  A clamped pair (Msum < 0) has K = 0 and no
-// gradient.  The pairs are those of the forward's default evaluation: the cells of the particle's
-// support bounding box whose closest point lies within the support radius.
+// The per-pair cell integrals are recomputed, not stored, with their derivatives in closed form
+// (box_grad.cuh): the derivative of a box mass with respect to a side is the kernel's integral over a face.  A
+// clamped pair (Msum < 0) has K = 0 and no gradient.  The pairs are those of the forward's default
+// evaluation: the cells of the particle's support bounding box whose closest point lies within the support
+// radius.
 //
-// The evaluation is the lattice form of the forward pass (lattice_tile.cuh) with derivatives: one CTA per
-// 8^3-cell tile walks the tile's particles in chunks; (A) the edge tiers of every (plane, edge line), in
-// swapped pairs, and (B) the octant value of every lattice point are computed once per particle with their
-// derivatives; (C) for each particle, each thread assembles the cells it owns from their 8 corners' octant
-// values (value and derivatives alike), weighs them with the cells' cotangents, and a fixed-order block
-// reduction writes the particle's partial gradient for this tile to its (tile, particle) entry.  (D) Each
-// particle's entries are then added in tile order.  Deterministic, no atomics on the gradients.
+// A box mass depends on offsets / H alone, so dT/dh = (ux dT/dx + uy dT/dy + uz dT/dz) / h with the derivatives
+// taken with respect to the particle's coordinates (u = plane - particle).
+//
+// One CTA takes a run of consecutive (tile, particle) entries, tile by tile: their planes, edge lines and lattice
+// points are formed once each as in box_tile.cuh, and then a warp takes each particle, assembles its cells from
+// their 8 corners (value and derivatives alike), weighs them with the cells' cotangents and writes the particle's
+// partial gradient for this tile to its entry.  An entry's partial depends on nothing else in the run, so the
+// runs are cut to fill the chip whatever the tiles hold.  k_adjoint_reduce adds each particle's entries in tile
+// order.  Deterministic, no atomics on the gradients.
+//
+// Against forward-mode dual numbers through the point-wise series (one CTA per tile, 255 registers with
+// spills): 100 k column particles on 80^3, cubic, forward and backward: 53.8 -> 17.2 ms; 2 k particles on 21 x 19 x 25 (36 tiles), Wendland C4:
+// 90.0 -> 5.2 ms.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <climits>
 
 #include "binning.cuh"
+#include "box_grad.cuh"
 #include "cart_common.cuh"
 #include "ctx.hpp"
-#include "dual.cuh"
 #include "engine.hpp"
-#include "kiwi_math.cuh"
+#include "kernel_tables.h"
 #include "lattice.cuh"
-#include "lattice_dual.cuh"
 #include "prims.cuh"
 
 namespace kiwi_b200 {
 
 namespace {
 
-constexpr int kAdjLatThreads = 256;
-constexpr int kAdjCellsPerThread = kTileCells / kAdjLatThreads;
+constexpr int kAdjThreads = 256, kAdjWarps = kAdjThreads / 32;
 constexpr int kAdjPMax = 32;
-constexpr int kAdjECap = 1536;  // edge slots per chunk (a full 8^3 particle box has 486)
-constexpr int kAdjPtCap = 2304; // lattice points per chunk (a full 8^3 particle box has 729)
-constexpr int kAdjERec = 8;     // D2, D3 as Dual3
-constexpr int kAdjTRec = 5;     // octant value and its derivatives with respect to x, y, z, h
-constexpr size_t kAdjDynSmem = sizeof(double) * (kAdjERec * kAdjECap + kAdjTRec * kAdjPtCap);
-static_assert(kAdjECap <= 2048, "packed edge-pair entries (11-bit slots)");
-// generic kernels: edge records of lattice_generic_edge in Dual3 (offsets with derivatives)
-constexpr int kAdjGenECap = kLatGenECap;
-constexpr int kAdjGenERec = lat_gen_dual_rec<3>();
-constexpr size_t kAdjGenDynSmem = sizeof(double) * (kAdjGenERec * kAdjGenECap + kAdjTRec * kAdjPtCap);
+constexpr int kAdjComps = 5;  // a point's T and its derivatives with respect to x, y, z, h
 
-static __constant__ KiwiKernelTable c_adj_tables[KIWI_NUM_KERNELS];
+static __constant__ KiwiBoxTable c_adj_box[KIWI_NUM_KERNELS];
+
+// Chunk capacities: two CTAs per SM (a full 8^3 box has 729 points, 243 edge lines and 27 planes).
+template <int NP>
+struct AdjCaps {
+    static constexpr int kN = NP ? NP : KIWI_BOX_PIECES;
+    static constexpr int kPt = NP ? 1024 : 800, kPair = NP ? 352 : 272, kPlane = NP ? 136 : 120;
+    static constexpr int kOffE = kAdjComps * kPt;
+    static constexpr int kOffP = kOffE + box_grad_edge_stride(kN) * kPair;
+    static constexpr int kEnd = kOffP + box_grad_plane_stride(kN) * kPlane;
+    static constexpr size_t kSmem = sizeof(double) * kEnd + sizeof(uint32_t) * 64 * kAdjWarps * kN;
+    static_assert(kPair <= 1024 && kPlane <= 512, "packed edge entries");
+};
 
 struct AdjGrads {
     double *x, *y, *z, *h, *m, *vx, *vy, *vz;
 };
 
-// |plane - x_axis| with its derivative with respect to the particle's coordinate on that axis
-__device__ __forceinline__ Dual3 dual_abs_offset(double off, int axis) {
-    Dual3 r(fabs(off));
-    r.d[axis] = off > 0.0 ? -1.0 : (off < 0.0 ? 1.0 : 0.0);
-    return r;
-}
-
-__device__ __forceinline__ Dual3 load_dual(const double* p) {
-    Dual3 r(p[0]);
-    r.d[0] = p[1];
-    r.d[1] = p[2];
-    r.d[2] = p[3];
-    return r;
-}
-
-__device__ __forceinline__ void store_dual(double* p, const Dual3& v) {
-    p[0] = v.v;
-    p[1] = v.d[0];
-    p[2] = v.d[1];
-    p[3] = v.d[2];
-}
-
-// The six edge tiers (with derivatives) of a lattice point, read from the chunk's table where lattice_point
-// uses them: slots in PointEdge order, D2 at +0 and D3 at +4 of each record.
-struct SmemDualEdges {
-    const double* rec;
-    int slot[6];
-    __device__ __forceinline__ Dual3 D2(int e) const { return load_dual(rec + kAdjERec * slot[e]); }
-    __device__ __forceinline__ Dual3 D3(int e) const { return load_dual(rec + kAdjERec * slot[e] + 4); }
-    __device__ __forceinline__ void leg_angles(int, const Dual3& a1, const Dual3& ia1, const Dual3& a2,
-                                               const Dual3& ia2, Dual3& pa, Dual3& pb) const {
-        kiwi_b200::leg_angles(a1, ia1, a2, ia2, pa, pb);
-    }
+struct AdjChunk {
+    double x[kAdjPMax], y[kAdjPMax], z[kAdjPMax], H[kAdjPMax], iH[kAdjPMax], m[kAdjPMax], vx[kAdjPMax], vy[kAdjPMax],
+        vz[kAdjPMax];
+    int lo[kAdjPMax][3], dim[kAdjPMax][3];  // lo relative to the tile
+    int loff[kAdjPMax], eoff[kAdjPMax], poff[kAdjPMax];
+    uint32_t entry[kAdjPMax];
+    uint32_t mag[kAdjPMax][3];   // div_magic of n1', n2' and n1' n2'
+    uint32_t cmag[kAdjPMax][2];  // div_magic of n2 and n1 n2
+    int np, ltot, etot, ptot;
 };
 
-__device__ __forceinline__ unsigned long long block_count(unsigned long long v) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    return v;
-}
-
-// (A)-(C) for one tile: list holds (tile, particle) entry indices (the entries of particle p are
-// offs[p] .. offs[p+1]-1); part receives 8 doubles per entry: dL/dm, dL/d(x, y, z, h), dL/d(vx, vy, vz)
-// over this tile's cells.
-//
-// The octant value T of a lattice point at offsets u = (ux, uy, uz) from the particle is sgn(ux) sgn(uy)
-// sgn(uz) G(|ux|, |uy|, |uz|), with G the kernel mass of the box spanned by the particle and the point
-// (lattice_point).  G is a mass fraction of a kernel of scale h, so G(a, b, c; h) = G(a/h, b/h, c/h; 1): it is
-// homogeneous of degree 0 in (a, b, c, h), whence dT/dh = (ux dT/dx + uy dT/dy + uz dT/dz) / h with the
-// derivatives taken with respect to the particle's coordinates (u = plane - particle).  The tiers are
-// therefore evaluated with three forward derivatives (Dual3, h held fixed) and dT/dh follows from them.
-//
-// GENERIC: the table-driven tiers of kernel `kernel` (support g.support_in_h x h): every edge line's record
-// (lattice_generic_edge in Dual3) in (A), the points' six vertex tiers together (lattice_generic_point in
-// Dual3) in (B).  The same homogeneity gives d/dh.
-template <bool GENERIC>
-__global__ void __launch_bounds__(kAdjLatThreads, 1) k_cart_adjoint_lattice(CartGeom g, DevParticles P, int kernel,
-                                                                          const uint32_t* __restrict__ list,
-                                                                          const int64_t* __restrict__ range,
-                                                                          const int64_t* __restrict__ offs,
-                                                                          const double* __restrict__ cot,
-                                                                          double* __restrict__ part,
-                                                                          DevStats* __restrict__ st) {
-    __shared__ double s_x[kAdjPMax], s_y[kAdjPMax], s_z[kAdjPMax], s_h[kAdjPMax], s_ih[kAdjPMax], s_m[kAdjPMax],
-        s_vx[kAdjPMax], s_vy[kAdjPMax], s_vz[kAdjPMax];
-    __shared__ int s_lo[kAdjPMax][3], s_dim[kAdjPMax][3], s_eoff[kAdjPMax], s_poff[kAdjPMax];
-    __shared__ uint32_t s_entry[kAdjPMax];
-    __shared__ uint32_t s_mag[kAdjPMax][4];  // div_magic of n0', n1', n2' and n1' n2'
-    __shared__ uint32_t s_plist[kAdjPtCap];
-    __shared__ uint32_t s_hlist[kAdjECap / 2];
-    __shared__ int s_np, s_etot, s_ptot, s_nexp, s_ncheap, s_nheavy, s_ninner;
-    __shared__ double s_red[kAdjLatThreads / 32][8];
-    __shared__ double s_pl[3][kTileX + 1];
-    extern __shared__ double s_adj[];
-    constexpr int kERec = GENERIC ? kAdjGenERec : kAdjERec;
-    constexpr int kECap = GENERIC ? kAdjGenECap : kAdjECap;
-    const KiwiKernelTable* K = GENERIC ? &c_adj_tables[kernel] : nullptr;
-    double* s_E = s_adj;
-    double* s_T = s_adj + kERec * kECap;
-
-    const int64_t t = blockIdx.x;
-    const int tz = (int)(t % g.ntz), ty = (int)((t / g.ntz) % g.nty), tx = (int)(t / ((int64_t)g.ntz * g.nty));
-    const int bx = tx * kTileX, by = ty * kTileY, bz = tz * kTileZ;
+// The partial gradients of the sorted entries [blockIdx.x per_block, ..): keys their tiles, list their entry
+// numbers, owner the particle of an entry; part receives 8 doubles per entry: dL/dm, dL/d(x, y, z, h),
+// dL/d(vx, vy, vz) over the entry's tile.
+template <int NP, int DEG>
+__global__ void __launch_bounds__(kAdjThreads, 2) k_cart_adjoint_box(CartGeom g, DevParticles P, int kernel,
+                                                                     const uint32_t* __restrict__ keys,
+                                                                     const uint32_t* __restrict__ list,
+                                                                     const uint32_t* __restrict__ owner, int64_t total,
+                                                                     int per_block, const double* __restrict__ cot,
+                                                                     double* __restrict__ part,
+                                                                     DevStats* __restrict__ st) {
+    using Caps = AdjCaps<NP>;
+    __shared__ AdjChunk s_cp;
+    __shared__ double s_pl[3][kTileX + 1], s_cc[3][kTileX];
+    __shared__ double s_C[NP ? 1 : (kBoxC + kBoxD + 1) * KIWI_BOX_PIECES];
+    __shared__ int64_t s_seg_end;
+    extern __shared__ double s_dyn[];
+    const KiwiBoxTable& T = NP ? c_adj_box[0] : c_adj_box[kernel];
+    const int n = NP ? NP : T.npiece;
+    const int kPS = box_grad_plane_stride(n), kES = box_grad_edge_stride(n);
+    double* const s_T = s_dyn;
+    double* const s_E = s_dyn + Caps::kOffE;
+    double* const s_P = s_dyn + Caps::kOffP;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1;
+    uint32_t* const s_q = reinterpret_cast<uint32_t*>(s_dyn + Caps::kEnd) + 64 * Caps::kN * warp;
+    constexpr int kCS = kBoxC + kBoxD + 1;
+    if (!NP)
+        for (int i = threadIdx.x; i < kCS * n; i += kAdjThreads) {
+            const int k = i / kCS, c = i % kCS;
+            s_C[i] = c < kBoxC ? T.reg[k].C[c] : (c < kBoxC + kBoxD ? T.reg[k].D[c - kBoxC] : T.reg[k].c);
+        }
     const int64_t ncell = (int64_t)g.nx * g.ny * g.nz;
-    unsigned long long n_eval = 0, n_neg = 0;
-    const int64_t beg = range[2 * t], end = range[2 * t + 1];
-    if (threadIdx.x < 3 * (kTileX + 1)) {
-        const int a = threadIdx.x / (kTileX + 1), l = threadIdx.x % (kTileX + 1);
-        const double mn = a == 0 ? g.x_min : (a == 1 ? g.y_min : g.z_min), d = a == 0 ? g.dpx : (a == 1 ? g.dpy : g.dpz);
-        s_pl[a][l] = add_rn(mn, mul_rn((double)((a == 0 ? bx : (a == 1 ? by : bz)) + l), d));
-    }
+    unsigned n_eval = 0, n_neg = 0;
+    const int64_t beg = (int64_t)blockIdx.x * per_block, end = min(beg + (int64_t)per_block, total);
 
     for (int64_t pos = beg; pos < end;) {
+        // the run of this tile's entries
+        const int64_t t = keys[pos];
+        __syncthreads();
         if (warp == 0) {
-            const int64_t idx = pos + lane;
-            int ne = 0, npt = 0, lo0 = 0, lo1 = 0, lo2 = 0, d0 = 0, d1 = 0, d2 = 0;
-            double px = 0, py = 0, pz = 0, ph = 0, pm = 0, pvx = 0, pvy = 0, pvz = 0;
-            uint32_t e = 0;
-            if (idx < end) {
-                e = list[idx];
-                int64_t lo = 0, hi = P.n - 1;  // the entry's particle: the last p with offs[p] <= e
-                while (lo < hi) {
-                    const int64_t mid = (lo + hi + 1) >> 1;
-                    if (offs[mid] <= (int64_t)e) lo = mid; else hi = mid - 1;
-                }
-                const int64_t p = lo;
-                px = P.x[p]; py = P.y[p]; pz = P.z[p]; ph = P.h[p];
-                pm = P.m[p]; pvx = P.vx[p]; pvy = P.vy[p]; pvz = P.vz[p];
-                CellBox b;
-                bool outside;
-                particle_cell_box(g, px, py, pz, ph, b, &outside);
-                lo0 = max(b.x0, bx); lo1 = max(b.y0, by); lo2 = max(b.z0, bz);
-                d0 = min(b.x1, bx + kTileX - 1) - lo0 + 1;
-                d1 = min(b.y1, by + kTileY - 1) - lo1 + 1;
-                d2 = min(b.z1, bz + kTileZ - 1) - lo2 + 1;
-                const int n0 = d0 + 1, n1 = d1 + 1, n2 = d2 + 1;
-                ne = 2 * (n0 * n1 + n0 * n2 + n1 * n2);
-                npt = n0 * n1 * n2;
+            int64_t e = pos;
+            for (;;) {  // at most per_block / 32 steps
+                const int64_t i = e + lane;
+                const unsigned same = __ballot_sync(0xffffffffu, i < end && keys[i] == (uint32_t)t);
+                e += __popc(same);
+                if (same != 0xffffffffu) break;
             }
-            int ie = ne, ip = npt;
-            for (int o = 1; o < 32; o <<= 1) {
-                const int ve = __shfl_up_sync(0xffffffffu, ie, o), vp = __shfl_up_sync(0xffffffffu, ip, o);
-                if (lane >= o) {
-                    ie += ve;
-                    ip += vp;
-                }
-            }
-            const bool take = (idx < end) && ie <= kECap && ip <= kAdjPtCap;
-            const int np = __popc(__ballot_sync(0xffffffffu, take));
-            if (take) {
-                s_x[lane] = px; s_y[lane] = py; s_z[lane] = pz; s_h[lane] = ph; s_ih[lane] = 1.0 / ph;
-                s_m[lane] = pm; s_vx[lane] = pvx; s_vy[lane] = pvy; s_vz[lane] = pvz;
-                s_lo[lane][0] = lo0; s_lo[lane][1] = lo1; s_lo[lane][2] = lo2;
-                s_dim[lane][0] = d0; s_dim[lane][1] = d1; s_dim[lane][2] = d2;
-                s_eoff[lane] = ie - ne;
-                s_poff[lane] = ip - npt;
-                s_entry[lane] = e;
-                s_mag[lane][0] = div_magic(d0 + 1);
-                s_mag[lane][1] = div_magic(d1 + 1);
-                s_mag[lane][2] = div_magic(d2 + 1);
-                s_mag[lane][3] = div_magic((d1 + 1) * (d2 + 1));
-            }
-            if (lane == np - 1) {
-                s_np = np;
-                s_etot = ie;
-                s_ptot = ip;
-                s_nexp = s_ncheap = s_nheavy = s_ninner = 0;
-            }
+            if (lane == 0) s_seg_end = e;
+        }
+        const int tz = (int)(t % g.ntz), ty = (int)((t / g.ntz) % g.nty), tx = (int)(t / ((int64_t)g.ntz * g.nty));
+        const int bx = tx * kTileX, by = ty * kTileY, bz = tz * kTileZ;
+        if (threadIdx.x >= 32 && threadIdx.x < 32 + 3 * (kTileX + 1)) {
+            const int i = threadIdx.x - 32, a = i / (kTileX + 1), l = i % (kTileX + 1);
+            const double mn = a == 0 ? g.x_min : (a == 1 ? g.y_min : g.z_min);
+            const double d = a == 0 ? g.dpx : (a == 1 ? g.dpy : g.dpz);
+            const int b0 = a == 0 ? bx : (a == 1 ? by : bz);
+            s_pl[a][l] = add_rn(mn, mul_rn((double)(b0 + l), d));
+            if (l < kTileX) s_cc[a][l] = cell_centre(mn, b0 + l, d);
         }
         __syncthreads();
-        const int np = s_np, etot = s_etot, ptot = s_ptot;
+        const int64_t seg_end = s_seg_end;
 
-        // (A) edge pairs, as the forward kernel walks them: pairs beyond 2h (or zero) get D2 = D3 = 0; the
-        // others are listed (slot ab | slot ba << 11 | particle << 22 | pair block << 27) with the two signed
-        // offsets parked in slot ab, and evaluated in (A2) by full warps.
-        {
-            const int qtot = etot >> 1;
-            const int qoff_l = lane < np ? (s_eoff[lane] >> 1) : INT_MAX;
-            for (int base = warp * 32; base < qtot; base += kAdjLatThreads) {
-                const int it = base + lane;
-                bool heavy = false, inner = false;
-                uint32_t hrec = 0;
-                const int j = warp_owner(base, qoff_l, lane);
-                const int qoff = __shfl_sync(0xffffffffu, qoff_l, j & 31);
-                if (it < qtot) {
-                    int e = it - qoff;
-                    const int n0 = s_dim[j][0] + 1, n1 = s_dim[j][1] + 1, n2 = s_dim[j][2] + 1;
-                    const int nxy = n0 * n1, nxz = n0 * n2, nyz = n1 * n2;
-                    const int blk = (e >= nxy) + (e >= nxy + nxz);
-                    e -= blk == 0 ? 0 : (blk == 1 ? nxy : nxy + nxz);
-                    const int a = blk == 2 ? 1 : 0, b = blk == 0 ? 1 : 2;
-                    const int nb = b == 1 ? n1 : n2, na = a == 0 ? n0 : n1;
-                    const int pi = div_by(e, s_mag[j][b]), qi = e - pi * nb;
-                    const int eb = s_eoff[j];
-                    const int sab = eb + (blk == 0 ? 0 : (blk == 1 ? nxy : 2 * nxy + nxz)) + pi * nb + qi;
-                    const int sba = eb + (blk == 0 ? nxy + nxz : (blk == 1 ? 2 * nxy + nxz + nyz : 2 * nxy + 2 * nxz + nyz)) +
-                                    qi * na + pi;
-                    const int la = s_lo[j][a] - (a == 0 ? bx : by), lb = s_lo[j][b] - (b == 1 ? by : bz);
-                    const double oa = s_pl[a][la + pi] - (a == 0 ? s_x[j] : s_y[j]);
-                    const double ob = s_pl[b][lb + qi] - (b == 1 ? s_y[j] : s_z[j]);
-                    const double h = s_h[j];
-                    if (GENERIC) {
-                        // both orientations' records, evaluated here (no pair list)
-                        const double H = mul_rn(g.support_in_h, h);
-                        const Dual3 pD = dual_abs_offset(oa, a), qD = dual_abs_offset(ob, b);
-                        lattice_generic_edge_dual<3>(K, H, pD, qD, s_E + kERec * sab);
-                        lattice_generic_edge_dual<3>(K, H, qD, pD, s_E + kERec * sba);
-                    } else {
-                    heavy = oa != 0.0 && ob != 0.0 && oa * oa + ob * ob <= 4.0 * (h * h);
-                    inner = heavy && oa * oa + ob * ob <= h * h;
-                    if (heavy) {
-                        s_E[kAdjERec * sab] = oa;
-                        s_E[kAdjERec * sab + 1] = ob;
-                        hrec = (uint32_t)sab | (uint32_t)sba << 11 | (uint32_t)j << 22 | (uint32_t)blk << 27;
-                    } else {
-#pragma unroll
-                        for (int k = 0; k < kAdjERec; ++k) s_E[kAdjERec * sab + k] = s_E[kAdjERec * sba + k] = 0.0;
-                    }
+        for (; pos < seg_end;) {
+            // (L) the next particles, as many as the capacities take
+            if (warp == 0) {
+                const int64_t idx = pos + lane;
+                int nl = 0, ne = 0, npt = 0, lo0 = 0, lo1 = 0, lo2 = 0, d0 = 0, d1 = 0, d2 = 0;
+                double px = 0, py = 0, pz = 0, ph = 1, pm = 0, pvx = 0, pvy = 0, pvz = 0;
+                uint32_t e = 0;
+                if (idx < seg_end) {
+                    e = list[idx];
+                    const uint32_t p = owner[e];
+                    px = P.x[p]; py = P.y[p]; pz = P.z[p]; ph = P.h[p];
+                    pm = P.m[p]; pvx = P.vx[p]; pvy = P.vy[p]; pvz = P.vz[p];
+                    CellBox b;
+                    bool outside;
+                    particle_cell_box(g, px, py, pz, ph, b, &outside);
+                    lo0 = max(b.x0 - bx, 0); lo1 = max(b.y0 - by, 0); lo2 = max(b.z0 - bz, 0);
+                    d0 = min(b.x1 - bx, kTileX - 1) - lo0 + 1;
+                    d1 = min(b.y1 - by, kTileY - 1) - lo1 + 1;
+                    d2 = min(b.z1 - bz, kTileZ - 1) - lo2 + 1;
+                    const int n0 = d0 + 1, n1 = d1 + 1, n2 = d2 + 1;
+                    nl = n0 + n1 + n2;
+                    ne = n0 * n1 + n0 * n2 + n1 * n2;
+                    npt = n0 * n1 * n2;
+                }
+                int il = nl, ie = ne, ip = npt;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int vl = __shfl_up_sync(0xffffffffu, il, o), ve = __shfl_up_sync(0xffffffffu, ie, o),
+                              vp = __shfl_up_sync(0xffffffffu, ip, o);
+                    if (lane >= o) {
+                        il += vl;
+                        ie += ve;
+                        ip += vp;
                     }
                 }
-                // pairs within h (two passes of the edge tiers) from the end of the list, the others from the
-                // front, so that each kind runs in warps of its own
-                const unsigned mm = __ballot_sync(0xffffffffu, heavy && !inner);
-                const unsigned mi = __ballot_sync(0xffffffffu, inner);
-                int hp = 0, hi = 0;
-                if (lane == 0) {
-                    if (mm) hp = atomicAdd(&s_nheavy, __popc(mm));
-                    if (mi) hi = atomicAdd(&s_ninner, __popc(mi));
+                const bool take = idx < seg_end && il <= Caps::kPlane && ie <= Caps::kPair && ip <= Caps::kPt;
+                const int np = __popc(__ballot_sync(0xffffffffu, take));
+                AdjChunk& c = s_cp;
+                if (take) {
+                    const double H = mul_rn(g.support_in_h, ph);
+                    c.x[lane] = px; c.y[lane] = py; c.z[lane] = pz; c.H[lane] = H; c.iH[lane] = 1.0 / H;
+                    c.m[lane] = pm; c.vx[lane] = pvx; c.vy[lane] = pvy; c.vz[lane] = pvz;
+                    c.lo[lane][0] = lo0; c.lo[lane][1] = lo1; c.lo[lane][2] = lo2;
+                    c.dim[lane][0] = d0; c.dim[lane][1] = d1; c.dim[lane][2] = d2;
+                    c.loff[lane] = il - nl;
+                    c.eoff[lane] = ie - ne;
+                    c.poff[lane] = ip - npt;
+                    c.entry[lane] = e;
+                    c.mag[lane][0] = div_magic(d1 + 1);
+                    c.mag[lane][1] = div_magic(d2 + 1);
+                    c.mag[lane][2] = div_magic((d1 + 1) * (d2 + 1));
+                    c.cmag[lane][0] = div_magic(d2);
+                    c.cmag[lane][1] = div_magic(d1 * d2);
                 }
-                hp = __shfl_sync(0xffffffffu, hp, 0);
-                hi = __shfl_sync(0xffffffffu, hi, 0);
-                const unsigned below = (1u << lane) - 1;
-                if (heavy) s_hlist[inner ? kAdjECap / 2 - 1 - hi - __popc(mi & below) : hp + __popc(mm & below)] = hrec;
+                if (lane == np - 1) {
+                    c.np = np;
+                    c.ltot = il;
+                    c.etot = ie;
+                    c.ptot = ip;
+                }
             }
-        }
+            __syncthreads();
+            const AdjChunk* const cp = &s_cp;
+            const int np = cp->np;
 
-        // (B0) the lattice points some evaluated cell reads, listed as in the forward kernel (the same padded
-        // test); a point on a particle plane has octant value 0 and no derivative, written here.
-        {
-            const int poff_l = lane < np ? s_poff[lane] : INT_MAX;
-            for (int base = warp * 32; base < ptot; base += kAdjLatThreads) {
-                const int pt = base + lane;
-                int cls = -1;  // -1 none, 0 within 2h, 1 beyond
-                uint32_t rec = 0;
-                const int jp = warp_owner(base, poff_l, lane);
-                const int poff = __shfl_sync(0xffffffffu, poff_l, jp & 31);
-                if (pt < ptot) {
-                    const int lp = pt - poff;
-                    const int n2 = s_dim[jp][2] + 1, n12 = (s_dim[jp][1] + 1) * n2;
-                    const int i = div_by(lp, s_mag[jp][3]), rem = lp - i * n12;
-                    const int jj = div_by(rem, s_mag[jp][2]), k = rem - jj * n2;
-                    const double ux = s_pl[0][s_lo[jp][0] - bx + i] - s_x[jp];
-                    const double uy = s_pl[1][s_lo[jp][1] - by + jj] - s_y[jp];
-                    const double uz = s_pl[2][s_lo[jp][2] - bz + k] - s_z[jp];
-                    const double h = s_h[jp], radius = mul_rn(g.support_in_h, h);
-                    const double ex = fmax(fabs(ux) - kNeedPad * g.dpx, 0.0);
-                    const double ey = fmax(fabs(uy) - kNeedPad * g.dpy, 0.0);
-                    const double ez = fmax(fabs(uz) - kNeedPad * g.dpz, 0.0);
-                    if (ex * ex + ey * ey + ez * ez < radius * radius) {
-                        if (ux == 0.0 || uy == 0.0 || uz == 0.0) {
+            // (A) planes
+            {
+                const int off_l = lane < np ? cp->loff[lane] : INT_MAX, tot = cp->ltot;
+                for (int base = warp * 32; base < tot; base += kAdjThreads) {
+                    const int j = warp_owner(base, off_l, lane), it = base + lane;
+                    const int off = __shfl_sync(0xffffffffu, off_l, j & 31);
+                    if (it < tot) {
+                        int l = it - off;
+                        const int n0 = cp->dim[j][0] + 1, n1 = cp->dim[j][1] + 1;
+                        const int a = (l >= n0) + (l >= n0 + n1);
+                        l -= a == 0 ? 0 : (a == 1 ? n0 : n0 + n1);
+                        const double c = a == 0 ? cp->x[j] : (a == 1 ? cp->y[j] : cp->z[j]);
+                        box_grad_plane<NP, DEG>(T, (s_pl[a][cp->lo[j][a] + l] - c) * cp->iH[j], s_P + kPS * it);
+                    }
+                }
+            }
+            __syncthreads();
+
+            // (E) edge lines, queued by piece as in box_tile
+            {
+                const int tot = cp->etot;
+                const int off_l = lane < np ? cp->eoff[lane] : INT_MAX;
+                int cnt[Caps::kN];
 #pragma unroll
-                            for (int c = 0; c < kAdjTRec; ++c) s_T[kAdjTRec * pt + c] = 0.0;
-                        } else {
-                            cls = (ux * ux + uy * uy + uz * uz < (GENERIC ? radius * radius : 4.0 * (h * h))) ? 0 : 1;
-                            rec = (uint32_t)jp | (uint32_t)i << 5 | (uint32_t)jj << 9 | (uint32_t)k << 13;
+                for (int c = 0; c < Caps::kN; ++c) cnt[c] = 0;
+                for (int base = warp * 32;; base += kAdjThreads) {
+                    const bool last = base >= tot;
+                    if (!last) {
+                        const int j = warp_owner(base, off_l, lane), it = base + lane;
+                        const int off = __shfl_sync(0xffffffffu, off_l, j & 31);
+                        int kind = -1;
+                        uint32_t rec = 0;
+                        if (it < tot) {
+                            int e = it - off;
+                            const int n0 = cp->dim[j][0] + 1, n1 = cp->dim[j][1] + 1, n2 = cp->dim[j][2] + 1;
+                            const int nxy = n0 * n1, nxz = n0 * n2;
+                            const int blk = (e >= nxy) + (e >= nxy + nxz);
+                            e -= blk == 0 ? 0 : (blk == 1 ? nxy : nxy + nxz);
+                            const int pi = div_by(e, cp->mag[j][blk == 0 ? 0 : 1]), qi = e - pi * (blk == 0 ? n1 : n2);
+                            const int la = cp->loff[j] + (blk == 2 ? n0 : 0) + pi;
+                            const int lb = cp->loff[j] + (blk == 0 ? n0 : n0 + n1) + qi;
+                            const double p = s_P[kPS * la], q = s_P[kPS * lb];
+                            const double D = fma(p, p, q * q);
+                            if (D >= 1.0 || p == 0.0 || q == 0.0) {
+                                double* const E = s_E + kES * it + 6 * n;
+                                E[0] = E[1] = E[2] = 0.0;
+                            } else {
+                                kind = 0;
+#pragma unroll
+                                for (int k = 0; k + 1 < n; ++k) kind += D >= T.scale[k].b * T.scale[k].b;
+                                rec = (uint32_t)it | (uint32_t)la << 10 | (uint32_t)lb << 19;
+                            }
+                        }
+#pragma unroll
+                        for (int c = 0; c < Caps::kN; ++c) {
+                            const unsigned m = __ballot_sync(0xffffffffu, kind == c);
+                            if (kind == c) s_q[64 * c + cnt[c] + __popc(m & below)] = rec;
+                            cnt[c] += __popc(m);
+                        }
+                        __syncwarp();
+                    }
+#pragma unroll
+                    for (int c = 0; c < Caps::kN; ++c) {
+                        if (cnt[c] >= 32 || (last && cnt[c] > 0)) {
+                            const int first = max(cnt[c] - 32, 0);
+                            if (first + lane < cnt[c]) {
+                                const uint32_t rec = s_q[64 * c + first + lane];
+                                box_grad_edge<NP, DEG>(T, c, s_P + kPS * ((rec >> 10) & 511u), s_P + kPS * (rec >> 19),
+                                                       s_E + kES * (rec & 1023u));
+                            }
+                            cnt[c] = first;
+                            __syncwarp();
                         }
                     }
+                    if (last) break;
                 }
-                const unsigned me = __ballot_sync(0xffffffffu, cls == 0), mc = __ballot_sync(0xffffffffu, cls == 1);
-                int pe = 0, pcb = 0;
-                if (lane == 0) {
-                    if (me) pe = atomicAdd(&s_nexp, __popc(me));
-                    if (mc) pcb = atomicAdd(&s_ncheap, __popc(mc));
-                }
-                pe = __shfl_sync(0xffffffffu, pe, 0);
-                pcb = __shfl_sync(0xffffffffu, pcb, 0);
-                const unsigned below = (1u << lane) - 1;
-                if (cls >= 0) s_plist[cls == 0 ? pe + __popc(me & below) : kAdjPtCap - 1 - pcb - __popc(mc & below)] = rec;
             }
-        }
-        __syncthreads();
+            __syncthreads();
 
-        // (A2) the listed edge pairs with their derivatives (the forward kernel's lattice_edge_pair in Dual3)
-        {
-            const int nmid = s_nheavy, ninner = s_ninner;
-            for (int li = threadIdx.x; li < nmid + ninner; li += kAdjLatThreads) {
-                const uint32_t rec = s_hlist[li < nmid ? li : kAdjECap / 2 - ninner + (li - nmid)];
-                const int sab = (int)(rec & 2047u), sba = (int)((rec >> 11) & 2047u), j = (int)((rec >> 22) & 31u);
-                const int blk = (int)(rec >> 27);
-                const int a = blk == 2 ? 1 : 0, b = blk == 0 ? 1 : 2;
-                const Dual3 pD = dual_abs_offset(s_E[kAdjERec * sab], a);
-                const Dual3 qD = dual_abs_offset(s_E[kAdjERec * sab + 1], b);
-                LatticeEdgeT<Dual3> e_pq, e_qp;
-                lattice_edge_pair(Dual3(s_h[j]), Dual3(s_ih[j]), pD, qD, e_pq, e_qp);
-                store_dual(s_E + kAdjERec * sab, e_pq.D2);
-                store_dual(s_E + kAdjERec * sab + 4, e_pq.D3);
-                store_dual(s_E + kAdjERec * sba, e_qp.D2);
-                store_dual(s_E + kAdjERec * sba + 4, e_qp.D3);
-            }
-        }
-        __syncthreads();
-
-        // (B) octant values with their derivatives
-        const int nexp = s_nexp, ncheap = s_ncheap;
-        for (int li = threadIdx.x; li < nexp + ncheap; li += kAdjLatThreads) {
-            const uint32_t rec = s_plist[li < nexp ? li : kAdjPtCap - ncheap + (li - nexp)];
-            const int jp = (int)(rec & 31u), i = (int)((rec >> 5) & 15u), jj = (int)((rec >> 9) & 15u),
-                      k = (int)((rec >> 13) & 15u);
-            const int n0 = s_dim[jp][0] + 1, n1 = s_dim[jp][1] + 1, n2 = s_dim[jp][2] + 1;
-            const int it = s_poff[jp] + (i * n1 + jj) * n2 + k;
-            const double ux = s_pl[0][s_lo[jp][0] - bx + i] - s_x[jp];
-            const double uy = s_pl[1][s_lo[jp][1] - by + jj] - s_y[jp];
-            const double uz = s_pl[2][s_lo[jp][2] - bz + k] - s_z[jp];
-            const int eb = s_eoff[jp];
-            const int nxy = n0 * n1, nxz = n0 * n2, nyz = n1 * n2;
-            const int slots[6] = {eb + i * n1 + jj, eb + nxy + i * n2 + k, eb + nxy + nxz + jj * n0 + i,
-                                  eb + 2 * nxy + nxz + jj * n2 + k, eb + 2 * nxy + nxz + nyz + k * n0 + i,
-                                  eb + 2 * nxy + 2 * nxz + nyz + k * n1 + jj};
-            const double sg = sgn(ux) * sgn(uy) * sgn(uz);
-            Dual3 f;
-            if (GENERIC) {
-                const GenEdgeRecsDual<3> R{s_E, {slots[0], slots[1], slots[2], slots[3], slots[4], slots[5]}};
-                f = sg * lattice_generic_point(K, mul_rn(g.support_in_h, s_h[jp]), dual_abs_offset(ux, 0),
-                                               dual_abs_offset(uy, 1), dual_abs_offset(uz, 2), R);
-            } else {
-                const SmemDualEdges PE{s_E, {slots[0], slots[1], slots[2], slots[3], slots[4], slots[5]}};
-                f = sg * lattice_point(Dual3(s_h[jp]), Dual3(s_ih[jp]), dual_abs_offset(ux, 0),
-                                       dual_abs_offset(uy, 1), dual_abs_offset(uz, 2), PE);
-            }
-            double* o = s_T + kAdjTRec * it;
-            o[0] = f.v;
-            o[1] = f.d[0];
-            o[2] = f.d[1];
-            o[3] = f.d[2];
-            o[4] = (ux * f.d[0] + uy * f.d[1] + uz * f.d[2]) * s_ih[jp];
-        }
-        __syncthreads();
-
-        // (C) per particle: each cell's value and derivatives as the alternating sum of its 8 corners,
-        // weighed by the cell's cotangents
-        for (int j = 0; j < np; ++j) {
-            double acc[8];
-#pragma unroll
-            for (int c = 0; c < 8; ++c) acc[c] = 0.0;
-            const double x0 = s_x[j], y0 = s_y[j], z0 = s_z[j];
-            const double radius = mul_rn(g.support_in_h, s_h[j]);
-            const int n2 = s_dim[j][2] + 1, n12 = (s_dim[j][1] + 1) * n2;
-#pragma unroll
-            for (int c = 0; c < kAdjCellsPerThread; ++c) {
-                const int li = threadIdx.x + c * kAdjLatThreads;
-                const int gz = bz + li % kTileZ, gy = by + (li / kTileZ) % kTileY, gx = bx + li / (kTileZ * kTileY);
-                const int i = gx - s_lo[j][0], jj = gy - s_lo[j][1], k = gz - s_lo[j][2];
-                if (i < 0 || jj < 0 || k < 0 || i >= s_dim[j][0] || jj >= s_dim[j][1] || k >= s_dim[j][2]) continue;
-                const double ex = fmax(fabs(x0 - cell_centre(g.x_min, gx, g.dpx)) - g.hpx, 0.0);
-                const double ey = fmax(fabs(y0 - cell_centre(g.y_min, gy, g.dpy)) - g.hpy, 0.0);
-                const double ez = fmax(fabs(z0 - cell_centre(g.z_min, gz, g.dpz)) - g.hpz, 0.0);
-                if (!(add_rn(add_rn(mul_rn(ex, ex), mul_rn(ey, ey)), mul_rn(ez, ez)) < mul_rn(radius, radius))) continue;
-                ++n_eval;
-                const double* Tp = s_T + kAdjTRec * (s_poff[j] + (i * (s_dim[j][1] + 1) + jj) * n2 + k);
-                // component comp of the cell's Msum: 0 the value, 1..4 d/d(x, y, z, h)
-                auto cell_sum = [&](int comp) {
-                    auto at = [&](int off) { return Tp[kAdjTRec * off + comp]; };
-                    const double m1 = (at(n12 + n2 + 1) - at(n12 + n2)) - (at(n12 + 1) - at(n12));
-                    const double m0 = (at(n2 + 1) - at(n2)) - (at(1) - at(0));
-                    return m1 - m0;
+            // (P) points
+            {
+                const int tot = cp->ptot;
+                const int off_l = lane < np ? cp->poff[lane] : INT_MAX;
+                int cnt = 0;
+                // a point's values, with the offsets' signs: d/d(particle x) of sgn T(|ux|, ..) = -sgn(uy) sgn(uz) T_x
+                auto put = [&](int it, int j, const double* rx, const double* ry, const double* rz, const double* v) {
+                    const double iH = cp->iH[j];
+                    const double x = rx[0], y = ry[0], z = rz[0];
+                    const double sx = x > 0.0 ? 1.0 : -1.0, sy = y > 0.0 ? 1.0 : -1.0, sz = z > 0.0 ? 1.0 : -1.0;
+                    const double tx_ = -sy * sz * v[1] * iH, ty_ = -sx * sz * v[2] * iH, tz_ = -sx * sy * v[3] * iH;
+                    s_T[it] = sx * sy * sz * v[0];
+                    s_T[Caps::kPt + it] = tx_;
+                    s_T[2 * Caps::kPt + it] = ty_;
+                    s_T[3 * Caps::kPt + it] = tz_;
+                    s_T[4 * Caps::kPt + it] = g.support_in_h * fma(x, tx_, fma(y, ty_, z * tz_));
                 };
-                const double msum = cell_sum(0);
-                if (msum < 0.0) {
-                    ++n_neg;
-                    continue;
+                for (int base = warp * 32;; base += kAdjThreads) {
+                    const bool last = base >= tot;
+                    if (!last) {
+                        const int j = warp_owner(base, off_l, lane), it = base + lane;
+                        const int off = __shfl_sync(0xffffffffu, off_l, j & 31);
+                        bool near = false;
+                        uint32_t rec = 0;
+                        if (it < tot) {
+                            const int lp = it - off;
+                            const int n0 = cp->dim[j][0] + 1, n1 = cp->dim[j][1] + 1, n2 = cp->dim[j][2] + 1;
+                            const int i = div_by(lp, cp->mag[j][2]), rem = lp - i * (n1 * n2);
+                            const int jj = div_by(rem, cp->mag[j][1]), k = rem - jj * n2;
+                            const double* const rx = s_P + kPS * (cp->loff[j] + i);
+                            const double* const ry = s_P + kPS * (cp->loff[j] + n0 + jj);
+                            const double* const rz = s_P + kPS * (cp->loff[j] + n0 + n1 + k);
+                            const double x = rx[0], y = ry[0], z = rz[0];
+                            if (x == 0.0 || y == 0.0 || z == 0.0) {
+#pragma unroll
+                                for (int c = 0; c < kAdjComps; ++c) s_T[c * Caps::kPt + it] = 0.0;
+                            } else if (fma(x, x, fma(y, y, z * z)) < 1.0) {
+                                near = true;
+                                rec = (uint32_t)j | (uint32_t)i << 5 | (uint32_t)jj << 9 | (uint32_t)k << 13;
+                            } else {
+                                const double* const E = s_E + kES * cp->eoff[j] + 6 * n;
+                                const double* const ez = E + kES * (i * n1 + jj);
+                                const double* const ey = E + kES * (n0 * n1 + i * n2 + k);
+                                const double* const ex = E + kES * (n0 * (n1 + n2) + jj * n2 + k);
+                                const double v[4] = {(ez[0] + ey[0]) + ex[0] +
+                                                         ((rx[bg_w(n, n)] + ry[bg_w(n, n)]) +
+                                                          (rz[bg_w(n, n)] + box_centre<NP>(T, n))),
+                                                     (ez[1] + ey[1]) + rx[bg_dw(n, n)], (ez[2] + ex[1]) + ry[bg_dw(n, n)],
+                                                     (ey[2] + ex[2]) + rz[bg_dw(n, n)]};
+                                put(it, j, rx, ry, rz, v);
+                            }
+                        }
+                        const unsigned m = __ballot_sync(0xffffffffu, near);
+                        if (near) s_q[cnt + __popc(m & below)] = rec;
+                        cnt += __popc(m);
+                        __syncwarp();
+                    }
+                    if (cnt >= 32 || (last && cnt > 0)) {
+                        const int first = max(cnt - 32, 0);
+                        if (first + lane < cnt) {
+                            const uint32_t rec = s_q[first + lane];
+                            const int j = (int)(rec & 31u), i = (int)((rec >> 5) & 15u), jj = (int)((rec >> 9) & 15u),
+                                      kk = (int)(rec >> 13);
+                            const int n0 = cp->dim[j][0] + 1, n1 = cp->dim[j][1] + 1, n2 = cp->dim[j][2] + 1;
+                            const double* const rx = s_P + kPS * (cp->loff[j] + i);
+                            const double* const ry = s_P + kPS * (cp->loff[j] + n0 + jj);
+                            const double* const rz = s_P + kPS * (cp->loff[j] + n0 + n1 + kk);
+                            const double r2 = fma(rx[0], rx[0], fma(ry[0], ry[0], rz[0] * rz[0]));
+                            int k = 0;
+#pragma unroll
+                            for (int s = 0; s + 1 < n; ++s) k += r2 >= T.scale[s].b * T.scale[s].b;
+                            const double* const E = s_E + kES * cp->eoff[j];
+                            const double* const ez = E + kES * (i * n1 + jj);
+                            const double* const ey = E + kES * (n0 * n1 + i * n2 + kk);
+                            const double* const ex = E + kES * (n0 * (n1 + n2) + jj * n2 + kk);
+                            double Cl[14], Dl[59], c0, v[4];
+                            const double *C = Cl, *D = Dl;
+                            if (NP == 2) {  // two pieces, few coefficients each: selected constants
+#pragma unroll
+                                for (int c = 0; c < 14; ++c) Cl[c] = k ? T.reg[1].C[c] : T.reg[0].C[c];
+#pragma unroll
+                                for (int c = 0; c < 59; ++c) Dl[c] = k ? T.reg[1].D[c] : T.reg[0].D[c];
+                                c0 = k ? T.reg[1].c : T.reg[0].c;
+                            } else {
+                                C = s_C + kCS * k;
+                                D = C + kBoxC;
+                                c0 = D[kBoxD];
+                            }
+                            box_inside_grad<DEG>(C, D, c0, T.deg, n, k, rx, ry, rz, ex, ey, ez, v);
+                            if (k > 0) {
+                                v[0] += (rx[bg_w(n, k)] + ry[bg_w(n, k)]) + (rz[bg_w(n, k)] + box_centre<NP>(T, k));
+                                v[1] += rx[bg_dw(n, k)];
+                                v[2] += ry[bg_dw(n, k)];
+                                v[3] += rz[bg_dw(n, k)];
+                            }
+                            put(cp->poff[j] + (i * n1 + jj) * n2 + kk, j, rx, ry, rz, v);
+                        }
+                        cnt = first;
+                        __syncwarp();
+                    }
+                    if (last) break;
                 }
-                if (msum == 0.0) continue;
-                const int64_t i3 = ((int64_t)gx * g.ny + gy) * g.nz + gz;
-                const double gM = cot[i3], gx_ = cot[ncell + i3], gy_ = cot[2 * ncell + i3], gz_ = cot[3 * ncell + i3];
-                const double gs = gM + s_vx[j] * gx_ + s_vy[j] * gy_ + s_vz[j] * gz_;
-                acc[0] += msum * gs;
-#pragma unroll
-                for (int comp = 1; comp <= 4; ++comp) acc[comp] += cell_sum(comp) * gs;
-                acc[5] += msum * gx_;
-                acc[6] += msum * gy_;
-                acc[7] += msum * gz_;
             }
-            // fixed-order block reduction: xor tree within each warp, then the warps in order
-#pragma unroll
-            for (int c = 0; c < 8; ++c)
-                for (int o = 16; o > 0; o >>= 1) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
-            if (lane == 0)
-#pragma unroll
-                for (int c = 0; c < 8; ++c) s_red[warp][c] = acc[c];
             __syncthreads();
-            if (threadIdx.x < 8) {
+
+            // (C) a warp per particle: its cells in box order over the lanes, weighed by the cotangents, and a
+            // fixed-order sum over the lanes
+            for (int j = warp; j < np; j += kAdjWarps) {
+                double acc[8];
+#pragma unroll
+                for (int c = 0; c < 8; ++c) acc[c] = 0.0;
+                const double x0 = cp->x[j], y0 = cp->y[j], z0 = cp->z[j], radius = cp->H[j];
+                const double vx = cp->vx[j], vy = cp->vy[j], vz = cp->vz[j];
+                const int l0 = cp->lo[j][0], l1 = cp->lo[j][1], l2 = cp->lo[j][2];
+                const int d1 = cp->dim[j][1], d2 = cp->dim[j][2], d12 = d1 * d2, nc = cp->dim[j][0] * d12;
+                const int n2 = d2 + 1, n12 = (d1 + 1) * n2;
+                for (int lc = lane; lc < nc; lc += 32) {
+                    const int i = div_by(lc, cp->cmag[j][1]), rem = lc - i * d12;
+                    const int jj = div_by(rem, cp->cmag[j][0]), k = rem - jj * d2;
+                    const double ex = fmax(fabs(x0 - s_cc[0][l0 + i]) - g.hpx, 0.0);
+                    const double ey = fmax(fabs(y0 - s_cc[1][l1 + jj]) - g.hpy, 0.0);
+                    const double ez = fmax(fabs(z0 - s_cc[2][l2 + k]) - g.hpz, 0.0);
+                    if (!(add_rn(add_rn(mul_rn(ex, ex), mul_rn(ey, ey)), mul_rn(ez, ez)) < mul_rn(radius, radius))) continue;
+                    ++n_eval;
+                    const double* const Tp = s_T + cp->poff[j] + (i * (d1 + 1) + jj) * n2 + k;
+                    // component c of the cell's Msum: 0 the value, 1..4 d/d(x, y, z, h)
+                    auto cell_sum = [&](int c) {
+                        const double* const q = Tp + c * Caps::kPt;
+                        const double m1 = (q[n12 + n2 + 1] - q[n12 + n2]) - (q[n12 + 1] - q[n12]);
+                        const double m0 = (q[n2 + 1] - q[n2]) - (q[1] - q[0]);
+                        return m1 - m0;
+                    };
+                    const double msum = cell_sum(0);
+                    if (msum < 0.0) {
+                        ++n_neg;
+                        continue;
+                    }
+                    if (msum == 0.0) continue;
+                    const int64_t i3 = ((int64_t)(bx + l0 + i) * g.ny + (by + l1 + jj)) * g.nz + (bz + l2 + k);
+                    const double gx = cot[ncell + i3], gy = cot[2 * ncell + i3], gz = cot[3 * ncell + i3];
+                    const double gs = fma(vz, gz, fma(vy, gy, fma(vx, gx, cot[i3])));
+                    acc[0] = fma(msum, gs, acc[0]);
+#pragma unroll
+                    for (int c = 1; c <= 4; ++c) acc[c] = fma(cell_sum(c), gs, acc[c]);
+                    acc[5] = fma(msum, gx, acc[5]);
+                    acc[6] = fma(msum, gy, acc[6]);
+                    acc[7] = fma(msum, gz, acc[7]);
+                }
+#pragma unroll
+                for (int c = 0; c < 8; ++c)
+                    for (int o = 16; o > 0; o >>= 1) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
                 double v = 0.0;
-                for (int w = 0; w < kAdjLatThreads / 32; ++w) v += s_red[w][threadIdx.x];
-                const double pm = s_m[j];
-                part[8 * (int64_t)s_entry[j] + threadIdx.x] = (threadIdx.x == 0) ? v : pm * v;
+#pragma unroll
+                for (int c = 0; c < 8; ++c) v = lane == c ? acc[c] : v;
+                if (lane < 8) part[8 * (int64_t)cp->entry[j] + lane] = lane == 0 ? v : cp->m[j] * v;
             }
+            pos += np;
             __syncthreads();
         }
-        pos += np;
     }
-    n_eval = block_count(n_eval);
-    n_neg = block_count(n_neg);
+    for (int o = 16; o > 0; o >>= 1) {
+        n_eval += __shfl_down_sync(0xffffffffu, n_eval, o);
+        n_neg += __shfl_down_sync(0xffffffffu, n_neg, o);
+    }
     if (lane == 0) {
-        if (n_eval) atomicAdd(&st->evaluated_pairs, n_eval);
-        if (n_neg) atomicAdd(&st->neg_clamped, n_neg);
+        if (n_eval) atomicAdd(&st->evaluated_pairs, (unsigned long long)n_eval);
+        if (n_neg) atomicAdd(&st->neg_clamped, (unsigned long long)n_neg);
     }
 }
 
-// (D) each particle's gradient: its entries' partial sums in tile order.
+// Each particle's gradient: its entries' partial sums in tile order.
 __global__ void k_adjoint_reduce(int64_t n, const int64_t* __restrict__ offs, const double* __restrict__ part,
                                  AdjGrads G) {
     const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -471,7 +476,7 @@ __global__ void k_adjoint_reduce(int64_t n, const int64_t* __restrict__ offs, co
 }  // namespace
 
 int adjoint_init_tables(KiwiCtx* ctx) {
-    KIWI_CUDA(ctx, cudaMemcpyToSymbol(c_adj_tables, kiwi_kernel_tables, sizeof(kiwi_kernel_tables)));
+    KIWI_CUDA(ctx, cudaMemcpyToSymbol(c_adj_box, kiwi_box_tables, sizeof(kiwi_box_tables)));
     return KIWI_OK;
 }
 
@@ -489,13 +494,11 @@ int cart_adjoint_dev(KiwiCtx* ctx, const DevParticles& P, const CartGeom& g, con
     // binning as the forward pass, with the sort carrying each (tile, particle) entry's index
     uint32_t* counts = nullptr;
     TileBox* boxes = nullptr;
-    int64_t *offs = nullptr, *range = nullptr;
+    int64_t* offs = nullptr;
     KIWI_TRY(scratch_t(ctx, S_COUNT, (size_t)std::max<int64_t>(n, 1), &counts));
     KIWI_TRY(scratch_t(ctx, S_BOX, (size_t)std::max<int64_t>(n, 1), &boxes));
     KIWI_TRY(scratch_t(ctx, S_OFFS, (size_t)std::max<int64_t>(n, 1) + 1, &offs));
-    KIWI_TRY(scratch_t(ctx, S_TILE_RANGE, (size_t)(2 * ntiles), &range));
     int64_t* d_total = offs + std::max<int64_t>(n, 1);
-    KIWI_CUDA(ctx, cudaMemsetAsync(range, 0, sizeof(int64_t) * 2 * ntiles, ctx->stream));
     if (n > 0) {
         k_tile_counts<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(g, P, counts, boxes, d_st);
         KIWI_LAUNCHED(ctx);
@@ -513,25 +516,33 @@ int cart_adjoint_dev(KiwiCtx* ctx, const DevParticles& P, const CartGeom& g, con
     KIWI_TRY(scratch_t(ctx, S_VALS1, (size_t)std::max<int64_t>(total, 1), &v1));
     KIWI_TRY(scratch_t(ctx, S_ADJ_PART, (size_t)8 * std::max<int64_t>(total, 1), &part));
     if (total > 0) {
+        uint32_t* owner = nullptr;
+        KIWI_TRY(scratch_t(ctx, S_ADJ_OWNER, (size_t)total, &owner));
         k_tile_emit<<<(unsigned)((total + 255) / 256), 256, 0, ctx->stream>>>(g, n, offs, boxes, 0, total, 0u, k0, v0,
-                                                                              true);
+                                                                              owner);
         KIWI_LAUNCHED(ctx);
         int key_bits = 1;
         while ((1LL << key_bits) < ntiles) ++key_bits;
         bool second = false;
         KIWI_TRY(radix_sort_pairs(ctx, k0, v0, k1, v1, total, key_bits, &second));
-        k_tile_ranges<<<(unsigned)((total + 255) / 256), 256, 0, ctx->stream>>>(second ? k1 : k0, total, range);
-        KIWI_LAUNCHED(ctx);
+        const uint32_t *sk = second ? k1 : k0, *sv = second ? v1 : v0;
+        // entries per CTA: about eight CTAs for each of the chip's 2 x SMs places, so that uneven entries level out,
+        // within 16 (two chunks of large boxes) .. 256
+        int sms = 148;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+        const int per = (int)std::min<int64_t>(256, std::max<int64_t>(16, total / (16 * (int64_t)sms)));
+        const unsigned blocks = (unsigned)((total + per - 1) / per);
+        const size_t smem = kc.cubic ? AdjCaps<2>::kSmem : AdjCaps<0>::kSmem;
         if (kc.cubic) {
-            KIWI_CUDA(ctx, cudaFuncSetAttribute(k_cart_adjoint_lattice<false>,
-                                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAdjDynSmem));
-            k_cart_adjoint_lattice<false><<<(unsigned)ntiles, kAdjLatThreads, kAdjDynSmem, ctx->stream>>>(
-                g, P, 0, second ? v1 : v0, range, offs, d_cot, part, d_st);
+            KIWI_CUDA(ctx, cudaFuncSetAttribute(k_cart_adjoint_box<2, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                (int)smem));
+            k_cart_adjoint_box<2, 3><<<blocks, kAdjThreads, smem, ctx->stream>>>(g, P, 0, sk, sv, owner, total, per,
+                                                                                 d_cot, part, d_st);
         } else {
-            KIWI_CUDA(ctx, cudaFuncSetAttribute(k_cart_adjoint_lattice<true>,
-                                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAdjGenDynSmem));
-            k_cart_adjoint_lattice<true><<<(unsigned)ntiles, kAdjLatThreads, kAdjGenDynSmem, ctx->stream>>>(
-                g, P, kc.kernel, second ? v1 : v0, range, offs, d_cot, part, d_st);
+            KIWI_CUDA(ctx, cudaFuncSetAttribute(k_cart_adjoint_box<0, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                (int)smem));
+            k_cart_adjoint_box<0, 0><<<blocks, kAdjThreads, smem, ctx->stream>>>(g, P, kc.kernel, sk, sv, owner, total,
+                                                                                 per, d_cot, part, d_st);
         }
         KIWI_LAUNCHED(ctx);
     }

@@ -163,14 +163,15 @@ KIWI_HD void box_edge(const KiwiBoxTable& T, int c, const double* A, const doubl
     const double p = fabs(A[0]), q = fabs(B[0]), ip = A[1], iq = B[1];
     const double P = fma(p, p, q * q), pq = p * q, S = pq * pq;
     const double lr = 0.5 * fm_log(P);  // ln of the line's distance (P >= kBoxTiny^2: normal)
-    double gsum = 0.0;
+    double gsum = 0.0, Qn = pq * box_q(T.reg[c].Q, d.q(), P, S);
 #ifdef __CUDACC__
 #pragma unroll
 #endif
     for (int k = 0; k < n; ++k) {
         if (k < c) continue;
-        const double Qk = pq * box_q(T.reg[k].Q, d.q(), P, S);
+        const double Qk = Qn;
         rec[k] = Qk;
+        Qn = k + 1 < n ? pq * box_q(T.reg[k + 1].Q, d.q(), P, S) : 0.0;
         rec[n + k] = fma(-Qk, lr, gsum);
         const KiwiBoxScale& s = T.scale[k];
         const double t2 = fma(s.b, s.b, -P);
@@ -179,7 +180,7 @@ KIWI_HD void box_edge(const KiwiBoxTable& T, int c, const double* A, const doubl
             const double anp = fm_atan_pos((p * ib) * (t * iq), (s.b * ip) * (q * it));
             const double anq = fm_atan_pos((q * ib) * (t * ip), (s.b * iq) * (p * it));
             double g = pq * (t * box_g(s.G, (DEG ? DEG : T.deg) / 2, P, S));
-            g = fma(pq * box_q(s.Q, d.q(), P, S), fm_log(s.b + t) - lr, g);
+            g = fma(Qk - Qn, fm_log(s.b + t) - lr, g);
             g = fma(-box_delta(t, t2, p, q, s.b), A[2 + 2 * n + k], g);
             g = fma(-box_delta(t, t2, q, p, s.b), B[2 + 2 * n + k], g);
             g = fma(anp, A[2 + 3 * n + k], g);

@@ -153,6 +153,7 @@ enum ScratchSlot {
     S_STATS2,        // device counters of a second pass
     S_VOR_MASK,      // Voronoi walk: per pair, the faces whose neighbour was processed earlier
     S_ADJ_PART,      // adjoint: partial gradients per (tile, particle) entry
+    S_ADJ_OWNER,     // adjoint: each entry's particle
     S_VOR_PVAL,      // inverse map: each visited pair's cell integral
     S_VOR_CMASS,     // inverse map: per-cell mass m_i
     S_INV_OUT,       // inverse map: given cell masses, recovered masses and coverage (host entry point)

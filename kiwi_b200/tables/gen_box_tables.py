@@ -35,6 +35,14 @@ the caps beyond two walls, (pi/2) m - (pi/2) sum_walls h(x) + sum_pairs g(x, y),
 
 f and h are stored in powers of b - p for p near b, where h is small, and in powers of p (f, a) for the rest.
 
+The derivative with respect to x is the kernel's integral over the box's face at x, from the same recurrences:
+
+  dT/dx = yz D(r, x^2, y^2 z^2) / r + y R(x^2, y^2) (atanh(z / r) - z / r) + z R(x^2, z^2) (atanh(y / r) - y / r)
+          - a'(x) A_x  inside,    -(pi/2) h'(x) + g_p(x, y) + g_p(x, z)  beyond b,
+  -g_p(p, q) = (phi - ang) f'(p) - ang h'(p) - q t A(p^2, q^2) - q R(p^2, q^2) atanh(t / b),
+
+D in powers of r - c like C, R and A (the triangle ending on the sphere) in powers of p^2 and p^2 + q^2.
+
 The polynomials of the arctangent and the logarithm (kiwi_b200/csrc/fastmath.cuh) interpolate
 atan(x) / x in x^2 on [0, 1] and atanh(s) / s in s^2 on [0, (3 - 2 sqrt 2)^2] at Chebyshev points, in
 exact rational arithmetic.
@@ -190,9 +198,47 @@ LAY_Q = [(i, 0) for i in range(1, 7)] + [(i, 1) for i in range(5)] + [(i, 2) for
 LAY_G = [(i, 0) for i in range(6)] + [(i, 1) for i in range(4)] + [(i, 2) for i in range(2)]
 
 
+# D: powers of r - c for each X^i S^j (X = x^2, S = y^2 z^2), largest total weight 12
+D_BLOCKS = [((i, j), 13 - 2 * i - 4 * j) for j in range(4) for i in range(7) if 13 - 2 * i - 4 * j > 0]
+LAY_R = [(i, j) for i in range(7) for j in range(7 - i)]   # X^i P^j
+LAY_A = [(i, j) for i in range(6) for j in range(6 - i)]
+
+
 def laid(poly, layout):
     assert set(poly) <= set(layout), (sorted(poly), layout)
     return [poly.get(m, Q(0)) for m in layout]
+
+
+def to_xp(a):
+    """A polynomial in (X, Y) as {(i, j): coef} of X^i P^j, P = X + Y (Y = P - X)."""
+    out = {}
+    for (i, j, k), v in a.items():
+        assert k == 0
+        for u in range(j + 1):
+            key = (i + u, j - u)
+            out[key] = out.get(key, Q(0)) + v * math.comb(j, u) * (-1) ** u
+    return {m: v for m, v in out.items() if v}
+
+
+def to_xes(a):
+    """A polynomial symmetric in (Y, Z) as {(i, l, j): coef} of X^i e1^l S^j, S = YZ, Y + Z = e1 - X."""
+    out, rest = {}, dict(a)
+    while rest:
+        m = max(rest, key=lambda t: (t[1], t[2], t[0]))
+        v, s = rest[m], m[1] - m[2]
+        assert s >= 0
+        rest = padd(rest, pmul({(m[0], 0, 0): Q(1)}, pmul(ppow(padd(YP, ZP), s), ppow(pmul(YP, ZP), m[2]))), -v)
+        for u in range(s + 1):
+            key = (m[0] + u, s - u, m[2])
+            out[key] = out.get(key, Q(0)) + v * math.comb(s, u) * (-1) ** u
+    return {m: v for m, v in out.items() if v}
+
+
+def face(n):
+    """The face moment of r^n: (yz [times r for odd n], y atanh(z / r)) coefficients, as polynomials in X, Y, Z."""
+    A, B = tri(n + 2)
+    s = Q(1, n + 2)
+    return pscale(padd(A, permuted(A, (0, 2, 1))), s), pscale(B, s), pscale(A, s)
 
 
 def add_into(dst, src, s):
@@ -214,7 +260,14 @@ def shifted(c, b):
 def region(w, c0):
     """Tables of one piece sum_n w[n] r^n: C (about r = c0), Q, a (rational, without the normalisation)."""
     C, QQ, a = {}, {}, [Q(0)] * 6
+    D, R = {}, {}
     for n, c in w.items():
+        A2, B1, _ = face(n)
+        for (i, l, j), v in to_xes(A2).items():
+            D.setdefault((i, j), [Q(0)] * 13)[2 * l + 1 + n % 2] += c * v
+        for (i, l, j), v in to_xes(padd(B1, permuted(B1, (0, 2, 1)))).items():
+            D.setdefault((i, j), [Q(0)] * 13)[2 * l] += c * v
+        add_into(R, to_xp(B1), c)
         V, B = moment(n)
         pairs = {}  # the three pairs' Q as a symmetric polynomial
         for (i, j), v in B.items():
@@ -233,7 +286,13 @@ def region(w, c0):
         assert not any(block[size:])
         flat += shifted(block[:size], c0)
     assert not C
-    return {"c": c0, "C": flat, "Q": laid(QQ, LAY_Q), "a": a}
+    dflat = []
+    for key, size in D_BLOCKS:
+        block = D.pop(key, [Q(0)] * 13)
+        assert not any(block[size:])
+        dflat += shifted(block[:size], c0)
+    assert not D
+    return {"c": c0, "C": flat, "Q": laid(QQ, LAY_Q), "a": a, "D": dflat, "R": laid(R, LAY_R)}
 
 
 def scale(d, b):
@@ -241,10 +300,14 @@ def scale(d, b):
     of b - p."""
     m = sum(c * b ** (n + 3) / (n + 3) for n, c in d.items())
     N = sum(c * b ** (n + 2) / ((n + 3) * (n + 2)) for n, c in d.items())
-    G, f, h = {}, [Q(0)] * 15, [Q(0)] * 15
+    G, f, h, A = {}, [Q(0)] * 15, [Q(0)] * 15, {}
     f[1] = N + m / b
     for n, c in d.items():
         add_into(G, edge_poly(n, b), c)
+        one, zpoly = {}, padd({(0, 0, 0): b * b}, PP, Q(-1))
+        for m3, v in face(n)[2].items():  # t^2 = b^2 - P, r = b
+            one = padd(one, pmul({(m3[0], m3[1], 0): v}, ppow(zpoly, m3[2])))
+        add_into(A, to_xp(one), c * (b if n % 2 else 1))
         v = c / ((n + 3) * (n + 2))
         if n % 2:
             h[n + 3] += v
@@ -255,8 +318,8 @@ def scale(d, b):
     h = [x - y for x, y in zip(h, f)]
     h[0] += m
     flip = lambda c: [v * (-1) ** i for i, v in enumerate(shifted(c, b))]  # noqa: E731
-    return {"b": b, "m": m, "G": laid(G, LAY_G), "Q": region(d, b)["Q"], "fp": fp, "ap": ap, "f": flip(f)[:14],
-            "h": flip(h)}
+    return {"b": b, "m": m, "G": laid(G, LAY_G), "fp": fp, "ap": ap, "f": flip(f)[:14],
+            "h": flip(h), "A": laid(A, LAY_A)}
 
 
 def kernel_box(K):
@@ -272,6 +335,11 @@ def kernel_box(K):
         scs.append(scale({n: c for n, c in d.items() if c}, b))
     top = max(n for p in polys for n in p)
     return {"key": K.key, "npiece": len(polys), "deg": top, "a3pi": a3, "reg": regs, "scale": scs}
+
+
+# the stored rows of a piece and of a difference kernel
+REG = ("C", "Q", "a", "D", "R")
+SCL = ("G", "fp", "ap", "f", "h", "A")
 
 
 # ---- the two univariate polynomials
@@ -338,9 +406,9 @@ def tables():
         a3 = t["a3pi"]
         rnd = lambda row: [rounded(v, a3) for v in row]  # noqa: E731
         out.append({"key": t["key"], "npiece": t["npiece"], "deg": t["deg"],
-                    "reg": [{"c": float(r["c"]), **{k: rnd(r[k]) for k in ("C", "Q", "a")}} for r in t["reg"]],
-                    "scale": [{"b": float(s["b"]), "m": rounded(s["m"], a3), "G": rnd(s["G"]), "Q": rnd(s["Q"]),
-                               **{k: rnd(s[k]) for k in ("fp", "ap", "f", "h")}} for s in t["scale"]]})
+                    "reg": [{"c": float(r["c"]), **{k: rnd(r[k]) for k in REG}} for r in t["reg"]],
+                    "scale": [{"b": float(s["b"]), "m": rounded(s["m"], a3), "G": rnd(s["G"]),
+                               **{k: rnd(s[k]) for k in SCL[1:]}} for s in t["scale"]]})
     return out
 
 
@@ -350,9 +418,9 @@ def _row(v):
 
 def header_text():
     T = tables()
-    zr = {"c": 0.0, "C": [0.0] * 39, "Q": [0.0] * 15, "a": [0.0] * 6}
-    zs = {"b": 0.0, "m": 0.0, "G": [0.0] * 12, "Q": [0.0] * 15, "fp": [0.0] * 7, "ap": [0.0] * 6,
-          "f": [0.0] * 14, "h": [0.0] * 15}
+    zr = {"c": 0.0, "C": [0.0] * 39, "Q": [0.0] * 15, "a": [0.0] * 6, "D": [0.0] * 84, "R": [0.0] * 28}
+    zs = {"b": 0.0, "m": 0.0, "G": [0.0] * 12, "fp": [0.0] * 7, "ap": [0.0] * 6,
+          "f": [0.0] * 14, "h": [0.0] * 15, "A": [0.0] * 21}
     L = [
         "// GENERATED by kiwi_b200/tables/gen_box_tables.py -- do not edit by hand.",
         "// Box-mass tables of the six SPH kernels (lengths in units of the support radius), normalised, derived in",
@@ -362,15 +430,16 @@ def header_text():
         "//   Q:    P^1..6 | S P^0..4 | S^2 P^0..2 | S^3        (P = p^2 + q^2, S = p^2 q^2)",
         "//   G:    P^0..5 | S P^0..3 | S^2 P^0..1",
         "//   a, ap: x^4, x^6, .. x^14       fp: p, p^3, .. p^13       f, h: (b - p)^0..",
+        "//   D:    (r - c)^0.. for each X^i S^j, i inner, 13 - 2 i - 4 j terms   R, A: X^i P^0.., i outer, total 6 and 5",
         "#pragma once",
         "",
         "#define KIWI_BOX_PIECES 3",
         "",
         "typedef struct KiwiBoxRegion {",
-        "    double c, C[39], Q[15], a[6];",
+        "    double c, C[39], Q[15], a[6], D[84], R[28];",
         "} KiwiBoxRegion;",
         "typedef struct KiwiBoxScale {",
-        "    double b, m, G[12], Q[15], fp[7], ap[6], f[14], h[15];",
+        "    double b, m, G[12], fp[7], ap[6], f[14], h[15], A[21];",
         "} KiwiBoxScale;",
         "typedef struct KiwiBoxTable {",
         "    int npiece;                       /* pieces: piece k holds scale[k-1].b <= r < scale[k].b */",
@@ -388,10 +457,10 @@ def header_text():
     for t in T:
         L.append(f"    {{ /* {t['key']} */ {t['npiece']}, {t['deg']},")
         L.append("      {" + ",\n       ".join(
-            "{" + _num(r["c"]) + ",\n        " + ",\n        ".join(_row(r[k]) for k in ("C", "Q", "a")) + "}"
+            "{" + _num(r["c"]) + ",\n        " + ",\n        ".join(_row(r[k]) for k in REG) + "}"
             for r in t["reg"] + [zr] * (3 - t["npiece"])) + "},")
         L.append("      {" + ",\n       ".join(
-            "{" + f"{_num(s['b'])}, {_num(s['m'])},\n        " + ",\n        ".join(_row(s[k]) for k in ("G", "Q", "fp", "ap", "f", "h")) +
+            "{" + f"{_num(s['b'])}, {_num(s['m'])},\n        " + ",\n        ".join(_row(s[k]) for k in SCL) +
             "}" for s in t["scale"] + [zs] * (3 - t["npiece"])) + "}},")
     L.append("};")
     L.append("")

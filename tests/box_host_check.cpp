@@ -1,6 +1,6 @@
 // Test-only: compiles the box-mass maths (kiwi_b200/csrc/box_math.cuh) for the host, so that tests/test_box_math.py
 // can check it against the float128 oracle without a GPU.
-#include "../kiwi_b200/csrc/box_math.cuh"
+#include "../kiwi_b200/csrc/box_grad.cuh"
 
 using namespace kiwi_b200;
 
@@ -34,6 +34,35 @@ double box_mass(const KiwiBoxTable& T, const double* o) {
                                pl[b][1], pl[b][2 + k]);
 }
 
+// The same with its derivatives: out = T, dT/dx, dT/dy, dT/dz.
+template <int NP, int DEG>
+void box_mass_grad(const KiwiBoxTable& T, const double* o, double* out) {
+    const int n = T.npiece;
+    double pl[3][32], e[3][32];
+    for (int a = 0; a < 3; ++a) box_grad_plane<NP, DEG>(T, o[a], pl[a]);
+    for (int i = 0; i < 3; ++i) {
+        const double *A = pl[i == 0 ? 1 : 0], *B = pl[i == 2 ? 1 : 2];
+        const int c = piece(T, fma(A[0], A[0], B[0] * B[0]));
+        for (int j = 0; j < 3; ++j) e[i][6 * n + j] = 0.0;
+        if (c < n) box_grad_edge<NP, DEG>(T, c, A, B, e[i]);
+    }
+    const int k = piece(T, fma(o[0], o[0], fma(o[1], o[1], o[2] * o[2])));
+    if (k < n) {
+        box_inside_grad<DEG>(T.reg[k].C, T.reg[k].D, T.reg[k].c, T.deg, n, k, pl[0], pl[1], pl[2], e[0], e[1], e[2], out);
+    } else {
+        const double *x = e[0] + 6 * n, *y = e[1] + 6 * n, *z = e[2] + 6 * n;
+        out[0] = x[0] + y[0] + z[0];
+        out[1] = z[1] + y[1];
+        out[2] = z[2] + x[1];
+        out[3] = y[2] + x[2];
+    }
+    out[0] += box_centre<NP>(T, k);
+    for (int a = 0; a < 3 && k > 0; ++a) {
+        out[0] += pl[a][bg_w(n, k)];
+        out[1 + a] += pl[a][bg_dw(n, k)];
+    }
+}
+
 }  // namespace
 
 extern "C" {
@@ -46,6 +75,11 @@ double bx_mass(int kernel, int fixed, const double* offsets) {
     const KiwiBoxTable& T = kiwi_box_tables[kernel];
     return fixed ? box_mass<2, 3>(T, offsets) : box_mass<0, 0>(T, offsets);
 }
+void bx_mass_grad(int kernel, int fixed, const double* offsets, double* out) {
+    const KiwiBoxTable& T = kiwi_box_tables[kernel];
+    if (fixed) box_mass_grad<2, 3>(T, offsets, out);
+    else box_mass_grad<0, 0>(T, offsets, out);
+}
 // The sum of the absolute values of a kernel's coefficients, for error bounds.
 double bx_coef_sum(int kernel) {
     const KiwiBoxTable& T = kiwi_box_tables[kernel];
@@ -55,7 +89,6 @@ double bx_coef_sum(int kernel) {
         for (double c : T.reg[k].Q) s += fabs(c);
         for (double c : T.reg[k].a) s += fabs(c);
         for (double c : T.scale[k].G) s += fabs(c);
-        for (double c : T.scale[k].Q) s += fabs(c);
     }
     return s;
 }

@@ -74,3 +74,25 @@ def test_cells_against_float128(bx, quad_oracle, kernel):
                     T[i] = np.sign(u).prod() * bx.bx_mass(kernel, fixed, (C.c_double * 3)(*np.abs(u)))
             cells = np.diff(np.diff(np.diff(T, axis=0), axis=1), axis=2)
             assert np.max(np.abs(np.maximum(cells, 0.0) - truth.astype(float))) <= bound
+
+
+@pytest.mark.parametrize("kernel", range(6), ids=KERNELS)
+def test_derivatives_against_differences(bx, kernel):
+    """dT/dx, dT/dy, dT/dz against extrapolated central differences of T over the pieces, near their breakpoints,
+    near a plane and beyond the support.  Bound: the kernels' third derivative jumps, so the differences err by
+    step^3 times the size of the kernel's coefficients, plus T's roundings over the step."""
+    bx.bx_mass_grad.argtypes = [C.c_int, C.c_int, C.POINTER(C.c_double), C.POINTER(C.c_double)]
+    rng = np.random.default_rng(5)
+    pts = np.concatenate([rng.uniform(0.02, 1.1, (60, 3)), 10.0 ** rng.uniform(-2, 0, (40, 3)),
+                          [[0.3, 0.4, 0.0051], [0.5, 0.5, 0.7071], [0.6, 0.8, 0.02], [0.2, 0.33, 0.999], [1.2, 1.3, 1.1]]])
+    step, size = 2.5e-4, max(1.0, bx.bx_coef_sum(kernel))
+    bound = 2 * step ** 3 * size + 16 * 8 * EPS * size / step
+    mass = lambda f, p: bx.bx_mass(kernel, f, (C.c_double * 3)(*p))  # noqa: E731
+    for fixed in ((0, 1) if kernel == 0 else (0,)):
+        for p in pts:
+            got = (C.c_double * 4)()
+            bx.bx_mass_grad(kernel, fixed, (C.c_double * 3)(*p), got)
+            assert abs(got[0] - mass(fixed, p)) <= 16 * EPS * size
+            for a in range(3):
+                d = [(mass(fixed, p + np.eye(3)[a] * s) - mass(fixed, p - np.eye(3)[a] * s)) / (2 * s) for s in (step, 2 * step)]
+                assert abs(got[1 + a] - (4 * d[0] - d[1]) / 3) <= bound
