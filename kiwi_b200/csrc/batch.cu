@@ -5,15 +5,15 @@
 // (item i's tiles follow item i-1's), so a single scan and a single stable sort build every tile list at
 // once; it groups the tiles by the tile body their item needs (cubic lattice, generic lattice, per-cell
 // gather), orders each group longest-first (by (tile, particle) entry count, ties by tile index) and
-// records one CUDA graph: counter resets and per-item mean velocities, then one k_batch_persistent launch
-// per group, whose CTAs pull tiles from a work counter and run the same tile bodies as the single-grid
-// kernels.  Every cell
-// is therefore summed in the same particle order with the same arithmetic as a single-grid call of the
+// records one CUDA graph: counter resets and per-item mean velocities, then one persistent launch per group,
+// whose CTAs pull work (tiles, or in the FP64 form segments of long lists) from a work counter and run the same
+// bodies as the single-grid kernels, then the sums of the cut tiles' segments.  Every cell is therefore summed in the same particle order with the same arithmetic as a single-grid call of the
 // same form: the batch's outputs equal the per-item outputs bit for bit.  kiwi_batch_run replays the graph.
 // kiwi_batch_tune times the launch shapes (tile order x resident CTAs per SM) and keeps the fastest.
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <utility>
 #include <vector>
 
 #include "../../include/kiwi_b200.h"
@@ -32,15 +32,20 @@ struct KiwiBatch {
     std::vector<void*> allocs;
     BatchItemDev* d_items = nullptr;
     int32_t* d_item_of_tile = nullptr;
-    // per tile-body family: its tiles in natural (item, tile) order and longest-first, and its counter
+    // per tile-body family: its work in natural (item, tile) order and longest-first (tiles, one int each, for the
+    // gather family; items of four ints, lattice_batch_work, for the lattice families), and its counter
     int32_t* d_natural[kBatchFamilies] = {};
     int32_t* d_lpt[kBatchFamilies] = {};
-    int64_t fam_tiles[kBatchFamilies] = {};
-    // both lattice families' tiles together (natural order and longest-first), for the merged launch
+    int64_t fam_tiles[kBatchFamilies] = {};  // work items
+    // both lattice families' work together (natural order and longest-first), for the merged launch
     int32_t* d_natural_m = nullptr;
     int32_t* d_lpt_m = nullptr;
     int64_t merged_tiles = 0;
     bool merge = false;
+    // the tiles whose lists are cut into segments (their first items) and their segments' raw sums
+    int32_t* d_cut = nullptr;
+    int64_t n_cut = 0;
+    double* d_sums = nullptr;
     const uint32_t* d_list = nullptr;
     int64_t* d_range = nullptr;
     unsigned long long* d_next = nullptr;  // kBatchFamilies counters
@@ -65,18 +70,6 @@ __global__ void k_gather_i64(const int64_t* __restrict__ src, const int64_t* __r
                              int64_t* __restrict__ dst) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) dst[i] = src[idx[i]];
-}
-
-// Longest-first sort keys for the tiles tiles[0 .. n): ~entries (ascending key = descending entry count),
-// value = tile index.
-__global__ void k_tile_weights(const int64_t* __restrict__ range, const int32_t* __restrict__ tiles, int64_t n,
-                               uint32_t* __restrict__ keys, uint32_t* __restrict__ vals) {
-    const int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (w >= n) return;
-    const int64_t t = tiles[w];
-    const int64_t e = range[2 * t + 1] - range[2 * t];
-    keys[w] = 0xffffffffu - (uint32_t)(e < 0xffffffffLL ? e : 0xffffffffLL);
-    vals[w] = (uint32_t)t;
 }
 
 template <class T>
@@ -110,17 +103,19 @@ int batch_enqueue(KiwiBatch* b) {
     for (int i = 0; i < b->n_items; ++i) KIWI_TRY(fp64_mean_velocity(ctx, b->items[i].P, b->d_meanv + 4 * i));
     for (int f = 0; f < kBatchFamilies; ++f) {
         if (b->merge && f == kBatchFamilyLatticeGeneric) continue;
-        if (b->merge && f == kBatchFamilyLattice) {
-            KIWI_TRY(fp64_batch_gather(ctx, kBatchFamilyLatticeMerged, b->d_items, b->d_item_of_tile,
-                                       b->lpt ? b->d_lpt_m : b->d_natural_m, b->merged_tiles, b->d_list, b->d_range,
-                                       b->d_next + f, b->sms * b->ctas_per_sm, mixed));
-            continue;
-        }
-        KIWI_TRY(fp64_batch_gather(ctx, f, b->d_items, b->d_item_of_tile, b->lpt ? b->d_lpt[f] : b->d_natural[f],
-                                   b->fam_tiles[f], b->d_list, b->d_range, b->d_next + f, b->sms * b->ctas_per_sm,
-                                   mixed));
+        const bool merged = b->merge && f == kBatchFamilyLattice;
+        const int64_t nwork = merged ? b->merged_tiles : b->fam_tiles[f];
+        if (nwork <= 0) continue;
+        const int32_t* work = merged ? (b->lpt ? b->d_lpt_m : b->d_natural_m) : (b->lpt ? b->d_lpt[f] : b->d_natural[f]);
+        if (f == kBatchFamilyGather)
+            KIWI_TRY(fp64_batch_gather(ctx, b->d_items, b->d_item_of_tile, work, nwork, b->d_list, b->d_range,
+                                       b->d_next + f, b->sms * b->ctas_per_sm));
+        else
+            KIWI_TRY(lattice_batch_gather(ctx, merged ? kBatchFamilyLatticeMerged : f, b->d_items, b->d_item_of_tile, work,
+                                          nwork, b->d_list, b->d_range, b->d_sums, b->d_next + f,
+                                          b->sms * b->ctas_per_sm, mixed));
     }
-    return KIWI_OK;
+    return lattice_batch_combine(ctx, b->d_items, b->d_item_of_tile, b->d_cut, b->n_cut, b->d_sums);
 }
 
 int batch_record(KiwiBatch* b) {
@@ -141,6 +136,66 @@ int batch_record(KiwiBatch* b) {
     b->graph = g;
     KIWI_CUDA(ctx, cudaGraphInstantiate(&b->exec, g, 0));
     return KIWI_OK;
+}
+
+// The families' work lists from the tiles' ranges, and the place of the cut tiles' sums.
+int batch_work(KiwiBatch* b) {
+    KiwiCtx* ctx = b->ctx;
+    std::vector<int64_t> range(2 * (size_t)b->n_tiles), grid_tiles((size_t)b->n_tiles);
+    KIWI_CUDA(ctx, cudaMemcpyAsync(range.data(), b->d_range, sizeof(int64_t) * range.size(), cudaMemcpyDeviceToHost,
+                                   ctx->stream));
+    KIWI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    const bool split = (b->precision & KIWI_FORM_MASK) == KIWI_FP64;
+    std::vector<int32_t> tiles[kBatchFamilies], both, slot((size_t)b->n_tiles, 0), cut, work;
+    int64_t places = 0;
+    for (int i = 0; i < b->n_items; ++i) {
+        const int f = batch_family(b->items[i].mode);
+        const int64_t nt = b->tile_base[i + 1] - b->tile_base[i];
+        for (int64_t t = b->tile_base[i]; t < b->tile_base[i + 1]; ++t) {
+            grid_tiles[(size_t)t] = nt;
+            tiles[f].push_back((int32_t)t);
+            if (f == kBatchFamilyGather) continue;
+            both.push_back((int32_t)t);
+            const int64_t nseg = split ? lattice_batch_segments(range[2 * (size_t)t + 1] - range[2 * (size_t)t], nt) : 1;
+            if (nseg <= 1) continue;
+            slot[(size_t)t] = (int32_t)places;
+            cut.insert(cut.end(), {(int32_t)t, 0, (int32_t)nseg, (int32_t)places});
+            places += nseg;
+        }
+    }
+    // one upload of all lists
+    std::vector<int32_t> all;
+    std::vector<std::pair<int32_t**, size_t>> place;
+    auto put = [&](const std::vector<int32_t>& v, int32_t** dst) {
+        place.push_back({dst, all.size()});
+        all.insert(all.end(), v.begin(), v.end());
+        all.resize((all.size() + 3) / 4 * 4);  // items are read as int4
+    };
+    for (int heaviest = 0; heaviest < 2; ++heaviest) {
+        for (int f = 0; f < kBatchFamilies; ++f) {
+            if (f == kBatchFamilyGather) {
+                work = tiles[f];
+                b->fam_tiles[f] = (int64_t)work.size();
+                if (heaviest)
+                    std::stable_sort(work.begin(), work.end(), [&](int32_t x, int32_t y) {
+                        return range[2 * (size_t)x + 1] - range[2 * (size_t)x] > range[2 * (size_t)y + 1] - range[2 * (size_t)y];
+                    });
+            } else {
+                b->fam_tiles[f] = lattice_batch_work(tiles[f], range, grid_tiles, slot, split, heaviest != 0, &work);
+            }
+            put(work, heaviest ? &b->d_lpt[f] : &b->d_natural[f]);
+        }
+        b->merged_tiles = lattice_batch_work(both, range, grid_tiles, slot, split, heaviest != 0, &work);
+        put(work, heaviest ? &b->d_lpt_m : &b->d_natural_m);
+    }
+    b->n_cut = (int64_t)cut.size() / 4;
+    put(cut, &b->d_cut);
+    int32_t* d_all = nullptr;
+    KIWI_TRY(balloc(b, all.size(), &d_all));
+    for (const auto& e : place) *e.first = d_all + e.second;
+    KIWI_CUDA(ctx, cudaMemcpyAsync(d_all, all.data(), sizeof(int32_t) * all.size(), cudaMemcpyHostToDevice, ctx->stream));
+    KIWI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));  // `all` is local
+    return balloc(b, (size_t)places * 4 * kTileCells, &b->d_sums);
 }
 
 int batch_build(KiwiBatch* b, const KiwiBatchItem* in) {
@@ -183,30 +238,6 @@ int batch_build(KiwiBatch* b, const KiwiBatchItem* in) {
     KIWI_TRY(balloc(b, (size_t)n, &b->d_items));
     KIWI_TRY(balloc(b, (size_t)b->n_tiles, &b->d_item_of_tile));
     KIWI_TRY(balloc(b, (size_t)2 * b->n_tiles, &b->d_range));
-    // each family's tiles in natural order (the tile ranges of its items, in item order)
-    std::vector<int32_t> nat[kBatchFamilies];
-    for (int i = 0; i < n; ++i) {
-        std::vector<int32_t>& v = nat[batch_family(b->items[i].mode)];
-        for (int64_t t = b->tile_base[i]; t < b->tile_base[i + 1]; ++t) v.push_back((int32_t)t);
-    }
-    for (int f = 0; f < kBatchFamilies; ++f) {
-        b->fam_tiles[f] = (int64_t)nat[f].size();
-        KIWI_TRY(balloc(b, nat[f].size(), &b->d_natural[f]));
-        KIWI_TRY(balloc(b, nat[f].size(), &b->d_lpt[f]));
-        if (!nat[f].empty())
-            KIWI_CUDA(ctx, cudaMemcpyAsync(b->d_natural[f], nat[f].data(), sizeof(int32_t) * nat[f].size(),
-                                           cudaMemcpyHostToDevice, ctx->stream));
-    }
-    std::vector<int32_t> nat_m;  // both lattice families, in item order
-    for (int i = 0; i < n; ++i)
-        if (batch_family(b->items[i].mode) != kBatchFamilyGather)
-            for (int64_t t = b->tile_base[i]; t < b->tile_base[i + 1]; ++t) nat_m.push_back((int32_t)t);
-    b->merged_tiles = (int64_t)nat_m.size();
-    KIWI_TRY(balloc(b, nat_m.size(), &b->d_natural_m));
-    KIWI_TRY(balloc(b, nat_m.size(), &b->d_lpt_m));
-    if (!nat_m.empty())
-        KIWI_CUDA(ctx, cudaMemcpyAsync(b->d_natural_m, nat_m.data(), sizeof(int32_t) * nat_m.size(),
-                                       cudaMemcpyHostToDevice, ctx->stream));
     KIWI_CUDA(ctx, cudaMemsetAsync(b->d_stats, 0, sizeof(DevStats) * n, ctx->stream));
     for (int i = 0; i < n; ++i) {
         b->items[i].st = b->d_stats + i;
@@ -258,7 +289,7 @@ int batch_build(KiwiBatch* b, const KiwiBatchItem* in) {
 
     // (2) entries of every item in one key space, one stable sort, per-tile ranges
     uint32_t *k0, *v0, *k1, *v1, *list = nullptr;
-    const size_t cap = (size_t)std::max<int64_t>(std::max<int64_t>(total, b->n_tiles), 1);
+    const size_t cap = (size_t)std::max<int64_t>(total, 1);
     KIWI_TRY(scratch_t(ctx, S_KEYS0, cap, &k0));
     KIWI_TRY(scratch_t(ctx, S_VALS0, cap, &v0));
     KIWI_TRY(scratch_t(ctx, S_KEYS1, cap, &k1));
@@ -285,24 +316,13 @@ int batch_build(KiwiBatch* b, const KiwiBatchItem* in) {
     }
     b->d_list = list;
 
-    // (3) which item owns each tile; the longest-first tile order
+    // (3) which item owns each tile; each family's work in natural and longest-first order
     for (int i = 0; i < n; ++i) {
         const int64_t nt = b->tile_base[i + 1] - b->tile_base[i];
         k_fill_i32<<<(unsigned)((nt + 255) / 256), 256, 0, ctx->stream>>>(b->d_item_of_tile + b->tile_base[i], nt, i);
         KIWI_LAUNCHED(ctx);
     }
-    for (int f = 0; f <= kBatchFamilies; ++f) {
-        const int64_t nf = f < kBatchFamilies ? b->fam_tiles[f] : b->merged_tiles;
-        if (nf <= 0) continue;
-        const int32_t* nat_f = f < kBatchFamilies ? b->d_natural[f] : b->d_natural_m;
-        int32_t* lpt_f = f < kBatchFamilies ? b->d_lpt[f] : b->d_lpt_m;
-        k_tile_weights<<<(unsigned)((nf + 255) / 256), 256, 0, ctx->stream>>>(b->d_range, nat_f, nf, k0, v0);
-        KIWI_LAUNCHED(ctx);
-        bool second = false;
-        KIWI_TRY(radix_sort_pairs(ctx, k0, v0, k1, v1, nf, 32, &second));
-        KIWI_CUDA(ctx, cudaMemcpyAsync(lpt_f, second ? v1 : v0, sizeof(int32_t) * nf, cudaMemcpyDeviceToDevice,
-                                       ctx->stream));
-    }
+    KIWI_TRY(batch_work(b));
     KIWI_CUDA(ctx, cudaMemcpyAsync(b->d_items, b->items.data(), sizeof(BatchItemDev) * n, cudaMemcpyHostToDevice,
                                    ctx->stream));
     DevStats* hs = nullptr;
@@ -313,7 +333,7 @@ int batch_build(KiwiBatch* b, const KiwiBatchItem* in) {
     b->item_skipped.resize(n);
     for (int i = 0; i < n; ++i) b->item_skipped[i] = (int64_t)h[i].skipped_outside;
 
-    KIWI_TRY(fp64_batch_prepare(ctx));
+    KIWI_TRY(lattice_batch_prepare(ctx));
     cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, ctx->device);
     return batch_record(b);
 }
@@ -365,7 +385,8 @@ int kiwi_batch_run(KiwiBatch* b, KiwiStats* item_stats, KiwiStats* total) {
     KIWI_TRY(batch_time_once(b, &ms));
     std::vector<DevStats> h(b->n_items);
     KIWI_CUDA(ctx, cudaMemcpy(h.data(), b->d_stats, sizeof(DevStats) * b->n_items, cudaMemcpyDeviceToHost));
-    int64_t kernels = b->n_items;  // mean velocities, then one gather launch per family present
+    // mean velocities, one launch per family present, the cut tiles' sums
+    int64_t kernels = b->n_items + (b->n_cut > 0 ? 1 : 0);
     for (int f = 0; f < kBatchFamilies; ++f) kernels += b->fam_tiles[f] > 0 ? 1 : 0;
     (void)launches0;
     KiwiStats sum{};

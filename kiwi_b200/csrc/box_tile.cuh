@@ -19,6 +19,12 @@
 // point within the support) and evaluates 32 of a kind at a time, so that no lane waits for another kind's work
 // and no list is shared between warps.
 //
+// A tile with a long list is cut into segments of box_segment() entries, each summed on its own (by CTAs of their
+// own, which leave raw sums for k_box_combine, or one after another in one CTA), and the segments' sums are
+// added in list order: a grid of few tiles, or a field with a few dense ones, then fills the chip.  The length
+// depends on the tile's own list and the grid's tile count alone, so that every call that maps a tile -- whole
+// grid, part, batch, allocation-free -- adds the same numbers in the same order.
+//
 // What bounds it: the FP64 pipe and the shared-memory loads of the records, about equally (a point within the
 // support issues about 150 FP64 instructions and 20 shared loads).
 #pragma once
@@ -30,6 +36,16 @@
 #include "lattice.cuh"
 
 namespace kiwi_b200 {
+
+// Entries per segment of a tile with cnt entries in a grid of ntiles tiles: 128 (where the whole grid has fewer
+// tiles than the chip has places, one tile in eight pieces or more) to 1024 (thousands of tiles: only outliers are cut),
+// and at most 16384 segments in the grid or 8 per tile beyond that, so that their sums stay small.
+__host__ __device__ __forceinline__ int64_t box_segment(int64_t cnt, int64_t ntiles) {
+    const int64_t s0 = ntiles / 4 < 128 ? 128 : (ntiles / 4 > 1024 ? 1024 : ntiles / 4);
+    const int64_t most = 16384 / ntiles < 8 ? 8 : (16384 / ntiles > 256 ? 256 : 16384 / ntiles);
+    const int64_t s1 = (cnt + most - 1) / most;
+    return s0 > s1 ? s0 : s1;
+}
 
 #ifndef KIWI_BOX_THREADS
 #define KIWI_BOX_THREADS 256
@@ -54,18 +70,20 @@ constexpr int kBoxPlaneCap = KIWI_BOX_PLANE_CAP;  // planes per chunk (a full bo
 constexpr int kBoxGenPtCap = 1792, kBoxGenPairCap = 640, kBoxGenPlaneCap = 256;
 static_assert(kBoxPairCap <= 1024 && kBoxPlaneCap <= 512, "packed edge entries");
 
-template <int NP>
+// SEQ: the segments of a tile one after another, which needs the cells' totals beside the segment's sums.
+template <int NP, bool SEQ = false>
 struct BoxCaps {
     static constexpr int kN = NP ? NP : KIWI_BOX_PIECES;
-    static constexpr int kPt = NP ? kBoxPtCap : kBoxGenPtCap;
-    static constexpr int kPair = NP ? kBoxPairCap : kBoxGenPairCap;
-    static constexpr int kPlane = NP ? kBoxPlaneCap : kBoxGenPlaneCap;
+    static constexpr int kPt = SEQ ? 1536 : (NP ? kBoxPtCap : kBoxGenPtCap);
+    static constexpr int kPair = SEQ ? (NP ? 768 : 512) : (NP ? kBoxPairCap : kBoxGenPairCap);
+    static constexpr int kPlane = SEQ ? 208 : (NP ? kBoxPlaneCap : kBoxGenPlaneCap);
     static constexpr int kQueues = kN;  // edge kinds; the point phase uses the first
     // dynamic shared memory, in doubles: the cells' sums, the octant values, the edge and plane records
     static constexpr int kOffT = 4 * kTileCells;
     static constexpr int kOffE = kOffT + kPt;
     static constexpr int kOffP = kOffE + box_edge_stride(kN) * kPair;
-    static constexpr int kEnd = kOffP + box_plane_stride(kN) * kPlane;
+    static constexpr int kOffS = kOffP + box_plane_stride(kN) * kPlane;
+    static constexpr int kEnd = kOffS + (SEQ ? 4 * kTileCells : 0);
     static constexpr size_t kSmem = sizeof(double) * kEnd + sizeof(uint32_t) * 64 * kBoxWarps * kQueues;
     // (C1) keeps the pairs' values in the edge records' place (with one piece the records are smaller)
     static_assert((NP ? box_edge_stride(kN) : box_edge_stride(1)) * kPair >= kPt, "pair values fit");
@@ -94,13 +112,52 @@ __device__ __forceinline__ double box_signed(double x, double a, double b, doubl
     return __hiloint2double(__double2hiint(x) ^ s, __double2loint(x));
 }
 
+// A cell's outputs from its sums (src/cartesian_grid.cpp:294-317).
+__device__ __forceinline__ void box_store(const CartGeom& g, const CartOutputs& out, int64_t t, int li, double M, double P1,
+                                          double P2, double P3) {
+    const int tz = (int)(t % g.ntz), ty = (int)((t / g.ntz) % g.nty), tx = (int)(t / ((int64_t)g.ntz * g.nty));
+    const int ix = tx * kTileX + li / (kTileZ * kTileY), iy = ty * kTileY + (li / kTileZ) % kTileY,
+              iz = tz * kTileZ + li % kTileZ;
+    if (ix >= g.nx || iy >= g.ny || iz >= g.nz) return;
+    const int64_t ncell = (int64_t)g.nx * g.ny * g.nz;
+    const int64_t i3 = ((int64_t)ix * g.ny + iy) * g.nz + iz;
+    if (out.density) out.density[i3] = M / g.cell_volume;
+    const bool has = M > 0.0;
+    if (out.vx) out.vx[i3] = has ? P1 / M : out.meanv[0];
+    if (out.vy) out.vy[i3] = has ? P2 / M : out.meanv[1];
+    if (out.vz) out.vz[i3] = has ? P3 / M : out.meanv[2];
+    if (out.raw4) {
+        out.raw4[i3] = M;
+        out.raw4[ncell + i3] = P1;
+        out.raw4[2 * ncell + i3] = P2;
+        out.raw4[3 * ncell + i3] = P3;
+    }
+}
+
+// A tile's cells from its segments' sums sums[segment][4][cell], added in list order (threads as the caller has).
+__device__ __forceinline__ void box_combine(const CartGeom& g, const CartOutputs& out, int64_t t, const double* sums,
+                                            int nseg) {
+    for (int li = threadIdx.x; li < kTileCells; li += blockDim.x) {
+        double a[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) a[c] = sums[c * kTileCells + li];
+        for (int s = 1; s < nseg; ++s)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) a[c] = add_rn(a[c], sums[(4 * (int64_t)s + c) * kTileCells + li]);
+        box_store(g, out, t, li, a[0], a[1], a[2], a[3]);
+    }
+}
+
+// The entries list[beg, end) of tile t: its outputs, or with `sums` their raw sums [4][cell].  SEQ: the list in
+// segments of `segment` entries, one after another.
 // NP, DEG: the kernel's pieces and largest power, known when compiling (the cubic spline: 2, 3), or 0 for any
 // kernel of the tables.  T: the kernel's table in constant memory.
-template <bool CULL, int NP, int DEG>
+template <bool CULL, int NP, int DEG, bool SEQ = false>
 __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& P, const uint32_t* __restrict__ list,
-                                         const int64_t* __restrict__ range, int64_t t_range, int64_t t,
-                                         const CartOutputs& out, DevStats* __restrict__ st, const KiwiBoxTable& T) {
-    using Caps = BoxCaps<NP>;
+                                         int64_t beg, int64_t end_all, int64_t segment, int64_t t,
+                                         const CartOutputs& out, double* __restrict__ sums, DevStats* __restrict__ st,
+                                         const KiwiBoxTable& T) {
+    using Caps = BoxCaps<NP, SEQ>;
     __shared__ BoxChunk s_cp[2];
     __shared__ double s_pl[3][kTileX + 1], s_cc[3][kTileX];
     __shared__ double s_C[NP ? 1 : (kBoxC + 1) * KIWI_BOX_PIECES];  // any kernel: c and C of its pieces (lanes differ in piece)
@@ -148,10 +205,12 @@ __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& 
         box_add_stat(&st->vertex_pyramids, n_vp);
         n_bbox = n_sphere = n_eval = n_neg = n_warn = n_eo = n_em = n_ei = n_vp = 0;
     };
-    const int64_t beg = range[2 * t_range], end = range[2 * t_range + 1];
+    // the end of the segment at hand (a chunk never crosses it)
+    auto segment_end = [&](int64_t at) { return SEQ ? min(at + segment, end_all) : end_all; };
+    int64_t end = segment_end(beg);
 
     // warp 0: the chunk of the particle list starting at `at` (as many particles as the capacities take)
-    auto load_chunk = [&](BoxChunk* dst, int64_t at) {
+    auto load_chunk = [&](BoxChunk* dst, int64_t at, int64_t end) {
         const int64_t idx = at + lane;
         int nl = 0, ne = 0, npt = 0, ncl = 0, lo0 = 0, lo1 = 0, lo2 = 0, d0 = 0, d1 = 0, d2 = 0;
         double px = 0, py = 0, pz = 0, ph = 1, pm = 0, pvx = 0, pvy = 0, pvz = 0;
@@ -226,17 +285,20 @@ __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& 
         }
     };
 
+    bool first_segment = true;
     BoxChunk* cp = &s_cp[0];
-    if (warp == 0 && beg < end) load_chunk(cp, beg);
+    if (warp == 0 && beg < end) load_chunk(cp, beg, end);
     __syncthreads();
     if (beg < end) form_planes(cp);
     __syncthreads();
 
-    for (int64_t pos = beg; pos < end;) {
+    for (int64_t pos = beg; pos < end_all;) {
         BoxChunk* const nx = cp == &s_cp[0] ? &s_cp[1] : &s_cp[0];
         const int np = cp->np;
-        const bool more = pos + np < end;
-        if (warp == 0 && more) load_chunk(nx, pos + np);
+        const bool more = pos + np < end_all;
+        const bool ends = SEQ && pos + np == end;  // the segment's last chunk
+        if (ends) end = segment_end(end);
+        if (warp == 0 && more) load_chunk(nx, pos + np, end);
 
         // (E) edge lines, block (x, y) over n0' x n1', (x, z) over n0' x n2', (y, z) over n1' x n2'
         {
@@ -448,7 +510,7 @@ __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& 
                 hit = i >= 0 && i < cp->dim[lane][0] && j0 < ly0 + 4 && j0 + cp->dim[lane][1] > ly0;
             }
             unsigned todo = __ballot_sync(0xffffffffu, hit);
-            if (todo == 0) continue;
+            if (todo == 0 && !ends) continue;
             double a0 = s_acc[li], a1 = s_acc[kTileCells + li];
             double a2 = s_acc[2 * kTileCells + li], a3 = s_acc[3 * kTileCells + li];
             for (; todo; todo &= todo - 1) {
@@ -463,11 +525,21 @@ __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& 
                 a2 = fma(mm, cp->vy[j], a2);
                 a3 = fma(mm, cp->vz[j], a3);
             }
+            if (SEQ && ends) {  // the first segment's sums as they are, the others' added
+                const double v[4] = {a0, a1, a2, a3};
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    double& tot = s_dyn[Caps::kOffS + q * kTileCells + li];
+                    tot = first_segment ? v[q] : add_rn(tot, v[q]);
+                }
+                a0 = a1 = a2 = a3 = 0.0;
+            }
             s_acc[li] = a0;
             s_acc[kTileCells + li] = a1;
             s_acc[2 * kTileCells + li] = a2;
             s_acc[3 * kTileCells + li] = a3;
         }
+        if (ends) first_segment = false;
         if (more) form_planes(nx);
         __syncthreads();
         pos += np;
@@ -478,27 +550,19 @@ __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& 
         }
     }
 
-    const double mvx = out.meanv[0], mvy = out.meanv[1], mvz = out.meanv[2];
-    const int64_t ncell = (int64_t)g.nx * g.ny * g.nz;
+    const double* const fin = SEQ && !first_segment ? s_dyn + Caps::kOffS : s_acc;
 #pragma unroll
     for (int c = 0; c < kBoxCells; ++c) {
         const int li = threadIdx.x + c * kBoxThreads;
         if (kTileCells % kBoxThreads && li >= kTileCells) break;
-        const int ix = bx + li / (kTileZ * kTileY), iy = by + (li / kTileZ) % kTileY, iz = bz + li % kTileZ;
-        if (ix >= g.nx || iy >= g.ny || iz >= g.nz) continue;
-        const int64_t i3 = ((int64_t)ix * g.ny + iy) * g.nz + iz;
-        const double M = s_acc[li];
-        if (out.density) out.density[i3] = M / g.cell_volume;
-        const bool has = M > 0.0;
-        const double P1 = s_acc[kTileCells + li], P2 = s_acc[2 * kTileCells + li], P3 = s_acc[3 * kTileCells + li];
-        if (out.vx) out.vx[i3] = has ? P1 / M : mvx;
-        if (out.vy) out.vy[i3] = has ? P2 / M : mvy;
-        if (out.vz) out.vz[i3] = has ? P3 / M : mvz;
-        if (out.raw4) {
-            out.raw4[i3] = M;
-            out.raw4[ncell + i3] = P1;
-            out.raw4[2 * ncell + i3] = P2;
-            out.raw4[3 * ncell + i3] = P3;
+        const double M = fin[li], P1 = fin[kTileCells + li], P2 = fin[2 * kTileCells + li], P3 = fin[3 * kTileCells + li];
+        if (sums) {
+            sums[li] = M;
+            sums[kTileCells + li] = P1;
+            sums[2 * kTileCells + li] = P2;
+            sums[3 * kTileCells + li] = P3;
+        } else {
+            box_store(g, out, t, li, M, P1, P2, P3);
         }
     }
     flush();

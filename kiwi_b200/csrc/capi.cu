@@ -163,7 +163,9 @@ int sph_to_grid_dev(KiwiCtx* ctx, const DevParticles& P, const CartGeom& g, cons
         k_tile_ranges<<<(unsigned)((total + 255) / 256), 256, 0, ctx->stream>>>(sk, total, range);
         KIWI_LAUNCHED(ctx);
     }
-    TileLists tl{sorted_vals, range, ntiles};
+    TileLists tl{sorted_vals, range, ntiles, total};
+    // the FP64 form orders its own work (lattice_cart_gather)
+    const bool own_order = (precision & KIWI_FORM_MASK) == KIWI_FP64 && !kc.tabulated && (kc.cubic || !(precision & KIWI_FULL_BOX));
     if (n_parts > 1) {
         // this part's tiles: a contiguous run of the tile order holding ~1/n_parts of the entries
         uint32_t *w = nullptr, *flags = nullptr;
@@ -189,7 +191,7 @@ int sph_to_grid_dev(KiwiCtx* ctx, const DevParticles& P, const CartGeom& g, cons
         KIWI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         tl.map = map;
         tl.nmap = nmap;
-    } else if (kTileLpt && !ctx->arena && ntiles > 1 && total > 0) {
+    } else if (kTileLpt && !ctx->arena && ntiles > 1 && total > 0 && !own_order) {
         // the whole grid, heaviest tiles first (by (tile, particle) entry count; ties in tile order), so that
         // the dense tiles of a clustered field do not start last and leave the SMs a tail
         uint32_t *lk0, *lv0, *lk1, *lv1;

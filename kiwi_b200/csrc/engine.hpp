@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <vector>
+
 #include "cart_common.cuh"
 #include "ctx.hpp"
 
@@ -35,6 +37,7 @@ struct TileLists {
     const uint32_t* list;
     const int64_t* range;
     int64_t ntiles;
+    int64_t total = 0;             // entries of all tiles
     const int32_t* map = nullptr;  // optional: run only tiles map[0 .. nmap) (device array)
     int64_t nmap = 0;
 };
@@ -85,13 +88,10 @@ struct BatchItemDev {
     DevStats* st;
 };
 
-// kiwi_fp64.cu: one persistent launch over the tiles order[0 .. ntiles) (global tile indices) of the items
-// of one family, taken from the work counter *next (zero before the launch); mixed: the lattice families'
-// FP32-mixed tile bodies.
-int fp64_batch_prepare(KiwiCtx* ctx);
-int fp64_batch_gather(KiwiCtx* ctx, int family, const BatchItemDev* d_items, const int32_t* d_item_of_tile,
-                      const int32_t* d_order, int64_t ntiles, const uint32_t* list, const int64_t* range,
-                      unsigned long long* d_next, int blocks, bool mixed);
+// kiwi_fp64.cu: one persistent launch of the gather family over the tiles order[0 .. ntiles) (global tile indices),
+// taken from the work counter *next (zero before the launch).
+int fp64_batch_gather(KiwiCtx* ctx, const BatchItemDev* d_items, const int32_t* d_item_of_tile, const int32_t* d_order,
+                      int64_t ntiles, const uint32_t* list, const int64_t* range, unsigned long long* d_next, int blocks);
 
 // mixed.cu: the FP32-mixed form (cubic spline).  cell_err (device, ncell doubles) receives each cell's
 // rounding-error bound and cell_mass (ncell doubles) its raw mass sum M.
@@ -143,8 +143,18 @@ int lattice_cart_gather(KiwiCtx* ctx, const CartGeom& g, const DevParticles& P, 
 int lattice_mixed_gather(KiwiCtx* ctx, const CartGeom& g, const DevParticles& P, const KernelChoice& k,
                          const TileLists& tl, const CartOutputs& out, DevStats* d_stats);
 int lattice_batch_prepare(KiwiCtx* ctx);
+// A batch's work (four ints per item: tile, segment, the tile's segments, the place of its sums): the items of
+// `tiles` given every tile's range, its grid's tile count and its place (host); split: long lists cut into
+// segments, else whole tiles; heaviest: in descending order of their entries.  Returns their number.
+int lattice_batch_work(const std::vector<int32_t>& tiles, const std::vector<int64_t>& range,
+                       const std::vector<int64_t>& grid_tiles, const std::vector<int32_t>& slot, bool split, bool heaviest,
+                       std::vector<int32_t>* work);
+int64_t lattice_batch_segments(int64_t cnt, int64_t grid_tiles);
+// sums: raw sums of the cut tiles' segments, 4 x kTileCells doubles each; d_cut: the cut tiles' first items.
 int lattice_batch_gather(KiwiCtx* ctx, int family, const BatchItemDev* d_items, const int32_t* d_item_of_tile,
-                         const int32_t* d_order, int64_t ntiles, const uint32_t* list, const int64_t* range,
+                         const int32_t* d_work, int64_t nwork, const uint32_t* list, const int64_t* range, double* sums,
                          unsigned long long* d_next, int blocks, bool mixed);
+int lattice_batch_combine(KiwiCtx* ctx, const BatchItemDev* d_items, const int32_t* d_item_of_tile, const int32_t* d_cut,
+                          int64_t n, const double* sums);
 
 }  // namespace kiwi_b200

@@ -7,6 +7,10 @@
 // explicitly rounded operations (cart_common.cuh), as in every other form.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <utility>
+#include <vector>
+
 #include "engine.hpp"
 #include "kernel_tables.h"
 
@@ -46,22 +50,117 @@ constexpr size_t kLatMergedDynSmem = kLatDynSmem > kLatGenDynSmem ? kLatDynSmem 
 #ifndef KIWI_BOX_MIN_BLOCKS
 #define KIWI_BOX_MIN_BLOCKS 2
 #endif
-#ifndef KIWI_BOX_GEN_MIN_BLOCKS
-#define KIWI_BOX_GEN_MIN_BLOCKS 2
-#endif
 constexpr int kBoxMinBlocks = KIWI_BOX_MIN_BLOCKS;
-constexpr int kBoxGenMinBlocks = KIWI_BOX_GEN_MIN_BLOCKS;
 constexpr size_t kBoxSmem = BoxCaps<2>::kSmem, kBoxGenSmem = BoxCaps<0>::kSmem;
 constexpr size_t kBoxMergedSmem = kBoxSmem > kBoxGenSmem ? kBoxSmem : kBoxGenSmem;
 
-template <bool CULL>
-__global__ void __launch_bounds__(kBoxThreads, kBoxMinBlocks) k_cart_box(CartGeom g, DevParticles P,
-                                                                         const uint32_t* __restrict__ list,
-                                                                         const int64_t* __restrict__ range,
-                                                                         const int32_t* __restrict__ tile_map,
-                                                                         CartOutputs out, DevStats* __restrict__ st) {
-    const int64_t t = tile_map ? (int64_t)tile_map[blockIdx.x] : (int64_t)blockIdx.x;
-    box_tile<CULL, 2, 3>(g, P, list, range, t, t, out, st, c_box[0]);
+// One piece of work: segment `seg` of the `nseg` of tile `tile`; its sums go to the partial sums' place slot + seg if
+// nseg > 1.
+struct BoxItem {
+    int32_t tile, seg, nseg, slot;
+};
+static_assert(sizeof(BoxItem) == sizeof(int4), "items are read as one int4");
+
+// Runs one item; range: the tile's list.
+template <bool CULL, int NP, int DEG>
+__device__ __forceinline__ void box_item(const BoxItem& it, const CartGeom& g, const DevParticles& P,
+                                         const uint32_t* __restrict__ list, const int64_t* __restrict__ range,
+                                         int64_t t, const CartOutputs& out, double* __restrict__ sums,
+                                         DevStats* __restrict__ st, const KiwiBoxTable& T) {
+    const int64_t lo = range[0], hi = range[1];
+    const int64_t len = box_segment(hi - lo, (int64_t)g.ntx * g.nty * g.ntz);
+    const int64_t beg = lo + it.seg * len, end = it.nseg > 1 ? min(beg + len, hi) : hi;
+    box_tile<CULL, NP, DEG>(g, P, list, beg, end, 0, t, out,
+                            it.nseg > 1 ? sums + (int64_t)(it.slot + it.seg) * 4 * kTileCells : nullptr, st, T);
+}
+
+// A kernel of pieces NP and powers DEG (0: any of the tables'), over items, or without them over the tiles
+// tile_map[0 ..) (every tile if null), each tile by one CTA: SEQ cuts it into its segments, else no list is longer
+// than one.
+template <bool CULL, int NP, int DEG, bool SEQ>
+__global__ void __launch_bounds__(kBoxThreads, kBoxMinBlocks)
+    k_cart_box(CartGeom g, DevParticles P, int kernel, const uint32_t* __restrict__ list,
+               const int64_t* __restrict__ range, const int32_t* __restrict__ tile_map, const BoxItem* __restrict__ items,
+               CartOutputs out, double* __restrict__ sums, DevStats* __restrict__ st) {
+    const KiwiBoxTable& T = NP ? c_box[0] : c_box[kernel];
+    if (SEQ) {
+        const int64_t t = tile_map ? (int64_t)tile_map[blockIdx.x] : (int64_t)blockIdx.x;
+        const int64_t lo = range[2 * t], hi = range[2 * t + 1];
+        box_tile<CULL, NP, DEG, true>(g, P, list, lo, hi, box_segment(hi - lo, (int64_t)g.ntx * g.nty * g.ntz), t, out,
+                                      nullptr, st, T);
+        return;
+    }
+    BoxItem it{tile_map ? tile_map[blockIdx.x] : (int)blockIdx.x, 0, 1, 0};
+    if (items) it = items[blockIdx.x];
+    box_item<CULL, NP, DEG>(it, g, P, list, range + 2 * (int64_t)it.tile, it.tile, out, sums, st, T);
+}
+
+// The cut tiles' outputs: one CTA per tile (its item of segment 0).
+__global__ void __launch_bounds__(256) k_box_combine(CartGeom g, const BoxItem* __restrict__ cut,
+                                                     const double* __restrict__ sums, CartOutputs out) {
+    const BoxItem it = cut[blockIdx.x];
+    box_combine(g, out, it.tile, sums + (int64_t)it.slot * 4 * kTileCells, it.nseg);
+}
+
+// The items of the tiles map[0 .. n) (every tile if null), heaviest first by 64 classes of their entry counts (the
+// order among the items, and among the places of their sums, does not affect any result).  counts: items, places
+// of sums, cut tiles, then the classes' sizes and their running starts (64 each).
+constexpr int kBoxClasses = 64;
+__device__ __forceinline__ int box_class(int64_t len, int64_t ntiles) {
+    const int64_t c = len * kBoxClasses / (box_segment(0, ntiles) + 1);
+    return kBoxClasses - 1 - (int)(c < kBoxClasses ? c : kBoxClasses - 1);
+}
+template <bool EMIT>
+__global__ void __launch_bounds__(256) k_box_items(const int64_t* __restrict__ range, int64_t ntiles,
+                                                   const int32_t* __restrict__ map, int64_t n, int* __restrict__ counts,
+                                                   BoxItem* __restrict__ items, BoxItem* __restrict__ cut) {
+    __shared__ int s_n[kBoxClasses], s_at[kBoxClasses];
+    if (threadIdx.x < kBoxClasses) s_n[threadIdx.x] = 0;
+    __syncthreads();
+    const int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    int t = 0, nseg = 0, full = 0, last = 0, at_full = 0, at_last = 0;
+    if (w < n) {
+        t = map ? map[w] : (int)w;
+        const int64_t cnt = range[2 * (int64_t)t + 1] - range[2 * (int64_t)t], len = box_segment(cnt, ntiles);
+        nseg = cnt > len ? (int)((cnt + len - 1) / len) : 1;
+        full = box_class(len, ntiles);
+        last = box_class(cnt - (nseg - 1) * len, ntiles);
+        if (nseg > 1) at_full = atomicAdd(&s_n[full], nseg - 1);
+        at_last = atomicAdd(&s_n[last], 1);
+    }
+    __syncthreads();
+    if (!EMIT) {
+        if (threadIdx.x < kBoxClasses && s_n[threadIdx.x]) atomicAdd(&counts[4 + threadIdx.x], s_n[threadIdx.x]);
+        int items_n = nseg, places = nseg > 1 ? nseg : 0, tiles = nseg > 1;
+        for (int o = 16; o > 0; o >>= 1) {
+            items_n += __shfl_down_sync(0xffffffffu, items_n, o);
+            places += __shfl_down_sync(0xffffffffu, places, o);
+            tiles += __shfl_down_sync(0xffffffffu, tiles, o);
+        }
+        if ((threadIdx.x & 31) == 0) {
+            if (items_n) atomicAdd(&counts[0], items_n);
+            if (places) {
+                atomicAdd(&counts[1], places);
+                atomicAdd(&counts[2], tiles);
+            }
+        }
+        return;
+    }
+    // the classes' first items, then this block's place in each
+    if (threadIdx.x < kBoxClasses) {
+        int first = 0;
+        for (int c = 0; c < (int)threadIdx.x; ++c) first += counts[4 + c];
+        s_at[threadIdx.x] = first + (s_n[threadIdx.x] ? atomicAdd(&counts[4 + kBoxClasses + threadIdx.x], s_n[threadIdx.x]) : 0);
+    }
+    __syncthreads();
+    if (w >= n) return;
+    int slot = 0;
+    if (nseg > 1) {
+        slot = atomicAdd(&counts[4 + 2 * kBoxClasses], nseg);
+        cut[atomicAdd(&counts[4 + 2 * kBoxClasses + 1], 1)] = BoxItem{t, 0, nseg, slot};
+    }
+    for (int s = 0; s + 1 < nseg; ++s) items[s_at[full] + at_full + s] = BoxItem{t, s, nseg, slot};
+    items[s_at[last] + at_last] = BoxItem{t, nseg - 1, nseg, slot};
 }
 
 // The FP32-mixed form of the cubic lattice kernel (support cells only): edge pairs and lattice points
@@ -77,17 +176,6 @@ __global__ void __launch_bounds__(kLatThreads, kLatMinBlocks) k_cart_lattice_mix
     lattice_tile<true, false, false, true>(g, P, list, range, t, t, out, st);
 }
 
-// Any kernel of the tables (support cells only).
-__global__ void __launch_bounds__(kBoxThreads, kBoxGenMinBlocks) k_cart_box_generic(CartGeom g, DevParticles P, int kernel,
-                                                                               const uint32_t* __restrict__ list,
-                                                                               const int64_t* __restrict__ range,
-                                                                               const int32_t* __restrict__ tile_map,
-                                                                               CartOutputs out,
-                                                                               DevStats* __restrict__ st) {
-    const int64_t t = tile_map ? (int64_t)tile_map[blockIdx.x] : (int64_t)blockIdx.x;
-    box_tile<true, 0, 0>(g, P, list, range, t, t, out, st, c_box[kernel]);
-}
-
 // The FP32-mixed form of the generic lattice kernel: edge records and vertex tiers in FP32 (FP64 islands
 // where a plane lies within 1e-3 h of the particle), records, cell assembly and per-cell sums in FP64.
 __global__ void __launch_bounds__(kLatThreads, kLatGenMinBlocks)
@@ -98,22 +186,23 @@ __global__ void __launch_bounds__(kLatThreads, kLatGenMinBlocks)
     lattice_tile<true, true, false, true>(g, P, list, range, t, t, out, st, &c_tables[kernel]);
 }
 
-// The tiles of a batch of grids, one persistent launch per lattice family, or one for both
-// (kBatchFamilyLatticeMerged: each tile takes its item's body): each CTA takes the next of the launch's
-// tiles (order[w]) from the work counter and runs the same tile body as the single-grid kernel, so every
-// cell's summation order is that of a single-grid call.  MIXED: the FP32-mixed tile bodies.
+// The work of a batch of grids, one persistent launch per lattice family, or one for both
+// (kBatchFamilyLatticeMerged: each item takes its grid's body): each CTA takes the next of the launch's
+// work items from the work counter and runs the same body as the single-grid kernel, so every
+// cell's summation order is that of a single-grid call.  MIXED: the FP32-mixed tile bodies (items are whole tiles).
 template <int FAMILY, bool MIXED>
 __global__ void __launch_bounds__(MIXED ? kLatThreads : kBoxThreads, 2)
     k_batch_lattice(const BatchItemDev* __restrict__ items, const int32_t* __restrict__ item_of_tile,
-                    const int32_t* __restrict__ order, int64_t ntiles, const uint32_t* __restrict__ list,
-                    const int64_t* __restrict__ range, unsigned long long* __restrict__ next) {
+                    const BoxItem* __restrict__ work, int64_t nwork, const uint32_t* __restrict__ list,
+                    const int64_t* __restrict__ range, double* __restrict__ sums, unsigned long long* __restrict__ next) {
     __shared__ long long s_w;
     for (;;) {
         if (threadIdx.x == 0) s_w = (long long)atomicAdd(next, 1ull);
         __syncthreads();
         const int64_t w = s_w;
-        if (w >= ntiles) break;
-        const int64_t tg = (int64_t)order[w];
+        if (w >= nwork) break;
+        const BoxItem wi = work[w];
+        const int64_t tg = wi.tile;
         const BatchItemDev& it = items[item_of_tile[tg]];
         const int64_t tl = tg - it.tile_base;
         const bool cubic = FAMILY == kBatchFamilyLattice || (FAMILY == kBatchFamilyLatticeMerged && it.mode == kBatchLattice);
@@ -121,11 +210,19 @@ __global__ void __launch_bounds__(MIXED ? kLatThreads : kBoxThreads, 2)
             if (cubic) lattice_tile<true, false, false, true>(it.g, it.P, list, range, tg, tl, it.out, it.st);
             else lattice_tile<true, true, false, true>(it.g, it.P, list, range, tg, tl, it.out, it.st, &c_tables[it.kernel]);
         } else {
-            if (cubic) box_tile<true, 2, 3>(it.g, it.P, list, range, tg, tl, it.out, it.st, c_box[0]);
-            else box_tile<true, 0, 0>(it.g, it.P, list, range, tg, tl, it.out, it.st, c_box[it.kernel]);
+            if (cubic) box_item<true, 2, 3>(wi, it.g, it.P, list, range + 2 * tg, tl, it.out, sums, it.st, c_box[0]);
+            else box_item<true, 0, 0>(wi, it.g, it.P, list, range + 2 * tg, tl, it.out, sums, it.st, c_box[it.kernel]);
         }
         __syncthreads();
     }
+}
+
+__global__ void __launch_bounds__(256) k_batch_combine(const BatchItemDev* __restrict__ items,
+                                                       const int32_t* __restrict__ item_of_tile,
+                                                       const BoxItem* __restrict__ cut, const double* __restrict__ sums) {
+    const BoxItem wi = cut[blockIdx.x];
+    const BatchItemDev& it = items[item_of_tile[wi.tile]];
+    box_combine(it.g, it.out, wi.tile - it.tile_base, sums + (int64_t)wi.slot * 4 * kTileCells, wi.nseg);
 }
 
 // The shared memory and block size of a batch launch.
@@ -139,22 +236,90 @@ constexpr size_t batch_smem() {
 
 }  // namespace
 
-template <class K, class... A>
-static int box_launch(KiwiCtx* ctx, K* kernel, size_t smem, dim3 grid, A... args) {
-    KIWI_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kernel<<<grid, kBoxThreads, smem, ctx->stream>>>(args...);
+template <bool CULL, int NP, int DEG, bool SEQ>
+static int box_launch(KiwiCtx* ctx, int64_t blocks, const CartGeom& g, const DevParticles& P, int kernel,
+                      const TileLists& tl, const BoxItem* items, const CartOutputs& out, double* sums, DevStats* st) {
+    constexpr size_t smem = BoxCaps<NP, SEQ>::kSmem;
+    KIWI_CUDA(ctx, cudaFuncSetAttribute(k_cart_box<CULL, NP, DEG, SEQ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)smem));
+    k_cart_box<CULL, NP, DEG, SEQ><<<(unsigned)blocks, kBoxThreads, smem, ctx->stream>>>(g, P, kernel, tl.list, tl.range,
+                                                                                      tl.map, items, out, sums, st);
     KIWI_LAUNCHED(ctx);
     return KIWI_OK;
 }
 
+template <bool SEQ>
+static int box_launch_kernel(KiwiCtx* ctx, int64_t blocks, const CartGeom& g, const DevParticles& P, const KernelChoice& k,
+                             const TileLists& tl, const BoxItem* items, const CartOutputs& out, double* sums,
+                             DevStats* st, bool full_box) {
+    if (!k.cubic) return box_launch<true, 0, 0, SEQ>(ctx, blocks, g, P, k.kernel, tl, items, out, sums, st);
+    if (full_box) return box_launch<false, 2, 3, SEQ>(ctx, blocks, g, P, 0, tl, items, out, sums, st);
+    return box_launch<true, 2, 3, SEQ>(ctx, blocks, g, P, 0, tl, items, out, sums, st);
+}
+
 int lattice_cart_gather(KiwiCtx* ctx, const CartGeom& g, const DevParticles& P, const KernelChoice& k,
                         const TileLists& tl, const CartOutputs& out, DevStats* d_stats, bool full_box) {
-    const dim3 grid((unsigned)(tl.map ? tl.nmap : tl.ntiles));
-    if (!k.cubic)
-        return box_launch(ctx, k_cart_box_generic, kBoxGenSmem, grid, g, P, k.kernel, tl.list, tl.range, tl.map, out,
-                          d_stats);
-    if (full_box) return box_launch(ctx, k_cart_box<false>, kBoxSmem, grid, g, P, tl.list, tl.range, tl.map, out, d_stats);
-    return box_launch(ctx, k_cart_box<true>, kBoxSmem, grid, g, P, tl.list, tl.range, tl.map, out, d_stats);
+    const int64_t n = tl.map ? tl.nmap : tl.ntiles;
+    // without scratch of its own (the allocation-free call), one CTA per tile cuts it
+    if (ctx->arena) return box_launch_kernel<true>(ctx, n, g, P, k, tl, nullptr, out, nullptr, d_stats, full_box);
+    // no list can be longer than a segment: the tiles as they are
+    const int64_t least = box_segment(0, tl.ntiles);
+    if (tl.total <= least) return box_launch_kernel<false>(ctx, n, g, P, k, tl, nullptr, out, nullptr, d_stats, full_box);
+    constexpr int kCounts = 4 + 2 * kBoxClasses + 2;
+    int* counts = nullptr;
+    KIWI_TRY(scratch_t(ctx, S_BOX_COUNTS, kCounts, &counts));
+    KIWI_CUDA(ctx, cudaMemsetAsync(counts, 0, sizeof(int) * kCounts, ctx->stream));
+    const unsigned nb = (unsigned)((n + 255) / 256);
+    k_box_items<false><<<nb, 256, 0, ctx->stream>>>(tl.range, tl.ntiles, tl.map, n, counts, nullptr, nullptr);
+    KIWI_LAUNCHED(ctx);
+    int h[3] = {0, 0, 0};
+    KIWI_CUDA(ctx, cudaMemcpyAsync(h, counts, sizeof h, cudaMemcpyDeviceToHost, ctx->stream));
+    KIWI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    BoxItem *items = nullptr, *cut = nullptr;
+    double* sums = nullptr;
+    KIWI_TRY(scratch_t(ctx, S_BOX_ITEMS, (size_t)h[0], &items));
+    KIWI_TRY(scratch_t(ctx, S_BOX_CUT, (size_t)(h[2] > 0 ? h[2] : 1), &cut));
+    if (h[1] > 0) KIWI_TRY(scratch_t(ctx, S_BOX_SUMS, (size_t)h[1] * 4 * kTileCells, &sums));
+    k_box_items<true><<<nb, 256, 0, ctx->stream>>>(tl.range, tl.ntiles, tl.map, n, counts, items, cut);
+    KIWI_LAUNCHED(ctx);
+    KIWI_TRY(box_launch_kernel<false>(ctx, h[0], g, P, k, tl, items, out, sums, d_stats, full_box));
+    if (h[2] > 0) {
+        k_box_combine<<<(unsigned)h[2], 256, 0, ctx->stream>>>(g, cut, sums, out);
+        KIWI_LAUNCHED(ctx);
+    }
+    return KIWI_OK;
+}
+
+// The work of a batch's tiles tiles[0 .. n) with their ranges (host): natural order, or heaviest segment first.
+int lattice_batch_work(const std::vector<int32_t>& tiles, const std::vector<int64_t>& range,
+                       const std::vector<int64_t>& grid_tiles, const std::vector<int32_t>& slot, bool split, bool heaviest,
+                       std::vector<int32_t>* work) {
+    std::vector<std::pair<int64_t, BoxItem>> v;
+    for (const int32_t t : tiles) {
+        const int64_t cnt = range[2 * (size_t)t + 1] - range[2 * (size_t)t];
+        const int64_t len = split ? box_segment(cnt, grid_tiles[(size_t)t]) : cnt;
+        const int nseg = cnt > len ? (int)((cnt + len - 1) / len) : 1;
+        for (int s = 0; s < nseg; ++s)
+            v.push_back({nseg > 1 ? std::min(len, cnt - s * len) : cnt, BoxItem{t, s, nseg, nseg > 1 ? slot[(size_t)t] : 0}});
+    }
+    if (heaviest) std::stable_sort(v.begin(), v.end(), [](const auto& a, const auto& b) { return a.first > b.first; });
+    work->clear();
+    for (const auto& e : v) work->insert(work->end(), {e.second.tile, e.second.seg, e.second.nseg, e.second.slot});
+    return (int)v.size();
+}
+
+int64_t lattice_batch_segments(int64_t cnt, int64_t grid_tiles) {
+    const int64_t len = box_segment(cnt, grid_tiles);
+    return cnt > len ? (cnt + len - 1) / len : 1;
+}
+
+int lattice_batch_combine(KiwiCtx* ctx, const BatchItemDev* d_items, const int32_t* d_item_of_tile, const int32_t* d_cut,
+                          int64_t n, const double* sums) {
+    if (n <= 0) return KIWI_OK;
+    k_batch_combine<<<(unsigned)n, 256, 0, ctx->stream>>>(d_items, d_item_of_tile, reinterpret_cast<const BoxItem*>(d_cut),
+                                                          sums);
+    KIWI_LAUNCHED(ctx);
+    return KIWI_OK;
 }
 
 int lattice_mixed_gather(KiwiCtx* ctx, const CartGeom& g, const DevParticles& P, const KernelChoice& k,
@@ -202,34 +367,35 @@ int lattice_batch_prepare(KiwiCtx* ctx) {
 }
 
 template <int FAMILY, bool MIXED>
-static void batch_launch_t(KiwiCtx* ctx, const BatchItemDev* d_items, const int32_t* d_item_of_tile,
-                           const int32_t* d_order, int64_t ntiles, const uint32_t* list, const int64_t* range,
+static void batch_launch_t(KiwiCtx* ctx, const BatchItemDev* d_items, const int32_t* d_item_of_tile, const BoxItem* work,
+                           int64_t nwork, const uint32_t* list, const int64_t* range, double* sums,
                            unsigned long long* d_next, int blocks) {
     k_batch_lattice<FAMILY, MIXED><<<blocks, MIXED ? kLatThreads : kBoxThreads, batch_smem<FAMILY, MIXED>(), ctx->stream>>>(
-        d_items, d_item_of_tile, d_order, ntiles, list, range, d_next);
+        d_items, d_item_of_tile, work, nwork, list, range, sums, d_next);
 }
 
 template <bool MIXED>
 static void batch_launch_form(KiwiCtx* ctx, int family, const BatchItemDev* d_items, const int32_t* d_item_of_tile,
-                              const int32_t* d_order, int64_t ntiles, const uint32_t* list, const int64_t* range,
-                              unsigned long long* d_next, int blocks) {
+                              const BoxItem* work, int64_t nwork, const uint32_t* list, const int64_t* range,
+                              double* sums, unsigned long long* d_next, int blocks) {
     if (family == kBatchFamilyLattice)
-        batch_launch_t<kBatchFamilyLattice, MIXED>(ctx, d_items, d_item_of_tile, d_order, ntiles, list, range, d_next, blocks);
+        batch_launch_t<kBatchFamilyLattice, MIXED>(ctx, d_items, d_item_of_tile, work, nwork, list, range, sums, d_next, blocks);
     else if (family == kBatchFamilyLatticeMerged)
-        batch_launch_t<kBatchFamilyLatticeMerged, MIXED>(ctx, d_items, d_item_of_tile, d_order, ntiles, list, range,
+        batch_launch_t<kBatchFamilyLatticeMerged, MIXED>(ctx, d_items, d_item_of_tile, work, nwork, list, range, sums,
                                                          d_next, blocks);
     else
-        batch_launch_t<kBatchFamilyLatticeGeneric, MIXED>(ctx, d_items, d_item_of_tile, d_order, ntiles, list, range,
+        batch_launch_t<kBatchFamilyLatticeGeneric, MIXED>(ctx, d_items, d_item_of_tile, work, nwork, list, range, sums,
                                                           d_next, blocks);
 }
 
 int lattice_batch_gather(KiwiCtx* ctx, int family, const BatchItemDev* d_items, const int32_t* d_item_of_tile,
-                         const int32_t* d_order, int64_t ntiles, const uint32_t* list, const int64_t* range,
+                         const int32_t* d_work, int64_t nwork, const uint32_t* list, const int64_t* range, double* sums,
                          unsigned long long* d_next, int blocks, bool mixed) {
+    const BoxItem* work = reinterpret_cast<const BoxItem*>(d_work);
     if (mixed)
-        batch_launch_form<true>(ctx, family, d_items, d_item_of_tile, d_order, ntiles, list, range, d_next, blocks);
+        batch_launch_form<true>(ctx, family, d_items, d_item_of_tile, work, nwork, list, range, sums, d_next, blocks);
     else
-        batch_launch_form<false>(ctx, family, d_items, d_item_of_tile, d_order, ntiles, list, range, d_next, blocks);
+        batch_launch_form<false>(ctx, family, d_items, d_item_of_tile, work, nwork, list, range, sums, d_next, blocks);
     KIWI_LAUNCHED(ctx);
     return KIWI_OK;
 }
