@@ -542,7 +542,7 @@ class Batch:
 
     def tune(self):
         """Times the launch shapes and keeps the fastest; returns (longest_first, ctas_per_sm) and sets
-        self.merged (both lattice families in one persistent launch)."""
+        self.merged (several families' launches side by side, in the FP32-mixed form in one launch)."""
         c = C.c_int(0)
         self.ctx.check(self.ctx._L.kiwi_batch_tune(self._h, C.byref(c)), "batch tune")
         self.merged = bool(c.value & 0x10000)

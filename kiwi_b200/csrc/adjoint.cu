@@ -52,8 +52,9 @@ static __constant__ KiwiBoxTable c_adj_box[KIWI_NUM_KERNELS];
 // Chunk capacities: two CTAs per SM (a full 8^3 box has 729 points, 243 edge lines and 27 planes).
 template <int NP>
 struct AdjCaps {
-    static constexpr int kN = NP ? NP : KIWI_BOX_PIECES;
-    static constexpr int kPt = NP ? 1024 : 800, kPair = NP ? 352 : 272, kPlane = NP ? 136 : 120;
+    static constexpr int kN = NP;
+    static constexpr int kPt = NP == 1 ? 1280 : (NP == 2 ? 1024 : 800), kPair = NP == 1 ? 512 : (NP == 2 ? 352 : 272),
+                         kPlane = NP == 1 ? 192 : (NP == 2 ? 136 : 120);
     static constexpr int kOffE = kAdjComps * kPt;
     static constexpr int kOffP = kOffE + box_grad_edge_stride(kN) * kPair;
     static constexpr int kEnd = kOffP + box_grad_plane_stride(kN) * kPlane;
@@ -79,8 +80,9 @@ struct AdjChunk {
 // The partial gradients of the sorted entries [blockIdx.x per_block, ..): keys their tiles, list their entry
 // numbers, owner the particle of an entry; part receives 8 doubles per entry: dL/dm, dL/d(x, y, z, h),
 // dL/d(vx, vy, vz) over the entry's tile.
-template <int NP, int DEG>
-__global__ void __launch_bounds__(kAdjThreads, 2) k_cart_adjoint_box(CartGeom g, DevParticles P, int kernel,
+// KERNEL: the kernel's table; NP, DEG: its pieces and largest power.
+template <int KERNEL, int NP, int DEG>
+__global__ void __launch_bounds__(kAdjThreads, 2) k_cart_adjoint_box(CartGeom g, DevParticles P,
                                                                      const uint32_t* __restrict__ keys,
                                                                      const uint32_t* __restrict__ list,
                                                                      const uint32_t* __restrict__ owner, int64_t total,
@@ -90,12 +92,11 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_cart_adjoint_box(CartGeom g,
     using Caps = AdjCaps<NP>;
     __shared__ AdjChunk s_cp;
     __shared__ double s_pl[3][kTileX + 1], s_cc[3][kTileX];
-    __shared__ double s_C[NP ? 1 : (kBoxC + kBoxD + 1) * KIWI_BOX_PIECES];
+    __shared__ double s_C[NP == 2 ? 1 : (kBoxC + kBoxD + 1) * NP];
     __shared__ int64_t s_seg_end;
     extern __shared__ double s_dyn[];
-    const KiwiBoxTable& T = NP ? c_adj_box[0] : c_adj_box[kernel];
-    const int n = NP ? NP : T.npiece;
-    const int kPS = box_grad_plane_stride(n), kES = box_grad_edge_stride(n);
+    const KiwiBoxTable& T = c_adj_box[KERNEL];
+    constexpr int n = NP, kPS = box_grad_plane_stride(NP), kES = box_grad_edge_stride(NP);
     double* const s_T = s_dyn;
     double* const s_E = s_dyn + Caps::kOffE;
     double* const s_P = s_dyn + Caps::kOffP;
@@ -103,7 +104,7 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_cart_adjoint_box(CartGeom g,
     const unsigned below = (1u << lane) - 1;
     uint32_t* const s_q = reinterpret_cast<uint32_t*>(s_dyn + Caps::kEnd) + 64 * Caps::kN * warp;
     constexpr int kCS = kBoxC + kBoxD + 1;
-    if (!NP)
+    if (NP != 2)
         for (int i = threadIdx.x; i < kCS * n; i += kAdjThreads) {
             const int k = i / kCS, c = i % kCS;
             s_C[i] = c < kBoxC ? T.reg[k].C[c] : (c < kBoxC + kBoxD ? T.reg[k].D[c - kBoxC] : T.reg[k].c);
@@ -532,18 +533,16 @@ int cart_adjoint_dev(KiwiCtx* ctx, const DevParticles& P, const CartGeom& g, con
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
         const int per = (int)std::min<int64_t>(256, std::max<int64_t>(16, total / (16 * (int64_t)sms)));
         const unsigned blocks = (unsigned)((total + per - 1) / per);
-        const size_t smem = kc.cubic ? AdjCaps<2>::kSmem : AdjCaps<0>::kSmem;
-        if (kc.cubic) {
-            KIWI_CUDA(ctx, cudaFuncSetAttribute(k_cart_adjoint_box<2, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                (int)smem));
-            k_cart_adjoint_box<2, 3><<<blocks, kAdjThreads, smem, ctx->stream>>>(g, P, 0, sk, sv, owner, total, per,
-                                                                                 d_cot, part, d_st);
-        } else {
-            KIWI_CUDA(ctx, cudaFuncSetAttribute(k_cart_adjoint_box<0, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                (int)smem));
-            k_cart_adjoint_box<0, 0><<<blocks, kAdjThreads, smem, ctx->stream>>>(g, P, kc.kernel, sk, sv, owner, total,
-                                                                                 per, d_cot, part, d_st);
-        }
+#define KIWI_ADJ_LAUNCH(K, NP, DEG)                                                                                      \
+    if (kc.kernel == K) {                                                                                               \
+        KIWI_CUDA(ctx, cudaFuncSetAttribute(k_cart_adjoint_box<K, NP, DEG>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+                                            (int)AdjCaps<NP>::kSmem));                                                  \
+        k_cart_adjoint_box<K, NP, DEG><<<blocks, kAdjThreads, AdjCaps<NP>::kSmem, ctx->stream>>>(g, P, sk, sv, owner,    \
+                                                                                             total, per, d_cot, part,   \
+                                                                                             d_st);                     \
+    }
+        KIWI_BOX_KERNELS(KIWI_ADJ_LAUNCH)
+#undef KIWI_ADJ_LAUNCH
         KIWI_LAUNCHED(ctx);
     }
     if (n > 0) {

@@ -37,10 +37,12 @@ struct KiwiBatch {
     int32_t* d_natural[kBatchFamilies] = {};
     int32_t* d_lpt[kBatchFamilies] = {};
     int64_t fam_tiles[kBatchFamilies] = {};  // work items
-    // both lattice families' work together (natural order and longest-first), for the merged launch
+    // FP32-mixed form: both lattice families' work together (natural order and longest-first), for the merged launch
     int32_t* d_natural_m = nullptr;
     int32_t* d_lpt_m = nullptr;
     int64_t merged_tiles = 0;
+    // FP32-mixed form: both families in one launch; FP64 form: the kernels' launches side by side (else one after
+    // another), so that one fills the places that another's last items leave
     bool merge = false;
     // the tiles whose lists are cut into segments (their first items) and their segments' raw sums
     int32_t* d_cut = nullptr;
@@ -94,27 +96,58 @@ void batch_free(KiwiBatch* b) {
     b->allocs.clear();
 }
 
-// The replayed work: reset the counters, the mean velocities, one persistent launch per family present.
+int families_present(const KiwiBatch* b) {
+    int k = 0;
+    for (int f = 0; f < kBatchFamilies; ++f) k += b->fam_tiles[f] > 0;
+    return k;
+}
+
+// The node(s) that the next captured operation of the stream will follow.
+int capture_front(KiwiCtx* ctx, std::vector<cudaGraphNode_t>* front) {
+    cudaStreamCaptureStatus status;
+    const cudaGraphNode_t* deps = nullptr;
+    size_t n = 0;
+    KIWI_CUDA(ctx, cudaStreamGetCaptureInfo(ctx->stream, &status, nullptr, nullptr, &deps, &n));
+    front->assign(deps, deps + n);
+    return KIWI_OK;
+}
+int capture_after(KiwiCtx* ctx, std::vector<cudaGraphNode_t> front) {
+    KIWI_CUDA(ctx, cudaStreamUpdateCaptureDependencies(ctx->stream, front.data(), front.size(),
+                                                       cudaStreamSetCaptureDependencies));
+    return KIWI_OK;
+}
+
+// The replayed work, captured: reset the counters, the mean velocities, one persistent launch per family present
+// (side by side: each follows the mean velocities alone), the cut tiles' sums.
 int batch_enqueue(KiwiBatch* b) {
     KiwiCtx* ctx = b->ctx;
     const bool mixed = (b->precision & KIWI_FORM_MASK) == KIWI_FP32_MIXED;
     KIWI_CUDA(ctx, cudaMemsetAsync(b->d_next, 0, sizeof(unsigned long long) * kBatchFamilies, ctx->stream));
     KIWI_CUDA(ctx, cudaMemsetAsync(b->d_stats, 0, sizeof(DevStats) * b->n_items, ctx->stream));
     for (int i = 0; i < b->n_items; ++i) KIWI_TRY(fp64_mean_velocity(ctx, b->items[i].P, b->d_meanv + 4 * i));
+    const bool merged = mixed && b->merge && b->fam_tiles[kBatchFamilyMixed] > 0 && b->fam_tiles[kBatchFamilyMixedGeneric] > 0;
+    const bool side = b->merge && (b->precision & KIWI_FORM_MASK) == KIWI_FP64 && families_present(b) > 1;
+    std::vector<cudaGraphNode_t> before, one, after;
+    if (side) KIWI_TRY(capture_front(ctx, &before));
     for (int f = 0; f < kBatchFamilies; ++f) {
-        if (b->merge && f == kBatchFamilyLatticeGeneric) continue;
-        const bool merged = b->merge && f == kBatchFamilyLattice;
-        const int64_t nwork = merged ? b->merged_tiles : b->fam_tiles[f];
-        if (nwork <= 0) continue;
+        if (b->fam_tiles[f] <= 0 || (merged && f == kBatchFamilyMixedGeneric)) continue;
         const int32_t* work = merged ? (b->lpt ? b->d_lpt_m : b->d_natural_m) : (b->lpt ? b->d_lpt[f] : b->d_natural[f]);
-        if (f == kBatchFamilyGather)
-            KIWI_TRY(fp64_batch_gather(ctx, b->d_items, b->d_item_of_tile, work, nwork, b->d_list, b->d_range,
-                                       b->d_next + f, b->sms * b->ctas_per_sm));
-        else
-            KIWI_TRY(lattice_batch_gather(ctx, merged ? kBatchFamilyLatticeMerged : f, b->d_items, b->d_item_of_tile, work,
-                                          nwork, b->d_list, b->d_range, b->d_sums, b->d_next + f,
-                                          b->sms * b->ctas_per_sm, mixed));
+        const int blocks = b->sms * b->ctas_per_sm;
+        if (f == kBatchFamilyGather) {
+            KIWI_TRY(fp64_batch_gather(ctx, b->d_items, b->d_item_of_tile, work, b->fam_tiles[f], b->d_list, b->d_range,
+                                       b->d_next + f, blocks));
+            continue;
+        }
+        if (side) KIWI_TRY(capture_after(ctx, before));
+        KIWI_TRY(lattice_batch_gather(ctx, merged ? kBatchFamilyMixedMerged : f, b->d_items, b->d_item_of_tile, work,
+                                      merged ? b->merged_tiles : b->fam_tiles[f], b->d_list, b->d_range, b->d_sums,
+                                      b->d_next + f, blocks, mixed));
+        if (side) {
+            KIWI_TRY(capture_front(ctx, &one));
+            after.insert(after.end(), one.begin(), one.end());
+        }
     }
+    if (side) KIWI_TRY(capture_after(ctx, after));
     return lattice_batch_combine(ctx, b->d_items, b->d_item_of_tile, b->d_cut, b->n_cut, b->d_sums);
 }
 
@@ -145,17 +178,17 @@ int batch_work(KiwiBatch* b) {
     KIWI_CUDA(ctx, cudaMemcpyAsync(range.data(), b->d_range, sizeof(int64_t) * range.size(), cudaMemcpyDeviceToHost,
                                    ctx->stream));
     KIWI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    const bool split = (b->precision & KIWI_FORM_MASK) == KIWI_FP64;
+    const bool split = (b->precision & KIWI_FORM_MASK) == KIWI_FP64, mixed = (b->precision & KIWI_FORM_MASK) == KIWI_FP32_MIXED;
     std::vector<int32_t> tiles[kBatchFamilies], both, slot((size_t)b->n_tiles, 0), cut, work;
     int64_t places = 0;
     for (int i = 0; i < b->n_items; ++i) {
-        const int f = batch_family(b->items[i].mode);
+        const int f = batch_family(b->items[i].mode, b->items[i].kernel, mixed);
         const int64_t nt = b->tile_base[i + 1] - b->tile_base[i];
         for (int64_t t = b->tile_base[i]; t < b->tile_base[i + 1]; ++t) {
             grid_tiles[(size_t)t] = nt;
             tiles[f].push_back((int32_t)t);
             if (f == kBatchFamilyGather) continue;
-            both.push_back((int32_t)t);
+            if (mixed) both.push_back((int32_t)t);
             const int64_t nseg = split ? lattice_batch_segments(range[2 * (size_t)t + 1] - range[2 * (size_t)t], nt) : 1;
             if (nseg <= 1) continue;
             slot[(size_t)t] = (int32_t)places;
@@ -366,6 +399,7 @@ int kiwi_batch_create(KiwiCtx* ctx, const KiwiBatchItem* items, int n_items, int
     b->ctx = ctx;
     b->n_items = n_items;
     b->precision = precision;
+    b->merge = form == KIWI_FP64;
     const int rc = batch_build(b, items);
     if (rc != KIWI_OK) {
         batch_free(b);
@@ -433,7 +467,7 @@ int kiwi_batch_tune(KiwiBatch* b, int* chosen) {
     float best = 1e30f;
     bool best_lpt = b->lpt, best_merge = b->merge;
     int best_ctas = b->ctas_per_sm;
-    const bool both = b->fam_tiles[kBatchFamilyLattice] > 0 && b->fam_tiles[kBatchFamilyLatticeGeneric] > 0;
+    const bool both = families_present(b) > 1 && b->fam_tiles[kBatchFamilyGather] == 0;
     for (int merge = both ? 1 : 0; merge >= 0; --merge) {
         for (int lpt = 1; lpt >= 0; --lpt) {
             for (int ctas = 1; ctas <= 2; ++ctas) {

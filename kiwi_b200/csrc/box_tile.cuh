@@ -74,9 +74,9 @@ static_assert(kBoxPairCap <= 1024 && kBoxPlaneCap <= 512, "packed edge entries")
 template <int NP, bool SEQ = false>
 struct BoxCaps {
     static constexpr int kN = NP ? NP : KIWI_BOX_PIECES;
-    static constexpr int kPt = SEQ ? 1536 : (NP ? kBoxPtCap : kBoxGenPtCap);
-    static constexpr int kPair = SEQ ? (NP ? 768 : 512) : (NP ? kBoxPairCap : kBoxGenPairCap);
-    static constexpr int kPlane = SEQ ? 208 : (NP ? kBoxPlaneCap : kBoxGenPlaneCap);
+    static constexpr int kPt = SEQ ? 1536 : (NP == 1 ? 3072 : (NP == 2 ? kBoxPtCap : kBoxGenPtCap));
+    static constexpr int kPair = SEQ ? (NP ? 768 : 512) : (NP == 1 ? 1024 : (NP == 2 ? kBoxPairCap : kBoxGenPairCap));
+    static constexpr int kPlane = SEQ ? 208 : (NP == 1 ? 448 : (NP == 2 ? kBoxPlaneCap : kBoxGenPlaneCap));
     static constexpr int kQueues = kN;  // edge kinds; the point phase uses the first
     // dynamic shared memory, in doubles: the cells' sums, the octant values, the edge and plane records
     static constexpr int kOffT = 4 * kTileCells;
@@ -160,7 +160,7 @@ __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& 
     using Caps = BoxCaps<NP, SEQ>;
     __shared__ BoxChunk s_cp[2];
     __shared__ double s_pl[3][kTileX + 1], s_cc[3][kTileX];
-    __shared__ double s_C[NP ? 1 : (kBoxC + 1) * KIWI_BOX_PIECES];  // any kernel: c and C of its pieces (lanes differ in piece)
+    __shared__ double s_C[NP == 2 ? 1 : (kBoxC + 1) * Caps::kN];  // any kernel: c and C of its pieces (lanes differ in piece)
     static_assert(kTileX == kTileY && kTileX == kTileZ, "cubic tiles");
     extern __shared__ double s_dyn[];
     const int n = NP ? NP : T.npiece;
@@ -183,7 +183,7 @@ __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& 
         s_pl[a][l] = add_rn(mn, mul_rn((double)(b0 + l), d));
         if (l < kTileX) s_cc[a][l] = cell_centre(mn, b0 + l, d);
     }
-    if (!NP)
+    if (NP != 2)
         for (int i = threadIdx.x; i < (kBoxC + 1) * n; i += kBoxThreads) {
             const int k = i / (kBoxC + 1), c = i % (kBoxC + 1);
             s_C[i] = c < kBoxC ? T.reg[k].C[c] : T.reg[k].c;

@@ -69,14 +69,14 @@ int cart_adjoint_dev(KiwiCtx* ctx, const DevParticles& P, const CartGeom& g, con
 // One grid of a batch (batch.cu): its geometry, particles and outputs, how its tiles are evaluated,
 // and where its tiles start in the batch's concatenated tile lists.
 enum BatchMode { kBatchLattice = 0, kBatchGatherCubic = 1, kBatchGatherGeneric = 2, kBatchLatticeGeneric = 3 };
-// tile-body families, one persistent launch each
-enum BatchFamily { kBatchFamilyLattice = 0, kBatchFamilyLatticeGeneric = 1, kBatchFamilyGather = 2, kBatchFamilies = 3 };
-// launch-only family: the tiles of both lattice families in one persistent launch, each tile taking its
-// item's body
-constexpr int kBatchFamilyLatticeMerged = 3;
-inline int batch_family(int mode) {
-    return mode == kBatchLattice ? kBatchFamilyLattice
-                                 : (mode == kBatchLatticeGeneric ? kBatchFamilyLatticeGeneric : kBatchFamilyGather);
+// families, one persistent launch each.  FP64 form: one per kernel of the tables (0 .. 5).  FP32-mixed form: the cubic
+// closed form (0) and the table-driven kernels (1).  Reference-order form: the per-cell gather.
+constexpr int kBatchFamilyMixed = 0, kBatchFamilyMixedGeneric = 1, kBatchFamilyGather = 6, kBatchFamilies = 7;
+// launch-only family (FP32-mixed form): both in one persistent launch, each tile taking its item's body
+constexpr int kBatchFamilyMixedMerged = 7;
+inline int batch_family(int mode, int kernel, bool mixed) {
+    if (mode == kBatchGatherCubic || mode == kBatchGatherGeneric) return kBatchFamilyGather;
+    return mixed ? (mode == kBatchLattice ? kBatchFamilyMixed : kBatchFamilyMixedGeneric) : kernel;
 }
 struct BatchItemDev {
     CartGeom g;
@@ -152,8 +152,8 @@ int lattice_batch_work(const std::vector<int32_t>& tiles, const std::vector<int6
 int64_t lattice_batch_segments(int64_t cnt, int64_t grid_tiles);
 // sums: raw sums of the cut tiles' segments, 4 x kTileCells doubles each; d_cut: the cut tiles' first items.
 int lattice_batch_gather(KiwiCtx* ctx, int family, const BatchItemDev* d_items, const int32_t* d_item_of_tile,
-                         const int32_t* d_work, int64_t nwork, const uint32_t* list, const int64_t* range, double* sums,
-                         unsigned long long* d_next, int blocks, bool mixed);
+                         const int32_t* d_work, int64_t nwork, const uint32_t* list,
+                         const int64_t* range, double* sums, unsigned long long* d_next, int blocks, bool mixed);
 int lattice_batch_combine(KiwiCtx* ctx, const BatchItemDev* d_items, const int32_t* d_item_of_tile, const int32_t* d_cut,
                           int64_t n, const double* sums);
 

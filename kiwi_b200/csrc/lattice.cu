@@ -51,8 +51,6 @@ constexpr size_t kLatMergedDynSmem = kLatDynSmem > kLatGenDynSmem ? kLatDynSmem 
 #define KIWI_BOX_MIN_BLOCKS 2
 #endif
 constexpr int kBoxMinBlocks = KIWI_BOX_MIN_BLOCKS;
-constexpr size_t kBoxSmem = BoxCaps<2>::kSmem, kBoxGenSmem = BoxCaps<0>::kSmem;
-constexpr size_t kBoxMergedSmem = kBoxSmem > kBoxGenSmem ? kBoxSmem : kBoxGenSmem;
 
 // One piece of work: segment `seg` of the `nseg` of tile `tile`; its sums go to the partial sums' place slot + seg if
 // nseg > 1.
@@ -74,15 +72,15 @@ __device__ __forceinline__ void box_item(const BoxItem& it, const CartGeom& g, c
                             it.nseg > 1 ? sums + (int64_t)(it.slot + it.seg) * 4 * kTileCells : nullptr, st, T);
 }
 
-// A kernel of pieces NP and powers DEG (0: any of the tables'), over items, or without them over the tiles
-// tile_map[0 ..) (every tile if null), each tile by one CTA: SEQ cuts it into its segments, else no list is longer
-// than one.
-template <bool CULL, int NP, int DEG, bool SEQ>
+// Kernel KERNEL of the tables (NP pieces, powers to DEG; KERNEL < 0: any, `kernel`, with both 0), over items, or
+// without them over the tiles tile_map[0 ..) (every tile if null), each tile by one CTA: SEQ cuts it into its
+// segments, else no list is longer than one.
+template <bool CULL, int KERNEL, int NP, int DEG, bool SEQ>
 __global__ void __launch_bounds__(kBoxThreads, kBoxMinBlocks)
     k_cart_box(CartGeom g, DevParticles P, int kernel, const uint32_t* __restrict__ list,
                const int64_t* __restrict__ range, const int32_t* __restrict__ tile_map, const BoxItem* __restrict__ items,
                CartOutputs out, double* __restrict__ sums, DevStats* __restrict__ st) {
-    const KiwiBoxTable& T = NP ? c_box[0] : c_box[kernel];
+    const KiwiBoxTable& T = c_box[KERNEL >= 0 ? KERNEL : kernel];
     if (SEQ) {
         const int64_t t = tile_map ? (int64_t)tile_map[blockIdx.x] : (int64_t)blockIdx.x;
         const int64_t lo = range[2 * t], hi = range[2 * t + 1];
@@ -186,16 +184,17 @@ __global__ void __launch_bounds__(kLatThreads, kLatGenMinBlocks)
     lattice_tile<true, true, false, true>(g, P, list, range, t, t, out, st, &c_tables[kernel]);
 }
 
-// The work of a batch of grids, one persistent launch per lattice family, or one for both
-// (kBatchFamilyLatticeMerged: each item takes its grid's body): each CTA takes the next of the launch's
-// work items from the work counter and runs the same body as the single-grid kernel, so every
-// cell's summation order is that of a single-grid call.  MIXED: the FP32-mixed tile bodies (items are whole tiles).
-template <int FAMILY, bool MIXED>
-__global__ void __launch_bounds__(MIXED ? kLatThreads : kBoxThreads, 2)
-    k_batch_lattice(const BatchItemDev* __restrict__ items, const int32_t* __restrict__ item_of_tile,
-                    const BoxItem* __restrict__ work, int64_t nwork, const uint32_t* __restrict__ list,
-                    const int64_t* __restrict__ range, double* __restrict__ sums, unsigned long long* __restrict__ next) {
+// The work of a batch's grids with one kernel (FP64 form), or one lattice family's (FP32-mixed form: whole tiles), in
+// one persistent launch: each CTA takes the next of the launch's work items from the work counter and runs the
+// same body as the single-grid kernel, so every cell's summation order is that of a single-grid call.
+template <int KERNEL, int NP, int DEG>
+__global__ void __launch_bounds__(kBoxThreads, 2)
+    k_batch_box(const BatchItemDev* __restrict__ items, const int32_t* __restrict__ item_of_tile,
+                const BoxItem* __restrict__ work, int64_t nwork, const uint32_t* __restrict__ list,
+                const int64_t* __restrict__ range, double* __restrict__ sums, unsigned long long* __restrict__ next) {
     __shared__ long long s_w;
+    __shared__ BatchItemDev s_it;  // (in shared memory: the body's registers are full)
+    static_assert(sizeof(BatchItemDev) % 8 == 0 && sizeof(BatchItemDev) / 8 <= kBoxThreads, "copied by one step");
     for (;;) {
         if (threadIdx.x == 0) s_w = (long long)atomicAdd(next, 1ull);
         __syncthreads();
@@ -203,16 +202,33 @@ __global__ void __launch_bounds__(MIXED ? kLatThreads : kBoxThreads, 2)
         if (w >= nwork) break;
         const BoxItem wi = work[w];
         const int64_t tg = wi.tile;
+        const int64_t* const src = reinterpret_cast<const int64_t*>(items + item_of_tile[tg]);
+        if (threadIdx.x < sizeof(BatchItemDev) / 8) reinterpret_cast<int64_t*>(&s_it)[threadIdx.x] = src[threadIdx.x];
+        __syncthreads();
+        box_item<true, NP, DEG>(wi, s_it.g, s_it.P, list, range + 2 * tg, tg - s_it.tile_base, s_it.out, sums, s_it.st,
+                                c_box[KERNEL]);
+        __syncthreads();
+    }
+}
+
+template <int FAMILY>
+__global__ void __launch_bounds__(kLatThreads, 2)
+    k_batch_mixed(const BatchItemDev* __restrict__ items, const int32_t* __restrict__ item_of_tile,
+                  const BoxItem* __restrict__ work, int64_t nwork, const uint32_t* __restrict__ list,
+                  const int64_t* __restrict__ range, unsigned long long* __restrict__ next) {
+    __shared__ long long s_w;
+    for (;;) {
+        if (threadIdx.x == 0) s_w = (long long)atomicAdd(next, 1ull);
+        __syncthreads();
+        const int64_t w = s_w;
+        if (w >= nwork) break;
+        const int64_t tg = work[w].tile;
         const BatchItemDev& it = items[item_of_tile[tg]];
         const int64_t tl = tg - it.tile_base;
-        const bool cubic = FAMILY == kBatchFamilyLattice || (FAMILY == kBatchFamilyLatticeMerged && it.mode == kBatchLattice);
-        if (MIXED) {
-            if (cubic) lattice_tile<true, false, false, true>(it.g, it.P, list, range, tg, tl, it.out, it.st);
-            else lattice_tile<true, true, false, true>(it.g, it.P, list, range, tg, tl, it.out, it.st, &c_tables[it.kernel]);
-        } else {
-            if (cubic) box_item<true, 2, 3>(wi, it.g, it.P, list, range + 2 * tg, tl, it.out, sums, it.st, c_box[0]);
-            else box_item<true, 0, 0>(wi, it.g, it.P, list, range + 2 * tg, tl, it.out, sums, it.st, c_box[it.kernel]);
-        }
+        if (FAMILY == kBatchFamilyMixed || (FAMILY == kBatchFamilyMixedMerged && it.mode == kBatchLattice))
+            lattice_tile<true, false, false, true>(it.g, it.P, list, range, tg, tl, it.out, it.st);
+        else
+            lattice_tile<true, true, false, true>(it.g, it.P, list, range, tg, tl, it.out, it.st, &c_tables[it.kernel]);
         __syncthreads();
     }
 }
@@ -225,24 +241,21 @@ __global__ void __launch_bounds__(256) k_batch_combine(const BatchItemDev* __res
     box_combine(it.g, it.out, wi.tile - it.tile_base, sums + (int64_t)wi.slot * 4 * kTileCells, wi.nseg);
 }
 
-// The shared memory and block size of a batch launch.
-template <int FAMILY, bool MIXED>
-constexpr size_t batch_smem() {
-    if (MIXED)
-        return FAMILY == kBatchFamilyLattice ? kLatDynSmem
-                                             : (FAMILY == kBatchFamilyLatticeMerged ? kLatMergedDynSmem : kLatGenDynSmem);
-    return FAMILY == kBatchFamilyLattice ? kBoxSmem : (FAMILY == kBatchFamilyLatticeMerged ? kBoxMergedSmem : kBoxGenSmem);
+template <int FAMILY>
+constexpr size_t mixed_smem() {
+    return FAMILY == kBatchFamilyMixed ? kLatDynSmem
+                                       : (FAMILY == kBatchFamilyMixedMerged ? kLatMergedDynSmem : kLatGenDynSmem);
 }
 
 }  // namespace
 
-template <bool CULL, int NP, int DEG, bool SEQ>
+template <bool CULL, int KERNEL, int NP, int DEG, bool SEQ>
 static int box_launch(KiwiCtx* ctx, int64_t blocks, const CartGeom& g, const DevParticles& P, int kernel,
                       const TileLists& tl, const BoxItem* items, const CartOutputs& out, double* sums, DevStats* st) {
     constexpr size_t smem = BoxCaps<NP, SEQ>::kSmem;
-    KIWI_CUDA(ctx, cudaFuncSetAttribute(k_cart_box<CULL, NP, DEG, SEQ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    KIWI_CUDA(ctx, cudaFuncSetAttribute(k_cart_box<CULL, KERNEL, NP, DEG, SEQ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)smem));
-    k_cart_box<CULL, NP, DEG, SEQ><<<(unsigned)blocks, kBoxThreads, smem, ctx->stream>>>(g, P, kernel, tl.list, tl.range,
+    k_cart_box<CULL, KERNEL, NP, DEG, SEQ><<<(unsigned)blocks, kBoxThreads, smem, ctx->stream>>>(g, P, kernel, tl.list, tl.range,
                                                                                       tl.map, items, out, sums, st);
     KIWI_LAUNCHED(ctx);
     return KIWI_OK;
@@ -252,9 +265,17 @@ template <bool SEQ>
 static int box_launch_kernel(KiwiCtx* ctx, int64_t blocks, const CartGeom& g, const DevParticles& P, const KernelChoice& k,
                              const TileLists& tl, const BoxItem* items, const CartOutputs& out, double* sums,
                              DevStats* st, bool full_box) {
-    if (!k.cubic) return box_launch<true, 0, 0, SEQ>(ctx, blocks, g, P, k.kernel, tl, items, out, sums, st);
-    if (full_box) return box_launch<false, 2, 3, SEQ>(ctx, blocks, g, P, 0, tl, items, out, sums, st);
-    return box_launch<true, 2, 3, SEQ>(ctx, blocks, g, P, 0, tl, items, out, sums, st);
+    if (k.kernel == 0 && full_box) return box_launch<false, 0, 2, 3, SEQ>(ctx, blocks, g, P, 0, tl, items, out, sums, st);
+    if (k.kernel == 0) return box_launch<true, 0, 2, 3, SEQ>(ctx, blocks, g, P, 0, tl, items, out, sums, st);
+    if constexpr (SEQ) {  // one CTA per tile (the allocation-free call): one body for the other kernels
+        return box_launch<true, -1, 0, 0, SEQ>(ctx, blocks, g, P, k.kernel, tl, items, out, sums, st);
+    } else {
+#define KIWI_BOX_LAUNCH(K, NP, DEG) \
+    if (k.kernel == K) return box_launch<true, K, NP, DEG, false>(ctx, blocks, g, P, K, tl, items, out, sums, st);
+        KIWI_BOX_OTHERS(KIWI_BOX_LAUNCH)
+#undef KIWI_BOX_LAUNCH
+        return set_err(ctx, KIWI_ERR_ARG, "unknown kernel %d", k.kernel);
+    }
 }
 
 int lattice_cart_gather(KiwiCtx* ctx, const CartGeom& g, const DevParticles& P, const KernelChoice& k,
@@ -347,55 +368,50 @@ int lattice_mixed_gather(KiwiCtx* ctx, const CartGeom& g, const DevParticles& P,
     return KIWI_OK;
 }
 
-template <int FAMILY, bool MIXED>
-static int batch_prepare_t(KiwiCtx* ctx) {
-    KIWI_CUDA(ctx, cudaFuncSetAttribute(k_batch_lattice<FAMILY, MIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)batch_smem<FAMILY, MIXED>()));
+template <class F>
+static int batch_attr(KiwiCtx* ctx, F* f, size_t smem) {
+    KIWI_CUDA(ctx, cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     return KIWI_OK;
 }
 
-template <bool MIXED>
-static int batch_prepare_form(KiwiCtx* ctx) {
-    KIWI_TRY((batch_prepare_t<kBatchFamilyLattice, MIXED>(ctx)));
-    KIWI_TRY((batch_prepare_t<kBatchFamilyLatticeGeneric, MIXED>(ctx)));
-    return batch_prepare_t<kBatchFamilyLatticeMerged, MIXED>(ctx);
-}
-
 int lattice_batch_prepare(KiwiCtx* ctx) {
-    KIWI_TRY(batch_prepare_form<false>(ctx));
-    return batch_prepare_form<true>(ctx);
+#define KIWI_BOX_ATTR(K, NP, DEG) KIWI_TRY(batch_attr(ctx, k_batch_box<K, NP, DEG>, BoxCaps<NP>::kSmem));
+    KIWI_BOX_KERNELS(KIWI_BOX_ATTR)
+#undef KIWI_BOX_ATTR
+    KIWI_TRY(batch_attr(ctx, k_batch_mixed<kBatchFamilyMixed>, mixed_smem<kBatchFamilyMixed>()));
+    KIWI_TRY(batch_attr(ctx, k_batch_mixed<kBatchFamilyMixedGeneric>, mixed_smem<kBatchFamilyMixedGeneric>()));
+    return batch_attr(ctx, k_batch_mixed<kBatchFamilyMixedMerged>, mixed_smem<kBatchFamilyMixedMerged>());
 }
 
-template <int FAMILY, bool MIXED>
-static void batch_launch_t(KiwiCtx* ctx, const BatchItemDev* d_items, const int32_t* d_item_of_tile, const BoxItem* work,
-                           int64_t nwork, const uint32_t* list, const int64_t* range, double* sums,
-                           unsigned long long* d_next, int blocks) {
-    k_batch_lattice<FAMILY, MIXED><<<blocks, MIXED ? kLatThreads : kBoxThreads, batch_smem<FAMILY, MIXED>(), ctx->stream>>>(
-        d_items, d_item_of_tile, work, nwork, list, range, sums, d_next);
-}
-
-template <bool MIXED>
-static void batch_launch_form(KiwiCtx* ctx, int family, const BatchItemDev* d_items, const int32_t* d_item_of_tile,
-                              const BoxItem* work, int64_t nwork, const uint32_t* list, const int64_t* range,
-                              double* sums, unsigned long long* d_next, int blocks) {
-    if (family == kBatchFamilyLattice)
-        batch_launch_t<kBatchFamilyLattice, MIXED>(ctx, d_items, d_item_of_tile, work, nwork, list, range, sums, d_next, blocks);
-    else if (family == kBatchFamilyLatticeMerged)
-        batch_launch_t<kBatchFamilyLatticeMerged, MIXED>(ctx, d_items, d_item_of_tile, work, nwork, list, range, sums,
-                                                         d_next, blocks);
-    else
-        batch_launch_t<kBatchFamilyLatticeGeneric, MIXED>(ctx, d_items, d_item_of_tile, work, nwork, list, range, sums,
-                                                          d_next, blocks);
+template <int FAMILY>
+static void batch_launch_mixed(cudaStream_t stream, const BatchItemDev* d_items, const int32_t* d_item_of_tile,
+                               const BoxItem* work, int64_t nwork, const uint32_t* list, const int64_t* range,
+                               unsigned long long* d_next, int blocks) {
+    k_batch_mixed<FAMILY><<<blocks, kLatThreads, mixed_smem<FAMILY>(), stream>>>(d_items, d_item_of_tile, work, nwork, list,
+                                                                              range, d_next);
 }
 
 int lattice_batch_gather(KiwiCtx* ctx, int family, const BatchItemDev* d_items, const int32_t* d_item_of_tile,
-                         const int32_t* d_work, int64_t nwork, const uint32_t* list, const int64_t* range, double* sums,
-                         unsigned long long* d_next, int blocks, bool mixed) {
+                         const int32_t* d_work, int64_t nwork, const uint32_t* list,
+                         const int64_t* range, double* sums, unsigned long long* d_next, int blocks, bool mixed) {
     const BoxItem* work = reinterpret_cast<const BoxItem*>(d_work);
-    if (mixed)
-        batch_launch_form<true>(ctx, family, d_items, d_item_of_tile, work, nwork, list, range, sums, d_next, blocks);
-    else
-        batch_launch_form<false>(ctx, family, d_items, d_item_of_tile, work, nwork, list, range, sums, d_next, blocks);
+    const cudaStream_t stream = ctx->stream;
+    if (mixed) {
+        if (family == kBatchFamilyMixed)
+            batch_launch_mixed<kBatchFamilyMixed>(stream, d_items, d_item_of_tile, work, nwork, list, range, d_next, blocks);
+        else if (family == kBatchFamilyMixedMerged)
+            batch_launch_mixed<kBatchFamilyMixedMerged>(stream, d_items, d_item_of_tile, work, nwork, list, range, d_next,
+                                                        blocks);
+        else
+            batch_launch_mixed<kBatchFamilyMixedGeneric>(stream, d_items, d_item_of_tile, work, nwork, list, range, d_next,
+                                                         blocks);
+    }
+#define KIWI_BOX_BATCH(K, NP, DEG)                                                                                  \
+    else if (family == K)                                                                                           \
+        k_batch_box<K, NP, DEG><<<blocks, kBoxThreads, BoxCaps<NP>::kSmem, stream>>>(d_items, d_item_of_tile, work, nwork, \
+                                                                                  list, range, sums, d_next);
+    KIWI_BOX_KERNELS(KIWI_BOX_BATCH)
+#undef KIWI_BOX_BATCH
     KIWI_LAUNCHED(ctx);
     return KIWI_OK;
 }
