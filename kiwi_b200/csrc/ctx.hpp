@@ -172,6 +172,8 @@ enum ScratchSlot {
     S_VOR_FVAL,      // Voronoi map: per (pair, face), the face's integral
     S_VOR_LINKS,     // Voronoi map: per face, its earlier twin in the cell and the neighbour's face back
     S_VOR_STAGE,     // Voronoi walk: the single walk's staging area
+    S_VOR_OWNER,     // Voronoi map: each pair's particle
+    S_VOR_PLANES,    // Voronoi map: the faces' planes
     S_BOX_COUNTS,    // box-mass gather: item counters and weight classes
     S_BOX_ITEMS,     // box-mass gather: work items
     S_BOX_CUT,       // box-mass gather: the cut tiles

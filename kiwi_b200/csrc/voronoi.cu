@@ -8,7 +8,7 @@
 //      visited cells, then it writes them (in walk order) at the particle's offset with, per visited
 //      cell, which of its faces lead to a cell the walk processed earlier.
 //  (2) a stable radix sort of the pairs by cell index: every cell's particles stay in ascending order.
-//  (3) k_vor_gather, one CTA per cell: the cell's faces are staged in shared memory, each thread takes
+//  (3) k_vor_faces and k_vor_sum (or k_vor_gather, both in one launch): the cell's faces are staged in shared memory, each thread takes
 //      one particle of the cell's list and evaluates compute_cell_integral (src/mapping.cpp:105-206): the
 //      sum over the cell's faces of the face walk, clamped at 0; the values are then added in particle
 //      order -- the reference's single-threaded summation order, no atomics -- and finalised as
@@ -21,21 +21,22 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 
 #include "../../include/kiwi_b200.h"
 #include "engine.hpp"
+#include "cone_math.cuh"
 #include "kiwi_math.cuh"
-#include "lattice.cuh"
 #include "prims.cuh"
 #include "tabulated.cuh"
 
 namespace kiwi_b200 {
 
 // kernel tables of this translation unit (constant memory is per translation unit)
-__constant__ KiwiKernelTable c_vor_tables[KIWI_NUM_KERNELS];
+__constant__ KiwiConeTable c_cones[6];
 
 int voronoi_init_tables(KiwiCtx* ctx) {
-    KIWI_CUDA(ctx, cudaMemcpyToSymbol(c_vor_tables, kiwi_kernel_tables, sizeof(kiwi_kernel_tables)));
+    KIWI_CUDA(ctx, cudaMemcpyToSymbol(c_cones, kiwi_cone_tables, sizeof(kiwi_cone_tables)));
     return KIWI_OK;
 }
 
@@ -53,6 +54,7 @@ struct VorCells {
     // is no cell)
     const int32_t* twin;
     const int64_t* back;
+    const double4* plane;  // per face: unit normal and offset (k_face_planes); zero for a face of under 3 vertices
 };
 
 // The face links of every cell (one thread per cell): what the walk and the gathers would otherwise look
@@ -84,13 +86,33 @@ __global__ void k_face_links(int64_t n_cells, const int64_t* __restrict__ face_o
     }
 }
 
+// Each face's plane from its first three vertices, as the reference takes it.
+__global__ void k_face_planes(int64_t n_faces, const int64_t* __restrict__ vert_off, const double* __restrict__ vxyz,
+                              double4* __restrict__ plane) {
+    const int64_t f = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (f >= n_faces) return;
+    const int64_t v = vert_off[f];
+    double4 r{0.0, 0.0, 0.0, 0.0};
+    if (vert_off[f + 1] - v >= 3) {
+        const double* q = vxyz + 3 * v;
+        const FacePlane g = face_plane(q);
+        r = double4{g.x, g.y, g.z, g.w};
+    }
+    plane[f] = r;
+}
+
 constexpr int kBfsWarpsPerBlock = 4;
+// The walk's visited cells in shared memory: an open-addressing table (cell -> queue position) and the queue, for
+// walks of up to kWalkCap cells (a particle visits about 120); a longer walk runs again in the slot's
+// global arrays.
+constexpr int kWalkBits = 10, kWalkSlots = 1 << kWalkBits, kWalkCap = 640;
+constexpr int kWalkClaim = 1 << 24;  // position values from here on: candidates' claims
 constexpr int kBfsCandCap = 512;  // a batch's discovery candidates listed per warp (larger batches: lane 0)
 constexpr int kGatherThreads = 128;
-constexpr int kGatherVertCap = 1536;  // vertices staged in shared memory per cell (36 KB)
+constexpr int kGatherVertCap = 1024;  // vertices staged in shared memory per cell (24 KB; a cell has about 80)
 // k_vor_faces: a face item packs (pair slot << 7 | face), for cells of at most 128 faces
 constexpr int kFaceItemMaxFaces = 128;
-constexpr int kFaceItemCap = 2048;  // 4 KB of items beside the 36 KB of staged vertices
+constexpr int kFaceItemCap = 2048;  // 4 KB of items beside the 24 KB of staged vertices
 // k_vor_faces: CTAs per SM the register allocation leaves room for (4: 128 registers a thread, a few
 // spilled; 8 % faster than 3 CTAs at 166 registers)
 #ifndef KIWI_VOR_FACES_MIN_BLOCKS
@@ -123,7 +145,8 @@ struct VorStage {
 // in order, and each unvisited neighbour whose face the kernel reaches is appended.  The lanes process 32
 // queued cells at a time and the appends are made in (cell, face) order, so the queue is the reference's
 // sequential queue.  A face whose neighbour already appeared on an earlier face of the same cell is a
-// face-cache hit in the reference and discovers nothing.  mark[cell] = (marker << 32) | queue position.
+// face-cache hit in the reference and discovers nothing.  The visited cells' queue positions stand in a shared table
+// (mark[cell] = (marker << 32) | queue position in the slot's global arrays for a walk that outgrows it).
 // Cells of more than 128 faces are refused (KIWI_ERR_LIMIT).
 // Pass 1 also records per (particle, cell) the faces whose neighbour the walk processed earlier (bit i:
 // face i of the cell, first 64 faces): the reference reuses that neighbour's cached, negated face value.
@@ -134,7 +157,325 @@ struct VorStage {
 // first face towards this cell, the neighbour being the particle's q-th visited cell; -2 - e it takes the
 // value of this cell's earlier face e towards the same neighbour -- the reference's face cache
 // (src/mapping.cpp:56-93), decided here once so that the map evaluates each face value once.
-__global__ void __launch_bounds__(32 * kBfsWarpsPerBlock) k_vor_bfs(VorCells C, DevParticles P,
+struct WalkShared {
+    int32_t cand[kBfsWarpsPerBlock][kBfsCandCap];
+    unsigned long long reach[kBfsWarpsPerBlock][32][2];
+    int32_t key[kBfsWarpsPerBlock][kWalkSlots], pos[kBfsWarpsPerBlock][kWalkSlots], queue[kBfsWarpsPerBlock][kWalkCap];
+};
+
+// A walk's visited cells: the shared table, or the slot's global arrays.
+template <bool SHARED>
+struct WalkCells {
+    int32_t *key, *pos, *queue;
+    long long* mark;
+    long long mk;
+    __device__ __forceinline__ static uint32_t slot_of(int32_t cell) {
+        return ((uint32_t)cell * 2654435761u) >> (32 - kWalkBits);
+    }
+    // the queue position of a cell, or -1
+    __device__ __forceinline__ int at(int32_t cell) const {
+        if (SHARED) {
+            for (uint32_t i = slot_of(cell);; i = (i + 1) & (kWalkSlots - 1)) {  // (never full: kWalkCap < kWalkSlots)
+                const int32_t k = key[i];
+                if (k == cell) return pos[i];
+                if (k < 0) return -1;
+            }
+        }
+        const long long mv = mark[cell];
+        return (mv >> 32) == mk ? (int)(mv & 0xffffffffLL) : -1;
+    }
+    // shared: the cell's place in the table, made if there is none
+    __device__ __forceinline__ uint32_t place(int32_t cell) {
+        for (uint32_t i = slot_of(cell);; i = (i + 1) & (kWalkSlots - 1)) {
+            const int32_t k = atomicCAS(&key[i], -1, cell);
+            if (k < 0 || k == cell) return i;
+        }
+    }
+};
+
+// One particle's walk (k_vor_bfs); returns its visited cells, or -1 if they outgrow the shared table.
+template <bool SHARED>
+__device__ __forceinline__ int vor_walk(const VorCells& C, WalkShared& sh, int warp, int lane, double x0, double y0,
+                                        double z0, double radius, int32_t k0, int pass, int64_t o, int64_t fcarry,
+                                        WalkCells<SHARED>& W, int32_t* __restrict__ pair_cells,
+                                        unsigned long long* __restrict__ pair_mask, int64_t* __restrict__ pair_foff,
+                                        int32_t* __restrict__ fsrc, int64_t& nface, unsigned long long& n_limit) {
+    nface = 0;  // this lane's share of the visited cells' faces
+    if (SHARED) {
+        for (int i = lane; i < kWalkSlots; i += 32) {
+            W.key[i] = -1;
+            W.pos[i] = INT_MAX;
+        }
+        __syncwarp();
+    }
+    if (lane == 0) {
+        W.queue[0] = k0;
+        if (SHARED) W.pos[W.place(k0)] = 0;
+        else W.mark[k0] = W.mk << 32;
+    }
+    __syncwarp();
+    auto reachable = [&](int64_t f) {
+        const int64_t v = C.vert_off[f];
+        const int nv = (int)(C.vert_off[f + 1] - v);
+        const int fast = nv < 3 ? 1 : face_reach_fast(x0, y0, z0, radius, C.plane[f], C.vxyz + 3 * v, nv);
+        if (fast >= 0) return fast != 0;
+        const FlatVerts V{C.vxyz + 3 * v};
+        return face_reachable(x0, y0, z0, radius, V, nv);
+    };
+    int head = 0, tail = 1;
+    while (head < tail) {
+        if (head > C.n_cells) {  // cannot happen: each cell enters the queue once
+            n_limit += (lane == 0);
+            break;
+        }
+        // The lanes take the next (up to) 32 queued cells, one each, and mark the faces to test: faces
+        // towards a neighbour not yet in the queue, skipping a face whose neighbour an earlier face of
+        // the same cell already named (a face-cache hit in the reference, which discovers nothing).  The
+        // warp tests them (the kernel reaches the face or not); the reachable ones are the discovery
+        // candidates, appended in (cell, face) order, skipping neighbours queued meanwhile: the
+        // reference's sequential queue.
+        const int batch = min(32, tail - head);
+        int64_t fa = 0, nf = 0;
+        unsigned long long cand0 = 0, cand1 = 0, earlier = 0, test0 = 0, test1 = 0;
+        if (lane < batch) {
+            const int rank = head + lane;
+            const int32_t cell = W.queue[rank];
+            fa = C.face_off[cell];
+            const int64_t fz = C.face_off[cell + 1];
+            nf = fz - fa;
+            nface += nf;
+            if (fz - fa > 128) n_limit += 1;  // a cell of more than 128 faces is not supported
+            for (int64_t f = fa; f < fz && f - fa < 128; ++f) {
+                const int32_t nb = C.face_nbr[f];
+                if (nb < 0 || nb >= C.n_cells) continue;
+                const int at = W.at(nb);
+                if (at >= 0) {
+                    if (at < rank && f - fa < 64) earlier |= 1ull << (f - fa);
+                    continue;
+                }
+                if (C.twin[f] >= 0) continue;  // an earlier face of this cell named nb already
+                if (f - fa < 64) test0 |= 1ull << (f - fa);
+                else test1 |= 1ull << (f - fa - 64);
+            }
+            if (pass == 1) {
+                pair_cells[o + rank] = cell;
+                pair_mask[o + rank] = earlier;
+            }
+        }
+        {
+            // The faces left to test (neighbour not queued, not a twin) as one list over the warp, in
+            // (cell, face) order, each lane testing every 32nd: a lane's own cell would leave the others
+            // idle through its faces, and the early batches hold one cell or a few.  A batch of more
+            // tests than the list holds is tested lane by lane.
+            const int nt_l = __popcll(test0) + __popcll(test1);
+            int t_incl = nt_l;
+            for (int d = 1; d < 32; d <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, t_incl, d);
+                if (lane >= d) t_incl += v;
+            }
+            const int n_test = __shfl_sync(0xffffffffu, t_incl, 31);
+            if (n_test <= kBfsCandCap) {
+                int32_t* items = sh.cand[warp];
+                int o_t = t_incl - nt_l;
+                for (int w = 0; w < 2; ++w) {
+                    unsigned long long bits = w == 0 ? test0 : test1;
+                    while (bits) {
+                        const int b = __ffsll((long long)bits) - 1;
+                        bits &= bits - 1;
+                        items[o_t++] = lane << 7 | (64 * w + b);
+                    }
+                }
+                sh.reach[warp][lane][0] = 0;
+                sh.reach[warp][lane][1] = 0;
+                __syncwarp();
+                for (int base = 0; base < n_test; base += 32) {
+                    const int i = base + lane;
+                    const int item = i < n_test ? items[i] : 0;
+                    const int src = item >> 7, fl = item & 127;
+                    const int64_t f = __shfl_sync(0xffffffffu, fa, src) + fl;
+                    if (i < n_test && reachable(f)) atomicOr(&sh.reach[warp][src][fl >> 6], 1ull << (fl & 63));
+                }
+                __syncwarp();
+                cand0 = sh.reach[warp][lane][0];
+                cand1 = sh.reach[warp][lane][1];
+                __syncwarp();
+            } else {
+                for (int w = 0; w < 2; ++w) {
+                    unsigned long long bits = w == 0 ? test0 : test1;
+                    while (bits) {
+                        const int b = __ffsll((long long)bits) - 1;
+                        bits &= bits - 1;
+                        if (reachable(fa + 64 * w + b)) {
+                            if (w == 0) cand0 |= 1ull << b;
+                            else cand1 |= 1ull << b;
+                        }
+                    }
+                }
+            }
+        }
+        if (pass == 1 && fsrc) {
+            // the cells' places in the face tables (a warp prefix sum in walk order) and each face's source
+            int64_t incl = nf;
+            for (int d = 1; d < 32; d <<= 1) {
+                const int64_t v = __shfl_up_sync(0xffffffffu, incl, d);
+                if (lane >= d) incl += v;
+            }
+            if (lane < batch) {
+                const int rank = head + lane;
+                const int64_t pf = fcarry + incl - nf;
+                pair_foff[o + rank] = pf;
+                for (int64_t f = fa; f < fa + nf; ++f) {
+                    const int32_t nb = C.face_nbr[f];
+                    int32_t code = -1;
+                    if (nb >= 0 && nb < C.n_cells) {
+                        const int at = W.at(nb);
+                        if (at >= 0 && at < rank && C.back[f] >= 0) code = at;
+                        if (code < 0 && C.twin[f] >= 0) code = -2 - C.twin[f];
+                    }
+                    fsrc[pf + (f - fa)] = code;
+                }
+            }
+            fcarry += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        int t = tail;
+        // the batch's candidates in (cell, face) order; each is queued if no earlier candidate names the
+        // same cell and it is not queued yet -- the sequential appends' queue, with every lane at work
+        const int nc_l = __popcll(cand0) + __popcll(cand1);
+        int c_incl = nc_l;
+        for (int d = 1; d < 32; d <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, c_incl, d);
+            if (lane >= d) c_incl += v;
+        }
+        const int n_cand = __shfl_sync(0xffffffffu, c_incl, 31);
+        if (SHARED && (n_cand > kBfsCandCap || tail + n_cand > kWalkCap)) return -1;
+        if (n_cand <= kBfsCandCap) {
+            int32_t* cl = sh.cand[warp];
+            int at = c_incl - nc_l;
+            for (int w = 0; w < 2; ++w) {
+                unsigned long long bits = w == 0 ? cand0 : cand1;
+                while (bits) {
+                    const int b = __ffsll((long long)bits) - 1;
+                    bits &= bits - 1;
+                    cl[at++] = C.face_nbr[fa + 64 * w + b];
+                }
+            }
+            __syncwarp();
+            if (SHARED) {
+                // the first candidate to name a cell claims it (none is queued: a queued cell is not tested)
+                for (int i = lane; i < n_cand; i += 32) atomicMin(&W.pos[W.place(cl[i])], kWalkClaim + i);
+                __syncwarp();
+            }
+            for (int base = 0; base < n_cand; base += 32) {
+                const int i = base + lane;
+                int32_t nb = -1;
+                bool keep = false;
+                if (i < n_cand) {
+                    nb = cl[i];
+                    if (SHARED) {
+                        keep = W.at(nb) == kWalkClaim + i;
+                    } else {
+                        keep = W.at(nb) < 0;
+                        for (int j = 0; keep && j < i; ++j) keep = cl[j] != nb;
+                    }
+                }
+                const unsigned kb = __ballot_sync(0xffffffffu, keep);
+                if (keep) {
+                    const int pos = t + __popc(kb & ((1u << lane) - 1));
+                    if (SHARED) W.pos[W.place(nb)] = pos;
+                    else W.mark[nb] = (W.mk << 32) | (long long)pos;
+                    W.queue[pos] = nb;
+                }
+                t += __popc(kb);
+                __syncwarp();
+            }
+        } else {
+            for (int L = 0; L < batch; ++L) {
+                unsigned long long c0 = __shfl_sync(0xffffffffu, cand0, L);
+                unsigned long long c1 = __shfl_sync(0xffffffffu, cand1, L);
+                const int64_t fl = __shfl_sync(0xffffffffu, fa, L);
+                if (lane == 0) {
+                    for (int w = 0; w < 2; ++w) {
+                        unsigned long long bits = w == 0 ? c0 : c1;
+                        while (bits) {
+                            const int b = __ffsll((long long)bits) - 1;
+                            bits &= bits - 1;
+                            const int32_t nb = C.face_nbr[fl + 64 * w + b];
+                            if (W.at(nb) < 0) {
+                                W.mark[nb] = (W.mk << 32) | (long long)t;
+                                W.queue[t++] = nb;
+                            }
+                        }
+                    }
+                }
+            }
+        }
+        tail = __shfl_sync(0xffffffffu, t, 0);
+        head += batch;
+        __syncwarp();
+    }
+    return tail;
+}
+
+// The single walk (pass 2): reserves the particle's pairs and faces in the staging area and writes them.  The table
+// holds every visited cell's queue position, so each face's source is decided as pass 1 decides it during its
+// walk (a neighbour processed earlier is one with a smaller queue position).
+template <bool SHARED>
+__device__ __forceinline__ void vor_stage(const VorCells& C, const WalkCells<SHARED>& W, int lane, int64_t p, int tail,
+                                          int64_t nface, const VorStage& stg) {
+    unsigned long long s0 = 0, fs0 = 0;
+    if (lane == 0) {
+        s0 = atomicAdd(&stg.ctr[0], (unsigned long long)tail);
+        fs0 = atomicAdd(&stg.ctr[1], (unsigned long long)nface);
+    }
+    s0 = __shfl_sync(0xffffffffu, s0, 0);
+    fs0 = __shfl_sync(0xffffffffu, fs0, 0);
+    if (s0 + tail > (unsigned long long)stg.cap_pairs || fs0 + nface > (unsigned long long)stg.cap_faces) {
+        if (lane == 0) atomicOr(&stg.ctr[2], 1ull);
+        return;
+    }
+    if (lane == 0) {
+        stg.start[p] = (int64_t)s0;
+        stg.fstart[p] = (int64_t)fs0;
+    }
+    int64_t fc = 0;
+    for (int base = 0; base < tail; base += 32) {
+        const int r = base + lane;
+        int32_t cell = 0;
+        int64_t fa = 0, nf = 0;
+        if (r < tail) {
+            cell = W.queue[r];
+            fa = C.face_off[cell];
+            nf = C.face_off[cell + 1] - fa;
+        }
+        int64_t incl = nf;
+        for (int d = 1; d < 32; d <<= 1) {
+            const int64_t v = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= d) incl += v;
+        }
+        if (r < tail) {
+            const int64_t fl = fc + incl - nf;
+            unsigned long long earlier = 0;
+            for (int64_t f = fa; f < fa + nf; ++f) {
+                const int32_t nb = C.face_nbr[f];
+                int32_t code = -1;
+                if (nb >= 0 && nb < C.n_cells) {
+                    const int at = W.at(nb);
+                    const bool before = at >= 0 && at < r;
+                    if (before && f - fa < 64) earlier |= 1ull << (f - fa);
+                    if (before && C.back[f] >= 0) code = at;
+                    if (code < 0 && C.twin[f] >= 0) code = -2 - C.twin[f];
+                }
+                stg.fsrc[fs0 + fl + (f - fa)] = code;
+            }
+            stg.cells[s0 + r] = cell;
+            stg.mask[s0 + r] = earlier;
+            stg.floc[s0 + r] = fl;
+        }
+        fc += __shfl_sync(0xffffffffu, incl, 31);
+    }
+}
+
+__global__ void __launch_bounds__(32 * kBfsWarpsPerBlock, 4) k_vor_bfs(VorCells C, DevParticles P,
                                                                     const int32_t* __restrict__ home,
                                                                     double support_in_h, int pass,
                                                                     unsigned long long* __restrict__ next,
@@ -149,12 +490,10 @@ __global__ void __launch_bounds__(32 * kBfsWarpsPerBlock) k_vor_bfs(VorCells C, 
                                                                     const int64_t* __restrict__ foffs,
                                                                     int64_t* __restrict__ pair_foff,
                                                                     int32_t* __restrict__ fsrc, VorStage stg) {
-    __shared__ int32_t s_cand[kBfsWarpsPerBlock][kBfsCandCap];
-    __shared__ unsigned long long s_reach[kBfsWarpsPerBlock][32][2];
+    extern __shared__ __align__(16) unsigned char s_walk[];
+    WalkShared& sh = *reinterpret_cast<WalkShared*>(s_walk);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t slot = (int64_t)blockIdx.x * kBfsWarpsPerBlock + warp;
-    long long* mark = mark_base + slot * C.n_cells;
-    int32_t* queue = queue_base + slot * C.n_cells;
     unsigned long long n_unresolved = 0, n_unmapped = 0, n_limit = 0;
     for (;;) {
         unsigned long long p = 0;
@@ -173,203 +512,22 @@ __global__ void __launch_bounds__(32 * kBfsWarpsPerBlock) k_vor_bfs(VorCells C, 
         }
         const double x0 = P.x[p], y0 = P.y[p], z0 = P.z[p];
         const double radius = mul_rn(support_in_h, h);
-        const long long mk = marker((int64_t)p, pass);
         const int64_t o = (pass == 1) ? offs[p] : 0;
-        if (lane == 0) {
-            queue[0] = k0;
-            mark[k0] = mk << 32;
+        const int64_t fcarry = (pass == 1 && fsrc) ? foffs[p] : 0;  // pass 1: the first cell's first face
+        int64_t nface = 0;
+        unsigned long long limit = 0;
+        WalkCells<true> W{sh.key[warp], sh.pos[warp], sh.queue[warp], nullptr, 0};
+        int tail = vor_walk<true>(C, sh, warp, lane, x0, y0, z0, radius, k0, pass, o, fcarry, W, pair_cells, pair_mask,
+                                  pair_foff, fsrc, nface, limit);
+        const bool shared = tail >= 0;
+        WalkCells<false> G{nullptr, nullptr, queue_base + slot * C.n_cells, mark_base + slot * C.n_cells,
+                           marker((int64_t)p, pass)};
+        if (!shared) {
+            limit = 0;
+            tail = vor_walk<false>(C, sh, warp, lane, x0, y0, z0, radius, k0, pass, o, fcarry, G, pair_cells, pair_mask,
+                                   pair_foff, fsrc, nface, limit);
         }
-        __syncwarp();
-        int head = 0, tail = 1;
-        int64_t nface = 0;                                  // pass 0: this lane's share of the face count
-        int64_t fcarry = (pass == 1 && fsrc) ? foffs[p] : 0;  // pass 1: the next cell's first face
-        while (head < tail) {
-            if (head > C.n_cells) {  // cannot happen: each cell enters the queue once
-                n_limit += (lane == 0);
-                break;
-            }
-            // The lanes take the next (up to) 32 queued cells, one each, and mark the faces to test: faces
-            // towards a neighbour not yet in the queue, skipping a face whose neighbour an earlier face of
-            // the same cell already named (a face-cache hit in the reference, which discovers nothing).  The
-            // warp tests them (the kernel reaches the face or not); the reachable ones are the discovery
-            // candidates, appended in (cell, face) order, skipping neighbours queued meanwhile: the
-            // reference's sequential queue.
-            const int batch = min(32, tail - head);
-            int64_t fa = 0, nf = 0;
-            unsigned long long cand0 = 0, cand1 = 0, earlier = 0, test0 = 0, test1 = 0;
-            if (lane < batch) {
-                const int rank = head + lane;
-                const int32_t cell = queue[rank];
-                fa = C.face_off[cell];
-                const int64_t fz = C.face_off[cell + 1];
-                nf = fz - fa;
-                nface += nf;
-                if (fz - fa > 128) n_limit += 1;  // a cell of more than 128 faces is not supported
-                for (int64_t f = fa; f < fz && f - fa < 128; ++f) {
-                    const int32_t nb = C.face_nbr[f];
-                    if (nb < 0 || nb >= C.n_cells) continue;
-                    const long long mv = mark[nb];
-                    const bool seen = (mv >> 32) == mk;
-                    if (seen) {
-                        if ((int)(mv & 0xffffffffLL) < rank && f - fa < 64) earlier |= 1ull << (f - fa);
-                        continue;
-                    }
-                    if (C.twin[f] >= 0) continue;  // an earlier face of this cell named nb already
-                    if (f - fa < 64) test0 |= 1ull << (f - fa);
-                    else test1 |= 1ull << (f - fa - 64);
-                }
-                if (pass == 1) {
-                    pair_cells[o + rank] = cell;
-                    pair_mask[o + rank] = earlier;
-                }
-            }
-            {
-                // The faces left to test (neighbour not queued, not a twin) as one list over the warp, in
-                // (cell, face) order, each lane testing every 32nd: a lane's own cell would leave the others
-                // idle through its faces, and the early batches hold one cell or a few.  A batch of more
-                // tests than the list holds is tested lane by lane.
-                const int nt_l = __popcll(test0) + __popcll(test1);
-                int t_incl = nt_l;
-                for (int d = 1; d < 32; d <<= 1) {
-                    const int v = __shfl_up_sync(0xffffffffu, t_incl, d);
-                    if (lane >= d) t_incl += v;
-                }
-                const int n_test = __shfl_sync(0xffffffffu, t_incl, 31);
-                if (n_test <= kBfsCandCap) {
-                    int32_t* items = s_cand[warp];
-                    int o_t = t_incl - nt_l;
-                    for (int w = 0; w < 2; ++w) {
-                        unsigned long long bits = w == 0 ? test0 : test1;
-                        while (bits) {
-                            const int b = __ffsll((long long)bits) - 1;
-                            bits &= bits - 1;
-                            items[o_t++] = lane << 7 | (64 * w + b);
-                        }
-                    }
-                    s_reach[warp][lane][0] = 0;
-                    s_reach[warp][lane][1] = 0;
-                    __syncwarp();
-                    for (int base = 0; base < n_test; base += 32) {
-                        const int i = base + lane;
-                        const int item = i < n_test ? items[i] : 0;
-                        const int src = item >> 7, fl = item & 127;
-                        const int64_t f = __shfl_sync(0xffffffffu, fa, src) + fl;
-                        if (i < n_test) {
-                            const FlatVerts V{C.vxyz + 3 * C.vert_off[f]};
-                            if (face_reachable(x0, y0, z0, radius, V, (int)(C.vert_off[f + 1] - C.vert_off[f])))
-                                atomicOr(&s_reach[warp][src][fl >> 6], 1ull << (fl & 63));
-                        }
-                    }
-                    __syncwarp();
-                    cand0 = s_reach[warp][lane][0];
-                    cand1 = s_reach[warp][lane][1];
-                    __syncwarp();
-                } else {
-                    for (int w = 0; w < 2; ++w) {
-                        unsigned long long bits = w == 0 ? test0 : test1;
-                        while (bits) {
-                            const int b = __ffsll((long long)bits) - 1;
-                            bits &= bits - 1;
-                            const int64_t f = fa + 64 * w + b;
-                            const FlatVerts V{C.vxyz + 3 * C.vert_off[f]};
-                            if (face_reachable(x0, y0, z0, radius, V, (int)(C.vert_off[f + 1] - C.vert_off[f]))) {
-                                if (w == 0) cand0 |= 1ull << b;
-                                else cand1 |= 1ull << b;
-                            }
-                        }
-                    }
-                }
-            }
-            if (pass == 1 && fsrc) {
-                // the cells' places in the face tables (a warp prefix sum in walk order) and each face's source
-                int64_t incl = nf;
-                for (int d = 1; d < 32; d <<= 1) {
-                    const int64_t v = __shfl_up_sync(0xffffffffu, incl, d);
-                    if (lane >= d) incl += v;
-                }
-                if (lane < batch) {
-                    const int rank = head + lane;
-                    const int64_t pf = fcarry + incl - nf;
-                    pair_foff[o + rank] = pf;
-                    for (int64_t f = fa; f < fa + nf; ++f) {
-                        const int32_t nb = C.face_nbr[f];
-                        int32_t code = -1;
-                        if (nb >= 0 && nb < C.n_cells) {
-                            const long long mv = mark[nb];
-                            if ((mv >> 32) == mk && (int)(mv & 0xffffffffLL) < rank && C.back[f] >= 0)
-                                code = (int32_t)(mv & 0xffffffffLL);
-                            if (code < 0 && C.twin[f] >= 0) code = -2 - C.twin[f];
-                        }
-                        fsrc[pf + (f - fa)] = code;
-                    }
-                }
-                fcarry += __shfl_sync(0xffffffffu, incl, 31);
-            }
-            int t = tail;
-            // the batch's candidates in (cell, face) order; each is queued if no earlier candidate names the
-            // same cell and it is not queued yet -- the sequential appends' queue, with every lane at work
-            const int nc_l = __popcll(cand0) + __popcll(cand1);
-            int c_incl = nc_l;
-            for (int d = 1; d < 32; d <<= 1) {
-                const int v = __shfl_up_sync(0xffffffffu, c_incl, d);
-                if (lane >= d) c_incl += v;
-            }
-            const int n_cand = __shfl_sync(0xffffffffu, c_incl, 31);
-            if (n_cand <= kBfsCandCap) {
-                int32_t* cl = s_cand[warp];
-                int o = c_incl - nc_l;
-                for (int w = 0; w < 2; ++w) {
-                    unsigned long long bits = w == 0 ? cand0 : cand1;
-                    while (bits) {
-                        const int b = __ffsll((long long)bits) - 1;
-                        bits &= bits - 1;
-                        cl[o++] = C.face_nbr[fa + 64 * w + b];
-                    }
-                }
-                __syncwarp();
-                for (int base = 0; base < n_cand; base += 32) {
-                    const int i = base + lane;
-                    int32_t nb = -1;
-                    bool keep = false;
-                    if (i < n_cand) {
-                        nb = cl[i];
-                        keep = (mark[nb] >> 32) != mk;
-                        for (int j = 0; keep && j < i; ++j) keep = cl[j] != nb;
-                    }
-                    const unsigned kb = __ballot_sync(0xffffffffu, keep);
-                    if (keep) {
-                        const int pos = t + __popc(kb & ((1u << lane) - 1));
-                        mark[nb] = (mk << 32) | (long long)pos;
-                        queue[pos] = nb;
-                    }
-                    t += __popc(kb);
-                }
-                __syncwarp();
-            } else {
-            for (int L = 0; L < batch; ++L) {
-                unsigned long long c0 = __shfl_sync(0xffffffffu, cand0, L);
-                unsigned long long c1 = __shfl_sync(0xffffffffu, cand1, L);
-                const int64_t fl = __shfl_sync(0xffffffffu, fa, L);
-                if (lane == 0) {
-                    for (int w = 0; w < 2; ++w) {
-                        unsigned long long bits = w == 0 ? c0 : c1;
-                        while (bits) {
-                            const int b = __ffsll((long long)bits) - 1;
-                            bits &= bits - 1;
-                            const int32_t nb = C.face_nbr[fl + 64 * w + b];
-                            if ((mark[nb] >> 32) != mk) {
-                                mark[nb] = (mk << 32) | (long long)t;
-                                queue[t++] = nb;
-                            }
-                        }
-                    }
-                }
-            }
-            }
-            tail = __shfl_sync(0xffffffffu, t, 0);
-            head += batch;
-            __syncwarp();
-        }
+        n_limit += limit;
         if (pass != 1 && fcounts) {
             for (int d = 16; d > 0; d >>= 1) nface += __shfl_down_sync(0xffffffffu, nface, d);
             nface = __shfl_sync(0xffffffffu, nface, 0);
@@ -380,60 +538,8 @@ __global__ void __launch_bounds__(32 * kBfsWarpsPerBlock) k_vor_bfs(VorCells C, 
             if (tail == 1) ++n_unmapped;
         }
         if (pass == 2) {
-            // the single walk: reserve this particle's pairs and faces, then write them.  The marks hold
-            // every visited cell's queue position, so each face's source is decided as pass 1 decides it
-            // during its walk (a neighbour processed earlier is one with a smaller queue position).
-            unsigned long long s0 = 0, fs0 = 0;
-            if (lane == 0) {
-                s0 = atomicAdd(&stg.ctr[0], (unsigned long long)tail);
-                fs0 = atomicAdd(&stg.ctr[1], (unsigned long long)nface);
-            }
-            s0 = __shfl_sync(0xffffffffu, s0, 0);
-            fs0 = __shfl_sync(0xffffffffu, fs0, 0);
-            if (s0 + tail > (unsigned long long)stg.cap_pairs || fs0 + nface > (unsigned long long)stg.cap_faces) {
-                if (lane == 0) atomicOr(&stg.ctr[2], 1ull);
-            } else {
-                if (lane == 0) {
-                    stg.start[p] = (int64_t)s0;
-                    stg.fstart[p] = (int64_t)fs0;
-                }
-                int64_t fc = 0;
-                for (int base = 0; base < tail; base += 32) {
-                    const int r = base + lane;
-                    int32_t cell = 0;
-                    int64_t fa = 0, nf = 0;
-                    if (r < tail) {
-                        cell = queue[r];
-                        fa = C.face_off[cell];
-                        nf = C.face_off[cell + 1] - fa;
-                    }
-                    int64_t incl = nf;
-                    for (int d = 1; d < 32; d <<= 1) {
-                        const int64_t v = __shfl_up_sync(0xffffffffu, incl, d);
-                        if (lane >= d) incl += v;
-                    }
-                    if (r < tail) {
-                        const int64_t fl = fc + incl - nf;
-                        unsigned long long earlier = 0;
-                        for (int64_t f = fa; f < fa + nf; ++f) {
-                            const int32_t nb = C.face_nbr[f];
-                            int32_t code = -1;
-                            if (nb >= 0 && nb < C.n_cells) {
-                                const long long mv = mark[nb];
-                                const bool before = (mv >> 32) == mk && (int)(mv & 0xffffffffLL) < r;
-                                if (before && f - fa < 64) earlier |= 1ull << (f - fa);
-                                if (before && C.back[f] >= 0) code = (int32_t)(mv & 0xffffffffLL);
-                                if (code < 0 && C.twin[f] >= 0) code = -2 - C.twin[f];
-                            }
-                            stg.fsrc[fs0 + fl + (f - fa)] = code;
-                        }
-                        stg.cells[s0 + r] = cell;
-                        stg.mask[s0 + r] = earlier;
-                        stg.floc[s0 + r] = fl;
-                    }
-                    fc += __shfl_sync(0xffffffffu, incl, 31);
-                }
-            }
+            if (shared) vor_stage(C, W, lane, (int64_t)p, tail, nface, stg);
+            else vor_stage(C, G, lane, (int64_t)p, tail, nface, stg);
         }
         __syncwarp();
     }
@@ -478,37 +584,52 @@ __global__ void k_vor_pairs(const int32_t* __restrict__ pair_cells, int64_t tota
     vals[k] = (uint32_t)k;
 }
 
-// The particle of pair k: the last p with offs[p] <= k.
-__device__ __forceinline__ int64_t pair_particle(const int64_t* __restrict__ offs, int64_t n, int64_t k) {
-    int64_t lo = 0, hi = n - 1;
-    while (lo < hi) {
-        const int64_t mid = (lo + hi + 1) >> 1;
-        if (offs[mid] <= k) lo = mid; else hi = mid - 1;
-    }
-    return lo;
+// owner[k] = the particle of pair k (one warp per particle).
+__global__ void k_vor_owner(int64_t n, const int64_t* __restrict__ counts, const int64_t* __restrict__ offs,
+                            uint32_t* __restrict__ owner) {
+    const int64_t p = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (p >= n) return;
+    const int64_t cnt = counts[p], o = offs[p];
+    for (int64_t r = threadIdx.x & 31; r < cnt; r += 32) owner[o + r] = (uint32_t)p;
 }
 
-// One face's integral for one particle (the face walk with the kernel's evaluator).  MODE: kVorGeneric,
-// kVorCubic (closed form) or kVorTab (lookups in tab; clamped indices counted in *nclamp).
-constexpr int kVorGeneric = 0, kVorCubic = 1, kVorTab = 2;
+// One face's integral for one particle: the cones of kernel MODE of the tables (0 .. 5; cone_math.cuh; R: its pieces
+// in shared memory), or kVorTab: lookups in tab (the face walk; clamped indices counted in *nclamp).  Out of line,
+// so that every kernel runs the same code on a face.
+constexpr int kVorTab = -1;
+template <int MODE>
+struct VorKernel {
+    static constexpr int kPieces = 1, kDeg = 1;
+};
+#define KIWI_VOR_KERNEL(K, NP, DEG) \
+    template <>                     \
+    struct VorKernel<K> {           \
+        static constexpr int kPieces = NP, kDeg = DEG; \
+    };
+KIWI_BOX_KERNELS(KIWI_VOR_KERNEL)
+#undef KIWI_VOR_KERNEL
 template <int MODE>
 static __device__ __noinline__ double vor_face(const double* verts, int nv, double x0, double y0, double z0, double h,
-                                               double radius, int kernel, const TabDev& tab, unsigned* nclamp) {
+                                               double radius, const KiwiConeRegion* R, const TabDev& tab,
+                                               unsigned* nclamp) {
     const FlatVerts V{verts};
-    if (MODE == kVorTab) {
+    if constexpr (MODE == kVorTab) {
         TabEval ev{tab, h, 0.0, 0.0, nclamp};
         return face_integral(x0, y0, z0, 2 * h, V, nv, (int*)nullptr, ev);
+    } else {
+        return cone_face<VorKernel<MODE>::kPieces, VorKernel<MODE>::kDeg>(c_cones[MODE], R, V, nv, x0, y0, z0,
+                                                                       fm_rcp(radius));
     }
-    if (MODE == kVorCubic) {
-        LenCubicEval ev;
-        ev.h = h;
-        ev.ih = 1.0 / h;
-        return face_integral(x0, y0, z0, 2 * h, V, nv, (int*)nullptr, ev);
+}
+// The kernel's pieces into shared memory (a barrier follows before they are read).
+template <int MODE>
+__device__ __forceinline__ void vor_stage_regions(KiwiConeRegion* R) {
+    if constexpr (MODE != kVorTab) {
+        constexpr int n = (int)(sizeof(KiwiConeRegion) / sizeof(double)) * VorKernel<MODE>::kPieces;
+        double* const dst = reinterpret_cast<double*>(R);
+        const double* const src = reinterpret_cast<const double*>(c_cones[MODE].reg);
+        for (int i = threadIdx.x; i < n; i += kGatherThreads) dst[i] = src[i];
     }
-    GenericEval ev;
-    ev.K = &c_vor_tables[kernel];
-    ev.H = radius;
-    return face_integral(x0, y0, z0, radius, V, nv, (int*)nullptr, ev);
 }
 
 __global__ void k_cell_ranges(const uint32_t* __restrict__ keys, int64_t total, int64_t* __restrict__ range) {
@@ -520,11 +641,11 @@ __global__ void k_cell_ranges(const uint32_t* __restrict__ keys, int64_t total, 
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(kGatherThreads) k_vor_gather(VorCells C, DevParticles P, int kernel,
-                                                                double support_in_h, const TabDev tab,
+__global__ void __launch_bounds__(kGatherThreads) k_vor_gather(VorCells C, DevParticles P, double support_in_h, const TabDev tab,
                                                                 const uint32_t* __restrict__ plist,
                                                                 const int64_t* __restrict__ range,
                                                                 const int64_t* __restrict__ offs,
+                                                                const uint32_t* __restrict__ owner,
                                                                 const int32_t* __restrict__ pair_cells,
                                                                 const unsigned long long* __restrict__ pair_mask,
                                                                 CartOutputs out, DevStats* __restrict__ st,
@@ -532,6 +653,8 @@ __global__ void __launch_bounds__(kGatherThreads) k_vor_gather(VorCells C, DevPa
     __shared__ double s_v[3 * kGatherVertCap];
     __shared__ double s_val[kGatherThreads], s_m[kGatherThreads], s_vx[kGatherThreads], s_vy[kGatherThreads],
         s_vz[kGatherThreads];
+    __shared__ KiwiConeRegion s_R[VorKernel<MODE>::kPieces];
+    vor_stage_regions<MODE>(s_R);
     const int64_t cell = blockIdx.x;
     const int64_t f0 = C.face_off[cell], f1 = C.face_off[cell + 1];
     const int64_t v0 = C.vert_off[f0], v1 = C.vert_off[f1];
@@ -548,7 +671,7 @@ __global__ void __launch_bounds__(kGatherThreads) k_vor_gather(VorCells C, DevPa
         double msum = 0.0;
         if (k < end) {
             const int64_t pk = plist[k];
-            const int64_t p = pair_particle(offs, P.n, pk);
+            const int64_t p = owner[pk];
             const int64_t seg = offs[p], rank = pk - seg;
             const unsigned long long mask = pair_mask[pk];
             const double x0 = P.x[p], y0 = P.y[p], z0 = P.z[p], h = P.h[p];
@@ -586,7 +709,7 @@ __global__ void __launch_bounds__(kGatherThreads) k_vor_gather(VorCells C, DevPa
                 const int nv = (int)(C.vert_off[src + 1] - C.vert_off[src]);
                 const double* verts = (src >= f0 && src < f1 && staged) ? s_v + 3 * (C.vert_off[src] - v0)
                                                                          : C.vxyz + 3 * C.vert_off[src];
-                const double val = vor_face<MODE>(verts, nv, x0, y0, z0, h, radius, kernel, tab, &n_clamp);
+                const double val = vor_face<MODE>(verts, nv, x0, y0, z0, h, radius, s_R, tab, &n_clamp);
                 if (sign < 0.0) msum -= val; else msum += val;
             }
             if (msum < 0.0) {
@@ -646,11 +769,13 @@ __global__ void __launch_bounds__(kGatherThreads) k_vor_gather(VorCells C, DevPa
 // every face value evaluated once per particle instead of once per side.
 template <int MODE>
 __global__ void __launch_bounds__(kGatherThreads, KIWI_VOR_FACES_MIN_BLOCKS)
-    k_vor_faces(VorCells C, DevParticles P, int kernel, double support_in_h, const TabDev tab,
+    k_vor_faces(VorCells C, DevParticles P, double support_in_h, const TabDev tab,
                 const uint32_t* __restrict__ plist, const int64_t* __restrict__ range,
                 const int64_t* __restrict__ pair_foff, const int32_t* __restrict__ fsrc,
-                const int64_t* __restrict__ offs, double* __restrict__ fval, DevStats* __restrict__ st) {
+                const uint32_t* __restrict__ owner, double* __restrict__ fval, DevStats* __restrict__ st) {
     __shared__ double s_v[3 * kGatherVertCap];
+    __shared__ KiwiConeRegion s_R[VorKernel<MODE>::kPieces];
+    vor_stage_regions<MODE>(s_R);
     const int64_t cell = blockIdx.x;
     const int64_t f0 = C.face_off[cell], f1 = C.face_off[cell + 1];
     const int64_t v0 = C.vert_off[f0], v1 = C.vert_off[f1];
@@ -665,7 +790,7 @@ __global__ void __launch_bounds__(kGatherThreads, KIWI_VOR_FACES_MIN_BLOCKS)
         // (a cell of more faces than an item packs; the walk refuses such a map afterwards)
         for (int64_t k = beg + threadIdx.x; k < end; k += kGatherThreads) {
             const int64_t pk = plist[k];
-            const int64_t p = pair_particle(offs, P.n, pk);
+            const int64_t p = owner[pk];
             const double h = P.h[p];
             const int64_t pf = pair_foff[pk];
 #pragma unroll 1
@@ -673,7 +798,7 @@ __global__ void __launch_bounds__(kGatherThreads, KIWI_VOR_FACES_MIN_BLOCKS)
                 if (fsrc[pf + (f - f0)] != -1) continue;
                 const int nv = (int)(C.vert_off[f + 1] - C.vert_off[f]);
                 fval[pf + (f - f0)] = vor_face<MODE>(C.vxyz + 3 * C.vert_off[f], nv, P.x[p], P.y[p], P.z[p], h,
-                                                     mul_rn(support_in_h, h), kernel, tab, &n_clamp);
+                                                     mul_rn(support_in_h, h), s_R, tab, &n_clamp);
             }
         }
     } else {
@@ -697,7 +822,7 @@ __global__ void __launch_bounds__(kGatherThreads, KIWI_VOR_FACES_MIN_BLOCKS)
             unsigned long long own0 = 0, own1 = 0;  // faces 0..63 and 64..127 this pair evaluates
             if (threadIdx.x < group && k < end) {
                 const int64_t pk = plist[k];
-                const int64_t p = pair_particle(offs, P.n, pk);
+                const int64_t p = owner[pk];
                 const int64_t pf = pair_foff[pk];
                 s_px[threadIdx.x] = P.x[p];
                 s_py[threadIdx.x] = P.y[p];
@@ -752,7 +877,7 @@ __global__ void __launch_bounds__(kGatherThreads, KIWI_VOR_FACES_MIN_BLOCKS)
                 const double* verts = staged ? s_v + 3 * (C.vert_off[f] - v0) : C.vxyz + 3 * C.vert_off[f];
                 const double h = s_ph[t];
                 fval[s_pf[t] + fl] = vor_face<MODE>(verts, nv, s_px[t], s_py[t], s_pz[t], h,
-                                                    mul_rn(support_in_h, h), kernel, tab, &n_clamp);
+                                                    mul_rn(support_in_h, h), s_R, tab, &n_clamp);
             }
             __syncthreads();
         }
@@ -765,6 +890,7 @@ __global__ void __launch_bounds__(kGatherThreads) k_vor_sum(VorCells C, DevParti
                                                              const uint32_t* __restrict__ plist,
                                                              const int64_t* __restrict__ range,
                                                              const int64_t* __restrict__ offs,
+                                                             const uint32_t* __restrict__ owner,
                                                              const int64_t* __restrict__ pair_foff,
                                                              const int32_t* __restrict__ fsrc,
                                                              const double* __restrict__ fval, CartOutputs out,
@@ -781,7 +907,7 @@ __global__ void __launch_bounds__(kGatherThreads) k_vor_sum(VorCells C, DevParti
         double msum = 0.0;
         if (k < end) {
             const int64_t pk = plist[k];
-            const int64_t p = pair_particle(offs, P.n, pk);
+            const int64_t p = owner[pk];
             const int64_t seg = offs[p];
             const int64_t pf = pair_foff[pk];
 #pragma unroll 1
@@ -874,7 +1000,7 @@ int voronoi_map_dev(KiwiCtx* ctx, const DevParticles& P, const int32_t* d_home, 
                     const KernelChoice& kc, const CartOutputs& out_in, KiwiStats* stats, const VorInverse* inv) {
     const int64_t launches0 = ctx->launches;
     const int64_t n = P.n, nc = cells.n_cells;
-    VorCells C{nc, cells.face_off, cells.vert_off, cells.vxyz, cells.face_nbr, cells.volume, nullptr, nullptr};
+    VorCells C{nc, cells.face_off, cells.vert_off, cells.vxyz, cells.face_nbr, cells.volume, nullptr, nullptr, nullptr};
     DevStats* d_stats = nullptr;
     double* d_meanv = nullptr;
     unsigned long long* d_next = nullptr;
@@ -902,11 +1028,18 @@ int voronoi_map_dev(KiwiCtx* ctx, const DevParticles& P, const int32_t* d_home, 
     KIWI_LAUNCHED(ctx);
     C.twin = d_twin;
     C.back = d_back;
+    double4* d_plane = nullptr;
+    KIWI_TRY(scratch_t(ctx, S_VOR_PLANES, nf_alloc, &d_plane));
+    if (n_faces > 0) {
+        k_face_planes<<<(unsigned)((n_faces + 255) / 256), 256, 0, ctx->stream>>>(n_faces, cells.vert_off, cells.vxyz, d_plane);
+        KIWI_LAUNCHED(ctx);
+    }
+    C.plane = d_plane;
 
     // BFS work slots: a visited marker and a queue of n_cells entries each
     int sms = 0;
     KIWI_CUDA(ctx, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
-    int64_t slots = (int64_t)sms * 8;
+    int64_t slots = (int64_t)sms * 4 * kBfsWarpsPerBlock;  // four blocks per SM
     const int64_t budget = (int64_t)16 << 30;  // bytes of BFS scratch at most
     while (slots > kBfsWarpsPerBlock && slots * nc * 12 > budget) slots /= 2;
     slots = std::max<int64_t>(kBfsWarpsPerBlock, (slots / kBfsWarpsPerBlock) * kBfsWarpsPerBlock);
@@ -924,6 +1057,7 @@ int voronoi_map_dev(KiwiCtx* ctx, const DevParticles& P, const int32_t* d_home, 
     KIWI_CUDA(ctx, cudaMemsetAsync(range, 0, sizeof(int64_t) * 2 * nc, ctx->stream));
 
     const double sup = kc.support_in_h;
+    KIWI_CUDA(ctx, cudaFuncSetAttribute(k_vor_bfs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WalkShared)));
     // pass 0: count the visited cells and their faces
     int64_t *fcounts = nullptr, *foffs = nullptr;
     KIWI_TRY(scratch_t(ctx, S_VOR_FCOUNT, (size_t)std::max<int64_t>(n, 1), &fcounts));
@@ -955,7 +1089,7 @@ int voronoi_map_dev(KiwiCtx* ctx, const DevParticles& P, const int32_t* d_home, 
             stg.cap_faces = cap_f;
             KIWI_CUDA(ctx, cudaMemsetAsync(stg.ctr, 0, 3 * sizeof(unsigned long long), ctx->stream));
             KIWI_CUDA(ctx, cudaMemsetAsync(d_next, 0, sizeof(unsigned long long), ctx->stream));
-            k_vor_bfs<<<blocks, 32 * kBfsWarpsPerBlock, 0, ctx->stream>>>(C, P, d_home, sup, 2, d_next, mark, queue,
+            k_vor_bfs<<<blocks, 32 * kBfsWarpsPerBlock, sizeof(WalkShared), ctx->stream>>>(C, P, d_home, sup, 2, d_next, mark, queue,
                                                                          counts, nullptr, nullptr, nullptr, d_stats,
                                                                          fcounts, nullptr, nullptr, nullptr, stg);
             KIWI_LAUNCHED(ctx);
@@ -969,7 +1103,7 @@ int voronoi_map_dev(KiwiCtx* ctx, const DevParticles& P, const int32_t* d_home, 
     if (!single) {
         KIWI_CUDA(ctx, cudaMemsetAsync(d_next, 0, sizeof(unsigned long long), ctx->stream));
         if (n > 0) {
-            k_vor_bfs<<<blocks, 32 * kBfsWarpsPerBlock, 0, ctx->stream>>>(C, P, d_home, sup, 0, d_next, mark, queue,
+            k_vor_bfs<<<blocks, 32 * kBfsWarpsPerBlock, sizeof(WalkShared), ctx->stream>>>(C, P, d_home, sup, 0, d_next, mark, queue,
                                                                          counts, nullptr, nullptr, nullptr, d_stats,
                                                                          fcounts, nullptr, nullptr, nullptr,
                                                                          VorStage{});
@@ -1002,6 +1136,8 @@ int voronoi_map_dev(KiwiCtx* ctx, const DevParticles& P, const int32_t* d_home, 
     uint32_t *k0, *v0, *k1, *v1;
     KIWI_TRY(scratch_t(ctx, S_VOR_PAIRS, (size_t)std::max<int64_t>(total, 1), &pair_cells));
     KIWI_TRY(scratch_t(ctx, S_VOR_MASK, (size_t)std::max<int64_t>(total, 1), &pair_mask));
+    uint32_t* owner = nullptr;
+    KIWI_TRY(scratch_t(ctx, S_VOR_OWNER, (size_t)std::max<int64_t>(total, 1), &owner));
     KIWI_TRY(scratch_t(ctx, S_KEYS0, (size_t)std::max<int64_t>(total, 1), &k0));
     KIWI_TRY(scratch_t(ctx, S_VALS0, (size_t)std::max<int64_t>(total, 1), &v0));
     KIWI_TRY(scratch_t(ctx, S_KEYS1, (size_t)std::max<int64_t>(total, 1), &k1));
@@ -1016,11 +1152,13 @@ int voronoi_map_dev(KiwiCtx* ctx, const DevParticles& P, const int32_t* d_home, 
         } else {
             // pass 1: write each particle's visited cells at its offset
             KIWI_CUDA(ctx, cudaMemsetAsync(d_next, 0, sizeof(unsigned long long), ctx->stream));
-            k_vor_bfs<<<blocks, 32 * kBfsWarpsPerBlock, 0, ctx->stream>>>(C, P, d_home, sup, 1, d_next, mark, queue,
+            k_vor_bfs<<<blocks, 32 * kBfsWarpsPerBlock, sizeof(WalkShared), ctx->stream>>>(C, P, d_home, sup, 1, d_next, mark, queue,
                                                                          counts, offs, pair_cells, pair_mask, d_stats,
                                                                          nullptr, foffs, pair_foff, fsrc, VorStage{});
             KIWI_LAUNCHED(ctx);
         }
+        k_vor_owner<<<(unsigned)((n * 32 + 255) / 256), 256, 0, ctx->stream>>>(n, counts, offs, owner);
+        KIWI_LAUNCHED(ctx);
         k_vor_pairs<<<(unsigned)((total + 255) / 256), 256, 0, ctx->stream>>>(pair_cells, total, k0, v0);
         KIWI_LAUNCHED(ctx);
         int key_bits = 1;
@@ -1036,30 +1174,28 @@ int voronoi_map_dev(KiwiCtx* ctx, const DevParticles& P, const int32_t* d_home, 
     if (nc > 0x7fffffffLL) return set_err(ctx, KIWI_ERR_ARG, "too many cells (%lld)", (long long)nc);
     double* pair_val = nullptr;
     if (inv) KIWI_TRY(scratch_t(ctx, S_VOR_PVAL, (size_t)std::max<int64_t>(total, 1), &pair_val));
+    const int mode = kc.tabulated ? kVorTab : kc.kernel;
     if (fsrc) {
-        if (kc.tabulated)
-            k_vor_faces<kVorTab><<<(unsigned)nc, kGatherThreads, 0, ctx->stream>>>(
-                C, P, kc.kernel, sup, kc.tab, plist, range, pair_foff, fsrc, offs, fval, d_stats);
-        else if (kc.cubic)
-            k_vor_faces<kVorCubic><<<(unsigned)nc, kGatherThreads, 0, ctx->stream>>>(
-                C, P, kc.kernel, sup, kc.tab, plist, range, pair_foff, fsrc, offs, fval, d_stats);
-        else
-            k_vor_faces<kVorGeneric><<<(unsigned)nc, kGatherThreads, 0, ctx->stream>>>(
-                C, P, kc.kernel, sup, kc.tab, plist, range, pair_foff, fsrc, offs, fval, d_stats);
+#define KIWI_VOR_FACES(K, NP, DEG)                                                                                  \
+    if (mode == K)                                                                                                  \
+        k_vor_faces<K><<<(unsigned)nc, kGatherThreads, 0, ctx->stream>>>(C, P, sup, kc.tab, plist, range, pair_foff, \
+                                                                         fsrc, owner, fval, d_stats);
+        KIWI_BOX_KERNELS(KIWI_VOR_FACES)
+        KIWI_VOR_FACES(kVorTab, 0, 0)
+#undef KIWI_VOR_FACES
         KIWI_LAUNCHED(ctx);
-        k_vor_sum<<<(unsigned)nc, kGatherThreads, 0, ctx->stream>>>(C, P, plist, range, offs, pair_foff, fsrc, fval,
+        k_vor_sum<<<(unsigned)nc, kGatherThreads, 0, ctx->stream>>>(C, P, plist, range, offs, owner, pair_foff, fsrc, fval,
                                                                      out, d_stats, pair_val);
         KIWI_LAUNCHED(ctx);
     } else {
-        if (kc.tabulated)
-            k_vor_gather<kVorTab><<<(unsigned)nc, kGatherThreads, 0, ctx->stream>>>(
-                C, P, kc.kernel, sup, kc.tab, plist, range, offs, pair_cells, pair_mask, out, d_stats, pair_val);
-        else if (kc.cubic)
-            k_vor_gather<kVorCubic><<<(unsigned)nc, kGatherThreads, 0, ctx->stream>>>(
-                C, P, kc.kernel, sup, kc.tab, plist, range, offs, pair_cells, pair_mask, out, d_stats, pair_val);
-        else
-            k_vor_gather<kVorGeneric><<<(unsigned)nc, kGatherThreads, 0, ctx->stream>>>(
-                C, P, kc.kernel, sup, kc.tab, plist, range, offs, pair_cells, pair_mask, out, d_stats, pair_val);
+#define KIWI_VOR_GATHER(K, NP, DEG)                                                                              \
+    if (mode == K)                                                                                               \
+        k_vor_gather<K><<<(unsigned)nc, kGatherThreads, 0, ctx->stream>>>(C, P, sup, kc.tab, plist, range, offs, \
+                                                                          owner, pair_cells, pair_mask, out,     \
+                                                                          d_stats, pair_val);
+        KIWI_BOX_KERNELS(KIWI_VOR_GATHER)
+        KIWI_VOR_GATHER(kVorTab, 0, 0)
+#undef KIWI_VOR_GATHER
         KIWI_LAUNCHED(ctx);
     }
     if (inv && n > 0) {

@@ -43,6 +43,15 @@ The derivative with respect to x is the kernel's integral over the box's face at
 
 D in powers of r - c like C, R and A (the triangle ending on the sphere) in powers of p^2 and p^2 + q^2.
 
+A face of a general cell is a sum over its edges' right triangles, whose cones' masses share all this: with
+delta = phi - ang at the triangle's far vertex, in piece k,
+
+  cone(r0, R0, t) = r0 R0 [t V(r, r0^2, p^2) / r + B(r0^2, p^2) (atanh(t / r) - t / r)] - delta a(r0)
+                    + sum_{s<k} [m_s delta - h_s(r0) phi + e_s(r0, R0)],
+  e(r0, R0) = r0 R0 [t_b A(r0^2, p^2) + B atanh(t_b / b)] - delta_b f(r0) + ang_b h(r0),
+
+the subscript b marking the point where the edge line leaves the sphere of radius b (kiwi_cone_tables).
+
 The polynomials of the arctangent and the logarithm (kiwi_b200/csrc/fastmath.cuh) interpolate
 atan(x) / x in x^2 on [0, 1] and atanh(s) / s in s^2 on [0, (3 - 2 sqrt 2)^2] at Chebyshev points, in
 exact rational arithmetic.
@@ -322,6 +331,54 @@ def scale(d, b):
             "h": flip(h), "A": laid(A, LAY_A)}
 
 
+V_BLOCKS = [((i, d - i), 13 - 2 * d) for d in range(7) for i in range(d + 1)]  # powers of r - c for each X^i P^j
+
+
+def to_xpr(a):
+    """A polynomial in (X, Y, Z) as {(i, j, l): coef} of X^i P^j r^(2l), Y = P - X, Z = r^2 - P."""
+    out = {}
+    for (i, j, k), v in a.items():
+        for u in range(j + 1):
+            for w in range(k + 1):
+                key = (i + u, j - u + k - w, w)
+                c = v * math.comb(j, u) * (-1) ** u * math.comb(k, w) * (-1) ** (k - w)
+                out[key] = out.get(key, Q(0)) + c
+    return {m: v for m, v in out.items() if v}
+
+
+def cone_region(w, c0):
+    V, B, a = {}, {}, [Q(0)] * 6
+    for n, c in w.items():
+        A1, B1 = tri(n + 2)
+        c = c / ((n + 3) * (n + 2))
+        for (i, j, l), v in to_xpr(A1).items():
+            V.setdefault((i, j), [Q(0)] * 13)[2 * l + 1 + n % 2] += c * v
+        b = to_xp(B1)
+        for (i, j), v in b.items():
+            V.setdefault((i, j), [Q(0)] * 13)[0] += c * v
+        add_into(B, b, c)
+        if n % 2:
+            a[(n - 1) // 2] += c
+    flat = []
+    for key, size in V_BLOCKS:
+        block = V.pop(key, [Q(0)] * 13)
+        assert not any(block[size:])
+        flat += shifted(block[:size], c0)
+    assert not V
+    return {"c": c0, "V": flat, "B": laid(B, LAY_R), "a": a}
+
+
+def cone_scale(d, b):
+    A, zpoly = {}, padd({(0, 0, 0): b * b}, PP, Q(-1))
+    for n, c in d.items():
+        one = {}
+        for m3, v in tri(n + 2)[0].items():  # t^2 = b^2 - P, r = b
+            one = padd(one, pmul({(m3[0], m3[1], 0): v}, ppow(zpoly, m3[2])))
+        add_into(A, to_xp(one), c * (b if n % 2 else 1) / ((n + 3) * (n + 2)))
+    s = scale(d, b)
+    return {"b": b, "m": s["m"], "fp": s["fp"], "ap": s["ap"], "f": s["f"], "h": s["h"], "A": laid(A, LAY_A)}
+
+
 def kernel_box(K):
     polys = [dict(p.c) for p in K.piece_polys()]
     a3 = K.a3_times_pi()
@@ -334,12 +391,20 @@ def kernel_box(K):
             d[n] = d.get(n, Q(0)) - c
         scs.append(scale({n: c for n, c in d.items() if c}, b))
     top = max(n for p in polys for n in p)
-    return {"key": K.key, "npiece": len(polys), "deg": top, "a3pi": a3, "reg": regs, "scale": scs}
+    cregs = [cone_region(p, b if K.spline else CENTRE * b) for p, b in zip(polys, K.breaks)]
+    cscs = []
+    for s, b in enumerate(K.breaks):
+        nxt = polys[s + 1] if s + 1 < len(polys) else {}
+        d = {n: polys[s].get(n, Q(0)) - nxt.get(n, Q(0)) for n in set(polys[s]) | set(nxt)}
+        cscs.append(cone_scale({n: c for n, c in d.items() if c}, b))
+    return {"creg": cregs, "cscale": cscs, "key": K.key, "npiece": len(polys), "deg": top, "a3pi": a3, "reg": regs, "scale": scs}
 
 
 # the stored rows of a piece and of a difference kernel
 REG = ("C", "Q", "a", "D", "R")
 SCL = ("G", "fp", "ap", "f", "h", "A")
+CREG = ("V", "B", "a")
+CSCL = ("fp", "ap", "f", "h", "A")
 
 
 # ---- the two univariate polynomials
@@ -406,6 +471,9 @@ def tables():
         a3 = t["a3pi"]
         rnd = lambda row: [rounded(v, a3) for v in row]  # noqa: E731
         out.append({"key": t["key"], "npiece": t["npiece"], "deg": t["deg"],
+                    "creg": [{"c": float(r["c"]), **{k: rnd(r[k]) for k in CREG}} for r in t["creg"]],
+                    "cscale": [{"b": float(s["b"]), "m": rounded(s["m"], a3), **{k: rnd(s[k]) for k in CSCL}}
+                               for s in t["cscale"]],
                     "reg": [{"c": float(r["c"]), **{k: rnd(r[k]) for k in REG}} for r in t["reg"]],
                     "scale": [{"b": float(s["b"]), "m": rounded(s["m"], a3), "G": rnd(s["G"]),
                                **{k: rnd(s[k]) for k in SCL[1:]}} for s in t["scale"]]})
@@ -462,6 +530,34 @@ def header_text():
         L.append("      {" + ",\n       ".join(
             "{" + f"{_num(s['b'])}, {_num(s['m'])},\n        " + ",\n        ".join(_row(s[k]) for k in SCL) +
             "}" for s in t["scale"] + [zs] * (3 - t["npiece"])) + "}},")
+    L.append("};")
+    L.append("")
+    zr = {"c": 0.0, "V": [0.0] * 140, "B": [0.0] * 28, "a": [0.0] * 6}
+    zs = {"b": 0.0, "m": 0.0, "fp": [0.0] * 7, "ap": [0.0] * 6, "f": [0.0] * 14, "h": [0.0] * 15, "A": [0.0] * 21}
+    L += [
+        "// The cones' tables.  V: (r - c)^0.. for each X^i P^j, by i + j, then i, 13 - 2 (i + j) terms; B like R.",
+        "typedef struct KiwiConeRegion {",
+        "    double c, V[140], B[28], a[6];",
+        "} KiwiConeRegion;",
+        "typedef struct KiwiConeScale {",
+        "    double b, m, fp[7], ap[6], f[14], h[15], A[21];",
+        "} KiwiConeScale;",
+        "typedef struct KiwiConeTable {",
+        "    int npiece, deg;",
+        "    KiwiConeRegion reg[KIWI_BOX_PIECES];",
+        "    KiwiConeScale scale[KIWI_BOX_PIECES];",
+        "} KiwiConeTable;",
+        "",
+        "KIWI_BOX_QUALIFIER KiwiConeTable kiwi_cone_tables[6] = {",
+    ]
+    for t in T:
+        L.append(f"    {{ /* {t['key']} */ {t['npiece']}, {t['deg']},")
+        L.append("      {" + ",\n       ".join(
+            "{" + _num(r["c"]) + ",\n        " + ",\n        ".join(_row(r[k]) for k in CREG) + "}"
+            for r in t["creg"] + [zr] * (3 - t["npiece"])) + "},")
+        L.append("      {" + ",\n       ".join(
+            "{" + f"{_num(s['b'])}, {_num(s['m'])},\n        " + ",\n        ".join(_row(s[k]) for k in CSCL) +
+            "}" for s in t["cscale"] + [zs] * (3 - t["npiece"])) + "}},")
     L.append("};")
     L.append("")
     L.append("// atan(x) / x in powers of x^2 on [0, 1], and atanh(s) / s in powers of s^2 on |s| <= 3 - 2 sqrt 2")

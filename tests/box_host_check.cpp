@@ -1,6 +1,7 @@
-// Test-only: compiles the box-mass maths (kiwi_b200/csrc/box_math.cuh) for the host, so that tests/test_box_math.py
-// can check it against the float128 oracle without a GPU.
-#include "../kiwi_b200/csrc/box_grad.cuh"
+// Test-only: compiles the box-mass maths (kiwi_b200/csrc/box_math.cuh) for the host, and the face integrals
+// (cone_math.cuh) for the host, so that tests/test_box_math.py can check them against the float128 oracle without a
+// GPU.
+#include "../kiwi_b200/csrc/cone_math.cuh"
 
 using namespace kiwi_b200;
 
@@ -79,6 +80,37 @@ void bx_mass_grad(int kernel, int fixed, const double* offsets, double* out) {
     const KiwiBoxTable& T = kiwi_box_tables[kernel];
     if (fixed) box_mass_grad<2, 3>(T, offsets, out);
     else box_mass_grad<0, 0>(T, offsets, out);
+}
+// A face's integral for a particle with support H, and whether the kernel reaches the face: the quick answer (-1: none)
+// and face_reachable's.
+double bx_face(int kernel, const double* verts, int nv, const double* p, double H) {
+    const FlatVerts V{verts};
+    const KiwiConeTable& T = kiwi_cone_tables[kernel];
+    switch (kernel) {
+#define FACE(K, NP, DEG) \
+    case K: return cone_face<NP, DEG>(T, T.reg, V, nv, p[0], p[1], p[2], 1.0 / H);
+        KIWI_BOX_KERNELS(FACE)
+#undef FACE
+    }
+    return NAN;
+}
+int bx_reach(const double* verts, int nv, const double* p, double radius, int* exact) {
+    const FlatVerts V{verts};
+    *exact = face_reachable(p[0], p[1], p[2], radius, V, nv) ? 1 : 0;
+    return face_reach_fast(p[0], p[1], p[2], radius, face_plane(verts), verts, nv);
+}
+double bx_cone_coef_sum(int kernel) {
+    const KiwiConeTable& T = kiwi_cone_tables[kernel];
+    double s = 0.0;
+    for (int k = 0; k < T.npiece; ++k) {
+        for (double c : T.reg[k].V) s += fabs(c);
+        for (double c : T.reg[k].B) s += fabs(c);
+        for (double c : T.reg[k].a) s += fabs(c);
+        for (double c : T.scale[k].A) s += fabs(c);
+        for (double c : T.scale[k].fp) s += fabs(c);
+        for (double c : T.scale[k].ap) s += fabs(c);
+    }
+    return s;
 }
 // The sum of the absolute values of a kernel's coefficients, for error bounds.
 double bx_coef_sum(int kernel) {

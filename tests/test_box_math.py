@@ -96,3 +96,68 @@ def test_derivatives_against_differences(bx, kernel):
             for a in range(3):
                 d = [(mass(fixed, p + np.eye(3)[a] * s) - mass(fixed, p - np.eye(3)[a] * s)) / (2 * s) for s in (step, 2 * step)]
                 assert abs(got[1 + a] - (4 * d[0] - d[1]) / 3) <= bound
+
+
+def _polygon(rng, n, scale, squash=1.0):
+    """A convex planar polygon of n vertices in a random plane."""
+    a = np.sort(rng.uniform(0, 2 * np.pi, n))
+    q, _ = np.linalg.qr(rng.standard_normal((3, 3)))
+    return (np.stack([np.cos(a), squash * np.sin(a), 0 * a], 1) * scale) @ q.T + rng.standard_normal(3) * scale
+
+
+@pytest.mark.parametrize("kernel", range(6), ids=KERNELS)
+def test_faces_against_float128(bx, quad_oracle, kernel):
+    """Faces of 3 to 9 vertices, slivers among them, particles anywhere about them, near a vertex, near an edge line
+    and near the plane.  Bound: each of the face's cones carries at most 16 roundings of terms no larger than the
+    table's coefficients allow, two cones and an edge share per vertex."""
+    dp = C.POINTER(C.c_double)
+    bx.bx_face.restype, bx.bx_face.argtypes = C.c_double, [C.c_int, dp, C.c_int, dp, C.c_double]
+    bx.bx_cone_coef_sum.restype, bx.bx_cone_coef_sum.argtypes = C.c_double, [C.c_int]
+    rng = np.random.default_rng(17)
+    size = max(1.0, bx.bx_cone_coef_sum(kernel))
+    for i in range(160):
+        n = 3 + i % 7
+        v = np.ascontiguousarray(_polygon(rng, n, 0.3, 1.0 if i % 4 else 0.02))
+        H = rng.uniform(0.2, 1.5)
+        p = v.mean(0) + rng.standard_normal(3) * 0.5 * H
+        if i % 5 == 1:
+            p = v[0] + rng.standard_normal(3) * 1e-5
+        if i % 5 == 2:
+            p = 0.5 * (v[0] + v[1]) + rng.standard_normal(3) * 1e-4
+        if i % 5 == 3:
+            p = v.mean(0) + rng.standard_normal(3) * 1e-7
+        want = quad_oracle.face_integral(*p, v, kernel=-1 if kernel == 0 else kernel, h=H / SUPPORT[kernel],
+                                         support=H)[0]
+        got = bx.bx_face(kernel, v.ctypes.data_as(dp), n, p.ctypes.data_as(dp), H)
+        assert abs(got - want) <= 3 * n * 16 * EPS * size, (i, got, want)
+
+
+def test_quick_reach_agrees(bx):
+    """Where the quick test answers, it answers as the reference's rule does: over scales, slivers, repeated vertices,
+    distances about the radius (down to 1e-9 of it), particles in the plane and beside vertices; and it does
+    answer almost always where the distance has a margin."""
+    dp = C.POINTER(C.c_double)
+    bx.bx_reach.argtypes = [dp, C.c_int, dp, C.c_double, C.POINTER(C.c_int)]
+    rng = np.random.default_rng(23)
+    open_, far = 0, 0
+    for i in range(20_000):
+        scale = 10.0 ** rng.integers(-9, 4) if i % 3 == 0 else 0.3
+        n = 3 + i % 8
+        v = _polygon(rng, n, scale, (1.0, 0.05, 1e-6)[i % 17 % 3])
+        if i % 11 == 0:
+            v[n - 1] = v[n - 2]
+        v = np.ascontiguousarray(v)
+        p = v.mean(0) + rng.standard_normal(3) * scale * 10.0 ** rng.uniform(-6, 1)
+        if i % 7 == 0:
+            p = v[0] + rng.standard_normal(3) * scale * 10.0 ** rng.uniform(-9, -1)
+        radius = scale * rng.uniform(0.1, 4.0)
+        if i % 2:  # a radius at a chosen distance from the face's vertices or plane
+            d = np.linalg.norm(p - v[rng.integers(n)])
+            radius = d * (1 + rng.choice([-1, 1]) * 10.0 ** rng.uniform(-9, -1))
+        ex = C.c_int(0)
+        got = bx.bx_reach(v.ctypes.data_as(dp), n, np.ascontiguousarray(p).ctypes.data_as(dp), radius, C.byref(ex))
+        assert got in (-1, ex.value), (i, got, ex.value)
+        if i % 2 == 0 and i % 3 and i % 11:
+            far += 1
+            open_ += got < 0
+    assert open_ < 0.02 * far
