@@ -34,6 +34,7 @@
 #include "box_math.cuh"
 #include "engine.hpp"
 #include "lattice.cuh"
+#include "tabulated.cuh"
 
 namespace kiwi_b200 {
 
@@ -66,27 +67,32 @@ constexpr int kBoxPMax = 32;                                            // parti
 constexpr int kBoxPtCap = KIWI_BOX_PT_CAP;        // lattice points per chunk (a full 8^3 box has 729)
 constexpr int kBoxPairCap = KIWI_BOX_PAIR_CAP;    // edge lines per chunk (a full box has 243)
 constexpr int kBoxPlaneCap = KIWI_BOX_PLANE_CAP;  // planes per chunk (a full box has 27)
+// The tabulated integral's records (box_tab_*): a plane's offset, fraction and index on the table's r0 axis; an edge
+// line's fractions and indices on the mu0 and cos phi axes for either of its two distances.
+constexpr int kTabPlane = 3, kTabEdge = 6;
 // The three-piece kernels' records are larger: fewer lines and planes in the same shared memory.
 constexpr int kBoxGenPtCap = 1792, kBoxGenPairCap = 640, kBoxGenPlaneCap = 256;
 static_assert(kBoxPairCap <= 1024 && kBoxPlaneCap <= 512, "packed edge entries");
 
 // SEQ: the segments of a tile one after another, which needs the cells' totals beside the segment's sums.
-template <int NP, bool SEQ = false>
+// TAB (with NP 1): the tabulated integral's records.
+template <int NP, bool SEQ = false, bool TAB = false>
 struct BoxCaps {
     static constexpr int kN = NP ? NP : KIWI_BOX_PIECES;
-    static constexpr int kPt = SEQ ? 1536 : (NP == 1 ? 3072 : (NP == 2 ? kBoxPtCap : kBoxGenPtCap));
-    static constexpr int kPair = SEQ ? (NP ? 768 : 512) : (NP == 1 ? 1024 : (NP == 2 ? kBoxPairCap : kBoxGenPairCap));
-    static constexpr int kPlane = SEQ ? 208 : (NP == 1 ? 448 : (NP == 2 ? kBoxPlaneCap : kBoxGenPlaneCap));
+    static constexpr int kPS = TAB ? kTabPlane : box_plane_stride(kN), kES = TAB ? kTabEdge : box_edge_stride(kN);
+    static constexpr int kPt = TAB ? 2304 : SEQ ? 1536 : (NP == 1 ? 3072 : (NP == 2 ? kBoxPtCap : kBoxGenPtCap));
+    static constexpr int kPair = TAB ? 900 : SEQ ? (NP ? 768 : 512) : (NP == 1 ? 1024 : (NP == 2 ? kBoxPairCap : kBoxGenPairCap));
+    static constexpr int kPlane = TAB ? 296 : SEQ ? 208 : (NP == 1 ? 448 : (NP == 2 ? kBoxPlaneCap : kBoxGenPlaneCap));
     static constexpr int kQueues = kN;  // edge kinds; the point phase uses the first
     // dynamic shared memory, in doubles: the cells' sums, the octant values, the edge and plane records
     static constexpr int kOffT = 4 * kTileCells;
     static constexpr int kOffE = kOffT + kPt;
-    static constexpr int kOffP = kOffE + box_edge_stride(kN) * kPair;
-    static constexpr int kOffS = kOffP + box_plane_stride(kN) * kPlane;
+    static constexpr int kOffP = kOffE + kES * kPair;
+    static constexpr int kOffS = kOffP + kPS * kPlane;
     static constexpr int kEnd = kOffS + (SEQ ? 4 * kTileCells : 0);
     static constexpr size_t kSmem = sizeof(double) * kEnd + sizeof(uint32_t) * 64 * kBoxWarps * kQueues;
     // (C1) keeps the pairs' values in the edge records' place (with one piece the records are smaller)
-    static_assert((NP ? box_edge_stride(kN) : box_edge_stride(1)) * kPair >= kPt, "pair values fit");
+    static_assert((NP ? kES : box_edge_stride(1)) * kPair >= kPt, "pair values fit");
 };
 
 // One chunk of a tile's particle list: the particles' data, their boxes clipped to the tile (lo, dim), their
@@ -110,6 +116,70 @@ __device__ __forceinline__ void box_add_stat(unsigned long long* dst, unsigned l
 __device__ __forceinline__ double box_signed(double x, double a, double b, double c) {
     const int s = (__double2hiint(a) ^ __double2hiint(b) ^ __double2hiint(c)) & (int)0x80000000;
     return __hiloint2double(__double2hiint(x) ^ s, __double2loint(x));
+}
+
+// The tabulated integral (tab_gridded_c at (cos phi, R_0) = (a1 / r, a1) and (a2 / r, a2) in a wall, r the corner's
+// distance in it): a corner's two lookups in a wall need the wall's bin on the r0 axis and, of every
+// pair (p, q) of the point's distances, the bins of p / sqrt(p^2 + q^2) on the mu0 axis (as the wall's distance over
+// the edge line's) and on the cos phi axis (as the leg over the corner's distance in the wall).  Those are formed once
+// per plane and per edge line here, and a point has its lookups left: 6 x 8 table
+// entries.  Indices carry whether they were clamped (counted per lookup) and whether they fall in the axis's last
+// bin (the lookup is then 0).
+constexpr int kTabClamped = 1 << 30, kTabLast = 1 << 29, kTabIndex = (1 << 29) - 1;
+__device__ __forceinline__ void box_tab_plane(const TabDev& t, const TabWidths& W, double u, double ih, double* rec) {
+    rec[0] = u;
+    if (u == 0.0) return;
+    double r0 = fabs(u) * ih, fx;
+    if (r0 > 2.0) r0 = 2.0;  // beyond 2h the pyramid mass depends on the angles alone
+    unsigned clamped = 0;
+    const int i = tab_index_fr(W, 0, r0, t.rl, t.nr01, t.nr0, fx, clamped);
+    rec[1] = fx;
+    rec[2] = __hiloint2double(0, i | (clamped ? kTabClamped : 0));
+}
+// One of the line's distances p against the other q: rec[0] the fraction on mu0, rec[1] on cos phi, rec[2] both
+// indices (mu0 in the low word, cos phi in the high word).
+__device__ __forceinline__ void box_tab_edge(const TabDev& t, const TabWidths& W, double p, double s, double is, double* rec) {
+    unsigned cj = 0, ck = 0;
+    double fy, fz;
+    const int j = tab_index_fr(W, 1, p / s, t.mul, t.nR_01 - 1, t.nR_0 - 1, fy, cj);
+    const int k = tab_index_fr(W, 2, p * is, t.cphil, t.nphi1 - 1, t.nphi - 1, fz, ck);
+    rec[0] = fy;
+    rec[1] = fz;
+    rec[2] = __hiloint2double(k | (ck ? kTabClamped : 0) | (k == t.nphi1 + t.nphi2 - 1 ? kTabLast : 0),
+                              j | (cj ? kTabClamped : 0) | (j == t.nR_01 + t.nR_02 - 1 ? kTabLast : 0));
+}
+// 32 bytes (aligned) in one load.  Not kept in L1: a scattered 32-byte read would hold a 128-byte line there, and those
+// lines were what bounded the reads in flight (17.8 -> 16.0 ms on 200 k particles, 120 x 125 x 130).
+__device__ __forceinline__ double4 box_tab_load(const double* p) {
+    double4 r;
+    asm("ld.global.nc.L1::no_allocate.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w) : "l"(p));
+    return r;
+}
+// One lookup: the wall's record, the mu0 side of one record and the cos phi side of another.
+__device__ __forceinline__ double box_tab_lookup(const TabDev& t, const double* wall, const double* mu, const double* phi,
+                                                 unsigned& nclamp) {
+    const int i = __double2loint(wall[2]) & kTabIndex, jw = __double2loint(mu[2]), kw = __double2hiint(phi[2]);
+    nclamp += ((jw & kTabClamped) != 0) + ((kw & kTabClamped) != 0);
+    if ((jw | kw) & kTabLast) return 0.0;
+    const int j = jw & kTabIndex, k = kw & kTabIndex;
+    const double fx = wall[1], fy = mu[0], fz = phi[1];
+    double4 a, b;  // rows j and j + 1: (i, k), (i + 1, k), (i, k + 1), (i + 1, k + 1)
+    const size_t at = ((size_t)i * (t.nR_0 + 1) + j) * (t.nphi + 1) + k;
+    if (t.v4) {
+        a = box_tab_load(t.v4 + 4 * at);
+        b = box_tab_load(t.v4 + 4 * (at + t.nphi + 1));
+    } else {
+        a = double4{tab_at(t, i, j, k), tab_at(t, i + 1, j, k), tab_at(t, i, j, k + 1), tab_at(t, i + 1, j, k + 1)};
+        b = double4{tab_at(t, i, j + 1, k), tab_at(t, i + 1, j + 1, k), tab_at(t, i, j + 1, k + 1),
+                    tab_at(t, i + 1, j + 1, k + 1)};
+    }
+    const double x00 = fx * a.y + (1 - fx) * a.x;
+    const double x10 = fx * b.y + (1 - fx) * b.x;
+    const double x01 = fx * a.w + (1 - fx) * a.z;
+    const double x11 = fx * b.w + (1 - fx) * b.z;
+    const double y0 = fy * x10 + (1 - fy) * x00;
+    const double y1 = fy * x11 + (1 - fy) * x01;
+    return fz * y1 + (1 - fz) * y0;
 }
 
 // A cell's outputs from its sums (src/cartesian_grid.cpp:294-317).
@@ -152,19 +222,24 @@ __device__ __forceinline__ void box_combine(const CartGeom& g, const CartOutputs
 // segments of `segment` entries, one after another.
 // NP, DEG: the kernel's pieces and largest power, known when compiling (the cubic spline: 2, 3), or 0 for any
 // kernel of the tables.  T: the kernel's table in constant memory.
-template <bool CULL, int NP, int DEG, bool SEQ = false>
+// TAB: the tabulated cubic integral, lookups in tab (NP 1, DEG 0, without CULL: outside the support the lookups do not
+// cancel exactly, and the reference keeps what they leave).
+template <bool CULL, int NP, int DEG, bool SEQ = false, bool TAB = false>
 __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& P, const uint32_t* __restrict__ list,
                                          int64_t beg, int64_t end_all, int64_t segment, int64_t t,
                                          const CartOutputs& out, double* __restrict__ sums, DevStats* __restrict__ st,
-                                         const KiwiBoxTable& T) {
-    using Caps = BoxCaps<NP, SEQ>;
+                                         const KiwiBoxTable& T, const TabDev tab = TabDev{}) {
+    using Caps = BoxCaps<NP, SEQ, TAB>;
+    static_assert(!TAB || !CULL, "the tabulated integral takes every cell of a box");
+    __shared__ TabWidths s_tw;
+    if (TAB && threadIdx.x == 0) s_tw = tab_widths(tab);
     __shared__ BoxChunk s_cp[2];
     __shared__ double s_pl[3][kTileX + 1], s_cc[3][kTileX];
-    __shared__ double s_C[NP == 2 ? 1 : (kBoxC + 1) * Caps::kN];  // any kernel: c and C of its pieces (lanes differ in piece)
+    __shared__ double s_C[NP == 2 || TAB ? 1 : (kBoxC + 1) * Caps::kN];  // any kernel: c and C of its pieces (lanes differ in piece)
     static_assert(kTileX == kTileY && kTileX == kTileZ, "cubic tiles");
     extern __shared__ double s_dyn[];
     const int n = NP ? NP : T.npiece;
-    const int kPS = box_plane_stride(n), kES = box_edge_stride(n);
+    const int kPS = TAB ? kTabPlane : box_plane_stride(n), kES = TAB ? kTabEdge : box_edge_stride(n);
     double* const s_acc = s_dyn;
     double* const s_T = s_dyn + Caps::kOffT;
     double* const s_E = s_dyn + Caps::kOffE;
@@ -183,7 +258,7 @@ __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& 
         s_pl[a][l] = add_rn(mn, mul_rn((double)(b0 + l), d));
         if (l < kTileX) s_cc[a][l] = cell_centre(mn, b0 + l, d);
     }
-    if (NP != 2)
+    if (NP != 2 && !TAB)
         for (int i = threadIdx.x; i < (kBoxC + 1) * n; i += kBoxThreads) {
             const int k = i / (kBoxC + 1), c = i % (kBoxC + 1);
             s_C[i] = c < kBoxC ? T.reg[k].C[c] : T.reg[k].c;
@@ -192,7 +267,7 @@ __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& 
 
     // work counters: 32-bit per thread, flushed to the 64-bit totals every 2^16 chunks and at the end
     unsigned n_bbox = 0, n_sphere = 0, n_eval = 0, n_neg = 0, n_warn = 0, n_eo = 0, n_em = 0, n_ei = 0, n_vp = 0,
-             n_chunks = 0;
+             n_clamp = 0, n_chunks = 0;
     auto flush = [&]() {
         box_add_stat(&st->bbox_pairs, n_bbox);
         box_add_stat(&st->sphere_pairs, n_sphere);
@@ -203,7 +278,8 @@ __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& 
         box_add_stat(&st->edge_middle, n_em);
         box_add_stat(&st->edge_inner, n_ei);
         box_add_stat(&st->vertex_pyramids, n_vp);
-        n_bbox = n_sphere = n_eval = n_neg = n_warn = n_eo = n_em = n_ei = n_vp = 0;
+        if (TAB) box_add_stat(&st->table_clamps, n_clamp);
+        n_bbox = n_sphere = n_eval = n_neg = n_warn = n_eo = n_em = n_ei = n_vp = n_clamp = 0;
     };
     // the end of the segment at hand (a chunk never crosses it)
     auto segment_end = [&](int64_t at) { return SEQ ? min(at + segment, end_all) : end_all; };
@@ -246,7 +322,7 @@ __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& 
         const int np = __popc(__ballot_sync(0xffffffffu, take));
         if (take) {
             const double H = mul_rn(g.support_in_h, ph);
-            dst->x[lane] = px; dst->y[lane] = py; dst->z[lane] = pz; dst->H[lane] = H; dst->iH[lane] = 1.0 / H;
+            dst->x[lane] = px; dst->y[lane] = py; dst->z[lane] = pz; dst->H[lane] = H; dst->iH[lane] = 1.0 / (TAB ? ph : H);
             dst->m[lane] = pm; dst->vx[lane] = pvx; dst->vy[lane] = pvy; dst->vz[lane] = pvz;
             dst->lo[lane][0] = lo0; dst->lo[lane][1] = lo1; dst->lo[lane][2] = lo2;
             dst->dim[lane][0] = d0; dst->dim[lane][1] = d1; dst->dim[lane][2] = d2;
@@ -280,7 +356,9 @@ __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& 
                 const int a = (l >= n0) + (l >= n0 + n1);
                 l -= a == 0 ? 0 : (a == 1 ? n0 : n0 + n1);
                 const double c = a == 0 ? cp->x[j] : (a == 1 ? cp->y[j] : cp->z[j]);
-                box_plane<NP, DEG>(T, (s_pl[a][cp->lo[j][a] + l] - c) * cp->iH[j], s_P + kPS * it);
+                const double u = s_pl[a][cp->lo[j][a] + l] - c;
+                if constexpr (TAB) box_tab_plane(tab, s_tw, u, cp->iH[j], s_P + kPS * it);
+                else box_plane<NP, DEG>(T, u * cp->iH[j], s_P + kPS * it);
             }
         }
     };
@@ -301,7 +379,32 @@ __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& 
         if (warp == 0 && more) load_chunk(nx, pos + np, end);
 
         // (E) edge lines, block (x, y) over n0' x n1', (x, z) over n0' x n2', (y, z) over n1' x n2'
-        {
+        auto line_planes = [&](int j, int e, int& la, int& lb) {  // the planes of particle j's line e
+            const int n0 = cp->dim[j][0] + 1, n1 = cp->dim[j][1] + 1, n2 = cp->dim[j][2] + 1;
+            const int nxy = n0 * n1, nxz = n0 * n2;
+            const int blk = (e >= nxy) + (e >= nxy + nxz);
+            e -= blk == 0 ? 0 : (blk == 1 ? nxy : nxy + nxz);
+            const int pi = div_by(e, cp->mag[j][blk == 0 ? 0 : 1]), qi = e - pi * (blk == 0 ? n1 : n2);
+            la = cp->loff[j] + (blk == 2 ? n0 : 0) + pi;
+            lb = cp->loff[j] + (blk == 0 ? n0 : n0 + n1) + qi;
+        };
+        if constexpr (TAB) {
+            const int off_l = lane < np ? cp->eoff[lane] : INT_MAX;
+            for (int base = warp * 32; base < cp->etot; base += kBoxThreads) {
+                const int j = warp_owner(base, off_l, lane), it = base + lane;
+                const int off = __shfl_sync(0xffffffffu, off_l, j & 31);
+                if (it < cp->etot) {
+                    int la, lb;
+                    line_planes(j, it - off, la, lb);
+                    const double p = fabs(s_P[kPS * la]), q = fabs(s_P[kPS * lb]);
+                    if (p != 0.0 && q != 0.0) {
+                        const double s = sqrt(p * p + q * q), is = 1.0 / s;
+                        box_tab_edge(tab, s_tw, p, s, is, s_E + kES * it);
+                        box_tab_edge(tab, s_tw, q, s, is, s_E + kES * it + 3);
+                    }
+                }
+            }
+        } else {
             const int tot = cp->etot;
             const int off_l = lane < np ? cp->eoff[lane] : INT_MAX;
             int cnt[Caps::kQueues];
@@ -315,14 +418,8 @@ __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& 
                     int kind = -1;
                     uint32_t rec = 0;
                     if (it < tot) {
-                        int e = it - off;
-                        const int n0 = cp->dim[j][0] + 1, n1 = cp->dim[j][1] + 1, n2 = cp->dim[j][2] + 1;
-                        const int nxy = n0 * n1, nxz = n0 * n2;
-                        const int blk = (e >= nxy) + (e >= nxy + nxz);
-                        e -= blk == 0 ? 0 : (blk == 1 ? nxy : nxy + nxz);
-                        const int pi = div_by(e, cp->mag[j][blk == 0 ? 0 : 1]), qi = e - pi * (blk == 0 ? n1 : n2);
-                        const int la = cp->loff[j] + (blk == 2 ? n0 : 0) + pi;
-                        const int lb = cp->loff[j] + (blk == 0 ? n0 : n0 + n1) + qi;
+                        int la, lb;
+                        line_planes(j, it - off, la, lb);
                         const double p = s_P[kPS * la], q = s_P[kPS * lb];
                         const double D = fma(p, p, q * q);
                         if (D >= 1.0 || p == 0.0 || q == 0.0) {
@@ -365,7 +462,38 @@ __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& 
         __syncthreads();
 
         // (P) lattice points
-        {
+        if constexpr (TAB) {
+            const int off_l = lane < np ? cp->poff[lane] : INT_MAX;
+            for (int base = warp * 32; base < cp->ptot; base += kBoxThreads) {
+                const int j = warp_owner(base, off_l, lane), it = base + lane;
+                const int off = __shfl_sync(0xffffffffu, off_l, j & 31);
+                if (it < cp->ptot) {
+                    const int lp = it - off;
+                    const int n0 = cp->dim[j][0] + 1, n1 = cp->dim[j][1] + 1, n2 = cp->dim[j][2] + 1;
+                    const int i = div_by(lp, cp->mag[j][2]), rem = lp - i * (n1 * n2);
+                    const int jj = div_by(rem, cp->mag[j][1]), k = rem - jj * n2;
+                    const double* const rx = s_P + kPS * (cp->loff[j] + i);
+                    const double* const ry = s_P + kPS * (cp->loff[j] + n0 + jj);
+                    const double* const rz = s_P + kPS * (cp->loff[j] + n0 + n1 + k);
+                    if (rx[0] == 0.0 || ry[0] == 0.0 || rz[0] == 0.0) {
+                        s_T[it] = 0.0;
+                    } else {
+                        // a line's first three entries are of its first axis's distance, the others of its second's
+                        const double* const E = s_E + kES * cp->eoff[j];
+                        const double* const xy = E + kES * (i * n1 + jj);
+                        const double* const xz = E + kES * (n0 * n1 + i * n2 + k);
+                        const double* const yz = E + kES * (n0 * (n1 + n2) + jj * n2 + k);
+                        double f = box_tab_lookup(tab, rx, xy, yz, n_clamp) + box_tab_lookup(tab, rx, xz, yz + 3, n_clamp);
+                        f = f + (box_tab_lookup(tab, ry, xy + 3, xz, n_clamp) + box_tab_lookup(tab, ry, yz, xz + 3, n_clamp));
+                        f = f + (box_tab_lookup(tab, rz, xz + 3, xy, n_clamp) + box_tab_lookup(tab, rz, yz + 3, xy + 3, n_clamp));
+                        n_clamp += ((__double2loint(rx[2]) & kTabClamped) != 0) + ((__double2loint(ry[2]) & kTabClamped) != 0) +
+                                   ((__double2loint(rz[2]) & kTabClamped) != 0);
+                        s_T[it] = box_signed(f, rx[0], ry[0], rz[0]);
+                        n_vp += 6;
+                    }
+                }
+            }
+        } else {
             const int tot = cp->ptot;
             const int off_l = lane < np ? cp->poff[lane] : INT_MAX;
             int cnt = 0;
@@ -566,6 +694,19 @@ __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& 
         }
     }
     flush();
+}
+
+// Runs one item; range: the tile's list.
+template <bool CULL, int NP, int DEG, bool TAB = false>
+__device__ __forceinline__ void box_item(const BoxItem& it, const CartGeom& g, const DevParticles& P,
+                                         const uint32_t* __restrict__ list, const int64_t* __restrict__ range,
+                                         int64_t t, const CartOutputs& out, double* __restrict__ sums,
+                                         DevStats* __restrict__ st, const KiwiBoxTable& T, const TabDev tab = TabDev{}) {
+    const int64_t lo = range[0], hi = range[1];
+    const int64_t len = box_segment(hi - lo, (int64_t)g.ntx * g.nty * g.ntz);
+    const int64_t beg = lo + it.seg * len, end = it.nseg > 1 ? min(beg + len, hi) : hi;
+    box_tile<CULL, NP, DEG, false, TAB>(g, P, list, beg, end, 0, t, out,
+                            it.nseg > 1 ? sums + (int64_t)(it.slot + it.seg) * 4 * kTileCells : nullptr, st, T, tab);
 }
 
 }  // namespace kiwi_b200

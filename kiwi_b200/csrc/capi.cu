@@ -112,6 +112,7 @@ int sph_to_grid_dev(KiwiCtx* ctx, const DevParticles& P, const CartGeom& g, cons
         if ((precision & KIWI_FORM_MASK) == KIWI_FP32_MIXED)
             return set_err(ctx, KIWI_ERR_UNSUPPORTED, "the FP32-mixed form is available for the analytic integral only");
         KIWI_TRY(table_ensure(ctx, &kc.tab));
+        if ((precision & KIWI_FORM_MASK) == KIWI_FP64) KIWI_TRY(table_blocks(ctx, &kc.tab));
     }
     const int64_t launches0 = ctx->launches;
     DevStats* d_stats = nullptr;
@@ -164,8 +165,8 @@ int sph_to_grid_dev(KiwiCtx* ctx, const DevParticles& P, const CartGeom& g, cons
         KIWI_LAUNCHED(ctx);
     }
     TileLists tl{sorted_vals, range, ntiles, total};
-    // the FP64 form orders its own work (lattice_cart_gather)
-    const bool own_order = (precision & KIWI_FORM_MASK) == KIWI_FP64 && !kc.tabulated && (kc.cubic || !(precision & KIWI_FULL_BOX));
+    // the FP64 form orders its own work (box_work_make)
+    const bool own_order = (precision & KIWI_FORM_MASK) == KIWI_FP64 && (kc.cubic || !(precision & KIWI_FULL_BOX));
     if (n_parts > 1) {
         // this part's tiles: a contiguous run of the tile order holding ~1/n_parts of the entries
         uint32_t *w = nullptr, *flags = nullptr;

@@ -14,6 +14,7 @@ namespace kiwi_b200 {
 // the sub-grid sizes and split points of its three axes and the values, laid out as the reference does.
 struct TabDev {
     const double* v = nullptr;
+    const double* v4 = nullptr;  // the table in blocks of four neighbours (table_blocks), or null
     int nr01 = 0, nR_01 = 0, nphi1 = 0, nr02 = 0, nR_02 = 0, nphi2 = 0, nr0 = 0, nR_0 = 0, nphi = 0;
     double rl = 0.0, mul = 0.0, cphil = 0.0;
 };

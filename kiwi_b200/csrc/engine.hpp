@@ -29,6 +29,9 @@ struct KernelChoice {
 
 // tabulated.cu: the context's density table, generating the canonical one if it holds none.
 int table_ensure(KiwiCtx* ctx, TabDev* out);
+// The same with the table also in blocks of four neighbours (four times its memory, 730 MB for the canonical shape,
+// released with it), unless that is over 4 GB or cannot be had.
+int table_blocks(KiwiCtx* ctx, TabDev* out);
 void table_free(KiwiCtx* ctx);
 
 // Tile lists built by the binning step: tile t owns list[range[2t] .. range[2t+1]) (particle indices in
@@ -134,6 +137,22 @@ int fp64_measure_peak(KiwiCtx* ctx, double* tflops);
 // lattice.cu: the lattice-factorised gather of the plain FP64 form for the cubic spline (every cell of the
 // support boxes with full_box, else the cells the supports reach) and the generic kernels (the cells the
 // supports reach), and the batch's persistent launches of those two families.
+// One piece of work: segment `seg` of the `nseg` of tile `tile`; its sums go to the partial sums' place slot + seg if
+// nseg > 1.
+struct BoxItem {
+    int32_t tile, seg, nseg, slot;
+};
+// The work of a box-mass gather over a call's tiles: items (heaviest first), or none when the tiles run as they are;
+// the places of the cut tiles' sums and the cut tiles, whose outputs box_work_finish forms.
+struct BoxWork {
+    const BoxItem* items = nullptr;
+    int64_t n = 0;
+    const BoxItem* cut = nullptr;
+    int64_t n_cut = 0;
+    double* sums = nullptr;
+};
+int box_work_make(KiwiCtx* ctx, const TileLists& tl, BoxWork* w);
+int box_work_finish(KiwiCtx* ctx, const CartGeom& g, const BoxWork& w, const CartOutputs& out);
 int lattice_init_tables(KiwiCtx* ctx);
 int adjoint_init_tables(KiwiCtx* ctx);
 int lattice_cart_gather(KiwiCtx* ctx, const CartGeom& g, const DevParticles& P, const KernelChoice& k,

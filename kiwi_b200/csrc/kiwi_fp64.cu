@@ -22,7 +22,10 @@ int fp64_init_tables(KiwiCtx* ctx) {
 
 }  // namespace kiwi_b200
 
-#include "lattice_tile.cuh"
+// The tabulated kernel waits on memory: more threads with fewer registers (200 k particles on 120 x 125 x 130: 256
+// threads, 3 CTAs per SM 13.7 ms, 384 and 2 CTAs 12.9 ms, 512 and 2 CTAs 13.6 ms).
+#define KIWI_BOX_THREADS 384
+#include "box_tile.cuh"
 
 namespace kiwi_b200 {
 
@@ -299,25 +302,20 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_cart_gather_tab(CartGe
 
 // ------------------------------------------------------------------ lattice form, tabulated integral
 
-// Resident CTAs per SM the register budget of the tabulated lattice kernel is sized for (its 30 KB of
-// shared memory fits more; four was slower).
-#ifndef KIWI_LATTICE_TAB_MIN_BLOCKS
-#define KIWI_LATTICE_TAB_MIN_BLOCKS 3
-#endif
-constexpr int kLatTabMinBlocks = KIWI_LATTICE_TAB_MIN_BLOCKS;
-
-// The lattice form with the tabulated integral, every cell of the particles' bounding boxes (outside the
-// support the lookups do not cancel exactly, and the reference keeps what they leave).  Built here, without
-// FMA contraction, so that every lookup lands on the reference's table entries with its weights.
-__global__ void __launch_bounds__(kLatThreads, kLatTabMinBlocks) k_cart_lattice_tab(CartGeom g, DevParticles P,
-                                                                                 const TabDev tab,
-                                                                                 const uint32_t* __restrict__ list,
-                                                                                 const int64_t* __restrict__ range,
-                                                                                 const int32_t* __restrict__ tile_map,
-                                                                                 CartOutputs out,
-                                                                                 DevStats* __restrict__ st) {
-    const int64_t t = tile_map ? (int64_t)tile_map[blockIdx.x] : (int64_t)blockIdx.x;
-    lattice_tile<false, false, true>(g, P, list, range, t, t, out, st, nullptr, tab);
+// The tabulated integral over every cell of the particles' bounding boxes, work items as the FP64 form's.  Built
+// here, without FMA contraction, so that every lookup lands on the reference's table entries with its weights.
+// Bound by the lookups' table reads: scattered 32-byte blocks (12 per point), about half of them from DRAM.  With the
+// indices formed per point and eight 8-byte reads per lookup, L1 was bound by its wavefronts at 21.9 ms; now 12.9.
+__global__ void __launch_bounds__(kBoxThreads, 2) k_cart_box_tab(CartGeom g, DevParticles P, const TabDev tab,
+                                                                 const uint32_t* __restrict__ list,
+                                                                 const int64_t* __restrict__ range,
+                                                                 const int32_t* __restrict__ tile_map,
+                                                                 const BoxItem* __restrict__ items, CartOutputs out,
+                                                                 double* __restrict__ sums, DevStats* __restrict__ st) {
+    BoxItem it{tile_map ? tile_map[blockIdx.x] : (int)blockIdx.x, 0, 1, 0};
+    if (items) it = items[blockIdx.x];
+    __shared__ KiwiBoxTable s_none;  // (unused: the tabulated body has no polynomial tables)
+    box_item<false, 1, 0, true>(it, g, P, list, range + 2 * (int64_t)it.tile, it.tile, out, sums, st, s_none, tab);
 }
 
 // The tiles of a batch of grids whose items take the per-cell gather (the lattice families run in
@@ -502,10 +500,14 @@ int fp64_cart_gather(KiwiCtx* ctx, const CartGeom& g, const DevParticles& P, con
     if (tl.map && tl.nmap <= 0) return KIWI_OK;
     const dim3 grid((unsigned)(tl.map ? tl.nmap : tl.ntiles));
     if (k.tabulated && !reference_order) {
-        KIWI_CUDA(ctx, cudaFuncSetAttribute(k_cart_lattice_tab, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)kLatTabDynSmem));
-        k_cart_lattice_tab<<<grid, kLatThreads, kLatTabDynSmem, ctx->stream>>>(g, P, k.tab, tl.list, tl.range, tl.map,
-                                                                               out, d_stats);
+        constexpr size_t smem = BoxCaps<1, false, true>::kSmem;
+        KIWI_CUDA(ctx, cudaFuncSetAttribute(k_cart_box_tab, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        BoxWork w;
+        KIWI_TRY(box_work_make(ctx, tl, &w));
+        k_cart_box_tab<<<(unsigned)w.n, kBoxThreads, smem, ctx->stream>>>(g, P, k.tab, tl.list, tl.range, tl.map, w.items,
+                                                                          out, w.sums, d_stats);
+        KIWI_LAUNCHED(ctx);
+        return box_work_finish(ctx, g, w, out);
     } else if (k.tabulated) {
         k_cart_gather_tab<<<grid, kThreads, 0, ctx->stream>>>(g, P, k.tab, tl.list, tl.range, tl.map, out, d_stats);
     } else if (!reference_order && (k.cubic || !full_box)) {

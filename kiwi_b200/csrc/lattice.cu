@@ -1,8 +1,7 @@
-// The lattice-factorised gather of the plain FP64 form (cubic spline closed form and table-driven generic
-// kernels) and the batch's persistent kernel for those two families.  This translation unit is built with
-// FMA contraction: the lattice form regroups the reference's sum (lattice_tile.cuh) and evaluates its tiers
-// in the triangles' own lengths (lattice_math.cuh), so it does not follow the reference's operation order
-// and gains nothing from rounding each product on its own; the quantities that integer results depend on
+// The box-mass gather of the plain FP64 form (box_tile.cuh), the lattice gather of the FP32-mixed form
+// (lattice_tile.cuh), and the batch's persistent kernels for both.  This translation unit is built with
+// FMA contraction: both regroup the reference's sum, so they do not follow its operation order
+// and gain nothing from rounding each product on its own; the quantities that integer results depend on
 // (bounding boxes, lattice planes, cell centres, the support test of the pair counters) are formed with
 // explicitly rounded operations (cart_common.cuh), as in every other form.
 #include <cuda_runtime.h>
@@ -51,26 +50,6 @@ constexpr size_t kLatMergedDynSmem = kLatDynSmem > kLatGenDynSmem ? kLatDynSmem 
 #define KIWI_BOX_MIN_BLOCKS 2
 #endif
 constexpr int kBoxMinBlocks = KIWI_BOX_MIN_BLOCKS;
-
-// One piece of work: segment `seg` of the `nseg` of tile `tile`; its sums go to the partial sums' place slot + seg if
-// nseg > 1.
-struct BoxItem {
-    int32_t tile, seg, nseg, slot;
-};
-static_assert(sizeof(BoxItem) == sizeof(int4), "items are read as one int4");
-
-// Runs one item; range: the tile's list.
-template <bool CULL, int NP, int DEG>
-__device__ __forceinline__ void box_item(const BoxItem& it, const CartGeom& g, const DevParticles& P,
-                                         const uint32_t* __restrict__ list, const int64_t* __restrict__ range,
-                                         int64_t t, const CartOutputs& out, double* __restrict__ sums,
-                                         DevStats* __restrict__ st, const KiwiBoxTable& T) {
-    const int64_t lo = range[0], hi = range[1];
-    const int64_t len = box_segment(hi - lo, (int64_t)g.ntx * g.nty * g.ntz);
-    const int64_t beg = lo + it.seg * len, end = it.nseg > 1 ? min(beg + len, hi) : hi;
-    box_tile<CULL, NP, DEG>(g, P, list, beg, end, 0, t, out,
-                            it.nseg > 1 ? sums + (int64_t)(it.slot + it.seg) * 4 * kTileCells : nullptr, st, T);
-}
 
 // Kernel KERNEL of the tables (NP pieces, powers to DEG; KERNEL < 0: any, `kernel`, with both 0), over items, or
 // without them over the tiles tile_map[0 ..) (every tile if null), each tile by one CTA: SEQ cuts it into its
@@ -171,7 +150,7 @@ __global__ void __launch_bounds__(kLatThreads, kLatMinBlocks) k_cart_lattice_mix
                                                                                 CartOutputs out,
                                                                                 DevStats* __restrict__ st) {
     const int64_t t = tile_map ? (int64_t)tile_map[blockIdx.x] : (int64_t)blockIdx.x;
-    lattice_tile<true, false, false, true>(g, P, list, range, t, t, out, st);
+    lattice_tile<false>(g, P, list, range, t, t, out, st);
 }
 
 // The FP32-mixed form of the generic lattice kernel: edge records and vertex tiers in FP32 (FP64 islands
@@ -181,7 +160,7 @@ __global__ void __launch_bounds__(kLatThreads, kLatGenMinBlocks)
                                  const int64_t* __restrict__ range, const int32_t* __restrict__ tile_map,
                                  CartOutputs out, DevStats* __restrict__ st) {
     const int64_t t = tile_map ? (int64_t)tile_map[blockIdx.x] : (int64_t)blockIdx.x;
-    lattice_tile<true, true, false, true>(g, P, list, range, t, t, out, st, &c_tables[kernel]);
+    lattice_tile<true>(g, P, list, range, t, t, out, st, &c_tables[kernel]);
 }
 
 // The work of a batch's grids with one kernel (FP64 form), or one lattice family's (FP32-mixed form: whole tiles), in
@@ -226,9 +205,9 @@ __global__ void __launch_bounds__(kLatThreads, 2)
         const BatchItemDev& it = items[item_of_tile[tg]];
         const int64_t tl = tg - it.tile_base;
         if (FAMILY == kBatchFamilyMixed || (FAMILY == kBatchFamilyMixedMerged && it.mode == kBatchLattice))
-            lattice_tile<true, false, false, true>(it.g, it.P, list, range, tg, tl, it.out, it.st);
+            lattice_tile<false>(it.g, it.P, list, range, tg, tl, it.out, it.st);
         else
-            lattice_tile<true, true, false, true>(it.g, it.P, list, range, tg, tl, it.out, it.st, &c_tables[it.kernel]);
+            lattice_tile<true>(it.g, it.P, list, range, tg, tl, it.out, it.st, &c_tables[it.kernel]);
         __syncthreads();
     }
 }
@@ -278,14 +257,12 @@ static int box_launch_kernel(KiwiCtx* ctx, int64_t blocks, const CartGeom& g, co
     }
 }
 
-int lattice_cart_gather(KiwiCtx* ctx, const CartGeom& g, const DevParticles& P, const KernelChoice& k,
-                        const TileLists& tl, const CartOutputs& out, DevStats* d_stats, bool full_box) {
+int box_work_make(KiwiCtx* ctx, const TileLists& tl, BoxWork* w) {
     const int64_t n = tl.map ? tl.nmap : tl.ntiles;
-    // without scratch of its own (the allocation-free call), one CTA per tile cuts it
-    if (ctx->arena) return box_launch_kernel<true>(ctx, n, g, P, k, tl, nullptr, out, nullptr, d_stats, full_box);
+    *w = BoxWork{};
+    w->n = n;
     // no list can be longer than a segment: the tiles as they are
-    const int64_t least = box_segment(0, tl.ntiles);
-    if (tl.total <= least) return box_launch_kernel<false>(ctx, n, g, P, k, tl, nullptr, out, nullptr, d_stats, full_box);
+    if (tl.total <= box_segment(0, tl.ntiles)) return KIWI_OK;
     constexpr int kCounts = 4 + 2 * kBoxClasses + 2;
     int* counts = nullptr;
     KIWI_TRY(scratch_t(ctx, S_BOX_COUNTS, kCounts, &counts));
@@ -297,18 +274,35 @@ int lattice_cart_gather(KiwiCtx* ctx, const CartGeom& g, const DevParticles& P, 
     KIWI_CUDA(ctx, cudaMemcpyAsync(h, counts, sizeof h, cudaMemcpyDeviceToHost, ctx->stream));
     KIWI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     BoxItem *items = nullptr, *cut = nullptr;
-    double* sums = nullptr;
     KIWI_TRY(scratch_t(ctx, S_BOX_ITEMS, (size_t)h[0], &items));
     KIWI_TRY(scratch_t(ctx, S_BOX_CUT, (size_t)(h[2] > 0 ? h[2] : 1), &cut));
-    if (h[1] > 0) KIWI_TRY(scratch_t(ctx, S_BOX_SUMS, (size_t)h[1] * 4 * kTileCells, &sums));
+    if (h[1] > 0) KIWI_TRY(scratch_t(ctx, S_BOX_SUMS, (size_t)h[1] * 4 * kTileCells, &w->sums));
     k_box_items<true><<<nb, 256, 0, ctx->stream>>>(tl.range, tl.ntiles, tl.map, n, counts, items, cut);
     KIWI_LAUNCHED(ctx);
-    KIWI_TRY(box_launch_kernel<false>(ctx, h[0], g, P, k, tl, items, out, sums, d_stats, full_box));
-    if (h[2] > 0) {
-        k_box_combine<<<(unsigned)h[2], 256, 0, ctx->stream>>>(g, cut, sums, out);
-        KIWI_LAUNCHED(ctx);
-    }
+    w->items = items;
+    w->n = h[0];
+    w->cut = cut;
+    w->n_cut = h[2];
     return KIWI_OK;
+}
+
+int box_work_finish(KiwiCtx* ctx, const CartGeom& g, const BoxWork& w, const CartOutputs& out) {
+    if (w.n_cut <= 0) return KIWI_OK;
+    k_box_combine<<<(unsigned)w.n_cut, 256, 0, ctx->stream>>>(g, w.cut, w.sums, out);
+    KIWI_LAUNCHED(ctx);
+    return KIWI_OK;
+}
+
+int lattice_cart_gather(KiwiCtx* ctx, const CartGeom& g, const DevParticles& P, const KernelChoice& k,
+                        const TileLists& tl, const CartOutputs& out, DevStats* d_stats, bool full_box) {
+    // without scratch of its own (the allocation-free call), one CTA per tile cuts it
+    if (ctx->arena)
+        return box_launch_kernel<true>(ctx, tl.map ? tl.nmap : tl.ntiles, g, P, k, tl, nullptr, out, nullptr, d_stats,
+                                       full_box);
+    BoxWork w;
+    KIWI_TRY(box_work_make(ctx, tl, &w));
+    KIWI_TRY(box_launch_kernel<false>(ctx, w.n, g, P, k, tl, w.items, out, w.sums, d_stats, full_box));
+    return box_work_finish(ctx, g, w, out);
 }
 
 // The work of a batch's tiles tiles[0 .. n) with their ranges (host): natural order, or heaviest segment first.

@@ -1,5 +1,5 @@
-// The tile body of the lattice-factorised gather (one CTA = one 8 x 8 x 8 cell tile), shared by the
-// single-grid kernels and the batch's persistent kernel.  A translation unit that includes this defines
+// The tile body of the FP32-mixed form's lattice-factorised gather (one CTA = one 8 x 8 x 8 cell tile), shared by
+// the single-grid kernels and the batch's persistent kernel.  A translation unit that includes this defines
 // `c_tables` (its __constant__ copy of the kernel tables) first.
 //
 // Per particle of the tile's list, the box of its support clipped to the tile (n0 x n1 x n2 cells) has
@@ -19,7 +19,6 @@
 #include "engine.hpp"
 #include "f32.cuh"
 #include "lattice.cuh"
-#include "tabulated.cuh"
 
 namespace kiwi_b200 {
 
@@ -59,7 +58,6 @@ constexpr int kLatCarveout = KIWI_LAT_CARVEOUT;
 constexpr size_t kLatAccSmem = sizeof(double) * 4 * kTileCells;
 constexpr size_t kLatDynSmem = kLatAccSmem + sizeof(double) * ((kLatAngles ? 3 : 2) * kLatECap2 + kLatPtCap);
 constexpr size_t kLatGenDynSmem = kLatAccSmem + sizeof(double) * (kLatGenERec * kLatGenECap + kLatPtCap);
-constexpr size_t kLatTabDynSmem = kLatAccSmem + sizeof(double) * kLatPtCap;
 
 // The six edge tiers of a lattice point (slots of the chunk's D2 / D3 tables in PointEdge order), read where
 // lattice_point uses them, as the real type T it is evaluated in.
@@ -117,23 +115,19 @@ struct LatChunk {
 // double-buffered: while warps 1-7 classify the current chunk's edge pairs and points, warp 0 loads the next
 // chunk (the particles' data, boxes and offsets) into the other buffer.
 // GENERIC: the table-driven tiers of kernel K (support radius support_in_h x h) instead of the cubic closed
-// form; edge tiers are lattice_generic_edge records.  TAB: the tabulated cubic integral (lookups in `tab`):
-// no edge tiers, and the points run in their natural order.  List order never affects the results.
-template <bool CULL, bool GENERIC = false, bool TAB = false, bool MIXED = false>
+// form; edge tiers are lattice_generic_edge records.  List order never affects the results.
+template <bool GENERIC>
 __device__ __forceinline__ void lattice_tile(const CartGeom& g, const DevParticles& P,
                                              const uint32_t* __restrict__ list, const int64_t* __restrict__ range,
                                              int64_t t_range, int64_t t, const CartOutputs& out,
-                                             DevStats* __restrict__ st, const KiwiKernelTable* K = nullptr,
-                                             const TabDev tab = TabDev{}) {
+                                             DevStats* __restrict__ st, const KiwiKernelTable* K = nullptr) {
     __shared__ LatChunk s_cp[2];
-    __shared__ TabWidths s_tw;               // TAB: the table's bin widths and their reciprocals
-    if (TAB && threadIdx.x == 0) s_tw = tab_widths(tab);  // read after the chunk load's barrier
     __shared__ int s_nexp, s_ncheap, s_nheavy, s_ninner;
-    __shared__ uint32_t s_plist[TAB ? 1 : kLatPtCap];
-    __shared__ uint32_t s_hlist[TAB ? 1 : kLatECap2 / 2];
+    __shared__ uint32_t s_plist[kLatPtCap];
+    __shared__ uint32_t s_hlist[kLatECap2 / 2];
     static_assert(kLatGenECap / 2 <= kLatECap2 / 2, "generic edge pairs fit the pair list");
     extern __shared__ double s_dyn[];
-    constexpr int kECap = GENERIC ? kLatGenECap : (TAB ? 0 : kLatECap2);
+    constexpr int kECap = GENERIC ? kLatGenECap : kLatECap2;
     // the owned cells' sums M, Px, Py, Pz: each thread's own entries (no sharing, no barrier), held in
     // registers only while (C) adds a chunk -- the point phase needs the registers
     double* s_acc = s_dyn;
@@ -141,7 +135,7 @@ __device__ __forceinline__ void lattice_tile(const CartGeom& g, const DevParticl
     double* s_D2 = s_chunk;
     double* s_D3 = s_chunk + kLatECap2;
     double* s_E = s_chunk;  // generic edge records
-    double* s_T = s_chunk + (GENERIC ? kLatGenERec * kLatGenECap : (TAB ? 0 : 2 * kLatECap2));
+    double* s_T = s_chunk + (GENERIC ? kLatGenERec * kLatGenECap : 2 * kLatECap2);
     // cubic: each edge pair's smaller in-plane angle (at its ab slot), or none
     double* s_A = kLatAngles ? s_T + kLatPtCap : nullptr;
 
@@ -168,7 +162,7 @@ __device__ __forceinline__ void lattice_tile(const CartGeom& g, const DevParticl
     // work counters: 32-bit per thread (a chunk adds at most a few hundred to any of them), flushed to the
     // 64-bit totals every 2^16 chunks and at the end
     unsigned n_bbox = 0, n_sphere = 0, n_eval = 0, n_neg = 0, n_warn = 0;
-    unsigned n_eo = 0, n_em = 0, n_ei = 0, n_vp = 0, n_clamp = 0, n_chunks = 0, n_island = 0;
+    unsigned n_eo = 0, n_em = 0, n_ei = 0, n_vp = 0, n_chunks = 0, n_island = 0;
     auto flush = [&]() {
         lat_add_stat(&st->bbox_pairs, n_bbox);
         lat_add_stat(&st->sphere_pairs, n_sphere);
@@ -179,9 +173,8 @@ __device__ __forceinline__ void lattice_tile(const CartGeom& g, const DevParticl
         lat_add_stat(&st->edge_middle, n_em);
         lat_add_stat(&st->edge_inner, n_ei);
         lat_add_stat(&st->vertex_pyramids, n_vp);
-        if (TAB) lat_add_stat(&st->table_clamps, n_clamp);
-        if (MIXED) lat_add_stat(&st->fp64_fallback, n_island);
-        n_bbox = n_sphere = n_eval = n_neg = n_warn = n_eo = n_em = n_ei = n_vp = n_clamp = n_island = 0;
+        lat_add_stat(&st->fp64_fallback, n_island);
+        n_bbox = n_sphere = n_eval = n_neg = n_warn = n_eo = n_em = n_ei = n_vp = n_island = 0;
     };
     const int64_t beg = range[2 * t_range], end = range[2 * t_range + 1];
     const double sup_in_h = g.support_in_h;
@@ -204,7 +197,7 @@ __device__ __forceinline__ void lattice_tile(const CartGeom& g, const DevParticl
             d1 = min(b.y1, by + kTileY - 1) - lo1 + 1;
             d2 = min(b.z1, bz + kTileZ - 1) - lo2 + 1;
             const int n0 = d0 + 1, n1 = d1 + 1, n2 = d2 + 1;
-            ne = TAB ? 0 : 2 * (n0 * n1 + n0 * n2 + n1 * n2);
+            ne = 2 * (n0 * n1 + n0 * n2 + n1 * n2);
             npt = n0 * n1 * n2;
             ncl = d0 * d1 * d2;
         }
@@ -259,7 +252,7 @@ __device__ __forceinline__ void lattice_tile(const CartGeom& g, const DevParticl
             // n1' x n2'; pair (p, q) of block (a, b) is edge ab[p][q] and edge ba[q][p].  Cubic: pairs beyond 2h
             // (and zero ones) get D2 = D3 = 0 here; the others are listed (slot ab | slot ba << 11 | particle <<
             // 22) with |u_a|, |u_b| parked in slot ab, and evaluated in (A2).  Generic: both records here.
-            if (!TAB) {
+            {
                 const int qtot = etot >> 1;
                 const int qoff_l = lane < np ? (cp->eoff[lane] >> 1) : INT_MAX;
                 for (int base = (warp - 1) * 32; base < qtot; base += kLatThreads - 32) {
@@ -345,14 +338,14 @@ __device__ __forceinline__ void lattice_tile(const CartGeom& g, const DevParticl
                 }
             }
 
-            // (B0) the lattice points some evaluated cell reads: with CULL, a point none of whose eight cells
+            // (B0) the lattice points some evaluated cell reads: a point none of whose eight cells
             // meets the support sphere is left out (the test bounds the distance to the 2 x 2 x 2 cells around
             // the point, their half-widths padded by 1e-6 of a cell so that rounding never drops a point an
             // evaluated cell reads).  A point on a particle plane (an offset of 0) has octant value 0, written
             // here; the others are listed, those within the support from the front of s_plist, those beyond it
             // from the end, so that each kind runs in warps of its own.  An entry packs (particle, i, j, k):
             // 5 + 3 x 4 bits.
-            if (!TAB) {
+            {
                 const int poff_l = lane < np ? cp->poff[lane] : INT_MAX;
                 for (int base = (warp - 1) * 32; base < ptot; base += kLatThreads - 32) {
                     const int pt = base + lane;
@@ -369,15 +362,11 @@ __device__ __forceinline__ void lattice_tile(const CartGeom& g, const DevParticl
                         const double uy = s_pl[1][cp->lo[jp][1] - by + jj] - cp->y[jp];
                         const double uz = s_pl[2][cp->lo[jp][2] - bz + k] - cp->z[jp];
                         const double h = cp->h[jp];
-                        bool keep = true;
-                        if (CULL) {
-                            const double radius = mul_rn(sup_in_h, h);
-                            const double ex = fmax(fabs(ux) - kNeedPad * g.dpx, 0.0);
-                            const double ey = fmax(fabs(uy) - kNeedPad * g.dpy, 0.0);
-                            const double ez = fmax(fabs(uz) - kNeedPad * g.dpz, 0.0);
-                            keep = ex * ex + ey * ey + ez * ez < radius * radius;
-                        }
-                        if (keep) {
+                        const double radius = mul_rn(sup_in_h, h);
+                        const double ex = fmax(fabs(ux) - kNeedPad * g.dpx, 0.0);
+                        const double ey = fmax(fabs(uy) - kNeedPad * g.dpy, 0.0);
+                        const double ez = fmax(fabs(uz) - kNeedPad * g.dpz, 0.0);
+                        if (ex * ex + ey * ey + ez * ez < radius * radius) {
                             if (ux == 0.0 || uy == 0.0 || uz == 0.0) {
                                 s_T[pt] = 0.0;
                             } else {
@@ -410,7 +399,7 @@ __device__ __forceinline__ void lattice_tile(const CartGeom& g, const DevParticl
                 const int sab = (int)(rec & 2047u), sba = (int)((rec >> 11) & 2047u), j = (int)(rec >> 22);
                 const double vp = s_E[kLatGenERec * sab], vq = s_E[kLatGenERec * sab + 1];
                 const double H = mul_rn(sup_in_h, cp->h[j]);
-                if (MIXED && fmin(vp, vq) >= kMixedIslandFrac * cp->h[j]) {
+                if (fmin(vp, vq) >= kMixedIslandFrac * cp->h[j]) {
                     lattice_generic_edge(K, H, F32(vp), F32(vq), s_E + kLatGenERec * sab);
                     lattice_generic_edge(K, H, F32(vq), F32(vp), s_E + kLatGenERec * sba);
                 } else {
@@ -420,7 +409,7 @@ __device__ __forceinline__ void lattice_tile(const CartGeom& g, const DevParticl
             }
             __syncthreads();
         }
-        if (!GENERIC && !TAB) {
+        if (!GENERIC) {
             const int nmid = s_nheavy, ninner = s_ninner;
             for (int li = threadIdx.x; li < nmid + ninner; li += kLatThreads) {
                 const uint32_t rec = s_hlist[li < nmid ? li : kLatECap2 / 2 - ninner + (li - nmid)];
@@ -431,7 +420,7 @@ __device__ __forceinline__ void lattice_tile(const CartGeom& g, const DevParticl
                 // which the walls with legs along a and b read
                 const double vmin = fmin(vp, vq), vmax = fmax(vp, vq);
                 if (kLatAngles) s_A[sab] = atan(vmin / vmax);
-                if (MIXED && vmin >= kMixedIslandFrac * cp->h[j]) {
+                if (vmin >= kMixedIslandFrac * cp->h[j]) {
                     LatticeEdgeT<F32> f_pq, f_qp;
                     lattice_edge_pair(F32(cp->h[j]), F32(cp->ih[j]), F32(vp), F32(vq), f_pq, f_qp);
                     e_pq = {(double)f_pq.D2.v, (double)f_pq.D3.v};
@@ -447,28 +436,14 @@ __device__ __forceinline__ void lattice_tile(const CartGeom& g, const DevParticl
             __syncthreads();
         }
         const int nexp = s_nexp, ncheap = s_ncheap;
-        const int nplist = TAB ? ptot : nexp + ncheap;
+        const int nplist = nexp + ncheap;
 
         // (B) octant values of the listed points
         for (int li = threadIdx.x; li < nplist; li += kLatThreads) {
-            int jp, i, jj, k, it;
-            if (TAB) {
-                it = li;
-                jp = chunk_search(cp->poff, np, it);
-                const int lp = it - cp->poff[jp];
-                const int n2 = cp->dim[jp][2] + 1, n12 = (cp->dim[jp][1] + 1) * n2;
-                i = div_by(lp, cp->mag[jp][3]);
-                const int rem = lp - i * n12;
-                jj = div_by(rem, cp->mag[jp][2]);
-                k = rem - jj * n2;
-            } else {
-                const uint32_t rec = s_plist[li < nexp ? li : kLatPtCap - ncheap + (li - nexp)];
-                jp = (int)(rec & 31u);
-                i = (int)((rec >> 5) & 15u);
-                jj = (int)((rec >> 9) & 15u);
-                k = (int)((rec >> 13) & 15u);
-                it = cp->poff[jp] + (i * (cp->dim[jp][1] + 1) + jj) * (cp->dim[jp][2] + 1) + k;
-            }
+            const uint32_t rec = s_plist[li < nexp ? li : kLatPtCap - ncheap + (li - nexp)];
+            const int jp = (int)(rec & 31u), i = (int)((rec >> 5) & 15u), jj = (int)((rec >> 9) & 15u),
+                      k = (int)((rec >> 13) & 15u);
+            const int it = cp->poff[jp] + (i * (cp->dim[jp][1] + 1) + jj) * (cp->dim[jp][2] + 1) + k;
             const double ux = s_pl[0][cp->lo[jp][0] - bx + i] - cp->x[jp];
             const double uy = s_pl[1][cp->lo[jp][1] - by + jj] - cp->y[jp];
             const double uz = s_pl[2][cp->lo[jp][2] - bz + k] - cp->z[jp];
@@ -476,43 +451,36 @@ __device__ __forceinline__ void lattice_tile(const CartGeom& g, const DevParticl
             double f = 0.0;
             if (sg != 0.0) {
                 const double ax = fabs(ux), ay = fabs(uy), az = fabs(uz);
-                if (TAB) {
-                    // two right-triangle vertex pyramids per wall; cos(phi) from the legs
-                    const double ih = cp->ih[jp];
-                    f = tab_pair(tab, s_tw, ih, ax, ay, az, n_clamp) + tab_pair(tab, s_tw, ih, ay, ax, az, n_clamp) +
-                        tab_pair(tab, s_tw, ih, az, ax, ay, n_clamp);
-                } else {
-                    const int n0 = cp->dim[jp][0] + 1, n1 = cp->dim[jp][1] + 1, n2 = cp->dim[jp][2] + 1;
-                    const int nxy = n0 * n1, nxz = n0 * n2, nyz = n1 * n2;
-                    const int eb = cp->eoff[jp];
-                    const int exy = eb + i * n1 + jj, exz = eb + nxy + i * n2 + k;
-                    const int eyx = eb + nxy + nxz + jj * n0 + i, eyz = eb + 2 * nxy + nxz + jj * n2 + k;
-                    const int ezx = eb + 2 * nxy + nxz + nyz + k * n0 + i, ezy = eb + 2 * nxy + 2 * nxz + nyz + k * n1 + jj;
-                    if (GENERIC) {
-                        const double H = mul_rn(sup_in_h, cp->h[jp]);
-                        const double *rxy = s_E + kLatGenERec * exy, *rxz = s_E + kLatGenERec * exz;
-                        const double *ryx = s_E + kLatGenERec * eyx, *ryz = s_E + kLatGenERec * eyz;
-                        const double *rzx = s_E + kLatGenERec * ezx, *rzy = s_E + kLatGenERec * ezy;
-                        if (MIXED && fmin(ax, fmin(ay, az)) >= kMixedIslandFrac * cp->h[jp]) {
-                            const F32 fx(ax), fy(ay), fz(az);
-                            f = (double)(lattice_generic_corner(K, H, fx, fy, fz, rxy, rxz) +
-                                         lattice_generic_corner(K, H, fy, fx, fz, ryx, ryz) +
-                                         lattice_generic_corner(K, H, fz, fx, fy, rzx, rzy)).v;
-                        } else {
-                            f = lattice_generic_corner(K, H, ax, ay, az, rxy, rxz) +
-                                lattice_generic_corner(K, H, ay, ax, az, ryx, ryz) +
-                                lattice_generic_corner(K, H, az, ax, ay, rzx, rzy);
-                            if (MIXED) ++n_island;
-                        }
+                const int n0 = cp->dim[jp][0] + 1, n1 = cp->dim[jp][1] + 1, n2 = cp->dim[jp][2] + 1;
+                const int nxy = n0 * n1, nxz = n0 * n2, nyz = n1 * n2;
+                const int eb = cp->eoff[jp];
+                const int exy = eb + i * n1 + jj, exz = eb + nxy + i * n2 + k;
+                const int eyx = eb + nxy + nxz + jj * n0 + i, eyz = eb + 2 * nxy + nxz + jj * n2 + k;
+                const int ezx = eb + 2 * nxy + nxz + nyz + k * n0 + i, ezy = eb + 2 * nxy + 2 * nxz + nyz + k * n1 + jj;
+                if (GENERIC) {
+                    const double H = mul_rn(sup_in_h, cp->h[jp]);
+                    const double *rxy = s_E + kLatGenERec * exy, *rxz = s_E + kLatGenERec * exz;
+                    const double *ryx = s_E + kLatGenERec * eyx, *ryz = s_E + kLatGenERec * eyz;
+                    const double *rzx = s_E + kLatGenERec * ezx, *rzy = s_E + kLatGenERec * ezy;
+                    if (fmin(ax, fmin(ay, az)) >= kMixedIslandFrac * cp->h[jp]) {
+                        const F32 fx(ax), fy(ay), fz(az);
+                        f = (double)(lattice_generic_corner(K, H, fx, fy, fz, rxy, rxz) +
+                                     lattice_generic_corner(K, H, fy, fx, fz, ryx, ryz) +
+                                     lattice_generic_corner(K, H, fz, fx, fy, rzx, rzy)).v;
                     } else {
-                        if (MIXED && fmin(ax, fmin(ay, az)) >= kMixedIslandFrac * cp->h[jp]) {
-                            const SmemPointEdges<F32> E{s_D2, s_D3, s_A, {exy, exz, eyx, eyz, ezx, ezy}};
-                            f = (double)lattice_point(F32(cp->h[jp]), F32(cp->ih[jp]), F32(ax), F32(ay), F32(az), E).v;
-                        } else {
-                            const SmemPointEdges<double> E{s_D2, s_D3, s_A, {exy, exz, eyx, eyz, ezx, ezy}};
-                            f = lattice_point(cp->h[jp], cp->ih[jp], ax, ay, az, E);
-                            if (MIXED) ++n_island;
-                        }
+                        f = lattice_generic_corner(K, H, ax, ay, az, rxy, rxz) +
+                            lattice_generic_corner(K, H, ay, ax, az, ryx, ryz) +
+                            lattice_generic_corner(K, H, az, ax, ay, rzx, rzy);
+                        ++n_island;
+                    }
+                } else {
+                    if (fmin(ax, fmin(ay, az)) >= kMixedIslandFrac * cp->h[jp]) {
+                        const SmemPointEdges<F32> E{s_D2, s_D3, s_A, {exy, exz, eyx, eyz, ezx, ezy}};
+                        f = (double)lattice_point(F32(cp->h[jp]), F32(cp->ih[jp]), F32(ax), F32(ay), F32(az), E).v;
+                    } else {
+                        const SmemPointEdges<double> E{s_D2, s_D3, s_A, {exy, exz, eyx, eyz, ezx, ezy}};
+                        f = lattice_point(cp->h[jp], cp->ih[jp], ax, ay, az, E);
+                        ++n_island;
                     }
                 }
                 n_vp += 6;
@@ -527,53 +495,8 @@ __device__ __forceinline__ void lattice_tile(const CartGeom& g, const DevParticl
         // (C) cells: the alternating sum of the 8 corners' octant values, added in particle order.  (C1) every
         // (particle, cell of its box) pair of the chunk, as one flat list over all threads: the support test,
         // the counters and the clamped alternating sum, into the chunk's edge-tier buffer (dead after (B));
-        // (C2) each thread adds, for the cells it owns, the chunk's pairs in particle order.  The tabulated
-        // body (no edge buffer) does both in the owners' loop.
-        if (TAB) {
-#pragma unroll
-    #pragma unroll
-            for (int c = 0; c < kLatCellsPerThread; ++c) {
-                const int li = threadIdx.x + c * kLatThreads;
-                const int lx = li / (kTileZ * kTileY), ly = (li / kTileZ) % kTileY, lz = li % kTileZ;
-                const int gx = bx + lx, gy = by + ly, gz = bz + lz;
-                double a0 = s_acc[li], a1 = s_acc[kTileCells + li];
-                double a2 = s_acc[2 * kTileCells + li], a3 = s_acc[3 * kTileCells + li];
-                for (int j = 0; j < np; ++j) {
-                    const int i = gx - cp->lo[j][0], jj = gy - cp->lo[j][1], k = gz - cp->lo[j][2];
-                    if (i < 0 || jj < 0 || k < 0 || i >= cp->dim[j][0] || jj >= cp->dim[j][1] || k >= cp->dim[j][2]) continue;
-                    ++n_bbox;
-                    const double radius = mul_rn(sup_in_h, cp->h[j]);
-                    const double ex = fmax(fabs(cp->x[j] - s_cc[0][lx]) - g.hpx, 0.0);
-                    const double ey = fmax(fabs(cp->y[j] - s_cc[1][ly]) - g.hpy, 0.0);
-                    const double ez = fmax(fabs(cp->z[j] - s_cc[2][lz]) - g.hpz, 0.0);
-                    // the support test of the pair counters, rounded as the host restatement rounds it
-                    const bool in = add_rn(add_rn(mul_rn(ex, ex), mul_rn(ey, ey)), mul_rn(ez, ez)) < mul_rn(radius, radius);
-                    n_sphere += in;
-                    if (CULL && !in) continue;
-                    ++n_eval;
-                    const int n2 = cp->dim[j][2] + 1, n12 = (cp->dim[j][1] + 1) * n2;
-                    const double* Tp = s_T + cp->poff[j] + (i * (cp->dim[j][1] + 1) + jj) * n2 + k;
-                    const double m1 = (Tp[n12 + n2 + 1] - Tp[n12 + n2]) - (Tp[n12 + 1] - Tp[n12]);
-                    const double m0 = (Tp[n2 + 1] - Tp[n2]) - (Tp[1] - Tp[0]);
-                    double msum = m1 - m0;
-                    if (msum < 0.0) {
-                        ++n_neg;
-                        if (msum <= -0.01) ++n_warn;
-                        msum = 0.0;
-                    }
-                    if (msum == 0.0) continue;
-                    const double mm = msum * cp->m[j];
-                    a0 += mm;
-                    a1 += mm * cp->vx[j];
-                    a2 += mm * cp->vy[j];
-                    a3 += mm * cp->vz[j];
-                }
-                s_acc[li] = a0;
-                s_acc[kTileCells + li] = a1;
-                s_acc[2 * kTileCells + li] = a2;
-                s_acc[3 * kTileCells + li] = a3;
-            }
-        } else {
+        // (C2) each thread adds, for the cells it owns, the chunk's pairs in particle order.
+        {
             double* const s_cm = s_chunk;  // (particle, cell) pair values at coff[j] + the cell's box index
             const int ctot = cp->ctot;
             const int coff_l = lane < np ? cp->coff[lane] : INT_MAX;
@@ -596,7 +519,7 @@ __device__ __forceinline__ void lattice_tile(const CartGeom& g, const DevParticl
                     const bool in = add_rn(add_rn(mul_rn(ex, ex), mul_rn(ey, ey)), mul_rn(ez, ez)) < mul_rn(radius, radius);
                     n_sphere += in;
                     double msum = 0.0;
-                    if (!CULL || in) {
+                    if (in) {
                         ++n_eval;
                         const int n2 = d2 + 1, n12 = (d1 + 1) * n2;
                         const double* Tp = s_T + cp->poff[j] + (i * (d1 + 1) + jj) * n2 + k;

@@ -54,12 +54,23 @@ __global__ void k_gridded_batch(TabDev t, int64_t n, const double* __restrict__ 
     if ((threadIdx.x & 31) == 0 && v) atomicAdd(clamps, v);
 }
 
+// One thread per entry: the four neighbours (i, k), (i + 1, k), (i, k + 1), (i + 1, k + 1) of row j together, so that a
+// lookup is two loads of 32 bytes (rows j and j + 1) instead of eight of 8.
+__global__ void k_tab_blocks(TabDev t, double4* __restrict__ out) {
+    const int nk = t.nphi + 1;
+    const int64_t row = (int64_t)(t.nR_0 + 1) * nk, e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= (int64_t)(t.nr0 + 1) * row) return;
+    const bool last = e % nk == t.nphi;  // (no lookup starts at the last k)
+    out[e] = double4{t.v[e], t.v[e + row], last ? 0.0 : t.v[e + 1], last ? 0.0 : t.v[e + row + 1]};
+}
+
 int64_t table_values(const TabDev& t) { return (int64_t)(t.nr0 + 2) * (t.nR_0 + 1) * (t.nphi + 1); }
 
 void table_release(KiwiCtx* ctx) {
     if (ctx->tab.v) {
         cudaStreamSynchronize(ctx->stream);
         cudaFree(const_cast<double*>(ctx->tab.v));
+        cudaFree(const_cast<double*>(ctx->tab.v4));
     }
     ctx->tab = TabDev{};
     ctx->tab_bytes = 0;
@@ -187,6 +198,22 @@ namespace kiwi_b200 {
 
 int table_ensure(KiwiCtx* ctx, TabDev* out) {
     if (!ctx->tab.v) KIWI_TRY(table_generate(ctx));
+    *out = ctx->tab;
+    return KIWI_OK;
+}
+
+int table_blocks(KiwiCtx* ctx, TabDev* out) {
+    const int64_t n = (int64_t)(ctx->tab.nr0 + 1) * (ctx->tab.nR_0 + 1) * (ctx->tab.nphi + 1);
+    if (!ctx->tab.v4 && n * (int64_t)sizeof(double4) <= ((int64_t)4 << 30)) {
+        double4* d = nullptr;
+        if (cudaMalloc(&d, sizeof(double4) * (size_t)n) == cudaSuccess) {
+            k_tab_blocks<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(ctx->tab, d);
+            ctx->tab.v4 = reinterpret_cast<const double*>(d);
+            KIWI_LAUNCHED(ctx);
+        } else {
+            cudaGetLastError();  // the lookups read the table itself
+        }
+    }
     *out = ctx->tab;
     return KIWI_OK;
 }

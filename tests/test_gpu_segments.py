@@ -68,3 +68,23 @@ def test_entry_points_agree(kiwi, ctx, kernel, n, shape):
         torch.cuda.synchronize()
         kiwi.sph_to_grid_device(dP, bounds, shape, ref, kernel=ki, ctx=ctx, precision="fp64_reference_order")
         assert_band_tolerance(whole["density"].cpu().numpy(), ref["density"].cpu().numpy(), (4e-10, 4e-9, 1e-7))
+
+
+def test_tabulated_parts_agree(kiwi, ctx):
+    """The tabulated integral's tiles are cut the same way: parts equal the whole, and the whole agrees with the
+    per-cell form to the rounding of the lookups' indices."""
+    import torch
+
+    ki = kiwi.make_kernel_integrator("cubic_spline", use_tabulated_integral=True)
+    bounds, shape, n = (0.0, 1.0) * 3, (17, 16, 9), 3000
+    nc = int(np.prod(shape))
+    dP = _particles(torch, n, 0.12, 5)
+    outs = []
+    for parts, form in ((1, "fp64"), (3, "fp64"), (1, "fp64_reference_order")):
+        out = {"density": torch.full((nc,), np.nan, dtype=torch.float64, device="cuda")}
+        torch.cuda.synchronize()
+        for p in range(parts):
+            st = kiwi.sph_to_grid_device(dP, bounds, shape, out, kernel=ki, ctx=ctx, part=p, n_parts=parts, precision=form)
+        outs.append((out["density"], st))
+    assert torch.equal(outs[0][0], outs[1][0])
+    assert_band_tolerance(outs[0][0].cpu().numpy(), outs[2][0].cpu().numpy(), (4e-10, 4e-9, 1e-7))
