@@ -129,7 +129,7 @@ KIWI_HD void box_grad_edge(const KiwiBoxTable& T, int c, const double* A, const 
         const KiwiBoxScale& s = T.scale[k];
         const double t2 = fma(s.b, s.b, -P);
         if (t2 > 0.0 && p < s.b && q < s.b) {
-            const double it = fm_rsqrt(t2), t = t2 * it, ib = 1.0 / s.b;
+            const double it = fm_rsqrt(t2), t = t2 * it, ib = s.ib;
             const double anp = fm_atan_pos((p * ib) * (t * iq), (s.b * ip) * (q * it));
             const double anq = fm_atan_pos((q * ib) * (t * ip), (s.b * iq) * (p * it));
             const double dep = box_delta(t, t2, p, q, s.b), deq = box_delta(t, t2, q, p, s.b);

@@ -9,15 +9,20 @@
 // src/kernel_integral.cpp:471-647).
 //
 // The list (ascending particle index) is walked in chunks, in phases separated by barriers:
-//   (E) edge lines; warp 0 first loads the next chunk (particles, boxes, offsets) into the other buffer;
+//   (E) edge lines, and warp 0 loads the next chunk (particles, boxes, offsets) into the other buffer;
 //   (P) points;
-//   (C1) every (particle, cell of its box) pair as one flat list: support test, counters, alternating sum;
+//   (C1) every (particle, cell of its box) pair as one flat list: support test, counters, alternating sum; and the
+//        next chunk's planes;
 //   (C2) each thread adds, for the cells it owns, the chunk's pairs in particle order, so that every cell's sum
-//        runs over its particles in ascending index order with no atomics; and the next chunk's planes.
-// Within (E) and (P) a warp walks its share of the flat list and sorts what it meets by cost: the cheap items
-// (lines and points beyond the support) it finishes at once, the others it queues by kind (a line by its piece, a
-// point within the support) and evaluates 32 of a kind at a time, so that no lane waits for another kind's work
-// and no list is shared between warps.
+//        runs over its particles in ascending index order with no atomics; and the next chunk's lines are listed.
+// An item's cost is its kind: a line or a point beyond the support is a few sums, one within it roots, logarithms and
+// arctangents, a line in an inner piece those of every piece from there on.  So that no lane waits for another kind's
+// work, lines are listed by kind over the whole CTA and taken 32 of a kind at a time, the costly kinds first, by
+// whichever warp is free; points (two kinds, forty batches a chunk) a warp sorts for itself, finishing the cheap ones
+// at once and queueing the others until it has 32.  Lines queued by warp and kind instead left half of the few
+// batches of a chunk part empty and the warps waiting at the barrier: 9 k particles on 37 x 41 x 149, quintic spline
+// (three kinds), 4.65 -> 3.7 ms; 150 k on 131 x 117 x 102, cubic, 5.0 -> 4.7 ms.  With one piece there is one
+// costly kind, and a warp's own queue is the faster (100 k on 128^3, Wendland C4: 8.5 against 9.1 ms).
 //
 // A tile with a long list is cut into segments of box_segment() entries, each summed on its own (by CTAs of their
 // own, which leave raw sums for k_box_combine, or one after another in one CTA), and the segments' sums are
@@ -72,7 +77,6 @@ constexpr int kBoxPlaneCap = KIWI_BOX_PLANE_CAP;  // planes per chunk (a full bo
 constexpr int kTabPlane = 3, kTabEdge = 6;
 // The three-piece kernels' records are larger: fewer lines and planes in the same shared memory.
 constexpr int kBoxGenPtCap = 1792, kBoxGenPairCap = 640, kBoxGenPlaneCap = 256;
-static_assert(kBoxPairCap <= 1024 && kBoxPlaneCap <= 512, "packed edge entries");
 
 // SEQ: the segments of a tile one after another, which needs the cells' totals beside the segment's sums.
 // TAB (with NP 1): the tabulated integral's records.
@@ -83,28 +87,56 @@ struct BoxCaps {
     static constexpr int kPt = TAB ? 2304 : SEQ ? 1536 : (NP == 1 ? 3072 : (NP == 2 ? kBoxPtCap : kBoxGenPtCap));
     static constexpr int kPair = TAB ? 900 : SEQ ? (NP ? 768 : 512) : (NP == 1 ? 1024 : (NP == 2 ? kBoxPairCap : kBoxGenPairCap));
     static constexpr int kPlane = TAB ? 296 : SEQ ? 208 : (NP == 1 ? 448 : (NP == 2 ? kBoxPlaneCap : kBoxGenPlaneCap));
-    static constexpr int kQueues = kN;  // edge kinds; the point phase uses the first
+    static constexpr int kKinds = kN + 1;  // of edge lines
+    static_assert(kKinds * kPair <= 2 * kPt || TAB, "the lines' lists fit the octant values' place");
+    static_assert(kPlane <= 512 && kPair <= 1024 && kPt <= 4096, "BoxGeo's fields");
     // dynamic shared memory, in doubles: the cells' sums, the octant values, the edge and plane records
     static constexpr int kOffT = 4 * kTileCells;
     static constexpr int kOffE = kOffT + kPt;
     static constexpr int kOffP = kOffE + kES * kPair;
     static constexpr int kOffS = kOffP + kPS * kPlane;
     static constexpr int kEnd = kOffS + (SEQ ? 4 * kTileCells : 0);
-    static constexpr size_t kSmem = sizeof(double) * kEnd + sizeof(uint32_t) * 64 * kBoxWarps * kQueues;
+    static constexpr size_t kSmem = sizeof(double) * kEnd + (TAB ? 0 : sizeof(uint2) * 64 * kBoxWarps);
     // (C1) keeps the pairs' values in the edge records' place (with one piece the records are smaller)
     static_assert((NP ? kES : box_edge_stride(1)) * kPair >= kPt, "pair values fit");
 };
 
-// One chunk of a tile's particle list: the particles' data, their boxes clipped to the tile (lo, dim), their
-// first plane, edge line, point and cell, and the magic divisors of their dimensions.
+// A particle's box clipped to the tile and its places in the chunk, packed so that a thread reads it in one 16-byte
+// load (eight to ten 4-byte loads otherwise).
+// x: the first plane (9 bits), edge line (10) and lattice point (13); y: the 16-bit magic divisors of n2' and n1' n2'
+// (x / n = x * ceil(2^16 / n) >> 16 for the at most 729 points); z: n1', n2' (4 each), n0' n1' (7), n0' (n1' + n2') (8),
+// n0' (4); w: the first cell (12), lo relative to the tile (3 each), the 10-bit magic divisor of n1' (the at most 81
+// lines of a block).
+struct BoxGeo {
+    int4 v;
+    __device__ __forceinline__ int plane() const { return v.x & 511; }
+    __device__ __forceinline__ int line() const { return (v.x >> 9) & 1023; }
+    __device__ __forceinline__ int point() const { return (int)((uint32_t)v.x >> 19); }
+    __device__ __forceinline__ int cell() const { return v.w & 4095; }
+    __device__ __forceinline__ int n1() const { return v.z & 15; }
+    __device__ __forceinline__ int n2() const { return (v.z >> 4) & 15; }
+    __device__ __forceinline__ int n01() const { return (v.z >> 8) & 127; }
+    __device__ __forceinline__ int n0_12() const { return (v.z >> 15) & 255; }
+    __device__ __forceinline__ int n0() const { return v.z >> 23; }
+    __device__ __forceinline__ int lo0() const { return (v.w >> 12) & 7; }
+    __device__ __forceinline__ int lo1() const { return (v.w >> 15) & 7; }
+    __device__ __forceinline__ int lo2() const { return (v.w >> 18) & 7; }
+    __device__ __forceinline__ int by_n2(int x) const { return (int)(((uint32_t)x * (v.y & 0xffffu)) >> 16); }
+    __device__ __forceinline__ int by_n12(int x) const { return (int)(((uint32_t)x * ((uint32_t)v.y >> 16)) >> 16); }
+    __device__ __forceinline__ int by_n1(int x) const { return (int)(((uint32_t)x * ((uint32_t)v.w >> 21)) >> 10); }
+};
+__device__ __forceinline__ uint32_t box_magic(int n, int bits) { return ((1u << bits) + (uint32_t)n - 1) / (uint32_t)n; }
+
+// One chunk of a tile's particle list: the particles' data, their boxes, and the 16-bit magic divisors of their cells'
+// dimensions n2 and n1 n2 (x / n = x * ceil(2^15 / n) >> 15 for the at most 512 cells).
 struct BoxChunk {
-    double x[kBoxPMax], y[kBoxPMax], z[kBoxPMax], H[kBoxPMax], iH[kBoxPMax], m[kBoxPMax], vx[kBoxPMax], vy[kBoxPMax],
-        vz[kBoxPMax];
-    int lo[kBoxPMax][3], dim[kBoxPMax][3];  // lo relative to the tile
-    int loff[kBoxPMax], eoff[kBoxPMax], poff[kBoxPMax], coff[kBoxPMax];
-    uint32_t mag[kBoxPMax][3];   // div_magic of n1', n2' and n1' n2'
-    uint32_t cmag[kBoxPMax][2];  // div_magic of n2 and n1 n2
+    double4 at[kBoxPMax];  // x, y, z and the support radius
+    double4 mv[kBoxPMax];  // mass, velocities
+    int4 geo[kBoxPMax];
+    double iH[kBoxPMax];
+    uint32_t cmag[kBoxPMax];
     int np, ltot, etot, ptot, ctot;
+    __device__ __forceinline__ BoxGeo box(int j) const { return BoxGeo{geo[j]}; }
 };
 
 __device__ __forceinline__ void box_add_stat(unsigned long long* dst, unsigned long long v) {
@@ -234,6 +266,10 @@ __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& 
     __shared__ TabWidths s_tw;
     if (TAB && threadIdx.x == 0) s_tw = tab_widths(tab);
     __shared__ BoxChunk s_cp[2];
+    constexpr bool kList = !TAB && NP != 1;
+    __shared__ int s_lines[Caps::kKinds], s_next;  // listed lines of each kind; (E)'s next batch
+    if (threadIdx.x < Caps::kKinds) s_lines[threadIdx.x] = 0;
+    if (threadIdx.x == 0) s_next = 0;
     __shared__ double s_pl[3][kTileX + 1], s_cc[3][kTileX];
     __shared__ double s_C[NP == 2 || TAB ? 1 : (kBoxC + 1) * Caps::kN];  // any kernel: c and C of its pieces (lanes differ in piece)
     static_assert(kTileX == kTileY && kTileX == kTileZ, "cubic tiles");
@@ -246,7 +282,8 @@ __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& 
     double* const s_P = s_dyn + Caps::kOffP;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1;
-    uint32_t* const s_q = reinterpret_cast<uint32_t*>(s_dyn + Caps::kEnd) + 64 * Caps::kQueues * warp;
+    uint2* const s_q = reinterpret_cast<uint2*>(s_dyn + Caps::kEnd) + 64 * warp;
+    uint32_t* const s_list = reinterpret_cast<uint32_t*>(s_T);
 
     const int tz = (int)(t % g.ntz), ty = (int)((t / g.ntz) % g.nty), tx = (int)(t / ((int64_t)g.ntz * g.nty));
     const int bx = tx * kTileX, by = ty * kTileY, bz = tz * kTileZ;
@@ -322,19 +359,15 @@ __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& 
         const int np = __popc(__ballot_sync(0xffffffffu, take));
         if (take) {
             const double H = mul_rn(g.support_in_h, ph);
-            dst->x[lane] = px; dst->y[lane] = py; dst->z[lane] = pz; dst->H[lane] = H; dst->iH[lane] = 1.0 / (TAB ? ph : H);
-            dst->m[lane] = pm; dst->vx[lane] = pvx; dst->vy[lane] = pvy; dst->vz[lane] = pvz;
-            dst->lo[lane][0] = lo0; dst->lo[lane][1] = lo1; dst->lo[lane][2] = lo2;
-            dst->dim[lane][0] = d0; dst->dim[lane][1] = d1; dst->dim[lane][2] = d2;
-            dst->loff[lane] = il - nl;
-            dst->eoff[lane] = ie - ne;
-            dst->poff[lane] = ip - npt;
-            dst->coff[lane] = ic - ncl;
-            dst->mag[lane][0] = div_magic(d1 + 1);
-            dst->mag[lane][1] = div_magic(d2 + 1);
-            dst->mag[lane][2] = div_magic((d1 + 1) * (d2 + 1));
-            dst->cmag[lane][0] = div_magic(d2);
-            dst->cmag[lane][1] = div_magic(d1 * d2);
+            dst->at[lane] = double4{px, py, pz, H};
+            dst->mv[lane] = double4{pm, pvx, pvy, pvz};
+            dst->iH[lane] = 1.0 / (TAB ? ph : H);
+            const int n0 = d0 + 1, n1 = d1 + 1, n2 = d2 + 1;
+            dst->geo[lane] = int4{(int)((uint32_t)(il - nl) | (uint32_t)(ie - ne) << 9 | (uint32_t)(ip - npt) << 19),
+                                  (int)(box_magic(n2, 16) | box_magic(n1 * n2, 16) << 16),
+                                  n1 | n2 << 4 | (n0 * n1) << 8 | (n0 * (n1 + n2)) << 15 | n0 << 23,
+                                  (int)((uint32_t)(ic - ncl) | (uint32_t)(lo0 | lo1 << 3 | lo2 << 6) << 12 | box_magic(n1, 10) << 21)};
+            dst->cmag[lane] = box_magic(d2, 15) | box_magic(d1 * d2, 15) << 16;
         }
         if (lane == np - 1) {
             dst->np = np;
@@ -346,21 +379,77 @@ __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& 
     };
     // all warps: a chunk's plane records
     auto form_planes = [&](const BoxChunk* cp) {
-        const int off_l = lane < cp->np ? cp->loff[lane] : INT_MAX, tot = cp->ltot;
+        const int off_l = lane < cp->np ? cp->box(lane).plane() : INT_MAX, tot = cp->ltot;
         for (int base = warp * 32; base < tot; base += kBoxThreads) {
             const int j = warp_owner(base, off_l, lane), it = base + lane;
-            const int off = __shfl_sync(0xffffffffu, off_l, j & 31);
             if (it < tot) {
-                int l = it - off;
-                const int n0 = cp->dim[j][0] + 1, n1 = cp->dim[j][1] + 1;
+                const BoxGeo b = cp->box(j);
+                int l = it - b.plane();
+                const int n0 = b.n0(), n1 = b.n1();
                 const int a = (l >= n0) + (l >= n0 + n1);
                 l -= a == 0 ? 0 : (a == 1 ? n0 : n0 + n1);
-                const double c = a == 0 ? cp->x[j] : (a == 1 ? cp->y[j] : cp->z[j]);
-                const double u = s_pl[a][cp->lo[j][a] + l] - c;
+                const double4 at = cp->at[j];
+                const double c = a == 0 ? at.x : (a == 1 ? at.y : at.z);
+                const double u = s_pl[a][(a == 0 ? b.lo0() : (a == 1 ? b.lo1() : b.lo2())) + l] - c;
                 if constexpr (TAB) box_tab_plane(tab, s_tw, u, cp->iH[j], s_P + kPS * it);
                 else box_plane<NP, DEG>(T, u * cp->iH[j], s_P + kPS * it);
             }
         }
+    };
+
+    // the planes of a box's line e: blocks (x, y) over n0' x n1', (x, z) over n0' x n2', (y, z) over n1' x n2'
+    auto line_planes = [&](const BoxGeo& b, int e, int& la, int& lb) {
+        const int n0 = b.n0(), n1 = b.n1(), n2 = b.n2();
+        const bool xy = e < b.n01(), yz = e >= b.n0_12();
+        const int base = b.plane();
+        e -= xy ? 0 : (yz ? b.n0_12() : b.n01());
+        const int pi = xy ? b.by_n1(e) : b.by_n2(e), qi = e - pi * (xy ? n1 : n2);
+        la = base + (yz ? n0 : 0) + pi;
+        lb = base + n0 + (xy ? 0 : n1) + qi;
+    };
+    // the kind of particle j's line: the piece it lies in, or n beyond the support and in a particle's plane (nothing to
+    // form); and the entry to form it from
+    auto line_kind = [&](const BoxChunk* cp, int j, int it, uint32_t& rec) {
+        const BoxGeo b = cp->box(j);
+        int la, lb;
+        line_planes(b, it - b.line(), la, lb);
+        const double p = s_P[kPS * la], q = s_P[kPS * lb];
+        const double D = fma(p, p, q * q);
+        rec = (uint32_t)it | (uint32_t)la << 10 | (uint32_t)lb << 19;
+        if (D >= 1.0 || p == 0.0 || q == 0.0) {
+            n_eo += 2;
+            return Caps::kN;
+        }
+        int kind = 0;
+#pragma unroll
+        for (int k = 0; k + 1 < n; ++k) kind += D >= T.scale[k].b * T.scale[k].b;
+        if (kind == 0) n_ei += 2;
+        else n_em += 2;
+        return kind;
+    };
+    // all warps: the lines of a chunk by kind, into the octant values' place (free from (C2) to (P)), in any order
+    auto list_lines = [&](const BoxChunk* cp) {
+        const int off_l = lane < cp->np ? cp->box(lane).line() : INT_MAX, tot = cp->etot;
+        for (int base = warp * 32; base < tot; base += kBoxThreads) {
+            const int j = warp_owner(base, off_l, lane), it = base + lane;
+            int kind = -1;
+            uint32_t rec = 0;
+            if (it < tot) kind = line_kind(cp, j, it, rec);
+#pragma unroll
+            for (int c = 0; c < Caps::kKinds; ++c) {
+                const unsigned m = __ballot_sync(0xffffffffu, kind == c);
+                if (m == 0) continue;
+                int at = 0;
+                if (lane == 0) at = atomicAdd(&s_lines[c], __popc(m));
+                at = __shfl_sync(0xffffffffu, at, 0);
+                if (kind == c) s_list[Caps::kPair * c + at + __popc(m & below)] = rec;
+            }
+        }
+    };
+    auto next_batch = [&]() {
+        int b = 0;
+        if (lane == 0) b = atomicAdd(&s_next, 1);
+        return __shfl_sync(0xffffffffu, b, 0);
     };
 
     bool first_segment = true;
@@ -368,6 +457,10 @@ __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& 
     if (warp == 0 && beg < end) load_chunk(cp, beg, end);
     __syncthreads();
     if (beg < end) form_planes(cp);
+    if constexpr (kList) {
+        __syncthreads();
+        if (beg < end) list_lines(cp);
+    }
     __syncthreads();
 
     for (int64_t pos = beg; pos < end_all;) {
@@ -378,24 +471,14 @@ __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& 
         if (ends) end = segment_end(end);
         if (warp == 0 && more) load_chunk(nx, pos + np, end);
 
-        // (E) edge lines, block (x, y) over n0' x n1', (x, z) over n0' x n2', (y, z) over n1' x n2'
-        auto line_planes = [&](int j, int e, int& la, int& lb) {  // the planes of particle j's line e
-            const int n0 = cp->dim[j][0] + 1, n1 = cp->dim[j][1] + 1, n2 = cp->dim[j][2] + 1;
-            const int nxy = n0 * n1, nxz = n0 * n2;
-            const int blk = (e >= nxy) + (e >= nxy + nxz);
-            e -= blk == 0 ? 0 : (blk == 1 ? nxy : nxy + nxz);
-            const int pi = div_by(e, cp->mag[j][blk == 0 ? 0 : 1]), qi = e - pi * (blk == 0 ? n1 : n2);
-            la = cp->loff[j] + (blk == 2 ? n0 : 0) + pi;
-            lb = cp->loff[j] + (blk == 0 ? n0 : n0 + n1) + qi;
-        };
+        // (E) edge lines
         if constexpr (TAB) {
-            const int off_l = lane < np ? cp->eoff[lane] : INT_MAX;
+            const int off_l = lane < np ? cp->box(lane).line() : INT_MAX;
             for (int base = warp * 32; base < cp->etot; base += kBoxThreads) {
                 const int j = warp_owner(base, off_l, lane), it = base + lane;
-                const int off = __shfl_sync(0xffffffffu, off_l, j & 31);
                 if (it < cp->etot) {
                     int la, lb;
-                    line_planes(j, it - off, la, lb);
+                    line_planes(cp->box(j), it - cp->box(j).line(), la, lb);
                     const double p = fabs(s_P[kPS * la]), q = fabs(s_P[kPS * lb]);
                     if (p != 0.0 && q != 0.0) {
                         const double s = sqrt(p * p + q * q), is = 1.0 / s;
@@ -404,85 +487,81 @@ __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& 
                     }
                 }
             }
-        } else {
+        } else if constexpr (!kList) {
             const int tot = cp->etot;
-            const int off_l = lane < np ? cp->eoff[lane] : INT_MAX;
-            int cnt[Caps::kQueues];
-#pragma unroll
-            for (int c = 0; c < Caps::kQueues; ++c) cnt[c] = 0;
+            const int off_l = lane < np ? cp->box(lane).line() : INT_MAX;
+            uint32_t* const s_ql = reinterpret_cast<uint32_t*>(s_q);
+            int cnt = 0;
             for (int base = warp * 32;; base += kBoxThreads) {
                 const bool last = base >= tot;
                 if (!last) {
                     const int j = warp_owner(base, off_l, lane), it = base + lane;
-                    const int off = __shfl_sync(0xffffffffu, off_l, j & 31);
-                    int kind = -1;
+                    bool near = false;
                     uint32_t rec = 0;
                     if (it < tot) {
-                        int la, lb;
-                        line_planes(j, it - off, la, lb);
-                        const double p = s_P[kPS * la], q = s_P[kPS * lb];
-                        const double D = fma(p, p, q * q);
-                        if (D >= 1.0 || p == 0.0 || q == 0.0) {
-                            s_E[kES * it + 2 * n] = 0.0;
-                            n_eo += 2;
-                        } else {
-                            kind = 0;
-#pragma unroll
-                            for (int k = 0; k + 1 < n; ++k) kind += D >= T.scale[k].b * T.scale[k].b;
-                            if (kind == 0) n_ei += 2;
-                            else n_em += 2;
-                            rec = (uint32_t)it | (uint32_t)la << 10 | (uint32_t)lb << 19;
-                        }
+                        near = line_kind(cp, j, it, rec) == 0;
+                        if (!near) s_E[kES * it + 2 * n] = 0.0;
                     }
-#pragma unroll
-                    for (int c = 0; c < Caps::kQueues; ++c) {
-                        const unsigned m = __ballot_sync(0xffffffffu, kind == c);
-                        if (kind == c) s_q[64 * c + cnt[c] + __popc(m & below)] = rec;
-                        cnt[c] += __popc(m);
-                    }
+                    const unsigned m = __ballot_sync(0xffffffffu, near);
+                    if (near) s_ql[cnt + __popc(m & below)] = rec;
+                    cnt += __popc(m);
                     __syncwarp();
                 }
-#pragma unroll
-                for (int c = 0; c < Caps::kQueues; ++c) {
-                    // (a queue gains at most 32 entries per step, so one batch per step keeps it below 32)
-                    if (cnt[c] >= 32 || (last && cnt[c] > 0)) {
-                        const int first = max(cnt[c] - 32, 0);
-                        if (first + lane < cnt[c]) {
-                            const uint32_t rec = s_q[64 * c + first + lane];
-                            box_edge<NP, DEG>(T, c, s_P + kPS * ((rec >> 10) & 511u), s_P + kPS * (rec >> 19),
-                                              s_E + kES * (rec & 1023u));
-                        }
-                        cnt[c] = first;
-                        __syncwarp();
+                // (the queue gains at most 32 entries per step, so one batch per step keeps it below 32)
+                if (cnt >= 32 || (last && cnt > 0)) {
+                    const int first = max(cnt - 32, 0);
+                    if (first + lane < cnt) {
+                        const uint32_t rec = s_ql[first + lane];
+                        box_edge<NP, DEG>(T, 0, s_P + kPS * ((rec >> 10) & 511u), s_P + kPS * (rec >> 19), s_E + kES * (rec & 1023u));
                     }
+                    cnt = first;
+                    __syncwarp();
                 }
                 if (last) break;
+            }
+        } else {
+            int nb = 0, first[Caps::kKinds];  // batches of each kind, the costly ones first
+#pragma unroll
+            for (int c = 0; c < Caps::kKinds; ++c) {
+                first[c] = nb;
+                nb += (s_lines[c] + 31) >> 5;
+            }
+            for (int b = next_batch(); b < nb; b = next_batch()) {
+#pragma unroll
+                for (int c = 0; c < Caps::kKinds; ++c) {
+                    if (b < first[c] || (c + 1 < Caps::kKinds && b >= first[c + 1])) continue;
+                    const int e = 32 * (b - first[c]) + lane;
+                    if (e >= s_lines[c]) continue;
+                    const uint32_t rec = s_list[Caps::kPair * c + e];
+                    double* const E = s_E + kES * (rec & 1023u);
+                    if (c == Caps::kN) E[2 * n] = 0.0;
+                    else box_edge<NP, DEG>(T, c, s_P + kPS * ((rec >> 10) & 511u), s_P + kPS * (rec >> 19), E);
+                }
             }
         }
         __syncthreads();
 
         // (P) lattice points
         if constexpr (TAB) {
-            const int off_l = lane < np ? cp->poff[lane] : INT_MAX;
+            const int off_l = lane < np ? cp->box(lane).point() : INT_MAX;
             for (int base = warp * 32; base < cp->ptot; base += kBoxThreads) {
                 const int j = warp_owner(base, off_l, lane), it = base + lane;
-                const int off = __shfl_sync(0xffffffffu, off_l, j & 31);
                 if (it < cp->ptot) {
-                    const int lp = it - off;
-                    const int n0 = cp->dim[j][0] + 1, n1 = cp->dim[j][1] + 1, n2 = cp->dim[j][2] + 1;
-                    const int i = div_by(lp, cp->mag[j][2]), rem = lp - i * (n1 * n2);
-                    const int jj = div_by(rem, cp->mag[j][1]), k = rem - jj * n2;
-                    const double* const rx = s_P + kPS * (cp->loff[j] + i);
-                    const double* const ry = s_P + kPS * (cp->loff[j] + n0 + jj);
-                    const double* const rz = s_P + kPS * (cp->loff[j] + n0 + n1 + k);
+                    const BoxGeo b = cp->box(j);
+                    const int lp = it - b.point(), n1 = b.n1(), n2 = b.n2();
+                    const int i = b.by_n12(lp), rem = lp - i * (n1 * n2);
+                    const int jj = b.by_n2(rem), k = rem - jj * n2;
+                    const double* const rx = s_P + kPS * (b.plane() + i);
+                    const double* const ry = s_P + kPS * (b.plane() + b.n0() + jj);
+                    const double* const rz = s_P + kPS * (b.plane() + b.n0() + n1 + k);
                     if (rx[0] == 0.0 || ry[0] == 0.0 || rz[0] == 0.0) {
                         s_T[it] = 0.0;
                     } else {
                         // a line's first three entries are of its first axis's distance, the others of its second's
-                        const double* const E = s_E + kES * cp->eoff[j];
+                        const double* const E = s_E + kES * b.line();
                         const double* const xy = E + kES * (i * n1 + jj);
-                        const double* const xz = E + kES * (n0 * n1 + i * n2 + k);
-                        const double* const yz = E + kES * (n0 * (n1 + n2) + jj * n2 + k);
+                        const double* const xz = E + kES * (b.n01() + i * n2 + k);
+                        const double* const yz = E + kES * (b.n0_12() + rem);
                         double f = box_tab_lookup(tab, rx, xy, yz, n_clamp) + box_tab_lookup(tab, rx, xz, yz + 3, n_clamp);
                         f = f + (box_tab_lookup(tab, ry, xy + 3, xz, n_clamp) + box_tab_lookup(tab, ry, yz, xz + 3, n_clamp));
                         f = f + (box_tab_lookup(tab, rz, xz + 3, xy, n_clamp) + box_tab_lookup(tab, rz, yz + 3, xy + 3, n_clamp));
@@ -495,34 +574,34 @@ __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& 
             }
         } else {
             const int tot = cp->ptot;
-            const int off_l = lane < np ? cp->poff[lane] : INT_MAX;
+            const int off_l = lane < np ? cp->box(lane).point() : INT_MAX;
             int cnt = 0;
             const double far_c = box_centre<NP>(T, n);
             for (int base = warp * 32;; base += kBoxThreads) {
                 const bool last = base >= tot;
                 if (!last) {
                     const int j = warp_owner(base, off_l, lane), it = base + lane;
-                    const int off = __shfl_sync(0xffffffffu, off_l, j & 31);
                     bool near = false;
-                    uint32_t rec = 0;
+                    uint2 rec{0, 0};
                     if (it < tot) {
-                        const int lp = it - off;
-                        const int n0 = cp->dim[j][0] + 1, n1 = cp->dim[j][1] + 1, n2 = cp->dim[j][2] + 1;
-                        const int i = div_by(lp, cp->mag[j][2]), rem = lp - i * (n1 * n2);
-                        const int jj = div_by(rem, cp->mag[j][1]), k = rem - jj * n2;
-                        const double* const rx = s_P + kPS * (cp->loff[j] + i);
-                        const double* const ry = s_P + kPS * (cp->loff[j] + n0 + jj);
-                        const double* const rz = s_P + kPS * (cp->loff[j] + n0 + n1 + k);
+                        const BoxGeo b = cp->box(j);
+                        const int lp = it - b.point(), n0 = b.n0(), n1 = b.n1(), n2 = b.n2();
+                        const int i = b.by_n12(lp), rem = lp - i * (n1 * n2);
+                        const int jj = b.by_n2(rem), k = rem - jj * n2;
+                        const int lx = b.plane() + i, dly = n0 - i + jj, dlz = n1 - jj + k;  // its planes, and its lines:
+                        const int exy = b.line() + i * n1 + jj, dxz = b.n01() + i * n2 + k - (i * n1 + jj), dyz = n2 * dly;
+                        const double* const rx = s_P + kPS * lx;
+                        const double* const ry = rx + kPS * dly;
+                        const double* const rz = ry + kPS * dlz;
                         const double x = rx[0], y = ry[0], z = rz[0];
                         if (x == 0.0 || y == 0.0 || z == 0.0) {
                             s_T[it] = 0.0;
                         } else if (fma(x, x, fma(y, y, z * z)) < 1.0) {
                             near = true;
-                            rec = (uint32_t)j | (uint32_t)i << 5 | (uint32_t)jj << 9 | (uint32_t)k << 13;
+                            rec = uint2{(uint32_t)(it | exy << 12 | lx << 22), (uint32_t)(dly | dlz << 5 | dxz << 10 | dyz << 18)};
                         } else {
-                            const double* const E = s_E + kES * cp->eoff[j] + 2 * n;
-                            const double f = (E[kES * (i * n1 + jj)] + E[kES * (n0 * n1 + i * n2 + k)]) +
-                                             E[kES * (n0 * (n1 + n2) + jj * n2 + k)] +
+                            const double* const E = s_E + kES * exy + 2 * n;
+                            const double f = (E[0] + E[kES * dxz]) + E[kES * (dxz + dyz)] +
                                              ((rx[1 + 2 * n] + ry[1 + 2 * n]) + (rz[1 + 2 * n] + far_c));
                             s_T[it] = box_signed(f, x, y, z);
                             n_vp += 6;
@@ -536,23 +615,20 @@ __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& 
                 if (cnt >= 32 || (last && cnt > 0)) {
                     const int first = max(cnt - 32, 0);
                     if (first + lane < cnt) {
-                        const uint32_t rec = s_q[first + lane];
-                        const int j = (int)(rec & 31u), i = (int)((rec >> 5) & 15u), jj = (int)((rec >> 9) & 15u),
-                                  kk = (int)(rec >> 13);
-                        const int n0 = cp->dim[j][0] + 1, n1 = cp->dim[j][1] + 1, n2 = cp->dim[j][2] + 1;
-                        const double* const rx = s_P + kPS * (cp->loff[j] + i);
-                        const double* const ry = s_P + kPS * (cp->loff[j] + n0 + jj);
-                        const double* const rz = s_P + kPS * (cp->loff[j] + n0 + n1 + kk);
+                        const uint2 rec = s_q[first + lane];
+                        const int it = (int)(rec.x & 4095u);
+                        const double* const rx = s_P + kPS * (int)(rec.x >> 22);
+                        const double* const ry = rx + kPS * (int)(rec.y & 31u);
+                        const double* const rz = ry + kPS * (int)((rec.y >> 5) & 31u);
                         const double x = rx[0], y = ry[0], z = rz[0];
                         const double ax = fabs(x), ay = fabs(y), az = fabs(z);
                         const double r2 = fma(x, x, fma(y, y, z * z));
                         int k = 0;  // the point's piece
 #pragma unroll
                         for (int s = 0; s + 1 < n; ++s) k += r2 >= T.scale[s].b * T.scale[s].b;
-                        const double* const E = s_E + kES * cp->eoff[j] + k;
-                        const double* const exy = E + kES * (i * n1 + jj);
-                        const double* const exz = E + kES * (n0 * n1 + i * n2 + kk);
-                        const double* const eyz = E + kES * (n0 * (n1 + n2) + jj * n2 + kk);
+                        const double* const exy = s_E + kES * (int)((rec.x >> 12) & 1023u) + k;
+                        const double* const exz = exy + kES * (int)((rec.y >> 10) & 255u);
+                        const double* const eyz = exz + kES * (int)(rec.y >> 18);
                         // the smallest offset first: the other two's angles are then at most pi/4
                         const bool mx = ax <= ay && ax <= az, my = !mx && ay <= az;
                         const double* const r0 = mx ? rx : (my ? ry : rz);
@@ -572,7 +648,7 @@ __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& 
                                                    exy[n], fabs(r0[0]), r0[2 + k], fabs(r1[0]), r1[1], r1[2 + k],
                                                    fabs(r2_[0]), r2_[1], r2_[2 + k]);
                         if (k > 0) f += ((rx[1 + n + k] + ry[1 + n + k]) + (rz[1 + n + k] + box_centre<NP>(T, k)));
-                        s_T[cp->poff[j] + (i * n1 + jj) * n2 + kk] = box_signed(f, x, y, z);
+                        s_T[it] = box_signed(f, x, y, z);
                         n_vp += 6;
                     }
                     cnt = first;
@@ -585,22 +661,26 @@ __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& 
 
         // (C1) the chunk's (particle, cell) pairs, into the edge records' place (dead after (P))
         double* const s_cm = s_E;
+        if (threadIdx.x < Caps::kKinds) s_lines[threadIdx.x] = 0;  // for the next chunk
+        if (threadIdx.x == 0) s_next = 0;
+        if (more) form_planes(nx);
         {
             const int tot = cp->ctot;
-            const int off_l = lane < np ? cp->coff[lane] : INT_MAX;
+            const int off_l = lane < np ? cp->box(lane).cell() : INT_MAX;
             for (int base = warp * 32; base < tot; base += kBoxThreads) {
                 const int j = warp_owner(base, off_l, lane), it = base + lane;
-                const int off = __shfl_sync(0xffffffffu, off_l, j & 31);
                 if (it < tot) {
-                    const int lc = it - off;
-                    const int d1 = cp->dim[j][1], d2 = cp->dim[j][2];
-                    const int i = div_by(lc, cp->cmag[j][1]), rem = lc - i * (d1 * d2);
-                    const int jj = div_by(rem, cp->cmag[j][0]), k = rem - jj * d2;
+                    const BoxGeo b = cp->box(j);
+                    const uint32_t cm = cp->cmag[j];
+                    const int lc = it - b.cell(), d1 = b.n1() - 1, d2 = b.n2() - 1;
+                    const int i = (int)(((uint32_t)lc * (cm >> 16)) >> 15), rem = lc - i * (d1 * d2);
+                    const int jj = (int)(((uint32_t)rem * (cm & 0xffffu)) >> 15), k = rem - jj * d2;
                     ++n_bbox;
-                    const double radius = cp->H[j];
-                    const double ex = fmax(fabs(cp->x[j] - s_cc[0][cp->lo[j][0] + i]) - g.hpx, 0.0);
-                    const double ey = fmax(fabs(cp->y[j] - s_cc[1][cp->lo[j][1] + jj]) - g.hpy, 0.0);
-                    const double ez = fmax(fabs(cp->z[j] - s_cc[2][cp->lo[j][2] + k]) - g.hpz, 0.0);
+                    const double4 at = cp->at[j];
+                    const double radius = at.w;
+                    const double ex = fmax(fabs(at.x - s_cc[0][b.lo0() + i]) - g.hpx, 0.0);
+                    const double ey = fmax(fabs(at.y - s_cc[1][b.lo1() + jj]) - g.hpy, 0.0);
+                    const double ez = fmax(fabs(at.z - s_cc[2][b.lo2() + k]) - g.hpz, 0.0);
                     // the support test of the pair counters, rounded as the host restatement rounds it
                     const bool in = add_rn(add_rn(mul_rn(ex, ex), mul_rn(ey, ey)), mul_rn(ez, ez)) < mul_rn(radius, radius);
                     n_sphere += in;
@@ -608,7 +688,7 @@ __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& 
                     if (!CULL || in) {
                         ++n_eval;
                         const int n2 = d2 + 1, n12 = (d1 + 1) * n2;
-                        const double* const Tp = s_T + cp->poff[j] + (i * (d1 + 1) + jj) * n2 + k;
+                        const double* const Tp = s_T + b.point() + i * n12 + jj * n2 + k;
                         const double m1 = (Tp[n12 + n2 + 1] - Tp[n12 + n2]) - (Tp[n12 + 1] - Tp[n12]);
                         const double m0 = (Tp[n2 + 1] - Tp[n2]) - (Tp[1] - Tp[0]);
                         msum = m1 - m0;
@@ -626,6 +706,7 @@ __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& 
 
         // (C2) the owned cells' sums: a warp's 32 cells are four z rows of one x slab; it visits the particles whose
         // boxes reach them
+        const BoxGeo mine = cp->box(lane < np ? lane : 0);
 #pragma unroll
         for (int c = 0; c < kBoxCells; ++c) {
             const int li = threadIdx.x + c * kBoxThreads;
@@ -634,8 +715,8 @@ __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& 
             const int ly0 = ly & ~3;
             bool hit = false;
             if (lane < np) {
-                const int i = lx - cp->lo[lane][0], j0 = cp->lo[lane][1];
-                hit = i >= 0 && i < cp->dim[lane][0] && j0 < ly0 + 4 && j0 + cp->dim[lane][1] > ly0;
+                const int i = lx - mine.lo0(), j0 = mine.lo1();
+                hit = i >= 0 && i < mine.n0() - 1 && j0 < ly0 + 4 && j0 + mine.n1() - 1 > ly0;
             }
             unsigned todo = __ballot_sync(0xffffffffu, hit);
             if (todo == 0 && !ends) continue;
@@ -643,15 +724,17 @@ __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& 
             double a2 = s_acc[2 * kTileCells + li], a3 = s_acc[3 * kTileCells + li];
             for (; todo; todo &= todo - 1) {
                 const int j = __ffs((int)todo) - 1;
-                const int i = lx - cp->lo[j][0], jj = ly - cp->lo[j][1], k = lz - cp->lo[j][2];
-                const int d1 = cp->dim[j][1], d2 = cp->dim[j][2];
+                const BoxGeo b = cp->box(j);
+                const int i = lx - b.lo0(), jj = ly - b.lo1(), k = lz - b.lo2();
+                const int d1 = b.n1() - 1, d2 = b.n2() - 1;
                 if ((unsigned)jj >= (unsigned)d1 || (unsigned)k >= (unsigned)d2) continue;
-                const double mm = s_cm[cp->coff[j] + (i * d1 + jj) * d2 + k] * cp->m[j];
+                const double4 mv = cp->mv[j];
+                const double mm = s_cm[b.cell() + (i * d1 + jj) * d2 + k] * mv.x;
                 if (mm == 0.0) continue;
                 a0 = add_rn(a0, mm);
-                a1 = fma(mm, cp->vx[j], a1);
-                a2 = fma(mm, cp->vy[j], a2);
-                a3 = fma(mm, cp->vz[j], a3);
+                a1 = fma(mm, mv.y, a1);
+                a2 = fma(mm, mv.z, a2);
+                a3 = fma(mm, mv.w, a3);
             }
             if (SEQ && ends) {  // the first segment's sums as they are, the others' added
                 const double v[4] = {a0, a1, a2, a3};
@@ -668,7 +751,8 @@ __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& 
             s_acc[3 * kTileCells + li] = a3;
         }
         if (ends) first_segment = false;
-        if (more) form_planes(nx);
+        if constexpr (kList)
+            if (more) list_lines(nx);
         __syncthreads();
         pos += np;
         cp = nx;

@@ -169,7 +169,7 @@ KIWI_HD double cone_face(const KiwiConeTable& T, const KiwiConeRegion* R, const 
                     const KiwiConeScale& g = T.scale[s];
                     const double t2 = fma(g.b, g.b, -P);
                     if (net[s] != 0 && t2 > 0.0 && r0 < g.b) {
-                        const double it = fm_rsqrt(t2), t = t2 * it, ib = 1.0 / g.b, iR = fm_rcp(R0);
+                        const double it = fm_rsqrt(t2), t = t2 * it, ib = g.ib, iR = fm_rcp(R0);
                         const double ang = fm_atan_pos((r0 * ib) * (t * iR), (g.b * R0) * (it * fm_rcp(r0)));
                         const double dB = box_xp(T.reg[s].B, 6, (DEG + 1) / 2, X, P) -
                                           (s + 1 < NP ? box_xp(T.reg[s + 1 < NP ? s + 1 : 0].B, 6, (DEG + 1) / 2, X, P) : 0.0);

@@ -507,7 +507,7 @@ def header_text():
         "    double c, C[39], Q[15], a[6], D[84], R[28];",
         "} KiwiBoxRegion;",
         "typedef struct KiwiBoxScale {",
-        "    double b, m, G[12], fp[7], ap[6], f[14], h[15], A[21];",
+        "    double b, ib, m, G[12], fp[7], ap[6], f[14], h[15], A[21];",
         "} KiwiBoxScale;",
         "typedef struct KiwiBoxTable {",
         "    int npiece;                       /* pieces: piece k holds scale[k-1].b <= r < scale[k].b */",
@@ -528,7 +528,7 @@ def header_text():
             "{" + _num(r["c"]) + ",\n        " + ",\n        ".join(_row(r[k]) for k in REG) + "}"
             for r in t["reg"] + [zr] * (3 - t["npiece"])) + "},")
         L.append("      {" + ",\n       ".join(
-            "{" + f"{_num(s['b'])}, {_num(s['m'])},\n        " + ",\n        ".join(_row(s[k]) for k in SCL) +
+            "{" + f"{_num(s['b'])}, {_num(1.0 / s['b'] if s['b'] else 0.0)}, {_num(s['m'])},\n        " + ",\n        ".join(_row(s[k]) for k in SCL) +
             "}" for s in t["scale"] + [zs] * (3 - t["npiece"])) + "}},")
     L.append("};")
     L.append("")
@@ -540,7 +540,7 @@ def header_text():
         "    double c, V[140], B[28], a[6];",
         "} KiwiConeRegion;",
         "typedef struct KiwiConeScale {",
-        "    double b, m, fp[7], ap[6], f[14], h[15], A[21];",
+        "    double b, ib, m, fp[7], ap[6], f[14], h[15], A[21];",
         "} KiwiConeScale;",
         "typedef struct KiwiConeTable {",
         "    int npiece, deg;",
@@ -556,7 +556,7 @@ def header_text():
             "{" + _num(r["c"]) + ",\n        " + ",\n        ".join(_row(r[k]) for k in CREG) + "}"
             for r in t["creg"] + [zr] * (3 - t["npiece"])) + "},")
         L.append("      {" + ",\n       ".join(
-            "{" + f"{_num(s['b'])}, {_num(s['m'])},\n        " + ",\n        ".join(_row(s[k]) for k in CSCL) +
+            "{" + f"{_num(s['b'])}, {_num(1.0 / s['b'] if s['b'] else 0.0)}, {_num(s['m'])},\n        " + ",\n        ".join(_row(s[k]) for k in CSCL) +
             "}" for s in t["cscale"] + [zs] * (3 - t["npiece"])) + "}},")
     L.append("};")
     L.append("")
