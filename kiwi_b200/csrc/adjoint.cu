@@ -16,15 +16,15 @@
 // taken with respect to the particle's coordinates (u = plane - particle).
 //
 // One CTA takes a run of consecutive (tile, particle) entries, tile by tile: their planes, edge lines and lattice
-// points are formed once each as in box_tile.cuh, and then a warp takes each particle, assembles its cells from
-// their 8 corners (value and derivatives alike), weighs them with the cells' cotangents and writes the particle's
-// partial gradient for this tile to its entry.  An entry's partial depends on nothing else in the run, so the
+// points are formed once each as in box_tile.cuh, and then each particle's cells are assembled from their 8 corners
+// (value and derivatives alike), weighed with the cells' cotangents and summed to the particle's partial gradient for
+// this tile, which goes to its entry.  An entry's partial depends on nothing else in the run, so the
 // runs are cut to fill the chip whatever the tiles hold.  k_adjoint_reduce adds each particle's entries in tile
 // order.  Deterministic, no atomics on the gradients.
 //
 // Against forward-mode dual numbers through the point-wise series (one CTA per tile, 255 registers with
-// spills): 100 k column particles on 80^3, cubic, forward and backward: 53.8 -> 17.2 ms; 2 k particles on 21 x 19 x 25 (36 tiles), Wendland C4:
-// 90.0 -> 5.2 ms.
+// spills): 100 k column particles on 80^3, cubic, forward and backward: 53.8 -> 13.5 ms; 2 k particles on 21 x 19 x 25 (36 tiles), Wendland C4:
+// 90.0 -> 1.3 ms.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -32,6 +32,7 @@
 
 #include "binning.cuh"
 #include "box_grad.cuh"
+#include "box_tile.cuh"
 #include "cart_common.cuh"
 #include "ctx.hpp"
 #include "engine.hpp"
@@ -43,46 +44,62 @@ namespace kiwi_b200 {
 
 namespace {
 
-constexpr int kAdjThreads = 256, kAdjWarps = kAdjThreads / 32;
+constexpr int kAdjThreads = 512, kAdjWarps = kAdjThreads / 32;
 constexpr int kAdjPMax = 32;
-constexpr int kAdjComps = 5;  // a point's T and its derivatives with respect to x, y, z, h
+constexpr int kAdjComps = 4;  // a point's T and its derivatives with respect to x, y, z
+constexpr int kAdjUnit = 128;  // cells a warp sums at a time
 
 static __constant__ KiwiBoxTable c_adj_box[KIWI_NUM_KERNELS];
 
-// Chunk capacities: two CTAs per SM (a full 8^3 box has 729 points, 243 edge lines and 27 planes).
+// Chunk capacities: one CTA per SM (a full 8^3 box has 729 points, 243 edge lines and 27 planes).
 template <int NP>
 struct AdjCaps {
-    static constexpr int kN = NP;
-    static constexpr int kPt = NP == 1 ? 1280 : (NP == 2 ? 1024 : 800), kPair = NP == 1 ? 512 : (NP == 2 ? 352 : 272),
-                         kPlane = NP == 1 ? 192 : (NP == 2 ? 136 : 120);
-    static constexpr int kOffE = kAdjComps * kPt;
-    static constexpr int kOffP = kOffE + box_grad_edge_stride(kN) * kPair;
-    static constexpr int kEnd = kOffP + box_grad_plane_stride(kN) * kPlane;
-    static constexpr size_t kSmem = sizeof(double) * kEnd + sizeof(uint32_t) * 64 * kAdjWarps * kN;
-    static_assert(kPair <= 1024 && kPlane <= 512, "packed edge entries");
+    static constexpr int kPt = NP == 1 ? 2688 : (NP == 2 ? 2190 : 2040), kPair = NP == 1 ? 1023 : (NP == 2 ? 740 : 576),
+                         kPlane = NP == 1 ? 352 : (NP == 2 ? 270 : 200);
+    static constexpr int kKinds = NP + 1;  // of edge lines (box_tile.cuh)
+    // dynamic shared memory, in doubles: the points' values (and before them the lists of lines), the lists of near
+    // and far points, the edge records (and after them the units' sums), the plane records
+    static constexpr int kOffL = kAdjComps * kPt;
+    static constexpr int kOffE = kOffL + kPt;
+    static constexpr int kOffP = kOffE + box_grad_edge_stride(NP) * kPair;
+    static constexpr int kEnd = kOffP + box_grad_plane_stride(NP) * kPlane;
+    static constexpr size_t kSmem = sizeof(double) * kEnd;
+    static_assert(kPair <= 1024 && kPlane <= 512 && kPt <= 4096, "BoxGeo's fields and the listed points'");
+    static_assert(kKinds * kPair <= 2 * kAdjComps * kPt, "the lists of lines fit");
+    static_assert(8 * (kAdjPMax + kPt / kAdjUnit) <= box_grad_edge_stride(NP) * kPair, "the units' sums fit");
 };
 
 struct AdjGrads {
     double *x, *y, *z, *h, *m, *vx, *vy, *vz;
 };
 
+// Consecutive entries of one tile: their particles and boxes (box_tile.cuh; a box's `cell` is its first unit), and the
+// tile's planes and cell centres.
 struct AdjChunk {
-    double x[kAdjPMax], y[kAdjPMax], z[kAdjPMax], H[kAdjPMax], iH[kAdjPMax], m[kAdjPMax], vx[kAdjPMax], vy[kAdjPMax],
-        vz[kAdjPMax];
-    int lo[kAdjPMax][3], dim[kAdjPMax][3];  // lo relative to the tile
-    int loff[kAdjPMax], eoff[kAdjPMax], poff[kAdjPMax];
-    uint32_t entry[kAdjPMax];
-    uint32_t mag[kAdjPMax][3];   // div_magic of n1', n2' and n1' n2'
-    uint32_t cmag[kAdjPMax][2];  // div_magic of n2 and n1 n2
-    int np, ltot, etot, ptot;
+    double4 at[kAdjPMax], mv[kAdjPMax];
+    int4 geo[kAdjPMax];
+    double iH[kAdjPMax];
+    uint32_t cmag[kAdjPMax], entry[kAdjPMax];
+    double pl[3][kTileX + 1], cc[3][kTileX];
+    int bx, by, bz;
+    int np, ltot, etot, ptot, utot;
+    __device__ __forceinline__ BoxGeo box(int j) const { return BoxGeo{geo[j]}; }
 };
 
 // The partial gradients of the sorted entries [blockIdx.x per_block, ..): keys their tiles, list their entry
 // numbers, owner the particle of an entry; part receives 8 doubles per entry: dL/dm, dL/d(x, y, z, h),
 // dL/d(vx, vy, vz) over the entry's tile.
+//
+// A chunk is a few boxes at most (a point's and a line's records are three to four times the forward's), so what a
+// phase gives to a warp has to be cut across boxes: lines by kind and points by piece are listed over the whole CTA and
+// taken 32 of a kind by whichever warp is free, and a box's cells are summed in units of kAdjUnit by different warps,
+// the units' sums then added in order.  One CTA holds the whole SM's shared memory: three full boxes instead of one in
+// each of two.  The kinds share one copy of the code: two copies of each evaluation overflowed the instruction cache.
+// Forward and backward of 100 k column particles on 80^3, cubic: 16.6 ms (warps sorting for themselves, a warp to a
+// box: half of the warps' time at the barriers) -> 15.3 (lists, units) -> 14.1 (one copy) -> 13.5 (one CTA per SM).
 // KERNEL: the kernel's table; NP, DEG: its pieces and largest power.
 template <int KERNEL, int NP, int DEG>
-__global__ void __launch_bounds__(kAdjThreads, 2) k_cart_adjoint_box(CartGeom g, DevParticles P,
+__global__ void __launch_bounds__(kAdjThreads, 1) k_cart_adjoint_box(CartGeom g, DevParticles P,
                                                                      const uint32_t* __restrict__ keys,
                                                                      const uint32_t* __restrict__ list,
                                                                      const uint32_t* __restrict__ owner, int64_t total,
@@ -90,346 +107,347 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_cart_adjoint_box(CartGeom g,
                                                                      double* __restrict__ part,
                                                                      DevStats* __restrict__ st) {
     using Caps = AdjCaps<NP>;
-    __shared__ AdjChunk s_cp;
-    __shared__ double s_pl[3][kTileX + 1], s_cc[3][kTileX];
-    __shared__ double s_C[NP == 2 ? 1 : (kBoxC + kBoxD + 1) * NP];
-    __shared__ int64_t s_seg_end;
+    __shared__ AdjChunk s_cp[2];
+    // listed lines by kind; near points of the first piece, of later ones, far points; (E)'s and (P)'s next batch
+    __shared__ int s_lines[Caps::kKinds], s_pts[3], s_next[2];
+    constexpr int kCS = kBoxC + kBoxD + 1;
+    __shared__ double s_C[kCS * NP];
     extern __shared__ double s_dyn[];
     const KiwiBoxTable& T = c_adj_box[KERNEL];
     constexpr int n = NP, kPS = box_grad_plane_stride(NP), kES = box_grad_edge_stride(NP);
     double* const s_T = s_dyn;
     double* const s_E = s_dyn + Caps::kOffE;
     double* const s_P = s_dyn + Caps::kOffP;
+    uint32_t* const s_list = reinterpret_cast<uint32_t*>(s_T);
+    uint32_t* const s_near = reinterpret_cast<uint32_t*>(s_dyn + Caps::kOffL);  // first piece from the front, others the back
+    uint32_t* const s_far = s_near + Caps::kPt;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1;
-    uint32_t* const s_q = reinterpret_cast<uint32_t*>(s_dyn + Caps::kEnd) + 64 * Caps::kN * warp;
-    constexpr int kCS = kBoxC + kBoxD + 1;
-    if (NP != 2)
-        for (int i = threadIdx.x; i < kCS * n; i += kAdjThreads) {
-            const int k = i / kCS, c = i % kCS;
-            s_C[i] = c < kBoxC ? T.reg[k].C[c] : (c < kBoxC + kBoxD ? T.reg[k].D[c - kBoxC] : T.reg[k].c);
-        }
+    for (int i = threadIdx.x; i < kCS * n; i += kAdjThreads) {
+        const int k = i / kCS, c = i % kCS;
+        s_C[i] = c < kBoxC ? T.reg[k].C[c] : (c < kBoxC + kBoxD ? T.reg[k].D[c - kBoxC] : T.reg[k].c);
+    }
+    auto reset = [&]() {
+        if (threadIdx.x < Caps::kKinds) s_lines[threadIdx.x] = 0;
+        if (threadIdx.x < 3) s_pts[threadIdx.x] = 0;
+        if (threadIdx.x < 2) s_next[threadIdx.x] = 0;
+    };
+    reset();
     const int64_t ncell = (int64_t)g.nx * g.ny * g.nz;
     unsigned n_eval = 0, n_neg = 0;
     const int64_t beg = (int64_t)blockIdx.x * per_block, end = min(beg + (int64_t)per_block, total);
 
-    for (int64_t pos = beg; pos < end;) {
-        // the run of this tile's entries
-        const int64_t t = keys[pos];
-        __syncthreads();
-        if (warp == 0) {
-            int64_t e = pos;
-            for (;;) {  // at most per_block / 32 steps
-                const int64_t i = e + lane;
-                const unsigned same = __ballot_sync(0xffffffffu, i < end && keys[i] == (uint32_t)t);
-                e += __popc(same);
-                if (same != 0xffffffffu) break;
-            }
-            if (lane == 0) s_seg_end = e;
-        }
+    // warp 0: the entries from `pos` on that lie in its tile, as many as the capacities take
+    auto load_chunk = [&](AdjChunk& c, int64_t pos) {
+        const uint32_t t = keys[pos];
         const int tz = (int)(t % g.ntz), ty = (int)((t / g.ntz) % g.nty), tx = (int)(t / ((int64_t)g.ntz * g.nty));
         const int bx = tx * kTileX, by = ty * kTileY, bz = tz * kTileZ;
-        if (threadIdx.x >= 32 && threadIdx.x < 32 + 3 * (kTileX + 1)) {
-            const int i = threadIdx.x - 32, a = i / (kTileX + 1), l = i % (kTileX + 1);
+        if (lane < 3 * (kTileX + 1)) {
+            const int a = lane / (kTileX + 1), l = lane % (kTileX + 1);
             const double mn = a == 0 ? g.x_min : (a == 1 ? g.y_min : g.z_min);
             const double d = a == 0 ? g.dpx : (a == 1 ? g.dpy : g.dpz);
             const int b0 = a == 0 ? bx : (a == 1 ? by : bz);
-            s_pl[a][l] = add_rn(mn, mul_rn((double)(b0 + l), d));
-            if (l < kTileX) s_cc[a][l] = cell_centre(mn, b0 + l, d);
+            c.pl[a][l] = add_rn(mn, mul_rn((double)(b0 + l), d));
+            if (l < kTileX) c.cc[a][l] = cell_centre(mn, b0 + l, d);
+        }
+        static_assert(3 * (kTileX + 1) <= 32, "a lane per plane of the tile");
+        const int64_t idx = pos + lane;
+        const bool in = idx < end && keys[idx] == t;
+        int nl = 0, ne = 0, npt = 0, nu = 0, lo0 = 0, lo1 = 0, lo2 = 0, d0 = 0, d1 = 0, d2 = 0;
+        double px = 0, py = 0, pz = 0, ph = 1, pm = 0, pvx = 0, pvy = 0, pvz = 0;
+        uint32_t e = 0;
+        if (in) {
+            e = list[idx];
+            const uint32_t p = owner[e];
+            px = P.x[p]; py = P.y[p]; pz = P.z[p]; ph = P.h[p];
+            pm = P.m[p]; pvx = P.vx[p]; pvy = P.vy[p]; pvz = P.vz[p];
+            CellBox b;
+            bool outside;
+            particle_cell_box(g, px, py, pz, ph, b, &outside);
+            lo0 = max(b.x0 - bx, 0); lo1 = max(b.y0 - by, 0); lo2 = max(b.z0 - bz, 0);
+            d0 = min(b.x1 - bx, kTileX - 1) - lo0 + 1;
+            d1 = min(b.y1 - by, kTileY - 1) - lo1 + 1;
+            d2 = min(b.z1 - bz, kTileZ - 1) - lo2 + 1;
+            const int n0 = d0 + 1, n1 = d1 + 1, n2 = d2 + 1;
+            nl = n0 + n1 + n2;
+            ne = n0 * n1 + n0 * n2 + n1 * n2;
+            npt = n0 * n1 * n2;
+            nu = (d0 * d1 * d2 + kAdjUnit - 1) / kAdjUnit;
+        }
+        int il = nl, ie = ne, ip = npt, iu = nu;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int vl = __shfl_up_sync(0xffffffffu, il, o), ve = __shfl_up_sync(0xffffffffu, ie, o),
+                      vp = __shfl_up_sync(0xffffffffu, ip, o), vu = __shfl_up_sync(0xffffffffu, iu, o);
+            if (lane >= o) {
+                il += vl;
+                ie += ve;
+                ip += vp;
+                iu += vu;
+            }
+        }
+        const bool fits = in && il <= Caps::kPlane && ie <= Caps::kPair && ip <= Caps::kPt;
+        const unsigned no = ~__ballot_sync(0xffffffffu, fits);  // the entries before the first that is not taken
+        const int np = no ? __ffs((int)no) - 1 : 32;
+        if (lane < np) {
+            const double H = mul_rn(g.support_in_h, ph);
+            c.at[lane] = double4{px, py, pz, H};
+            c.mv[lane] = double4{pm, pvx, pvy, pvz};
+            c.iH[lane] = 1.0 / H;
+            c.entry[lane] = e;
+            c.geo[lane] = box_geo(d0 + 1, d1 + 1, d2 + 1, lo0, lo1, lo2, il - nl, ie - ne, ip - npt, iu - nu);
+            c.cmag[lane] = box_cell_magic(d1, d2);
+        }
+        if (lane == np - 1) {
+            c.np = np;
+            c.ltot = il;
+            c.etot = ie;
+            c.ptot = ip;
+            c.utot = iu;
+            c.bx = bx; c.by = by; c.bz = bz;
+        }
+    };
+    // all warps: a chunk's plane records
+    auto form_planes = [&](const AdjChunk* cp) {
+        const int off_l = lane < cp->np ? cp->box(lane).plane() : INT_MAX, tot = cp->ltot;
+        for (int base = warp * 32; base < tot; base += kAdjThreads) {
+            const int j = warp_owner(base, off_l, lane), it = base + lane;
+            if (it < tot) {
+                const BoxGeo b = cp->box(j);
+                int l = it - b.plane();
+                const int n0 = b.n0(), n1 = b.n1();
+                const int a = (l >= n0) + (l >= n0 + n1);
+                l -= a == 0 ? 0 : (a == 1 ? n0 : n0 + n1);
+                const double4 at = cp->at[j];
+                const double c = a == 0 ? at.x : (a == 1 ? at.y : at.z);
+                const int lo = a == 0 ? b.lo0() : (a == 1 ? b.lo1() : b.lo2());
+                box_grad_plane<NP, DEG>(T, (cp->pl[a][lo + l] - c) * cp->iH[j], s_P + kPS * it);
+            }
+        }
+    };
+    // a lane's item to a list: its place, counted in *count from `first` up or down
+    auto append = [&](bool mine, int* count, uint32_t* first, bool down, uint32_t rec) {
+        const unsigned m = __ballot_sync(0xffffffffu, mine);
+        if (m == 0) return;
+        int at = 0;
+        if (lane == 0) at = atomicAdd(count, __popc(m));
+        at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & below);
+        if (mine) first[down ? -at : at] = rec;
+    };
+    // all warps: a chunk's lines by kind and its points by piece, in any order
+    auto list_items = [&](const AdjChunk* cp) {
+        {
+            const int off_l = lane < cp->np ? cp->box(lane).line() : INT_MAX, tot = cp->etot;
+            for (int base = warp * 32; base < tot; base += kAdjThreads) {
+                const int j = warp_owner(base, off_l, lane), it = base + lane;
+                int kind = -1;
+                uint32_t rec = 0;
+                if (it < tot) {
+                    const BoxGeo b = cp->box(j);
+                    int la, lb;
+                    b.line_planes(it - b.line(), la, lb);
+                    const double p = s_P[kPS * la], q = s_P[kPS * lb];
+                    const double D = fma(p, p, q * q);
+                    rec = (uint32_t)it | (uint32_t)la << 10 | (uint32_t)lb << 19;
+                    kind = n;
+                    if (D < 1.0 && p != 0.0 && q != 0.0) {
+                        kind = 0;
+#pragma unroll
+                        for (int k = 0; k + 1 < n; ++k) kind += D >= T.scale[k].b * T.scale[k].b;
+                    }
+                }
+#pragma unroll
+                for (int c = 0; c < Caps::kKinds; ++c) append(kind == c, &s_lines[c], s_list + Caps::kPair * c, false, rec);
+            }
+        }
+        {
+            const int off_l = lane < cp->np ? cp->box(lane).point() : INT_MAX, tot = cp->ptot;
+            // (from the last warp on: the first ones had the lines' last share)
+            for (int base = (kAdjWarps - 1 - warp) * 32; base < tot; base += kAdjThreads) {
+                const int j = warp_owner(base, off_l, lane), it = base + lane;
+                int kind = -1;
+                uint32_t rec = 0;
+                if (it < tot) {
+                    const BoxGeo b = cp->box(j);
+                    const int lp = it - b.point(), n0 = b.n0(), n1 = b.n1(), n2 = b.n2();
+                    const int i = b.by_n12(lp), rem = lp - i * (n1 * n2);
+                    const int jj = b.by_n2(rem), k = rem - jj * n2;
+                    const double* const rx = s_P + kPS * (b.plane() + i);
+                    const double* const ry = s_P + kPS * (b.plane() + n0 + jj);
+                    const double* const rz = s_P + kPS * (b.plane() + n0 + n1 + k);
+                    const double x = rx[0], y = ry[0], z = rz[0];
+                    const double r2 = fma(x, x, fma(y, y, z * z));
+                    rec = (uint32_t)(it | j << 12 | i << 17 | jj << 21 | k << 25);
+                    kind = x == 0.0 || y == 0.0 || z == 0.0 || !(r2 < 1.0)
+                               ? 2
+                               : (n > 1 && r2 >= T.scale[0].b * T.scale[0].b ? 1 : 0);
+                }
+                append(kind == 0, &s_pts[0], s_near, false, rec);
+                if (n > 1) append(kind == 1, &s_pts[1], s_near + Caps::kPt - 1, true, rec);
+                append(kind == 2, &s_pts[2], s_far, false, rec);
+            }
+        }
+    };
+    auto next_batch = [&](int* counter) {
+        int b = 0;
+        if (lane == 0) b = atomicAdd(counter, 1);
+        return __shfl_sync(0xffffffffu, b, 0);
+    };
+
+    const AdjChunk* cp = &s_cp[0];
+    if (warp == 0) load_chunk(s_cp[0], beg);
+    __syncthreads();
+    form_planes(cp);
+    __syncthreads();
+    list_items(cp);
+    __syncthreads();
+
+    for (int64_t pos = beg; pos < end;) {
+        AdjChunk& nx = cp == &s_cp[0] ? s_cp[1] : s_cp[0];
+        const int np = cp->np;
+        const bool more = pos + np < end;
+        if (warp == 0 && more) load_chunk(nx, pos + np);
+
+        // (E) edge lines
+        {
+            int nb = 0, first[Caps::kKinds];  // batches of each kind, the costly ones first
+#pragma unroll
+            for (int c = 0; c < Caps::kKinds; ++c) {
+                first[c] = nb;
+                nb += (s_lines[c] + 31) >> 5;
+            }
+            for (int b = next_batch(&s_next[0]); b < nb; b = next_batch(&s_next[0])) {
+                int c = 0, f = 0;
+#pragma unroll
+                for (int k = 1; k < Caps::kKinds; ++k)
+                    if (b >= first[k]) c = k, f = first[k];
+                const int e = 32 * (b - f) + lane;
+                if (e >= s_lines[c]) continue;
+                const uint32_t rec = s_list[Caps::kPair * c + e];
+                double* const E = s_E + kES * (rec & 1023u);
+                if (c == n) E[6 * n] = E[6 * n + 1] = E[6 * n + 2] = 0.0;
+                else box_grad_edge<NP, DEG>(T, c, s_P + kPS * ((rec >> 10) & 511u), s_P + kPS * (rec >> 19), E);
+            }
         }
         __syncthreads();
-        const int64_t seg_end = s_seg_end;
 
-        for (; pos < seg_end;) {
-            // (L) the next particles, as many as the capacities take
-            if (warp == 0) {
-                const int64_t idx = pos + lane;
-                int nl = 0, ne = 0, npt = 0, lo0 = 0, lo1 = 0, lo2 = 0, d0 = 0, d1 = 0, d2 = 0;
-                double px = 0, py = 0, pz = 0, ph = 1, pm = 0, pvx = 0, pvy = 0, pvz = 0;
-                uint32_t e = 0;
-                if (idx < seg_end) {
-                    e = list[idx];
-                    const uint32_t p = owner[e];
-                    px = P.x[p]; py = P.y[p]; pz = P.z[p]; ph = P.h[p];
-                    pm = P.m[p]; pvx = P.vx[p]; pvy = P.vy[p]; pvz = P.vz[p];
-                    CellBox b;
-                    bool outside;
-                    particle_cell_box(g, px, py, pz, ph, b, &outside);
-                    lo0 = max(b.x0 - bx, 0); lo1 = max(b.y0 - by, 0); lo2 = max(b.z0 - bz, 0);
-                    d0 = min(b.x1 - bx, kTileX - 1) - lo0 + 1;
-                    d1 = min(b.y1 - by, kTileY - 1) - lo1 + 1;
-                    d2 = min(b.z1 - bz, kTileZ - 1) - lo2 + 1;
-                    const int n0 = d0 + 1, n1 = d1 + 1, n2 = d2 + 1;
-                    nl = n0 + n1 + n2;
-                    ne = n0 * n1 + n0 * n2 + n1 * n2;
-                    npt = n0 * n1 * n2;
-                }
-                int il = nl, ie = ne, ip = npt;
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int vl = __shfl_up_sync(0xffffffffu, il, o), ve = __shfl_up_sync(0xffffffffu, ie, o),
-                              vp = __shfl_up_sync(0xffffffffu, ip, o);
-                    if (lane >= o) {
-                        il += vl;
-                        ie += ve;
-                        ip += vp;
+        // (P) points
+        {
+            const int nn[3] = {s_pts[0], s_pts[1], s_pts[2]};
+            const int b1 = (nn[0] + 31) >> 5, b2 = b1 + ((nn[1] + 31) >> 5), nb = b2 + ((nn[2] + 31) >> 5);
+            // a point's values, with the offsets' signs: d/d(particle x) of sgn T(|ux|, ..) = -sgn(uy) sgn(uz) T_x
+            auto put = [&](int it, int j, double x, double y, double z, const double* v) {
+                const double iH = cp->iH[j];
+                const double sx = x > 0.0 ? 1.0 : -1.0, sy = y > 0.0 ? 1.0 : -1.0, sz = z > 0.0 ? 1.0 : -1.0;
+                s_T[it] = sx * sy * sz * v[0];
+                s_T[Caps::kPt + it] = -sy * sz * v[1] * iH;
+                s_T[2 * Caps::kPt + it] = -sx * sz * v[2] * iH;
+                s_T[3 * Caps::kPt + it] = -sx * sy * v[3] * iH;
+            };
+            for (int b = next_batch(&s_next[1]); b < nb; b = next_batch(&s_next[1])) {
+                const int kind = b < b1 ? 0 : (b < b2 ? 1 : 2);
+                const int e = 32 * (b - (kind == 0 ? 0 : (kind == 1 ? b1 : b2))) + lane;
+                if (e >= (kind == 0 ? nn[0] : (kind == 1 ? nn[1] : nn[2]))) continue;
+                const uint32_t rec = kind == 0 ? s_near[e] : (kind == 1 ? s_near[Caps::kPt - 1 - e] : s_far[e]);
+                const int it = (int)(rec & 4095u), j = (int)((rec >> 12) & 31u), i = (int)((rec >> 17) & 15u),
+                          jj = (int)((rec >> 21) & 15u), kk = (int)(rec >> 25);
+                const BoxGeo bg = cp->box(j);
+                const int n0 = bg.n0(), n1 = bg.n1(), n2 = bg.n2();
+                const double* const rx = s_P + kPS * (bg.plane() + i);
+                const double* const ry = s_P + kPS * (bg.plane() + n0 + jj);
+                const double* const rz = s_P + kPS * (bg.plane() + n0 + n1 + kk);
+                const double* const E = s_E + kES * bg.line();
+                const double* const ez = E + kES * (i * n1 + jj);
+                const double* const ey = E + kES * (bg.n01() + i * n2 + kk);
+                const double* const ex = E + kES * (bg.n0_12() + jj * n2 + kk);
+                const double x = rx[0], y = ry[0], z = rz[0];
+                double v[4] = {0.0, 0.0, 0.0, 0.0};
+                if (kind == 2) {
+                    if (x != 0.0 && y != 0.0 && z != 0.0) {
+                        v[0] = (ez[6 * n] + ey[6 * n]) + ex[6 * n] +
+                               ((rx[bg_w(n, n)] + ry[bg_w(n, n)]) + (rz[bg_w(n, n)] + box_centre<NP>(T, n)));
+                        v[1] = (ez[6 * n + 1] + ey[6 * n + 1]) + rx[bg_dw(n, n)];
+                        v[2] = (ez[6 * n + 2] + ex[6 * n + 1]) + ry[bg_dw(n, n)];
+                        v[3] = (ey[6 * n + 2] + ex[6 * n + 2]) + rz[bg_dw(n, n)];
+                    }
+                } else {
+                    int k = kind;  // the point's piece
+                    if (NP > 2 && kind == 1) {
+                        const double r2 = fma(x, x, fma(y, y, z * z));
+#pragma unroll
+                        for (int s = 1; s + 1 < n; ++s) k += r2 >= T.scale[s].b * T.scale[s].b;
+                    }
+                    const double* const C = s_C + kCS * k;
+                    box_inside_grad<DEG>(C, C + kBoxC, C[kBoxC + kBoxD], T.deg, n, k, rx, ry, rz, ex, ey, ez, v);
+                    if (kind > 0) {
+                        v[0] += (rx[bg_w(n, k)] + ry[bg_w(n, k)]) + (rz[bg_w(n, k)] + box_centre<NP>(T, k));
+                        v[1] += rx[bg_dw(n, k)];
+                        v[2] += ry[bg_dw(n, k)];
+                        v[3] += rz[bg_dw(n, k)];
                     }
                 }
-                const bool take = idx < seg_end && il <= Caps::kPlane && ie <= Caps::kPair && ip <= Caps::kPt;
-                const int np = __popc(__ballot_sync(0xffffffffu, take));
-                AdjChunk& c = s_cp;
-                if (take) {
-                    const double H = mul_rn(g.support_in_h, ph);
-                    c.x[lane] = px; c.y[lane] = py; c.z[lane] = pz; c.H[lane] = H; c.iH[lane] = 1.0 / H;
-                    c.m[lane] = pm; c.vx[lane] = pvx; c.vy[lane] = pvy; c.vz[lane] = pvz;
-                    c.lo[lane][0] = lo0; c.lo[lane][1] = lo1; c.lo[lane][2] = lo2;
-                    c.dim[lane][0] = d0; c.dim[lane][1] = d1; c.dim[lane][2] = d2;
-                    c.loff[lane] = il - nl;
-                    c.eoff[lane] = ie - ne;
-                    c.poff[lane] = ip - npt;
-                    c.entry[lane] = e;
-                    c.mag[lane][0] = div_magic(d1 + 1);
-                    c.mag[lane][1] = div_magic(d2 + 1);
-                    c.mag[lane][2] = div_magic((d1 + 1) * (d2 + 1));
-                    c.cmag[lane][0] = div_magic(d2);
-                    c.cmag[lane][1] = div_magic(d1 * d2);
-                }
-                if (lane == np - 1) {
-                    c.np = np;
-                    c.ltot = il;
-                    c.etot = ie;
-                    c.ptot = ip;
-                }
+                put(it, j, x, y, z, v);
             }
-            __syncthreads();
-            const AdjChunk* const cp = &s_cp;
-            const int np = cp->np;
+        }
+        __syncthreads();
 
-            // (A) planes
-            {
-                const int off_l = lane < np ? cp->loff[lane] : INT_MAX, tot = cp->ltot;
-                for (int base = warp * 32; base < tot; base += kAdjThreads) {
-                    const int j = warp_owner(base, off_l, lane), it = base + lane;
-                    const int off = __shfl_sync(0xffffffffu, off_l, j & 31);
-                    if (it < tot) {
-                        int l = it - off;
-                        const int n0 = cp->dim[j][0] + 1, n1 = cp->dim[j][1] + 1;
-                        const int a = (l >= n0) + (l >= n0 + n1);
-                        l -= a == 0 ? 0 : (a == 1 ? n0 : n0 + n1);
-                        const double c = a == 0 ? cp->x[j] : (a == 1 ? cp->y[j] : cp->z[j]);
-                        box_grad_plane<NP, DEG>(T, (s_pl[a][cp->lo[j][a] + l] - c) * cp->iH[j], s_P + kPS * it);
-                    }
-                }
-            }
-            __syncthreads();
-
-            // (E) edge lines, queued by piece as in box_tile
-            {
-                const int tot = cp->etot;
-                const int off_l = lane < np ? cp->eoff[lane] : INT_MAX;
-                int cnt[Caps::kN];
-#pragma unroll
-                for (int c = 0; c < Caps::kN; ++c) cnt[c] = 0;
-                for (int base = warp * 32;; base += kAdjThreads) {
-                    const bool last = base >= tot;
-                    if (!last) {
-                        const int j = warp_owner(base, off_l, lane), it = base + lane;
-                        const int off = __shfl_sync(0xffffffffu, off_l, j & 31);
-                        int kind = -1;
-                        uint32_t rec = 0;
-                        if (it < tot) {
-                            int e = it - off;
-                            const int n0 = cp->dim[j][0] + 1, n1 = cp->dim[j][1] + 1, n2 = cp->dim[j][2] + 1;
-                            const int nxy = n0 * n1, nxz = n0 * n2;
-                            const int blk = (e >= nxy) + (e >= nxy + nxz);
-                            e -= blk == 0 ? 0 : (blk == 1 ? nxy : nxy + nxz);
-                            const int pi = div_by(e, cp->mag[j][blk == 0 ? 0 : 1]), qi = e - pi * (blk == 0 ? n1 : n2);
-                            const int la = cp->loff[j] + (blk == 2 ? n0 : 0) + pi;
-                            const int lb = cp->loff[j] + (blk == 0 ? n0 : n0 + n1) + qi;
-                            const double p = s_P[kPS * la], q = s_P[kPS * lb];
-                            const double D = fma(p, p, q * q);
-                            if (D >= 1.0 || p == 0.0 || q == 0.0) {
-                                double* const E = s_E + kES * it + 6 * n;
-                                E[0] = E[1] = E[2] = 0.0;
-                            } else {
-                                kind = 0;
-#pragma unroll
-                                for (int k = 0; k + 1 < n; ++k) kind += D >= T.scale[k].b * T.scale[k].b;
-                                rec = (uint32_t)it | (uint32_t)la << 10 | (uint32_t)lb << 19;
-                            }
-                        }
-#pragma unroll
-                        for (int c = 0; c < Caps::kN; ++c) {
-                            const unsigned m = __ballot_sync(0xffffffffu, kind == c);
-                            if (kind == c) s_q[64 * c + cnt[c] + __popc(m & below)] = rec;
-                            cnt[c] += __popc(m);
-                        }
-                        __syncwarp();
-                    }
-#pragma unroll
-                    for (int c = 0; c < Caps::kN; ++c) {
-                        if (cnt[c] >= 32 || (last && cnt[c] > 0)) {
-                            const int first = max(cnt[c] - 32, 0);
-                            if (first + lane < cnt[c]) {
-                                const uint32_t rec = s_q[64 * c + first + lane];
-                                box_grad_edge<NP, DEG>(T, c, s_P + kPS * ((rec >> 10) & 511u), s_P + kPS * (rec >> 19),
-                                                       s_E + kES * (rec & 1023u));
-                            }
-                            cnt[c] = first;
-                            __syncwarp();
-                        }
-                    }
-                    if (last) break;
-                }
-            }
-            __syncthreads();
-
-            // (P) points
-            {
-                const int tot = cp->ptot;
-                const int off_l = lane < np ? cp->poff[lane] : INT_MAX;
-                int cnt = 0;
-                // a point's values, with the offsets' signs: d/d(particle x) of sgn T(|ux|, ..) = -sgn(uy) sgn(uz) T_x
-                auto put = [&](int it, int j, const double* rx, const double* ry, const double* rz, const double* v) {
-                    const double iH = cp->iH[j];
-                    const double x = rx[0], y = ry[0], z = rz[0];
-                    const double sx = x > 0.0 ? 1.0 : -1.0, sy = y > 0.0 ? 1.0 : -1.0, sz = z > 0.0 ? 1.0 : -1.0;
-                    const double tx_ = -sy * sz * v[1] * iH, ty_ = -sx * sz * v[2] * iH, tz_ = -sx * sy * v[3] * iH;
-                    s_T[it] = sx * sy * sz * v[0];
-                    s_T[Caps::kPt + it] = tx_;
-                    s_T[2 * Caps::kPt + it] = ty_;
-                    s_T[3 * Caps::kPt + it] = tz_;
-                    s_T[4 * Caps::kPt + it] = g.support_in_h * fma(x, tx_, fma(y, ty_, z * tz_));
-                };
-                for (int base = warp * 32;; base += kAdjThreads) {
-                    const bool last = base >= tot;
-                    if (!last) {
-                        const int j = warp_owner(base, off_l, lane), it = base + lane;
-                        const int off = __shfl_sync(0xffffffffu, off_l, j & 31);
-                        bool near = false;
-                        uint32_t rec = 0;
-                        if (it < tot) {
-                            const int lp = it - off;
-                            const int n0 = cp->dim[j][0] + 1, n1 = cp->dim[j][1] + 1, n2 = cp->dim[j][2] + 1;
-                            const int i = div_by(lp, cp->mag[j][2]), rem = lp - i * (n1 * n2);
-                            const int jj = div_by(rem, cp->mag[j][1]), k = rem - jj * n2;
-                            const double* const rx = s_P + kPS * (cp->loff[j] + i);
-                            const double* const ry = s_P + kPS * (cp->loff[j] + n0 + jj);
-                            const double* const rz = s_P + kPS * (cp->loff[j] + n0 + n1 + k);
-                            const double x = rx[0], y = ry[0], z = rz[0];
-                            if (x == 0.0 || y == 0.0 || z == 0.0) {
-#pragma unroll
-                                for (int c = 0; c < kAdjComps; ++c) s_T[c * Caps::kPt + it] = 0.0;
-                            } else if (fma(x, x, fma(y, y, z * z)) < 1.0) {
-                                near = true;
-                                rec = (uint32_t)j | (uint32_t)i << 5 | (uint32_t)jj << 9 | (uint32_t)k << 13;
-                            } else {
-                                const double* const E = s_E + kES * cp->eoff[j] + 6 * n;
-                                const double* const ez = E + kES * (i * n1 + jj);
-                                const double* const ey = E + kES * (n0 * n1 + i * n2 + k);
-                                const double* const ex = E + kES * (n0 * (n1 + n2) + jj * n2 + k);
-                                const double v[4] = {(ez[0] + ey[0]) + ex[0] +
-                                                         ((rx[bg_w(n, n)] + ry[bg_w(n, n)]) +
-                                                          (rz[bg_w(n, n)] + box_centre<NP>(T, n))),
-                                                     (ez[1] + ey[1]) + rx[bg_dw(n, n)], (ez[2] + ex[1]) + ry[bg_dw(n, n)],
-                                                     (ey[2] + ex[2]) + rz[bg_dw(n, n)]};
-                                put(it, j, rx, ry, rz, v);
-                            }
-                        }
-                        const unsigned m = __ballot_sync(0xffffffffu, near);
-                        if (near) s_q[cnt + __popc(m & below)] = rec;
-                        cnt += __popc(m);
-                        __syncwarp();
-                    }
-                    if (cnt >= 32 || (last && cnt > 0)) {
-                        const int first = max(cnt - 32, 0);
-                        if (first + lane < cnt) {
-                            const uint32_t rec = s_q[first + lane];
-                            const int j = (int)(rec & 31u), i = (int)((rec >> 5) & 15u), jj = (int)((rec >> 9) & 15u),
-                                      kk = (int)(rec >> 13);
-                            const int n0 = cp->dim[j][0] + 1, n1 = cp->dim[j][1] + 1, n2 = cp->dim[j][2] + 1;
-                            const double* const rx = s_P + kPS * (cp->loff[j] + i);
-                            const double* const ry = s_P + kPS * (cp->loff[j] + n0 + jj);
-                            const double* const rz = s_P + kPS * (cp->loff[j] + n0 + n1 + kk);
-                            const double r2 = fma(rx[0], rx[0], fma(ry[0], ry[0], rz[0] * rz[0]));
-                            int k = 0;
-#pragma unroll
-                            for (int s = 0; s + 1 < n; ++s) k += r2 >= T.scale[s].b * T.scale[s].b;
-                            const double* const E = s_E + kES * cp->eoff[j];
-                            const double* const ez = E + kES * (i * n1 + jj);
-                            const double* const ey = E + kES * (n0 * n1 + i * n2 + kk);
-                            const double* const ex = E + kES * (n0 * (n1 + n2) + jj * n2 + kk);
-                            double Cl[14], Dl[59], c0, v[4];
-                            const double *C = Cl, *D = Dl;
-                            if (NP == 2) {  // two pieces, few coefficients each: selected constants
-#pragma unroll
-                                for (int c = 0; c < 14; ++c) Cl[c] = k ? T.reg[1].C[c] : T.reg[0].C[c];
-#pragma unroll
-                                for (int c = 0; c < 59; ++c) Dl[c] = k ? T.reg[1].D[c] : T.reg[0].D[c];
-                                c0 = k ? T.reg[1].c : T.reg[0].c;
-                            } else {
-                                C = s_C + kCS * k;
-                                D = C + kBoxC;
-                                c0 = D[kBoxD];
-                            }
-                            box_inside_grad<DEG>(C, D, c0, T.deg, n, k, rx, ry, rz, ex, ey, ez, v);
-                            if (k > 0) {
-                                v[0] += (rx[bg_w(n, k)] + ry[bg_w(n, k)]) + (rz[bg_w(n, k)] + box_centre<NP>(T, k));
-                                v[1] += rx[bg_dw(n, k)];
-                                v[2] += ry[bg_dw(n, k)];
-                                v[3] += rz[bg_dw(n, k)];
-                            }
-                            put(cp->poff[j] + (i * n1 + jj) * n2 + kk, j, rx, ry, rz, v);
-                        }
-                        cnt = first;
-                        __syncwarp();
-                    }
-                    if (last) break;
-                }
-            }
-            __syncthreads();
-
-            // (C) a warp per particle: its cells in box order over the lanes, weighed by the cotangents, and a
-            // fixed-order sum over the lanes
-            for (int j = warp; j < np; j += kAdjWarps) {
+        // (C) a warp per unit: its cells in box order over the lanes, weighed by the cotangents, and a fixed-order sum
+        // over the lanes, into the edge records' place (dead after (P)); and the next chunk's planes
+        double* const s_sum = s_E;
+        {
+            const int off_l = lane < np ? cp->box(lane).cell() : INT_MAX;
+            for (int u = warp; u < cp->utot; u += kAdjWarps) {
+                const int j = __popc(__ballot_sync(0xffffffffu, off_l <= u)) - 1;
                 double acc[8];
 #pragma unroll
                 for (int c = 0; c < 8; ++c) acc[c] = 0.0;
-                const double x0 = cp->x[j], y0 = cp->y[j], z0 = cp->z[j], radius = cp->H[j];
-                const double vx = cp->vx[j], vy = cp->vy[j], vz = cp->vz[j];
-                const int l0 = cp->lo[j][0], l1 = cp->lo[j][1], l2 = cp->lo[j][2];
-                const int d1 = cp->dim[j][1], d2 = cp->dim[j][2], d12 = d1 * d2, nc = cp->dim[j][0] * d12;
-                const int n2 = d2 + 1, n12 = (d1 + 1) * n2;
-                for (int lc = lane; lc < nc; lc += 32) {
-                    const int i = div_by(lc, cp->cmag[j][1]), rem = lc - i * d12;
-                    const int jj = div_by(rem, cp->cmag[j][0]), k = rem - jj * d2;
-                    const double ex = fmax(fabs(x0 - s_cc[0][l0 + i]) - g.hpx, 0.0);
-                    const double ey = fmax(fabs(y0 - s_cc[1][l1 + jj]) - g.hpy, 0.0);
-                    const double ez = fmax(fabs(z0 - s_cc[2][l2 + k]) - g.hpz, 0.0);
+                const BoxGeo b = cp->box(j);
+                const double4 at = cp->at[j], mv = cp->mv[j];
+                const double radius = at.w, sih = g.support_in_h * cp->iH[j];
+                const int d1 = b.n1() - 1, d2 = b.n2() - 1, n2 = d2 + 1, n12 = (d1 + 1) * n2;
+                const int l0 = b.lo0(), l1 = b.lo1(), l2 = b.lo2();
+                const int c0 = kAdjUnit * (u - b.cell()), c1 = min(c0 + kAdjUnit, (b.n0() - 1) * d1 * d2);
+                for (int lc = c0 + lane; lc < c1; lc += 32) {
+                    int i, jj, k;
+                    box_cell(cp->cmag[j], lc, d1, d2, i, jj, k);
+                    const double ex = fmax(fabs(at.x - cp->cc[0][l0 + i]) - g.hpx, 0.0);
+                    const double ey = fmax(fabs(at.y - cp->cc[1][l1 + jj]) - g.hpy, 0.0);
+                    const double ez = fmax(fabs(at.z - cp->cc[2][l2 + k]) - g.hpz, 0.0);
                     if (!(add_rn(add_rn(mul_rn(ex, ex), mul_rn(ey, ey)), mul_rn(ez, ez)) < mul_rn(radius, radius))) continue;
                     ++n_eval;
-                    const double* const Tp = s_T + cp->poff[j] + (i * (d1 + 1) + jj) * n2 + k;
-                    // component c of the cell's Msum: 0 the value, 1..4 d/d(x, y, z, h)
-                    auto cell_sum = [&](int c) {
-                        const double* const q = Tp + c * Caps::kPt;
-                        const double m1 = (q[n12 + n2 + 1] - q[n12 + n2]) - (q[n12 + 1] - q[n12]);
-                        const double m0 = (q[n2 + 1] - q[n2]) - (q[1] - q[0]);
-                        return m1 - m0;
-                    };
-                    const double msum = cell_sum(0);
+                    const double* const Tp = s_T + b.point() + i * n12 + jj * n2 + k;
+                    const double m1 = (Tp[n12 + n2 + 1] - Tp[n12 + n2]) - (Tp[n12 + 1] - Tp[n12]);
+                    const double m0 = (Tp[n2 + 1] - Tp[n2]) - (Tp[1] - Tp[0]);
+                    const double msum = m1 - m0;
                     if (msum < 0.0) {
                         ++n_neg;
                         continue;
                     }
                     if (msum == 0.0) continue;
-                    const int64_t i3 = ((int64_t)(bx + l0 + i) * g.ny + (by + l1 + jj)) * g.nz + (bz + l2 + k);
+                    const int64_t i3 = ((int64_t)(cp->bx + l0 + i) * g.ny + (cp->by + l1 + jj)) * g.nz + (cp->bz + l2 + k);
                     const double gx = cot[ncell + i3], gy = cot[2 * ncell + i3], gz = cot[3 * ncell + i3];
-                    const double gs = fma(vz, gz, fma(vy, gy, fma(vx, gx, cot[i3])));
+                    const double gs = fma(mv.w, gz, fma(mv.z, gy, fma(mv.y, gx, cot[i3])));
                     acc[0] = fma(msum, gs, acc[0]);
-#pragma unroll
-                    for (int c = 1; c <= 4; ++c) acc[c] = fma(cell_sum(c), gs, acc[c]);
                     acc[5] = fma(msum, gx, acc[5]);
                     acc[6] = fma(msum, gy, acc[6]);
                     acc[7] = fma(msum, gz, acc[7]);
+                    // each derivative's sum over the corners of either plane of its axis: their difference is the cell's,
+                    // and weighed with the planes' offsets it is that axis's part of d/dh
+                    double dh = 0.0;
+#pragma unroll
+                    for (int a = 0; a < 3; ++a) {
+                        const double* const q = Tp + (a + 1) * Caps::kPt;
+                        const double z11 = q[n12 + n2 + 1] - q[n12 + n2], z10 = q[n12 + 1] - q[n12], z01 = q[n2 + 1] - q[n2],
+                                     z00 = q[1] - q[0];
+                        const double hi = a == 0 ? z11 - z10 : (a == 1 ? z11 - z01
+                                                                       : (q[n12 + n2 + 1] - q[n12 + 1]) - (q[n2 + 1] - q[1]));
+                        const double lo = a == 0 ? z01 - z00 : (a == 1 ? z10 - z00 : (q[n12 + n2] - q[n12]) - (q[n2] - q[0]));
+                        const int l = a == 0 ? l0 + i : (a == 1 ? l1 + jj : l2 + k);
+                        const double x0 = a == 0 ? at.x : (a == 1 ? at.y : at.z);
+                        acc[1 + a] = fma(hi - lo, gs, acc[1 + a]);
+                        dh = fma(cp->pl[a][l + 1] - x0, hi, dh);
+                        dh = fma(-(cp->pl[a][l] - x0), lo, dh);
+                    }
+                    acc[4] = fma(sih * dh, gs, acc[4]);
                 }
 #pragma unroll
                 for (int c = 0; c < 8; ++c)
@@ -437,11 +455,26 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_cart_adjoint_box(CartGeom g,
                 double v = 0.0;
 #pragma unroll
                 for (int c = 0; c < 8; ++c) v = lane == c ? acc[c] : v;
-                if (lane < 8) part[8 * (int64_t)cp->entry[j] + lane] = lane == 0 ? v : cp->m[j] * v;
+                if (lane < 8) s_sum[8 * u + lane] = v;
             }
-            pos += np;
-            __syncthreads();
         }
+        reset();
+        if (more) form_planes(&nx);
+        __syncthreads();
+
+        // each entry's units in order; and the next chunk's lists
+        if (threadIdx.x < 8 * np) {
+            const int j = threadIdx.x >> 3, c = threadIdx.x & 7;
+            const int u1 = j + 1 < np ? cp->box(j + 1).cell() : cp->utot;
+            int u = cp->box(j).cell();
+            double v = s_sum[8 * u + c];
+            for (++u; u < u1; ++u) v += s_sum[8 * u + c];
+            part[8 * (int64_t)cp->entry[j] + c] = c == 0 ? v : cp->mv[j].x * v;
+        }
+        if (more) list_items(&nx);
+        __syncthreads();
+        pos += np;
+        cp = &nx;
     }
     for (int o = 16; o > 0; o >>= 1) {
         n_eval += __shfl_down_sync(0xffffffffu, n_eval, o);
@@ -527,7 +560,7 @@ int cart_adjoint_dev(KiwiCtx* ctx, const DevParticles& P, const CartGeom& g, con
         bool second = false;
         KIWI_TRY(radix_sort_pairs(ctx, k0, v0, k1, v1, total, key_bits, &second));
         const uint32_t *sk = second ? k1 : k0, *sv = second ? v1 : v0;
-        // entries per CTA: about eight CTAs for each of the chip's 2 x SMs places, so that uneven entries level out,
+        // entries per CTA: about sixteen CTAs for each of the chip's SMs, so that uneven entries level out,
         // within 16 (two chunks of large boxes) .. 256
         int sms = 148;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);

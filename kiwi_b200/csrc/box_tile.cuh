@@ -21,7 +21,7 @@
 // whichever warp is free; points (two kinds, forty batches a chunk) a warp sorts for itself, finishing the cheap ones
 // at once and queueing the others until it has 32.  Lines queued by warp and kind instead left half of the few
 // batches of a chunk part empty and the warps waiting at the barrier: 9 k particles on 37 x 41 x 149, quintic spline
-// (three kinds), 4.65 -> 3.7 ms; 150 k on 131 x 117 x 102, cubic, 5.0 -> 4.7 ms.  With one piece there is one
+// (three kinds), 4.65 -> 3.7 ms, and 3.2 with one copy of the evaluation for all kinds; 150 k on 131 x 117 x 102, cubic, 5.0 -> 4.7 ms.  With one piece there is one
 // costly kind, and a warp's own queue is the faster (100 k on 128^3, Wendland C4: 8.5 against 9.1 ms).
 //
 // A tile with a long list is cut into segments of box_segment() entries, each summed on its own (by CTAs of their
@@ -124,11 +124,35 @@ struct BoxGeo {
     __device__ __forceinline__ int by_n2(int x) const { return (int)(((uint32_t)x * (v.y & 0xffffu)) >> 16); }
     __device__ __forceinline__ int by_n12(int x) const { return (int)(((uint32_t)x * ((uint32_t)v.y >> 16)) >> 16); }
     __device__ __forceinline__ int by_n1(int x) const { return (int)(((uint32_t)x * ((uint32_t)v.w >> 21)) >> 10); }
+    // the planes of line e: blocks (x, y) over n0' x n1', (x, z) over n0' x n2', (y, z) over n1' x n2'
+    __device__ __forceinline__ void line_planes(int e, int& la, int& lb) const {
+        const int a0 = n0(), a1 = n1(), a2 = n2();
+        const bool xy = e < n01(), yz = e >= n0_12();
+        e -= xy ? 0 : (yz ? n0_12() : n01());
+        const int pi = xy ? by_n1(e) : by_n2(e), qi = e - pi * (xy ? a1 : a2);
+        la = plane() + (yz ? a0 : 0) + pi;
+        lb = plane() + a0 + (xy ? 0 : a1) + qi;
+    }
 };
 __device__ __forceinline__ uint32_t box_magic(int n, int bits) { return ((1u << bits) + (uint32_t)n - 1) / (uint32_t)n; }
+// The entry of a box of n0' x n1' x n2' planes.
+__device__ __forceinline__ int4 box_geo(int n0, int n1, int n2, int lo0, int lo1, int lo2, int plane, int line, int point,
+                                        int cell) {
+    return int4{(int)((uint32_t)plane | (uint32_t)line << 9 | (uint32_t)point << 19),
+                (int)(box_magic(n2, 16) | box_magic(n1 * n2, 16) << 16),
+                n1 | n2 << 4 | (n0 * n1) << 8 | (n0 * (n1 + n2)) << 15 | n0 << 23,
+                (int)((uint32_t)cell | (uint32_t)(lo0 | lo1 << 3 | lo2 << 6) << 12 | box_magic(n1, 10) << 21)};
+}
+// The 16-bit magic divisors of a box's n2 and n1 n2 cells (x / n = x * ceil(2^15 / n) >> 15 for the at most 512).
+__device__ __forceinline__ uint32_t box_cell_magic(int d1, int d2) { return box_magic(d2, 15) | box_magic(d1 * d2, 15) << 16; }
+__device__ __forceinline__ void box_cell(uint32_t magic, int lc, int d1, int d2, int& i, int& j, int& k) {
+    i = (int)(((uint32_t)lc * (magic >> 16)) >> 15);
+    const int rem = lc - i * (d1 * d2);
+    j = (int)(((uint32_t)rem * (magic & 0xffffu)) >> 15);
+    k = rem - j * d2;
+}
 
-// One chunk of a tile's particle list: the particles' data, their boxes, and the 16-bit magic divisors of their cells'
-// dimensions n2 and n1 n2 (x / n = x * ceil(2^15 / n) >> 15 for the at most 512 cells).
+// One chunk of a tile's particle list: the particles' data and their boxes.
 struct BoxChunk {
     double4 at[kBoxPMax];  // x, y, z and the support radius
     double4 mv[kBoxPMax];  // mass, velocities
@@ -362,12 +386,8 @@ __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& 
             dst->at[lane] = double4{px, py, pz, H};
             dst->mv[lane] = double4{pm, pvx, pvy, pvz};
             dst->iH[lane] = 1.0 / (TAB ? ph : H);
-            const int n0 = d0 + 1, n1 = d1 + 1, n2 = d2 + 1;
-            dst->geo[lane] = int4{(int)((uint32_t)(il - nl) | (uint32_t)(ie - ne) << 9 | (uint32_t)(ip - npt) << 19),
-                                  (int)(box_magic(n2, 16) | box_magic(n1 * n2, 16) << 16),
-                                  n1 | n2 << 4 | (n0 * n1) << 8 | (n0 * (n1 + n2)) << 15 | n0 << 23,
-                                  (int)((uint32_t)(ic - ncl) | (uint32_t)(lo0 | lo1 << 3 | lo2 << 6) << 12 | box_magic(n1, 10) << 21)};
-            dst->cmag[lane] = box_magic(d2, 15) | box_magic(d1 * d2, 15) << 16;
+            dst->geo[lane] = box_geo(d0 + 1, d1 + 1, d2 + 1, lo0, lo1, lo2, il - nl, ie - ne, ip - npt, ic - ncl);
+            dst->cmag[lane] = box_cell_magic(d1, d2);
         }
         if (lane == np - 1) {
             dst->np = np;
@@ -397,22 +417,12 @@ __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& 
         }
     };
 
-    // the planes of a box's line e: blocks (x, y) over n0' x n1', (x, z) over n0' x n2', (y, z) over n1' x n2'
-    auto line_planes = [&](const BoxGeo& b, int e, int& la, int& lb) {
-        const int n0 = b.n0(), n1 = b.n1(), n2 = b.n2();
-        const bool xy = e < b.n01(), yz = e >= b.n0_12();
-        const int base = b.plane();
-        e -= xy ? 0 : (yz ? b.n0_12() : b.n01());
-        const int pi = xy ? b.by_n1(e) : b.by_n2(e), qi = e - pi * (xy ? n1 : n2);
-        la = base + (yz ? n0 : 0) + pi;
-        lb = base + n0 + (xy ? 0 : n1) + qi;
-    };
     // the kind of particle j's line: the piece it lies in, or n beyond the support and in a particle's plane (nothing to
     // form); and the entry to form it from
     auto line_kind = [&](const BoxChunk* cp, int j, int it, uint32_t& rec) {
         const BoxGeo b = cp->box(j);
         int la, lb;
-        line_planes(b, it - b.line(), la, lb);
+        b.line_planes(it - b.line(), la, lb);
         const double p = s_P[kPS * la], q = s_P[kPS * lb];
         const double D = fma(p, p, q * q);
         rec = (uint32_t)it | (uint32_t)la << 10 | (uint32_t)lb << 19;
@@ -478,7 +488,7 @@ __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& 
                 const int j = warp_owner(base, off_l, lane), it = base + lane;
                 if (it < cp->etot) {
                     int la, lb;
-                    line_planes(cp->box(j), it - cp->box(j).line(), la, lb);
+                    cp->box(j).line_planes(it - cp->box(j).line(), la, lb);
                     const double p = fabs(s_P[kPS * la]), q = fabs(s_P[kPS * lb]);
                     if (p != 0.0 && q != 0.0) {
                         const double s = sqrt(p * p + q * q), is = 1.0 / s;
@@ -527,16 +537,16 @@ __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& 
                 nb += (s_lines[c] + 31) >> 5;
             }
             for (int b = next_batch(); b < nb; b = next_batch()) {
+                int c = 0, f = 0;
 #pragma unroll
-                for (int c = 0; c < Caps::kKinds; ++c) {
-                    if (b < first[c] || (c + 1 < Caps::kKinds && b >= first[c + 1])) continue;
-                    const int e = 32 * (b - first[c]) + lane;
-                    if (e >= s_lines[c]) continue;
-                    const uint32_t rec = s_list[Caps::kPair * c + e];
-                    double* const E = s_E + kES * (rec & 1023u);
-                    if (c == Caps::kN) E[2 * n] = 0.0;
-                    else box_edge<NP, DEG>(T, c, s_P + kPS * ((rec >> 10) & 511u), s_P + kPS * (rec >> 19), E);
-                }
+                for (int k = 1; k < Caps::kKinds; ++k)
+                    if (b >= first[k]) c = k, f = first[k];
+                const int e = 32 * (b - f) + lane;
+                if (e >= s_lines[c]) continue;
+                const uint32_t rec = s_list[Caps::kPair * c + e];
+                double* const E = s_E + kES * (rec & 1023u);
+                if (c == Caps::kN) E[2 * n] = 0.0;
+                else box_edge<NP, DEG>(T, c, s_P + kPS * ((rec >> 10) & 511u), s_P + kPS * (rec >> 19), E);
             }
         }
         __syncthreads();
@@ -671,10 +681,9 @@ __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& 
                 const int j = warp_owner(base, off_l, lane), it = base + lane;
                 if (it < tot) {
                     const BoxGeo b = cp->box(j);
-                    const uint32_t cm = cp->cmag[j];
-                    const int lc = it - b.cell(), d1 = b.n1() - 1, d2 = b.n2() - 1;
-                    const int i = (int)(((uint32_t)lc * (cm >> 16)) >> 15), rem = lc - i * (d1 * d2);
-                    const int jj = (int)(((uint32_t)rem * (cm & 0xffffu)) >> 15), k = rem - jj * d2;
+                    const int d1 = b.n1() - 1, d2 = b.n2() - 1;
+                    int i, jj, k;
+                    box_cell(cp->cmag[j], it - b.cell(), d1, d2, i, jj, k);
                     ++n_bbox;
                     const double4 at = cp->at[j];
                     const double radius = at.w;
