@@ -53,8 +53,8 @@ delta = phi - ang at the triangle's far vertex, in piece k,
 the subscript b marking the point where the edge line leaves the sphere of radius b (kiwi_cone_tables).
 
 The polynomials of the arctangent and the logarithm (kiwi_b200/csrc/fastmath.cuh) interpolate
-atan(x) / x in x^2 on [0, 1] and atanh(s) / s in s^2 on [0, (3 - 2 sqrt 2)^2] at Chebyshev points, in
-exact rational arithmetic.
+atan(x) / x in x^2 on [0, 1] and (log(1 + f) - f) / f^2 in f about 0 at Chebyshev points, in exact rational
+arithmetic; the logarithm's argument is reduced by a table of reciprocals with their logarithms.
 
 Usage:  python gen_box_tables.py            (write the header)
         python gen_box_tables.py --check    (exit 1 if the committed header is stale)
@@ -63,6 +63,7 @@ from __future__ import annotations
 
 import math
 import os
+import struct
 import sys
 from decimal import Decimal, getcontext
 from fractions import Fraction as Q
@@ -436,24 +437,34 @@ def atan_over_x(z):
     return tot.limit_denominator(10 ** 50)
 
 
-def atanh_over_s(z):
-    tot, term = Q(0), Q(1)
-    for k in range(60):
-        tot += term / (2 * k + 1)
-        term = Q((term * z).limit_denominator(10 ** 60))
-        if term < Q(1, 10 ** 40):
-            break
-    return tot.limit_denominator(10 ** 50)
+def log1p_rest(f):
+    """(log(1 + f) - f) / f^2 for small f."""
+    return sum(Q((-1) ** (k + 1), k + 2) * f ** k for k in range(30))
 
 
-def chebyshev_poly(fn, hi, n):
-    nodes = [Q(0.5 * hi * (1 + math.cos(math.pi * (2 * k + 1) / (2 * n)))).limit_denominator(10 ** 12)
+def chebyshev_poly(fn, lo, hi, n):
+    nodes = [Q(0.5 * (lo + hi) + 0.5 * (hi - lo) * math.cos(math.pi * (2 * k + 1) / (2 * n))).limit_denominator(10 ** 12)
              for k in range(n)]
     return interpolate([fn(z) for z in nodes], nodes)
 
 
-N_ATAN, N_LOG = 22, 9
-LOG_HI = (3 - 2 * math.sqrt(2)) ** 2 * 1.0001
+N_ATAN, N_LOG, LOG_BITS = 22, 5, 6
+LOG_HI0 = 0x3fe6a09e  # the high word of sqrt(1/2)
+
+
+def log_table():
+    """Per cell of 2^(20 - LOG_BITS) high words from sqrt(1/2) on: the reciprocal of its middle and minus that
+    reciprocal's logarithm; 1 and 0 in the cell that holds 1.  And the largest |m reciprocal - 1| of any cell."""
+    def value(hi):
+        return struct.unpack("<d", struct.pack("<Q", hi << 32))[0]
+
+    out, most = [], 0.0
+    for i in range(1 << LOG_BITS):
+        lo, hi = (value(LOG_HI0 + ((i + k) << (20 - LOG_BITS))) for k in (0, 1))
+        inv = 1.0 if lo < 1.0 < hi else 2.0 / (lo + hi)
+        out += [inv, float(-Decimal(inv).ln()) + 0.0]
+        most = max(most, abs(lo * inv - 1.0), abs(hi * inv - 1.0))
+    return out, most
 
 
 def rounded(v, a3=None):
@@ -560,11 +571,16 @@ def header_text():
             "}" for s in t["cscale"] + [zs] * (3 - t["npiece"])) + "}},")
     L.append("};")
     L.append("")
-    L.append("// atan(x) / x in powers of x^2 on [0, 1], and atanh(s) / s in powers of s^2 on |s| <= 3 - 2 sqrt 2")
+    L.append("// atan(x) / x in powers of x^2 on [0, 1], and (log(1 + f) - f) / f^2 in powers of f")
     L.append(f"#define KIWI_N_ATAN {N_ATAN}")
-    L.append("#define KIWI_ATAN_COEFS " + ", ".join(_num(float(c)) for c in chebyshev_poly(atan_over_x, 1.0, N_ATAN)))
+    L.append("#define KIWI_ATAN_COEFS " + ", ".join(_num(float(c)) for c in chebyshev_poly(atan_over_x, 0.0, 1.0, N_ATAN)))
+    table, most = log_table()
+    L.append(f"// the logarithm's cells: pairs (reciprocal of the middle, minus its logarithm); |f| <= {most:.6f}")
+    L.append(f"#define KIWI_LOG_BITS {LOG_BITS}")
+    L.append(f"#define KIWI_LOG_HI0 0x{LOG_HI0:x}")
+    L.append("#define KIWI_LOG_TABLE " + ", ".join(_num(v) for v in table))
     L.append(f"#define KIWI_N_LOG {N_LOG}")
-    L.append("#define KIWI_LOG_COEFS " + ", ".join(_num(float(c)) for c in chebyshev_poly(atanh_over_s, LOG_HI, N_LOG)))
+    L.append("#define KIWI_LOG_COEFS " + ", ".join(_num(float(c)) for c in chebyshev_poly(log1p_rest, -most, most, N_LOG)))
     L.append("")
     return "\n".join(L)
 
