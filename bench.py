@@ -44,7 +44,7 @@ sys.path.insert(0, ROOT)
 TRANS_FLOPS = 20.0
 WORK_PER_SUPPORT_PAIR = 10166.4 + TRANS_FLOPS * 481.9
 WORK_PER_BBOX_PAIR = 9142.7 + TRANS_FLOPS * 435.6
-# The lattice-factorised kernel's own work items (orc_edge_cost / orc_lattice_vertex_cost of the counting
+# The FP32-mixed lattice kernel's own work items (orc_edge_cost / orc_lattice_vertex_cost of the counting
 # oracle, averaged over 3,000 random inputs per class): an edge tier beyond 2h 37 flops; between h and 2h
 # 127 flops + 6 transcendentals; within h 209 flops + 12; a vertex pyramid 121 flops + 4; the assembly of
 # one cell from 24 corner values ~60 flops.
@@ -53,10 +53,19 @@ EDGE_MIDDLE = 127.0 + TRANS_FLOPS * 6
 EDGE_INNER = 209.0 + TRANS_FLOPS * 12
 VERTEX_PYRAMID = 121.0 + TRANS_FLOPS * 4
 CELL_ASSEMBLY = 60.0
+# The FP64 box-mass kernel's work items (cubic spline, counted in box_math.cuh; a line counts as two edge tiers, a
+# point as six vertex pyramids): a line beyond the support 5 flops, within it 60 flops + 6 transcendentals for the
+# outer piece alone and 105 + 11 for both; a point within the support 75 + 5, beyond it 12, of which the former are
+# 26 % on the default workload (counted over 3,000 of its particles); a cell ~12 flops.
+BOX_EDGE_OUTER = 2.5
+BOX_EDGE_MIDDLE = 30.0 + TRANS_FLOPS * 3
+BOX_EDGE_INNER = 52.5 + TRANS_FLOPS * 5.5
+BOX_VERTEX_PYRAMID = (0.26 * (75.0 + TRANS_FLOPS * 5) + 0.74 * 12.0) / 6
+BOX_CELL_ASSEMBLY = 12.0
 
-# DRAM bytes (read + write) of one k_cart_lattice launch on the default workload (2 M particles, 256^3) from
+# DRAM bytes (read + write) of one k_cart_box launch on the default workload (2 M particles, 256^3) from
 # a one-pass ncu capture, and the commit whose kernel was captured.
-LATTICE_TRAFFIC = {"bytes": 948.439296e6 + 511.081984e6, "commit": "9c39bf1", "kernel": "k_cart_lattice"}
+LATTICE_TRAFFIC = {"bytes": 889.018880e6 + 551.887360e6, "commit": "acf9e1d", "kernel": "k_cart_box"}
 
 L2_BYTES = 126 * 1024 * 1024
 # the tabulated integral: one trilinear lookup reads 8 table entries
@@ -1005,12 +1014,12 @@ def main():
             kname = ("k_cart_lattice_f32 (FP32 lattice tiers with rounding bounds; flagged tiles recomputed in FP64)"
                      if args.precision == "fp32_mixed_guaranteed" else
                      "k_cart_lattice_mixed (FP32 lattice tiers, FP64 islands and assembly)" if is32 else
-                     "k_cart_lattice (FP64 lattice-factorised cell-integral gather)" if args.kernel == "cubic_spline"
-                     else "k_cart_lattice_generic (FP64 lattice form, table-driven tiers; work items costed at the "
-                          "cubic tiers' rates)")
-            work = (items["edge_tiers_outer"] * EDGE_OUTER + items["edge_tiers_middle"] * EDGE_MIDDLE +
-                    items["edge_tiers_inner"] * EDGE_INNER + items["vertex_pyramids"] * VERTEX_PYRAMID +
-                    evaluated * CELL_ASSEMBLY) / args.steps
+                     "k_cart_box (FP64 box-mass gather)" if args.kernel == "cubic_spline"
+                     else "k_cart_box (FP64 box-mass gather; work items costed at the cubic spline's rates)")
+            eo, em, ei, vp, cell = ((EDGE_OUTER, EDGE_MIDDLE, EDGE_INNER, VERTEX_PYRAMID, CELL_ASSEMBLY) if is32 else
+                                    (BOX_EDGE_OUTER, BOX_EDGE_MIDDLE, BOX_EDGE_INNER, BOX_VERTEX_PYRAMID, BOX_CELL_ASSEMBLY))
+            work = (items["edge_tiers_outer"] * eo + items["edge_tiers_middle"] * em + items["edge_tiers_inner"] * ei +
+                    items["vertex_pyramids"] * vp + evaluated * cell) / args.steps
             work_per_pair = work / max(evaluated_per_launch, 1)
         else:
             kname = "k_cart_gather (FP64 cell-integral gather, reference evaluation order)"
@@ -1033,7 +1042,7 @@ def main():
             # each vertex pyramid is one trilinear lookup: 8 table entries (64 bytes) from a 182 MB table
             lookups = items.get("vertex_pyramids", 0) / args.steps
             ach = lookups * TAB_BYTES_PER_LOOKUP / (g_ms * 1e-3) / 1e9
-            tab_roofline = {"bound": "hbm", "kernel": "k_cart_lattice_tab (FP64 lattice form, tabulated integral)",
+            tab_roofline = {"bound": "hbm", "kernel": "k_cart_box_tab (FP64 box form, tabulated integral)",
                             "achieved": ach, "peak": hbm_peak, "unit": "GB/s",
                             "frac": ach / hbm_peak if hbm_peak else None, "traffic": None,
                             "algorithmic_bytes": "64 bytes (8 table entries) per lookup x lookups per launch",

@@ -34,7 +34,7 @@ int lattice_init_tables(KiwiCtx* ctx) {
 
 namespace {
 
-// Resident CTAs per SM the register budget is sized for: two for both kernels (128 registers).  The cubic
+// Resident CTAs per SM of the FP32-mixed kernels: two (128 registers), as measured in the FP64 form of this body: the cubic
 // kernel's shared memory would fit three, but at the 80 registers three need, its point-wise tiers spill:
 // 3.59 G support pairs/s at three against 3.84 G at two on the 2 M-particle log-normal cube.
 #ifndef KIWI_LATTICE_MIN_BLOCKS

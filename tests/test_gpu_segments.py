@@ -88,3 +88,30 @@ def test_tabulated_parts_agree(kiwi, ctx):
         outs.append((out["density"], st))
     assert torch.equal(outs[0][0], outs[1][0])
     assert_band_tolerance(outs[0][0].cpu().numpy(), outs[2][0].cpu().numpy(), (4e-10, 4e-9, 1e-7))
+
+
+# small boxes (chunks of 32 entries), boxes that fill their tiles (chunks of two or three) and both mixed
+@pytest.mark.parametrize("kernel", ["cubic_spline", "quintic_spline", "wendland_c4"])
+@pytest.mark.parametrize("hmin,hmax", [(0.002, 0.02), (0.3, 0.5), (0.002, 0.5)])
+def test_adjoint_does_not_depend_on_the_other_particles(kiwi, ctx, kernel, hmin, hmax):
+    """At given cotangents a particle's gradient is its own entries' sums: the same bits whatever else is mapped."""
+    import torch
+
+    ki = kiwi.make_kernel_integrator(kernel)
+    bounds, shape, n = (0.0, 1.0) * 3, (17, 16, 23), 200
+    dP = _particles(torch, n, 0.5, 3)
+    dP["h"] = hmin + (dP["h"] - dP["h"].min()) / 0.5 * (hmax - hmin)
+    cot = torch.from_numpy(np.random.default_rng(4).standard_normal(4 * int(np.prod(shape)))).cuda()
+
+    def gradients(P):
+        g = {k: torch.full((P["x"].numel(),), np.nan, dtype=torch.float64, device="cuda") for k in P}
+        torch.cuda.synchronize()
+        kiwi.sph_to_grid_adjoint_device(P, bounds, shape, cot, g, kernel=ki, ctx=ctx)
+        return g
+
+    every = gradients(dP)
+    assert all(torch.isfinite(v).all() for v in every.values())
+    for idx in (slice(0, 1), slice(0, None, 7), slice(5, 120)):
+        some = gradients({k: v[idx].contiguous() for k, v in dP.items()})
+        for k in every:
+            assert torch.equal(some[k], every[k][idx]), k
