@@ -3,9 +3,9 @@
 //
 // kiwi_batch_create bins every item's particles into its own grid's cell tiles with one shared key space
 // (item i's tiles follow item i-1's), so a single scan and a single stable sort build every tile list at
-// once; it groups the tiles by the tile body their item needs (cubic lattice, generic lattice, per-cell
-// gather), orders each group longest-first (by (tile, particle) entry count, ties by tile index) and
-// records one CUDA graph: counter resets and per-item mean velocities, then one persistent launch per group,
+// once; it groups the tiles by the tile body their item needs (one box-mass body per SPH kernel, per-cell
+// gather, the FP32-mixed form's two), orders each group longest-first (by (tile, particle) entry count, ties by tile index) and
+// records one CUDA graph: counter resets and per-item mean velocities, then one persistent launch per group, side by side,
 // whose CTAs pull work (tiles, or in the FP64 form segments of long lists) from a work counter and run the same
 // bodies as the single-grid kernels, then the sums of the cut tiles' segments.  Every cell is therefore summed in the same particle order with the same arithmetic as a single-grid call of the
 // same form: the batch's outputs equal the per-item outputs bit for bit.  kiwi_batch_run replays the graph.
