@@ -61,6 +61,16 @@ struct ConeWall {
     }
 };
 
+// The normal of a face's plane from its first three vertices, u and w the second's and third's offsets from the first,
+// with the roundings of face_integral_impl (src/kernel_integral.cpp:471-647): products rounded on their own, so that three vertices in
+// a line give exactly 0 as there, and not what an fma leaves of a product.
+struct FaceNormal {
+    double x, y, z;
+};
+KIWI_HD FaceNormal face_normal(double ux, double uy, double uz, double wx, double wy, double wz) {
+    return {fm_mul(uy, wz) - fm_mul(wy, uz), fm_mul(uz, wx) - fm_mul(wz, ux), fm_mul(ux, wy) - fm_mul(wx, uy)};
+}
+
 // The integral of a face with vertices V (nv of them, in order) for a particle at (x0, y0, z0), iH = 1 / H.  R: the
 // table's pieces, where the caller keeps them (threads differ in piece).
 template <int NP, int DEG, class Verts>
@@ -68,20 +78,10 @@ KIWI_HD double cone_face(const KiwiConeTable& T, const KiwiConeRegion* R, const 
                          double z0, double iH) {
     if (nv < 3) return 0.0;
     const double x1 = V.x(0), y1 = V.y(0), z1 = V.z(0);
-    double A, B, C;  // the plane's normal from the first three vertices, as the reference takes it
-    {
-        const double ux = V.x(1) - x1, uy = V.y(1) - y1, uz = V.z(1) - z1;
-        const double wx = V.x(2) - x1, wy = V.y(2) - y1, wz = V.z(2) - z1;
-        A = fma(uy, wz, -(wy * uz));
-        B = fma(uz, wx, -(wz * ux));
-        C = fma(ux, wy, -(wx * uy));
-    }
-    const double n2 = fma(A, A, fma(B, B, C * C));
-    if (!(n2 > 0.0)) return 0.0;
-    const double in = 1.0 / sqrt(n2);
-    A *= in;
-    B *= in;
-    C *= in;
+    const FaceNormal nrm = face_normal(V.x(1) - x1, V.y(1) - y1, V.z(1) - z1, V.x(2) - x1, V.y(2) - y1, V.z(2) - z1);
+    const double n2 = fma(nrm.x, nrm.x, fma(nrm.y, nrm.y, fm_mul(nrm.z, nrm.z)));
+    if (!(n2 > 0.0)) return 0.0;  // no plane: the reference's angles are undefined there and it adds nothing
+    const double in = 1.0 / sqrt(n2), A = nrm.x * in, B = nrm.y * in, C = nrm.z * in;
     const double rs = fma(A, x0 - x1, fma(B, y0 - y1, C * (z0 - z1)));  // signed distance
     const double r0 = fabs(rs) * iH;
     if (!(r0 > kBoxTiny)) return 0.0;
@@ -194,11 +194,9 @@ struct FacePlane {
     double x, y, z, w;
 };
 KIWI_HD FacePlane face_plane(const double* q) {
-    const double ux = q[3] - q[0], uy = q[4] - q[1], uz = q[5] - q[2];
-    const double wx = q[6] - q[0], wy = q[7] - q[1], wz = q[8] - q[2];
-    const double A = uy * wz - wy * uz, B = uz * wx - wz * ux, C = ux * wy - wx * uy;
-    const double in = 1.0 / sqrt(A * A + B * B + C * C);
-    return {A * in, B * in, C * in, -(A * q[0] + B * q[1] + C * q[2]) * in};
+    const FaceNormal n = face_normal(q[3] - q[0], q[4] - q[1], q[5] - q[2], q[6] - q[0], q[7] - q[1], q[8] - q[2]);
+    const double in = 1.0 / sqrt(n.x * n.x + n.y * n.y + n.z * n.z);
+    return {n.x * in, n.y * in, n.z * in, -(n.x * q[0] + n.y * q[1] + n.z * q[2]) * in};
 }
 
 // Whether the kernel reaches a face: face_reachable's rule (the reference's, src/kernel_integral.cpp:533-645) decided

@@ -16,6 +16,15 @@
 
 namespace kiwi_b200 {
 
+// a b, rounded on its own: a sum that takes it is not contracted into an fma.
+KIWI_HD double fm_mul(double a, double b) {
+#ifdef __CUDA_ARCH__
+    return __dmul_rn(a, b);
+#else
+    return fma(a, b, -0.0);
+#endif
+}
+
 // 1 / d for normal d > 0, to rounding: the hardware's approximation y (at least 18 bits), then
 // y (1 + e + e^2 + e^3) with e = 1 - d y.
 KIWI_HD double fm_rcp(double d) {

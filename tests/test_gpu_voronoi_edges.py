@@ -1,0 +1,50 @@
+"""Voronoi maps of tessellations and particles that the other tests do not hold."""
+import numpy as np
+import pytest
+
+from conftest import random_particles
+from test_gpu_voronoi import _cells_as_lists, _lists_as_cells, lattice_cells
+
+pytestmark = pytest.mark.gpu
+
+
+def _home(P, n, d):
+    return ((np.floor(P["x"] / d) * n + np.floor(P["y"] / d)) * n + np.floor(P["z"] / d)).astype(np.int32)
+
+
+def _close(got, want):
+    for band, tol in ((1e-2, 4e-10), (1e-4, 4e-9), (1e-6, 1e-7)):
+        m = want > band * want.max()
+        assert np.max(np.abs(got[m] - want[m]) / want[m]) < tol, band
+
+
+def test_face_that_starts_on_an_edge(kiwi, ctx, oracle):
+    """A cell whose faces start with a vertex on an edge (three vertices in a line) has no plane there by the reference's
+    rule: such faces add 0 and every walk passes them.  The tessellation is turned, so that the offsets' products
+    round."""
+    n = 8
+    geo, d = lattice_cells(n, 0.0, 1.0)
+    cells = _cells_as_lists(geo)
+    c = (4 * n + 3) * n + 4
+    turn, _ = np.linalg.qr(np.random.default_rng(9).standard_normal((3, 3)))
+    for i, (v, b) in enumerate(cells[c]):
+        step = 0.5 * (v[1] - v[0])
+        cells[c][i] = (np.concatenate([v[:1], [v[0] + step], v[1:]]), b)
+    P = random_particles(60, 21, box=(0.3, 0.7), hmin=0.05, hmax=0.12)
+    home = _home(P, n, d)
+    g = _lists_as_cells(cells, geo["volume"])
+    g["vxyz"] = np.ascontiguousarray((g["vxyz"].reshape(-1, 3) @ turn.T).reshape(-1))
+    # the second and third vertices' offsets from the first exactly in the ratio 1 : 2 after the turn
+    vx, vo = g["vxyz"].reshape(-1, 3), g["vert_off"]
+    for f in range(g["face_off"][c], g["face_off"][c + 1]):
+        a = vo[f]
+        half = np.round(0.5 * (vx[a + 2] - vx[a]) * 2.0 ** 40) / 2.0 ** 40
+        vx[a] = np.round(vx[a] * 2.0 ** 40) / 2.0 ** 40
+        vx[a + 1], vx[a + 2] = vx[a] + half, vx[a] + 2 * half
+        assert not np.any(np.cross(vx[a + 1] - vx[a], vx[a + 2] - vx[a]))
+    X = np.stack([P["x"], P["y"], P["z"]], 1) @ turn.T
+    P["x"], P["y"], P["z"] = (np.ascontiguousarray(X[:, i]) for i in range(3))
+    o = oracle.map_voronoi(P, home, g)
+    v = kiwi.map_voronoi(P, home, g, raw=True, ctx=ctx)
+    assert v.stats["visited_pairs"] == o[5]
+    _close(v.raw[0], o[4][0])
