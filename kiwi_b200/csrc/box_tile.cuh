@@ -737,9 +737,10 @@ __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& 
                 const int i = lx - b.lo0(), jj = ly - b.lo1(), k = lz - b.lo2();
                 const int d1 = b.n1() - 1, d2 = b.n2() - 1;
                 if ((unsigned)jj >= (unsigned)d1 || (unsigned)k >= (unsigned)d2) continue;
+                const double msum = s_cm[b.cell() + (i * d1 + jj) * d2 + k];
+                if (msum == 0.0) continue;  // (not by its mass: a mass or velocity that is not finite shows in its cells)
                 const double4 mv = cp->mv[j];
-                const double mm = s_cm[b.cell() + (i * d1 + jj) * d2 + k] * mv.x;
-                if (mm == 0.0) continue;
+                const double mm = msum * mv.x;
                 a0 = add_rn(a0, mm);
                 a1 = fma(mm, mv.y, a1);
                 a2 = fma(mm, mv.z, a2);
