@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1) k_cart_adjoint_box(CartGeom g,
                     const double D = fma(p, p, q * q);
                     rec = (uint32_t)it | (uint32_t)la << 10 | (uint32_t)lb << 19;
                     kind = n;
-                    if (D < 1.0 && p != 0.0 && q != 0.0) {
+                    if (D < 1.0 && !(bg_on(p) && bg_on(q))) {
                         kind = 0;
 #pragma unroll
                         for (int k = 0; k + 1 < n; ++k) kind += D >= T.scale[k].b * T.scale[k].b;
@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1) k_cart_adjoint_box(CartGeom g,
                     const double x = rx[0], y = ry[0], z = rz[0];
                     const double r2 = fma(x, x, fma(y, y, z * z));
                     rec = (uint32_t)(it | j << 12 | i << 17 | jj << 21 | k << 25);
-                    kind = x == 0.0 || y == 0.0 || z == 0.0 || !(r2 < 1.0)
+                    kind = (int)bg_on(x) + (int)bg_on(y) + (int)bg_on(z) > 1 || !(r2 < 1.0)
                                ? 2
                                : (n > 1 && r2 >= T.scale[0].b * T.scale[0].b ? 1 : 0);
                 }
@@ -334,10 +334,12 @@ __global__ void __launch_bounds__(kAdjThreads, 1) k_cart_adjoint_box(CartGeom g,
         {
             const int nn[3] = {s_pts[0], s_pts[1], s_pts[2]};
             const int b1 = (nn[0] + 31) >> 5, b2 = b1 + ((nn[1] + 31) >> 5), nb = b2 + ((nn[2] + 31) >> 5);
-            // a point's values, with the offsets' signs: d/d(particle x) of sgn T(|ux|, ..) = -sgn(uy) sgn(uz) T_x
+            // a point's values, with the offsets' signs: d/d(particle x) of sgn T(|ux|, ..) = -sgn(uy) sgn(uz) T_x; the sign
+            // of a plane through the particle is 0, which leaves the derivative across it (none where two planes meet)
+            auto sign = [](double u) { return bg_on(u) ? 0.0 : (u > 0.0 ? 1.0 : -1.0); };
             auto put = [&](int it, int j, double x, double y, double z, const double* v) {
                 const double iH = cp->iH[j];
-                const double sx = x > 0.0 ? 1.0 : -1.0, sy = y > 0.0 ? 1.0 : -1.0, sz = z > 0.0 ? 1.0 : -1.0;
+                const double sx = sign(x), sy = sign(y), sz = sign(z);
                 s_T[it] = sx * sy * sz * v[0];
                 s_T[Caps::kPt + it] = -sy * sz * v[1] * iH;
                 s_T[2 * Caps::kPt + it] = -sx * sz * v[2] * iH;
@@ -362,7 +364,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1) k_cart_adjoint_box(CartGeom g,
                 const double x = rx[0], y = ry[0], z = rz[0];
                 double v[4] = {0.0, 0.0, 0.0, 0.0};
                 if (kind == 2) {
-                    if (x != 0.0 && y != 0.0 && z != 0.0) {
+                    if ((int)bg_on(x) + (int)bg_on(y) + (int)bg_on(z) < 2) {
                         v[0] = (ez[6 * n] + ey[6 * n]) + ex[6 * n] +
                                ((rx[bg_w(n, n)] + ry[bg_w(n, n)]) + (rz[bg_w(n, n)] + box_centre<NP>(T, n)));
                         v[1] = (ez[6 * n + 1] + ey[6 * n + 1]) + rx[bg_dw(n, n)];

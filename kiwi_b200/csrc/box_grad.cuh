@@ -51,16 +51,17 @@ KIWI_HD double box_xp(const double* c, int full, int D, double X, double P) {
     return s;
 }
 
+// The record of the plane at signed offset u.  T is odd in u: on a plane through the particle it is 0, and so are its
+// derivatives along the plane, but not the one across it, whose terms tend to their values at u = 0.  Such a plane's record is
+// that of the smallest offset, by which bg_on tells it.
+KIWI_HD bool bg_on(double u) { return fabs(u) <= kBoxTiny; }
 template <int NP, int DEG>
 KIWI_HD void box_grad_plane(const KiwiBoxTable& T, double u, double* rec) {
     const int n = NP ? NP : T.npiece;
     const BoxDegree<DEG> d{T.deg};
-    const double p = fabs(u), p2 = p * p;
-    if (p < kBoxTiny) {
-        rec[0] = 0.0;
-        return;
-    }
-    rec[0] = u;
+    const bool on = fabs(u) < kBoxTiny;
+    const double p = on ? kBoxTiny : fabs(u), p2 = p * p;
+    rec[0] = on ? kBoxTiny : u;
     rec[1] = 1.0 / p;
     double w = 0.0, dw = 0.0;
 #ifdef __CUDACC__
