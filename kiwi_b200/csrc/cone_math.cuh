@@ -201,19 +201,22 @@ KIWI_HD FacePlane face_plane(const double* q) {
 
 // Whether the kernel reaches a face: face_reachable's rule (the reference's, src/kernel_integral.cpp:533-645) decided
 // from squared lengths and products, without its three roots, two divisions and two arccosines per vertex; 1 or 0
-// where the decision has a margin, -1 where it has none (the caller then takes face_reachable).  The reference's
-// own roundings move its distance by up to 1e-8 of the face's extent (R_0 = r12 sqrt(1 - cos^2)) and its side test's
-// threshold is 1e-9 of max(extent, 1); the margins here are 1e-5 of the radius and a tenth of that threshold, for
-// faces of up to 100 radii and coordinates of up to 1e5 (beyond which the answer is -1).  Of 400 k tests
+// where the decision has a margin, -1 where it has none (the caller then takes face_reachable).  What the two may differ by:
+// the plane's distance, the foot point and with them every length by the roundings of the coordinates, below err = 1e-14 of
+// their size (each is a handful of sums of products with a unit normal, formed from the same A, B, C); R_0 = r12 sqrt(1 - cos^2)
+// and the legs from arccosines by up to 1e-8 of the face's extent.  The margins are err and 1e-5 of the radius, for faces of
+// up to 100 radii and coordinates of up to 1e7 radii (beyond which the answer is -1 unless the plane alone decides); for the
+// side tests, whose threshold is 1e-9 of max(extent, 1), err and a tenth of the threshold.  So it answers in any unit of length,
+// and only where coordinates leave the radius fewer than seven digits it does not.  Of 400 k tests
 // about the cells of a jittered tessellation none was left to face_reachable.  (Walk of 64 k particles: 30.3 ms with
 // face_reachable and the visited marks in global memory, 9.2 ms.)
 template <class Plane>
 KIWI_HD int face_reach_fast(double x0, double y0, double z0, double radius, const Plane pl, const double* v, int nv) {
-    const double mag = fabs(x0) + fabs(y0) + fabs(z0);
+    const double mag = (fabs(x0) + fabs(y0) + fabs(z0)) + (fabs(v[0]) + fabs(v[1]) + fabs(v[2])), err = 1e-14 * mag;
     const double r0 = fma(pl.x, x0, fma(pl.y, y0, fma(pl.z, z0, pl.w)));
-    const double ar0 = fabs(r0), tol = fma(1e-9, radius, 1e-12 * (mag + fabs(pl.w)));
-    if (ar0 >= radius + tol && mag < 1e5) return 0;
-    if (!(ar0 < radius - tol) || !(mag < 1e5)) return -1;
+    const double ar0 = fabs(r0), tol = fma(1e-9, radius, err);
+    if (ar0 >= radius + tol) return 0;
+    if (!(ar0 < radius - tol) || !(mag < 1e7 * radius)) return -1;
     const double rr = radius * radius, near = rr * (1.0 - 1e-5), r02 = r0 * r0;
     const double xp = fma(-r0, pl.x, x0), yp = fma(-r0, pl.y, y0), zp = fma(-r0, pl.z, z0);
     bool inside = true, have = false, positive = false, sure = true;
@@ -235,9 +238,9 @@ KIWI_HD int face_reach_fast(double x0, double y0, double z0, double radius, cons
         if (sure && r02 + d2 < near) return 1;  // within reach whatever the side tests say
         const double side = fma(fma(ey, az, -(ez * ay)), pl.x, fma(fma(ez, ax, -(ex * az)), pl.y, fma(ex, ay, -(ey * ax)) * pl.z));
         const double m = fmax(fmax(fabs(ax), fabs(ay)), fmax(fabs(az), 1.0));
-        const double s2 = side * side, eps2 = 1e-18 * len2 * (m * m);
-        if (s2 > 0.81 * eps2 && s2 < 1.21 * eps2) sure = false;
-        if (s2 > eps2) {
+        const double lo = fmax(fma(0.9e-9, m, -err), 0.0), hi = fma(1.1e-9, m, err), s2 = side * side;
+        if (s2 >= lo * lo * len2 && s2 <= hi * hi * len2) sure = false;
+        if (s2 > hi * hi * len2) {
             if (!have) {
                 positive = side > 0.0;
                 have = true;

@@ -48,3 +48,21 @@ def test_face_that_starts_on_an_edge(kiwi, ctx, oracle):
     v = kiwi.map_voronoi(P, home, g, raw=True, ctx=ctx)
     assert v.stats["visited_pairs"] == o[5]
     _close(v.raw[0], o[4][0])
+
+
+@pytest.mark.parametrize("unit,shift", [(2.0 ** 21, 0.0), (2.0 ** 62, 0.0), (1.0, 3.0e4), (2.0 ** -10, 3.0)])
+def test_units_and_offsets(kiwi, ctx, oracle, unit, shift):
+    """Any unit of length, and a domain far from the origin: the walk visits the reference's pairs."""
+    n = 8
+    geo, d = lattice_cells(n, 0.0, 1.0)
+    P = random_particles(60, 33, box=(0.2, 0.8), hmin=0.04, hmax=0.12)
+    home = _home(P, n, d)
+    g = dict(geo, vxyz=np.ascontiguousarray(geo["vxyz"].reshape(-1) * unit + shift), volume=geo["volume"] * unit ** 3)
+    for k in ("x", "y", "z"):
+        P[k] = P[k] * unit + shift
+    P["h"] = P["h"] * unit
+    o = oracle.map_voronoi(P, home, g)
+    v = kiwi.map_voronoi(P, home, g, raw=True, ctx=ctx)
+    assert v.stats["visited_pairs"] == o[5]
+    if shift == 0.0:  # (else the coordinates' roundings, which the two take differently, are in the masses)
+        _close(v.raw[0], o[4][0])
