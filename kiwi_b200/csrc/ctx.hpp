@@ -142,8 +142,8 @@ enum ScratchSlot {
     S_MISC1,
     S_MISC2,
     S_MISC3,
-    S_VOR_MARK,      // Voronoi walk: visited markers per work slot
-    S_VOR_QUEUE,     // Voronoi walk: queues per work slot
+    S_VOR_MARK,      // Voronoi walk: visited markers per warp of the long walks
+    S_VOR_QUEUE,     // Voronoi walk: queues per warp of the long walks
     S_VOR_PAIRS,     // Voronoi walk: visited cells of every particle
     S_VOR_NEXT,      // Voronoi walk: particle counter
     S_VOR_CSR,       // staged cell geometry (host entry point)
@@ -175,6 +175,7 @@ enum ScratchSlot {
     S_VOR_STAGE,     // Voronoi walk: the single walk's staging area
     S_VOR_OWNER,     // Voronoi map: each pair's particle
     S_VOR_PLANES,    // Voronoi map: the faces' planes
+    S_VOR_OVER,      // Voronoi walk: the particles whose walks outgrow the shared table
     S_BOX_COUNTS,    // box-mass gather: item counters and weight classes
     S_BOX_ITEMS,     // box-mass gather: work items
     S_BOX_CUT,       // box-mass gather: the cut tiles

@@ -103,8 +103,9 @@ __global__ void k_face_planes(int64_t n_faces, const int64_t* __restrict__ vert_
 
 constexpr int kBfsWarpsPerBlock = 4;
 // The walk's visited cells in shared memory: an open-addressing table (cell -> queue position) and the queue, for
-// walks of up to kWalkCap cells (a particle visits about 120); a longer walk runs again in the slot's
-// global arrays.
+// walks of up to kWalkCap cells (a particle visits about 120).  A longer walk is listed and runs in a launch of its own,
+// in global arrays of n_cells entries per warp, which only that launch needs: with them behind every warp of the
+// common one, a map of 64 k cells held 1.9 GB for nothing and cleared 1.2 GB of it (0.2 ms).
 constexpr int kWalkBits = 10, kWalkSlots = 1 << kWalkBits, kWalkCap = 640;
 constexpr int kWalkClaim = 1 << 24;  // position values from here on: candidates' claims
 constexpr int kBfsCandCap = 512;  // a batch's discovery candidates listed per warp (larger batches: lane 0)
@@ -146,7 +147,8 @@ struct VorStage {
 // queued cells at a time and the appends are made in (cell, face) order, so the queue is the reference's
 // sequential queue.  A face whose neighbour already appeared on an earlier face of the same cell is a
 // face-cache hit in the reference and discovers nothing.  The visited cells' queue positions stand in a shared table
-// (mark[cell] = (marker << 32) | queue position in the slot's global arrays for a walk that outgrows it).
+// (SHARED; a walk that outgrows it is listed in `over` and left to the other form), or as
+// mark[cell] = (marker << 32) | queue position in the warp's global arrays, for the listed particles.
 // Cells of more than 128 faces are refused (KIWI_ERR_LIMIT).
 // Pass 1 also records per (particle, cell) the faces whose neighbour the walk processed earlier (bit i:
 // face i of the cell, first 64 faces): the reference reuses that neighbour's cached, negated face value.
@@ -157,13 +159,14 @@ struct VorStage {
 // first face towards this cell, the neighbour being the particle's q-th visited cell; -2 - e it takes the
 // value of this cell's earlier face e towards the same neighbour -- the reference's face cache
 // (src/mapping.cpp:56-93), decided here once so that the map evaluates each face value once.
+template <bool SHARED>
 struct WalkShared {
     int32_t cand[kBfsWarpsPerBlock][kBfsCandCap];
     unsigned long long reach[kBfsWarpsPerBlock][32][2];
-    int32_t key[kBfsWarpsPerBlock][kWalkSlots], pos[kBfsWarpsPerBlock][kWalkSlots], queue[kBfsWarpsPerBlock][kWalkCap];
+    int32_t cells[kBfsWarpsPerBlock][SHARED ? 2 * kWalkSlots + kWalkCap : 1];  // the table's keys and positions, the queue
 };
 
-// A walk's visited cells: the shared table, or the slot's global arrays.
+// A walk's visited cells: the shared table, or the warp's global arrays.
 template <bool SHARED>
 struct WalkCells {
     int32_t *key, *pos, *queue;
@@ -195,7 +198,7 @@ struct WalkCells {
 
 // One particle's walk (k_vor_bfs); returns its visited cells, or -1 if they outgrow the shared table.
 template <bool SHARED>
-__device__ __forceinline__ int vor_walk(const VorCells& C, WalkShared& sh, int warp, int lane, double x0, double y0,
+__device__ __forceinline__ int vor_walk(const VorCells& C, WalkShared<SHARED>& sh, int warp, int lane, double x0, double y0,
                                         double z0, double radius, int32_t k0, int pass, int64_t o, int64_t fcarry,
                                         WalkCells<SHARED>& W, int32_t* __restrict__ pair_cells,
                                         unsigned long long* __restrict__ pair_mask, int64_t* __restrict__ pair_foff,
@@ -475,10 +478,14 @@ __device__ __forceinline__ void vor_stage(const VorCells& C, const WalkCells<SHA
     }
 }
 
+// Pass 0 counts, pass 1 writes, pass 2 does both through the staging area.  The n_over particles of `over` in the global
+// form; in the shared form all, those that outgrow the table appended to `over` (passes 0 and 2) with a count of 0.
+template <bool SHARED>
 __global__ void __launch_bounds__(32 * kBfsWarpsPerBlock, 4) k_vor_bfs(VorCells C, DevParticles P,
                                                                     const int32_t* __restrict__ home,
                                                                     double support_in_h, int pass,
                                                                     unsigned long long* __restrict__ next,
+                                                                    uint32_t* __restrict__ over, int64_t n_over,
                                                                     long long* __restrict__ mark_base,
                                                                     int32_t* __restrict__ queue_base,
                                                                     int64_t* __restrict__ counts,
@@ -491,15 +498,17 @@ __global__ void __launch_bounds__(32 * kBfsWarpsPerBlock, 4) k_vor_bfs(VorCells 
                                                                     int64_t* __restrict__ pair_foff,
                                                                     int32_t* __restrict__ fsrc, VorStage stg) {
     extern __shared__ __align__(16) unsigned char s_walk[];
-    WalkShared& sh = *reinterpret_cast<WalkShared*>(s_walk);
+    WalkShared<SHARED>& sh = *reinterpret_cast<WalkShared<SHARED>*>(s_walk);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t slot = (int64_t)blockIdx.x * kBfsWarpsPerBlock + warp;
+    const unsigned long long n = (unsigned long long)(SHARED ? P.n : n_over);
     unsigned long long n_unresolved = 0, n_unmapped = 0, n_limit = 0;
     for (;;) {
         unsigned long long p = 0;
         if (lane == 0) p = atomicAdd(next, 1ull);
         p = __shfl_sync(0xffffffffu, p, 0);
-        if (p >= (unsigned long long)P.n) break;
+        if (p >= n) break;
+        if (!SHARED) p = over[p];
         const double h = P.h[p];
         const int32_t k0 = home[p];
         if (!(h > 0.0) || k0 < 0 || k0 >= C.n_cells) {
@@ -516,16 +525,19 @@ __global__ void __launch_bounds__(32 * kBfsWarpsPerBlock, 4) k_vor_bfs(VorCells 
         const int64_t fcarry = (pass == 1 && fsrc) ? foffs[p] : 0;  // pass 1: the first cell's first face
         int64_t nface = 0;
         unsigned long long limit = 0;
-        WalkCells<true> W{sh.key[warp], sh.pos[warp], sh.queue[warp], nullptr, 0};
-        int tail = vor_walk<true>(C, sh, warp, lane, x0, y0, z0, radius, k0, pass, o, fcarry, W, pair_cells, pair_mask,
-                                  pair_foff, fsrc, nface, limit);
-        const bool shared = tail >= 0;
-        WalkCells<false> G{nullptr, nullptr, queue_base + slot * C.n_cells, mark_base + slot * C.n_cells,
-                           marker((int64_t)p, pass)};
-        if (!shared) {
-            limit = 0;
-            tail = vor_walk<false>(C, sh, warp, lane, x0, y0, z0, radius, k0, pass, o, fcarry, G, pair_cells, pair_mask,
-                                   pair_foff, fsrc, nface, limit);
+        WalkCells<SHARED> W;
+        if (SHARED) W = {sh.cells[warp], sh.cells[warp] + kWalkSlots, sh.cells[warp] + 2 * kWalkSlots, nullptr, 0};
+        else W = {nullptr, nullptr, queue_base + slot * C.n_cells, mark_base + slot * C.n_cells, marker((int64_t)p, pass)};
+        const int tail = vor_walk<SHARED>(C, sh, warp, lane, x0, y0, z0, radius, k0, pass, o, fcarry, W, pair_cells,
+                                          pair_mask, pair_foff, fsrc, nface, limit);
+        if (SHARED && tail < 0) {
+            if (lane == 0 && pass != 1) {
+                over[atomicAdd(next + 1, 1ull)] = (uint32_t)p;
+                counts[p] = 0;
+                if (fcounts) fcounts[p] = 0;
+            }
+            __syncwarp();
+            continue;
         }
         n_limit += limit;
         if (pass != 1 && fcounts) {
@@ -537,10 +549,7 @@ __global__ void __launch_bounds__(32 * kBfsWarpsPerBlock, 4) k_vor_bfs(VorCells 
             counts[p] = tail;
             if (tail == 1) ++n_unmapped;
         }
-        if (pass == 2) {
-            if (shared) vor_stage(C, W, lane, (int64_t)p, tail, nface, stg);
-            else vor_stage(C, G, lane, (int64_t)p, tail, nface, stg);
-        }
+        if (pass == 2) vor_stage(C, W, lane, (int64_t)p, tail, nface, stg);
         __syncwarp();
     }
     n_unresolved = warp_sum_u64(n_unresolved);
@@ -1044,33 +1053,54 @@ int voronoi_map_dev(KiwiCtx* ctx, const DevParticles& P, const int32_t* d_home, 
     }
     C.plane = d_plane;
 
-    // BFS work slots: a visited marker and a queue of n_cells entries each
     int sms = 0;
     KIWI_CUDA(ctx, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
-    int64_t slots = (int64_t)sms * 4 * kBfsWarpsPerBlock;  // four blocks per SM
-    const int64_t budget = (int64_t)16 << 30;  // bytes of BFS scratch at most
-    while (slots > kBfsWarpsPerBlock && slots * nc * 12 > budget) slots /= 2;
-    slots = std::max<int64_t>(kBfsWarpsPerBlock, (slots / kBfsWarpsPerBlock) * kBfsWarpsPerBlock);
-    const int blocks = (int)(slots / kBfsWarpsPerBlock);
-    long long* mark = nullptr;
-    int32_t* queue = nullptr;
+    uint32_t* over = nullptr;  // the particles whose walks outgrow the shared table
+    KIWI_TRY(scratch_t(ctx, S_VOR_OVER, (size_t)std::max<int64_t>(n, 1), &over));
     int64_t *counts = nullptr, *offs = nullptr, *range = nullptr;
-    KIWI_TRY(scratch_t(ctx, S_VOR_MARK, (size_t)(slots * nc), &mark));
-    KIWI_TRY(scratch_t(ctx, S_VOR_QUEUE, (size_t)(slots * nc), &queue));
     KIWI_TRY(scratch_t(ctx, S_COUNT, (size_t)std::max<int64_t>(n, 1) * 2, &counts));
     KIWI_TRY(scratch_t(ctx, S_OFFS, (size_t)std::max<int64_t>(n, 1) + 1, &offs));
     KIWI_TRY(scratch_t(ctx, S_TILE_RANGE, (size_t)(2 * nc), &range));
     int64_t* d_total = offs + std::max<int64_t>(n, 1);
-    KIWI_CUDA(ctx, cudaMemsetAsync(mark, 0xff, sizeof(long long) * slots * nc, ctx->stream));
     KIWI_CUDA(ctx, cudaMemsetAsync(range, 0, sizeof(int64_t) * 2 * nc, ctx->stream));
 
     const double sup = kc.support_in_h;
-    KIWI_CUDA(ctx, cudaFuncSetAttribute(k_vor_bfs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WalkShared)));
-    // pass 0: count the visited cells and their faces
+    constexpr size_t smem = sizeof(WalkShared<true>), smem_long = sizeof(WalkShared<false>);
+    KIWI_CUDA(ctx, cudaFuncSetAttribute(k_vor_bfs<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    static_assert(smem_long <= 48 * 1024, "no opt-in needed");
     int64_t *fcounts = nullptr, *foffs = nullptr;
     KIWI_TRY(scratch_t(ctx, S_VOR_FCOUNT, (size_t)std::max<int64_t>(n, 1), &fcounts));
     KIWI_TRY(scratch_t(ctx, S_VOR_FOFFS, (size_t)std::max<int64_t>(n, 1) + 1, &foffs));
     int64_t* d_ftotal = foffs + std::max<int64_t>(n, 1);
+    const int walk_blocks = (int)std::min<int64_t>((int64_t)sms * 4, (n + kBfsWarpsPerBlock - 1) / kBfsWarpsPerBlock);
+    // The listed particles' walks in global arrays (a visited marker and a queue of n_cells entries per warp): sixteen
+    // warps per SM while the arrays are small, else eight as far as they stay within a budget.
+    long long* mark = nullptr;
+    int32_t* queue = nullptr;
+    int64_t slots = 0;
+    auto long_walks = [&](int pass, unsigned long long n_over, const int64_t* w_offs, int32_t* w_cells,
+                          unsigned long long* w_mask, int64_t* w_fcounts, const int64_t* w_foffs, int64_t* w_pfoff,
+                          int32_t* w_fsrc, const VorStage& w_stg) -> int {
+        if (n_over == 0) return KIWI_OK;
+        if (!mark) {
+            slots = (int64_t)sms * 4 * kBfsWarpsPerBlock;
+            const int64_t budget = (int64_t)16 << 30, small = (int64_t)2 << 30;
+            if (slots * nc * 12 > small) slots /= 2;
+            while (slots > kBfsWarpsPerBlock && slots * nc * 12 > budget) slots /= 2;
+            slots = std::min<int64_t>(slots, (int64_t)n_over + kBfsWarpsPerBlock - 1);
+            slots = std::max<int64_t>(kBfsWarpsPerBlock, (slots / kBfsWarpsPerBlock) * kBfsWarpsPerBlock);
+            KIWI_TRY(scratch_t(ctx, S_VOR_MARK, (size_t)(slots * nc), &mark));
+            KIWI_TRY(scratch_t(ctx, S_VOR_QUEUE, (size_t)(slots * nc), &queue));
+            // (a marker is distinct for every particle and pass: cleared once per map)
+            KIWI_CUDA(ctx, cudaMemsetAsync(mark, 0xff, sizeof(long long) * slots * nc, ctx->stream));
+        }
+        KIWI_CUDA(ctx, cudaMemsetAsync(d_next, 0, sizeof(unsigned long long), ctx->stream));
+        k_vor_bfs<false><<<(unsigned)(slots / kBfsWarpsPerBlock), 32 * kBfsWarpsPerBlock, smem_long, ctx->stream>>>(
+            C, P, d_home, sup, pass, d_next, over, (int64_t)n_over, mark, queue, counts, w_offs, w_cells, w_mask, d_stats,
+            w_fcounts, w_foffs, w_pfoff, w_fsrc, w_stg);
+        KIWI_LAUNCHED(ctx);
+        return KIWI_OK;
+    };
     // One walk when an earlier map on this context gave the totals to reserve (with room to spare): each
     // particle's pairs and face sources go to a staging area and are laid out particle by particle after;
     // otherwise (or if the reservation overflows) one walk counts and a second writes.
@@ -1096,34 +1126,49 @@ int voronoi_map_dev(KiwiCtx* ctx, const DevParticles& P, const int32_t* d_home, 
             stg.cap_pairs = cap_p;
             stg.cap_faces = cap_f;
             KIWI_CUDA(ctx, cudaMemsetAsync(stg.ctr, 0, 3 * sizeof(unsigned long long), ctx->stream));
-            KIWI_CUDA(ctx, cudaMemsetAsync(d_next, 0, sizeof(unsigned long long), ctx->stream));
-            k_vor_bfs<<<blocks, 32 * kBfsWarpsPerBlock, sizeof(WalkShared), ctx->stream>>>(C, P, d_home, sup, 2, d_next, mark, queue,
-                                                                         counts, nullptr, nullptr, nullptr, d_stats,
-                                                                         fcounts, nullptr, nullptr, nullptr, stg);
+            KIWI_CUDA(ctx, cudaMemsetAsync(d_next, 0, 2 * sizeof(unsigned long long), ctx->stream));
+            k_vor_bfs<true><<<walk_blocks, 32 * kBfsWarpsPerBlock, smem, ctx->stream>>>(
+                C, P, d_home, sup, 2, d_next, over, 0, nullptr, nullptr, counts, nullptr, nullptr, nullptr, d_stats, fcounts,
+                nullptr, nullptr, nullptr, stg);
             KIWI_LAUNCHED(ctx);
-            unsigned long long ovf = 0;
+            unsigned long long ovf = 0, n_over = 0;
             KIWI_CUDA(ctx, cudaMemcpyAsync(&ovf, stg.ctr + 2, sizeof ovf, cudaMemcpyDeviceToHost, ctx->stream));
+            KIWI_CUDA(ctx, cudaMemcpyAsync(&n_over, d_next + 1, sizeof n_over, cudaMemcpyDeviceToHost, ctx->stream));
             KIWI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+            if (ovf == 0 && n_over > 0) {
+                KIWI_TRY(long_walks(2, n_over, nullptr, nullptr, nullptr, fcounts, nullptr, nullptr, nullptr, stg));
+                KIWI_CUDA(ctx, cudaMemcpyAsync(&ovf, stg.ctr + 2, sizeof ovf, cudaMemcpyDeviceToHost, ctx->stream));
+                KIWI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+            }
             single = ovf == 0;
             if (!single) KIWI_CUDA(ctx, cudaMemsetAsync(d_stats, 0, sizeof(DevStats), ctx->stream));
         }
     }
-    if (!single) {
-        KIWI_CUDA(ctx, cudaMemsetAsync(d_next, 0, sizeof(unsigned long long), ctx->stream));
-        if (n > 0) {
-            k_vor_bfs<<<blocks, 32 * kBfsWarpsPerBlock, sizeof(WalkShared), ctx->stream>>>(C, P, d_home, sup, 0, d_next, mark, queue,
-                                                                         counts, nullptr, nullptr, nullptr, d_stats,
-                                                                         fcounts, nullptr, nullptr, nullptr,
-                                                                         VorStage{});
-            KIWI_LAUNCHED(ctx);
-        }
+    // pass 0: count the visited cells and their faces
+    if (!single && n > 0) {
+        KIWI_CUDA(ctx, cudaMemsetAsync(d_next, 0, 2 * sizeof(unsigned long long), ctx->stream));
+        k_vor_bfs<true><<<walk_blocks, 32 * kBfsWarpsPerBlock, smem, ctx->stream>>>(
+            C, P, d_home, sup, 0, d_next, over, 0, nullptr, nullptr, counts, nullptr, nullptr, nullptr, d_stats, fcounts,
+            nullptr, nullptr, nullptr, VorStage{});
+        KIWI_LAUNCHED(ctx);
     }
-    KIWI_TRY(exclusive_scan<int64_t>(ctx, counts, n, offs, d_total));
-    KIWI_TRY(exclusive_scan<int64_t>(ctx, fcounts, n, foffs, d_ftotal));
     int64_t total = 0, total_faces = 0;
-    KIWI_CUDA(ctx, cudaMemcpyAsync(&total, d_total, sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
-    KIWI_CUDA(ctx, cudaMemcpyAsync(&total_faces, d_ftotal, sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
-    KIWI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    unsigned long long n_over = 0;
+    auto totals = [&]() -> int {
+        KIWI_TRY(exclusive_scan<int64_t>(ctx, counts, n, offs, d_total));
+        KIWI_TRY(exclusive_scan<int64_t>(ctx, fcounts, n, foffs, d_ftotal));
+        KIWI_CUDA(ctx, cudaMemcpyAsync(&total, d_total, sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
+        KIWI_CUDA(ctx, cudaMemcpyAsync(&total_faces, d_ftotal, sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
+        if (!single && n > 0)
+            KIWI_CUDA(ctx, cudaMemcpyAsync(&n_over, d_next + 1, sizeof n_over, cudaMemcpyDeviceToHost, ctx->stream));
+        KIWI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        return KIWI_OK;
+    };
+    KIWI_TRY(totals());
+    if (n_over > 0) {  // (the listed particles count as 0 so far)
+        KIWI_TRY(long_walks(0, n_over, nullptr, nullptr, nullptr, fcounts, nullptr, nullptr, nullptr, VorStage{}));
+        KIWI_TRY(totals());
+    }
     ctx->vor_pairs_hint = total;
     ctx->vor_faces_hint = total_faces;
     // the face tables (each (pair, face) value evaluated once) when they fit a memory budget; else the
@@ -1160,10 +1205,11 @@ int voronoi_map_dev(KiwiCtx* ctx, const DevParticles& P, const int32_t* d_home, 
         } else {
             // pass 1: write each particle's visited cells at its offset
             KIWI_CUDA(ctx, cudaMemsetAsync(d_next, 0, sizeof(unsigned long long), ctx->stream));
-            k_vor_bfs<<<blocks, 32 * kBfsWarpsPerBlock, sizeof(WalkShared), ctx->stream>>>(C, P, d_home, sup, 1, d_next, mark, queue,
-                                                                         counts, offs, pair_cells, pair_mask, d_stats,
-                                                                         nullptr, foffs, pair_foff, fsrc, VorStage{});
+            k_vor_bfs<true><<<walk_blocks, 32 * kBfsWarpsPerBlock, smem, ctx->stream>>>(
+                C, P, d_home, sup, 1, d_next, over, 0, nullptr, nullptr, counts, offs, pair_cells, pair_mask, d_stats,
+                nullptr, foffs, pair_foff, fsrc, VorStage{});
             KIWI_LAUNCHED(ctx);
+            KIWI_TRY(long_walks(1, n_over, offs, pair_cells, pair_mask, nullptr, foffs, pair_foff, fsrc, VorStage{}));
         }
         k_vor_owner<<<(unsigned)((n * 32 + 255) / 256), 256, 0, ctx->stream>>>(n, counts, offs, owner);
         KIWI_LAUNCHED(ctx);

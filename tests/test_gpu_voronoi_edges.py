@@ -66,3 +66,49 @@ def test_units_and_offsets(kiwi, ctx, oracle, unit, shift):
     assert v.stats["visited_pairs"] == o[5]
     if shift == 0.0:  # (else the coordinates' roundings, which the two take differently, are in the masses)
         _close(v.raw[0], o[4][0])
+
+
+# walks longer than the shared table holds (640 cells; here up to all 4,096), alone, and one in seven among short ones
+@pytest.mark.parametrize("n_part,every", [(3, 1), (300, 7)])
+@pytest.mark.parametrize("kernel", [0, 4])
+def test_long_walks(kiwi, oracle, n_part, every, kernel):
+    """The walks that outgrow the shared table run in a launch of their own: the reference's pairs, and the same bits from
+    a context's first map (two walks), its second (one, staged), a larger map after a smaller one (the staging area
+    overflows), the single-launch gather and the inverse map's pairs."""
+    n = 16
+    geo, d = lattice_cells(n, 0.0, 1.0)
+    P = random_particles(n_part, 7, box=(0.05, 0.95), hmin=0.04, hmax=0.13)
+    P["h"][::every] = np.linspace(0.25, 0.9, len(P["h"][::every]))
+    home = _home(P, n, d)
+    ki = kiwi.KernelIntegrator(kernel=kernel)
+    o = oracle.map_voronoi(P, home, geo, kernel=kernel if kernel > 0 else -1, support_in_h=2.0)
+    assert o[5] > 640 * len(P["h"][::every])
+    ctx = kiwi.Context(0)
+    maps = [kiwi.map_voronoi(P, home, geo, kernel=ki, raw=True, ctx=ctx) for _ in range(2)]
+    ctx.set_voronoi_face_tables(False)
+    maps.append(kiwi.map_voronoi(P, home, geo, kernel=ki, raw=True, ctx=ctx))
+    other = kiwi.Context(0)
+    kiwi.map_voronoi({k: v[:2] for k, v in P.items()}, home[:2], geo, kernel=ki, ctx=other)
+    maps.append(kiwi.map_voronoi(P, home, geo, kernel=ki, raw=True, ctx=other))
+    for v in maps:
+        assert v.stats["visited_pairs"] == o[5]
+        assert np.array_equal(v.raw, maps[0].raw)
+    assert np.max(np.abs(maps[0].raw[0] - o[4][0])) <= 1e-9 * o[4][0].max()
+    inv = [kiwi.inverse_map_voronoi(P, home, geo, kernel=ki, ctx=c) for c in (other, kiwi.Context(0))]
+    assert np.array_equal(inv[0].m_recovered, inv[1].m_recovered)
+
+
+def test_short_walks_hold_no_global_arrays(kiwi):
+    """A map of short walks takes memory for its cells, faces and pairs alone: 27,000 cells under 100 MB."""
+    torch = pytest.importorskip("torch")
+    n = 30
+    geo, d = lattice_cells(n, 0.0, 1.0)
+    P = random_particles(20, 5, box=(0.2, 0.8), hmin=0.02, hmax=0.05)
+    ctx = kiwi.Context(0)
+    tiny, dt = lattice_cells(3, 0.0, 1.0)
+    kiwi.map_voronoi(P, _home(P, 3, dt), tiny, ctx=ctx)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    kiwi.map_voronoi(P, _home(P, n, d), geo, ctx=ctx)
+    torch.cuda.synchronize()
+    assert free - torch.cuda.mem_get_info()[0] < 100e6
