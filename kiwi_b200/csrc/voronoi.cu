@@ -663,15 +663,15 @@ __global__ void __launch_bounds__(kGatherThreads) k_vor_gather(VorCells C, DevPa
     __shared__ double s_val[kGatherThreads], s_m[kGatherThreads], s_vx[kGatherThreads], s_vy[kGatherThreads],
         s_vz[kGatherThreads];
     __shared__ KiwiConeRegion s_R[VorKernel<MODE>::kPieces];
-    vor_stage_regions<MODE>(s_R);
     const int64_t cell = blockIdx.x;
+    const int64_t beg = range[2 * cell], end = range[2 * cell + 1];
+    if (beg < end) vor_stage_regions<MODE>(s_R);
     const int64_t f0 = C.face_off[cell], f1 = C.face_off[cell + 1];
     const int64_t v0 = C.vert_off[f0], v1 = C.vert_off[f1];
     const bool staged = (v1 - v0) <= kGatherVertCap;
-    if (staged)
+    if (staged && beg < end)
         for (int64_t i = threadIdx.x; i < 3 * (v1 - v0); i += kGatherThreads) s_v[i] = C.vxyz[3 * v0 + i];
     __syncthreads();
-    const int64_t beg = range[2 * cell], end = range[2 * cell + 1];
     double M = 0.0, Px = 0.0, Py = 0.0, Pz = 0.0;
     unsigned long long n_neg = 0, n_warn = 0;
     unsigned n_clamp = 0;
@@ -784,15 +784,16 @@ __global__ void __launch_bounds__(kGatherThreads, KIWI_VOR_FACES_MIN_BLOCKS)
                 const uint32_t* __restrict__ owner, double* __restrict__ fval, DevStats* __restrict__ st) {
     __shared__ double s_v[3 * kGatherVertCap];
     __shared__ KiwiConeRegion s_R[VorKernel<MODE>::kPieces];
-    vor_stage_regions<MODE>(s_R);
     const int64_t cell = blockIdx.x;
+    const int64_t beg = range[2 * cell], end = range[2 * cell + 1];
+    if (beg == end) return;  // (before the staging: a few particles on many cells)
+    vor_stage_regions<MODE>(s_R);
     const int64_t f0 = C.face_off[cell], f1 = C.face_off[cell + 1];
     const int64_t v0 = C.vert_off[f0], v1 = C.vert_off[f1];
     const bool staged = (v1 - v0) <= kGatherVertCap;
     if (staged)
         for (int64_t i = threadIdx.x; i < 3 * (v1 - v0); i += kGatherThreads) s_v[i] = C.vxyz[3 * v0 + i];
     __syncthreads();
-    const int64_t beg = range[2 * cell], end = range[2 * cell + 1];
     const int nf = (int)(f1 - f0);
     unsigned n_clamp = 0;
     if (nf > kFaceItemMaxFaces) {
@@ -911,12 +912,14 @@ __global__ void __launch_bounds__(kGatherThreads) k_vor_sum(VorCells C, DevParti
     const int64_t cell = blockIdx.x;
     const int64_t f0 = C.face_off[cell], f1 = C.face_off[cell + 1];
     const int nf = (int)(f1 - f0);
-    for (int f = threadIdx.x; f < min(nf, kFaceItemMaxFaces); f += kGatherThreads) {
-        const int32_t nb = C.face_nbr[f0 + f];
-        s_back[f] = nb >= 0 && nb < C.n_cells && C.back[f0 + f] >= 0 ? (int32_t)(C.back[f0 + f] - C.face_off[nb]) : 0;
-    }
-    __syncthreads();
     const int64_t beg = range[2 * cell], end = range[2 * cell + 1];
+    if (beg < end) {
+        for (int f = threadIdx.x; f < min(nf, kFaceItemMaxFaces); f += kGatherThreads) {
+            const int32_t nb = C.face_nbr[f0 + f];
+            s_back[f] = nb >= 0 && nb < C.n_cells && C.back[f0 + f] >= 0 ? (int32_t)(C.back[f0 + f] - C.face_off[nb]) : 0;
+        }
+        __syncthreads();
+    }
     double sum = 0.0;  // threads 0 .. 3: M, Px, Py, Pz
     unsigned long long n_neg = 0, n_warn = 0;
     for (int64_t base = beg; base < end; base += kGatherThreads) {
