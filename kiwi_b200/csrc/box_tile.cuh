@@ -45,13 +45,19 @@ namespace kiwi_b200 {
 
 // Entries per segment of a tile with cnt entries in a grid of ntiles tiles: 128 (where the whole grid has fewer
 // tiles than the chip has places, one tile in eight pieces or more) to 1024 (thousands of tiles: only outliers are cut),
-// and at most 16384 segments in the grid or 8 per tile beyond that, so that their sums stay small.
+// and at most box_most segments in a tile: 16384 in the grid, or 8 per tile beyond that.
+__host__ __device__ __forceinline__ int64_t box_most(int64_t ntiles) {
+    return 16384 / ntiles < 8 ? 8 : (16384 / ntiles > 256 ? 256 : 16384 / ntiles);
+}
 __host__ __device__ __forceinline__ int64_t box_segment(int64_t cnt, int64_t ntiles) {
     const int64_t s0 = ntiles / 4 < 128 ? 128 : (ntiles / 4 > 1024 ? 1024 : ntiles / 4);
-    const int64_t most = 16384 / ntiles < 8 ? 8 : (16384 / ntiles > 256 ? 256 : 16384 / ntiles);
-    const int64_t s1 = (cnt + most - 1) / most;
+    const int64_t s1 = (cnt + box_most(ntiles) - 1) / box_most(ntiles);
     return s0 > s1 ? s0 : s1;
 }
+// Segments whose raw sums are held at a time (16 KB each: 268 MB).  A call with more takes its tiles in runs, one after
+// another: 8 segments a tile would be eight times the outputs of a grid whose every list is long (34 GB on 512^3).  The
+// 2 M particles of the log-normal cube on 256^3 have 7405.
+constexpr int64_t kBoxPlaces = 16384;
 
 #ifndef KIWI_BOX_THREADS
 #define KIWI_BOX_THREADS 256
@@ -737,10 +743,9 @@ __device__ __forceinline__ void box_tile(const CartGeom& g, const DevParticles& 
                 const int i = lx - b.lo0(), jj = ly - b.lo1(), k = lz - b.lo2();
                 const int d1 = b.n1() - 1, d2 = b.n2() - 1;
                 if ((unsigned)jj >= (unsigned)d1 || (unsigned)k >= (unsigned)d2) continue;
-                const double msum = s_cm[b.cell() + (i * d1 + jj) * d2 + k];
-                if (msum == 0.0) continue;  // (not by its mass: a mass or velocity that is not finite shows in its cells)
                 const double4 mv = cp->mv[j];
-                const double mm = msum * mv.x;
+                const double msum = s_cm[b.cell() + (i * d1 + jj) * d2 + k], mm = msum * mv.x;
+                if (msum == 0.0) continue;  // (not by mm: a mass or velocity that is not finite shows in its cells)
                 a0 = add_rn(a0, mm);
                 a1 = fma(mm, mv.y, a1);
                 a2 = fma(mm, mv.z, a2);
