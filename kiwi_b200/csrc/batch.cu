@@ -4,15 +4,17 @@
 // kiwi_batch_create bins every item's particles into its own grid's cell tiles with one shared key space
 // (item i's tiles follow item i-1's), so a single scan and a single stable sort build every tile list at
 // once; it groups the tiles by the tile body their item needs (one box-mass body per SPH kernel, per-cell
-// gather, the FP32-mixed form's two), orders each group longest-first (by (tile, particle) entry count, ties by tile index) and
-// records one CUDA graph: counter resets and per-item mean velocities, then one persistent launch per group, side by side,
-// whose CTAs pull work (tiles, or in the FP64 form segments of long lists) from a work counter and run the same
-// bodies as the single-grid kernels, then the sums of the cut tiles' segments.  Every cell is therefore summed in the same particle order with the same arithmetic as a single-grid call of the
-// same form: the batch's outputs equal the per-item outputs bit for bit.  kiwi_batch_run replays the graph.
+// gather, the FP32-mixed form's two), orders each group longest-first (by (tile, particle) entry count, ties by tile
+// index) and records one CUDA graph: counter resets and per-item mean velocities, then one persistent launch per group,
+// side by side, whose CTAs pull work (tiles, or in the FP64 form segments of long lists) from a work counter and run
+// the same bodies as the single-grid kernels, then the sums of the cut tiles' segments (in several runs where those are
+// many).  Every cell is therefore summed in the same particle order with the same arithmetic as a single-grid call of
+// the same form: the batch's outputs equal the per-item outputs bit for bit.  kiwi_batch_run replays the graph.
 // kiwi_batch_tune times the launch shapes (tile order x resident CTAs per SM) and keeps the fastest.
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <new>
 #include <utility>
 #include <vector>
 
@@ -32,22 +34,23 @@ struct KiwiBatch {
     std::vector<void*> allocs;
     BatchItemDev* d_items = nullptr;
     int32_t* d_item_of_tile = nullptr;
-    // per tile-body family: its work in natural (item, tile) order and longest-first (tiles, one int each, for the
-    // gather family; items of four ints, lattice_batch_work, for the lattice families), and its counter
-    int32_t* d_natural[kBatchFamilies] = {};
-    int32_t* d_lpt[kBatchFamilies] = {};
-    int64_t fam_tiles[kBatchFamilies] = {};  // work items
-    // FP32-mixed form: both lattice families' work together (natural order and longest-first), for the merged launch
-    int32_t* d_natural_m = nullptr;
-    int32_t* d_lpt_m = nullptr;
-    int64_t merged_tiles = 0;
+    // The tiles in runs of consecutive ones, one after another, so that the segments' sums of a run fit kBatchPlaces
+    // (nearly always one run).  Per run and tile-body family: its work in natural (item, tile) order and longest-first
+    // (tiles, one int each, for the gather family; items of four ints, lattice_batch_work, for the lattice families);
+    // FP32-mixed form: both lattice families' work together, for the merged launch; and the tiles whose lists are cut
+    // into segments (their first items).
+    struct Run {
+        int32_t *natural[kBatchFamilies] = {}, *lpt[kBatchFamilies] = {}, *natural_m = nullptr, *lpt_m = nullptr;
+        int64_t items[kBatchFamilies] = {}, merged = 0;
+        int32_t* cut = nullptr;
+        int64_t n_cut = 0;
+    };
+    std::vector<Run> runs;
+    int64_t fam_items[kBatchFamilies] = {};  // work items of all runs
     // FP32-mixed form: both families in one launch; FP64 form: the kernels' launches side by side (else one after
     // another), so that one fills the places that another's last items leave
     bool merge = false;
-    // the tiles whose lists are cut into segments (their first items) and their segments' raw sums
-    int32_t* d_cut = nullptr;
-    int64_t n_cut = 0;
-    double* d_sums = nullptr;
+    double* d_sums = nullptr;  // the segments' raw sums of one run
     const uint32_t* d_list = nullptr;
     int64_t* d_range = nullptr;
     unsigned long long* d_next = nullptr;  // kBatchFamilies counters
@@ -98,7 +101,7 @@ void batch_free(KiwiBatch* b) {
 
 int families_present(const KiwiBatch* b) {
     int k = 0;
-    for (int f = 0; f < kBatchFamilies; ++f) k += b->fam_tiles[f] > 0;
+    for (int f = 0; f < kBatchFamilies; ++f) k += b->fam_items[f] > 0;
     return k;
 }
 
@@ -117,38 +120,45 @@ int capture_after(KiwiCtx* ctx, std::vector<cudaGraphNode_t> front) {
     return KIWI_OK;
 }
 
-// The replayed work, captured: reset the counters, the mean velocities, one persistent launch per family present
-// (side by side: each follows the mean velocities alone), the cut tiles' sums.
-int batch_enqueue(KiwiBatch* b) {
+// The replayed work of one run, captured: one persistent launch per family present (side by side: each follows what came
+// before the run alone), the cut tiles' sums.
+int batch_enqueue_run(KiwiBatch* b, const KiwiBatch::Run& r) {
     KiwiCtx* ctx = b->ctx;
     const bool mixed = (b->precision & KIWI_FORM_MASK) == KIWI_FP32_MIXED;
-    KIWI_CUDA(ctx, cudaMemsetAsync(b->d_next, 0, sizeof(unsigned long long) * kBatchFamilies, ctx->stream));
-    KIWI_CUDA(ctx, cudaMemsetAsync(b->d_stats, 0, sizeof(DevStats) * b->n_items, ctx->stream));
-    for (int i = 0; i < b->n_items; ++i) KIWI_TRY(fp64_mean_velocity(ctx, b->items[i].P, b->d_meanv + 4 * i));
-    const bool merged = mixed && b->merge && b->fam_tiles[kBatchFamilyMixed] > 0 && b->fam_tiles[kBatchFamilyMixedGeneric] > 0;
+    const bool merged = mixed && b->merge && r.items[kBatchFamilyMixed] > 0 && r.items[kBatchFamilyMixedGeneric] > 0;
     const bool side = b->merge && (b->precision & KIWI_FORM_MASK) == KIWI_FP64 && families_present(b) > 1;
+    KIWI_CUDA(ctx, cudaMemsetAsync(b->d_next, 0, sizeof(unsigned long long) * kBatchFamilies, ctx->stream));
     std::vector<cudaGraphNode_t> before, one, after;
     if (side) KIWI_TRY(capture_front(ctx, &before));
     for (int f = 0; f < kBatchFamilies; ++f) {
-        if (b->fam_tiles[f] <= 0 || (merged && f == kBatchFamilyMixedGeneric)) continue;
-        const int32_t* work = merged ? (b->lpt ? b->d_lpt_m : b->d_natural_m) : (b->lpt ? b->d_lpt[f] : b->d_natural[f]);
+        if (r.items[f] <= 0 || (merged && f == kBatchFamilyMixedGeneric)) continue;
+        const int32_t* work = merged ? (b->lpt ? r.lpt_m : r.natural_m) : (b->lpt ? r.lpt[f] : r.natural[f]);
         const int blocks = b->sms * b->ctas_per_sm;
         if (f == kBatchFamilyGather) {
-            KIWI_TRY(fp64_batch_gather(ctx, b->d_items, b->d_item_of_tile, work, b->fam_tiles[f], b->d_list, b->d_range,
+            KIWI_TRY(fp64_batch_gather(ctx, b->d_items, b->d_item_of_tile, work, r.items[f], b->d_list, b->d_range,
                                        b->d_next + f, blocks));
             continue;
         }
         if (side) KIWI_TRY(capture_after(ctx, before));
         KIWI_TRY(lattice_batch_gather(ctx, merged ? kBatchFamilyMixedMerged : f, b->d_items, b->d_item_of_tile, work,
-                                      merged ? b->merged_tiles : b->fam_tiles[f], b->d_list, b->d_range, b->d_sums,
-                                      b->d_next + f, blocks, mixed));
+                                      merged ? r.merged : r.items[f], b->d_list, b->d_range, b->d_sums, b->d_next + f,
+                                      blocks, mixed));
         if (side) {
             KIWI_TRY(capture_front(ctx, &one));
             after.insert(after.end(), one.begin(), one.end());
         }
     }
     if (side) KIWI_TRY(capture_after(ctx, after));
-    return lattice_batch_combine(ctx, b->d_items, b->d_item_of_tile, b->d_cut, b->n_cut, b->d_sums);
+    return lattice_batch_combine(ctx, b->d_items, b->d_item_of_tile, r.cut, r.n_cut, b->d_sums);
+}
+
+// The replayed work, captured: reset the counters, the mean velocities, the runs.
+int batch_enqueue(KiwiBatch* b) {
+    KiwiCtx* ctx = b->ctx;
+    KIWI_CUDA(ctx, cudaMemsetAsync(b->d_stats, 0, sizeof(DevStats) * b->n_items, ctx->stream));
+    for (int i = 0; i < b->n_items; ++i) KIWI_TRY(fp64_mean_velocity(ctx, b->items[i].P, b->d_meanv + 4 * i));
+    for (const KiwiBatch::Run& r : b->runs) KIWI_TRY(batch_enqueue_run(b, r));
+    return KIWI_OK;
 }
 
 int batch_record(KiwiBatch* b) {
@@ -171,7 +181,30 @@ int batch_record(KiwiBatch* b) {
     return KIWI_OK;
 }
 
-// The families' work lists from the tiles' ranges, and the place of the cut tiles' sums.
+// The work items (`ints` ints each) in descending order of their weights, equal ones in their order: two counting
+// passes over 11 bits (weights beyond 22 bits count as equal).
+std::vector<int32_t> heaviest_first(const std::vector<int32_t>& work, const std::vector<int64_t>& weight, int ints) {
+    const size_t n = weight.size();
+    constexpr int kBits = 11, kBins = 1 << kBits;
+    std::vector<uint32_t> key(n), order(n), next(n);
+    for (size_t i = 0; i < n; ++i) {
+        key[i] = (uint32_t)((1 << 2 * kBits) - 1 - std::min<int64_t>(weight[i], (1 << 2 * kBits) - 1));
+        order[i] = (uint32_t)i;
+    }
+    for (int pass = 0; pass < 2; ++pass) {
+        std::vector<size_t> at(kBins + 1, 0);
+        for (size_t i = 0; i < n; ++i) ++at[((key[i] >> pass * kBits) & (kBins - 1)) + 1];
+        for (int c = 0; c < kBins; ++c) at[c + 1] += at[c];
+        for (size_t i = 0; i < n; ++i) next[at[(key[order[i]] >> pass * kBits) & (kBins - 1)]++] = order[i];
+        order.swap(next);
+    }
+    std::vector<int32_t> out;
+    out.reserve(work.size());
+    for (const uint32_t i : order) out.insert(out.end(), work.begin() + (size_t)i * ints, work.begin() + (size_t)(i + 1) * ints);
+    return out;
+}
+
+// The families' work lists from the tiles' ranges, run by run, and the place of the cut tiles' sums.
 int batch_work(KiwiBatch* b) {
     KiwiCtx* ctx = b->ctx;
     std::vector<int64_t> range(2 * (size_t)b->n_tiles), grid_tiles((size_t)b->n_tiles);
@@ -180,55 +213,90 @@ int batch_work(KiwiBatch* b) {
     KIWI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     const bool split = (b->precision & KIWI_FORM_MASK) == KIWI_FP64, mixed = (b->precision & KIWI_FORM_MASK) == KIWI_FP32_MIXED;
     std::vector<int32_t> tiles[kBatchFamilies], both, slot((size_t)b->n_tiles, 0), cut, work;
-    int64_t places = 0;
+    std::vector<int64_t> weight;
+    for (int i = 0; i < b->n_items; ++i)
+        for (int64_t t = b->tile_base[i]; t < b->tile_base[i + 1]; ++t) grid_tiles[(size_t)t] = b->tile_base[i + 1] - b->tile_base[i];
+    auto segments = [&](int64_t t) {
+        return split ? lattice_batch_segments(range[2 * (size_t)t + 1] - range[2 * (size_t)t], grid_tiles[(size_t)t]) : 1;
+    };
+    // the sums' buffer: all segments' or kBatchPlaces; half as many as long as it cannot be had (a tile has at most 256)
+    int64_t cap = 0, places = 0;
+    for (int64_t t = 0; t < b->n_tiles && cap < kBatchPlaces; ++t) cap += segments(t) > 1 ? segments(t) : 0;
+    for (cap = std::min(cap, kBatchPlaces);; cap /= 2) {
+        const int rc = balloc(b, (size_t)cap * 4 * kTileCells, &b->d_sums);
+        if (rc == KIWI_OK) break;
+        if (rc != KIWI_ERR_ALLOC || cap < 512) return rc;
+        ctx->err.clear();
+    }
+    // one upload of all lists; their places are known once it is made
+    std::vector<int32_t> all;
+    struct Place {
+        size_t run, at;
+        int32_t* KiwiBatch::Run::*list;
+        int32_t* (KiwiBatch::Run::*lists)[kBatchFamilies];
+        int family;
+    };
+    std::vector<Place> where;
+    auto put = [&](const std::vector<int32_t>& v, Place p) {
+        p.run = b->runs.size() - 1;
+        p.at = all.size();
+        where.push_back(p);
+        all.insert(all.end(), v.begin(), v.end());
+        all.resize((all.size() + 3) / 4 * 4);  // items are read as int4
+    };
+    auto close_run = [&]() {
+        using Run = KiwiBatch::Run;
+        b->runs.emplace_back();
+        Run& r = b->runs.back();
+        for (int f = 0; f < kBatchFamilies; ++f) {
+            const int ints = f == kBatchFamilyGather ? 1 : 4;
+            if (f == kBatchFamilyGather) {
+                work = tiles[f];
+                weight.clear();
+                for (const int32_t t : work) weight.push_back(range[2 * (size_t)t + 1] - range[2 * (size_t)t]);
+            } else {
+                lattice_batch_work(tiles[f], range, grid_tiles, slot, split, &work, &weight);
+            }
+            r.items[f] = (int64_t)weight.size();
+            b->fam_items[f] += r.items[f];
+            put(work, {0, 0, nullptr, &Run::natural, f});
+            put(heaviest_first(work, weight, ints), {0, 0, nullptr, &Run::lpt, f});
+            tiles[f].clear();
+        }
+        lattice_batch_work(both, range, grid_tiles, slot, split, &work, &weight);
+        r.merged = (int64_t)weight.size();
+        put(work, {0, 0, &Run::natural_m, nullptr, 0});
+        put(heaviest_first(work, weight, 4), {0, 0, &Run::lpt_m, nullptr, 0});
+        r.n_cut = (int64_t)cut.size() / 4;
+        put(cut, {0, 0, &Run::cut, nullptr, 0});
+        both.clear();
+        cut.clear();
+        places = 0;
+    };
     for (int i = 0; i < b->n_items; ++i) {
         const int f = batch_family(b->items[i].mode, b->items[i].kernel, mixed);
-        const int64_t nt = b->tile_base[i + 1] - b->tile_base[i];
         for (int64_t t = b->tile_base[i]; t < b->tile_base[i + 1]; ++t) {
-            grid_tiles[(size_t)t] = nt;
+            const int64_t nseg = segments(t);
+            if (nseg > 1 && places + nseg > cap) close_run();
             tiles[f].push_back((int32_t)t);
             if (f == kBatchFamilyGather) continue;
             if (mixed) both.push_back((int32_t)t);
-            const int64_t nseg = split ? lattice_batch_segments(range[2 * (size_t)t + 1] - range[2 * (size_t)t], nt) : 1;
             if (nseg <= 1) continue;
             slot[(size_t)t] = (int32_t)places;
             cut.insert(cut.end(), {(int32_t)t, 0, (int32_t)nseg, (int32_t)places});
             places += nseg;
         }
     }
-    // one upload of all lists
-    std::vector<int32_t> all;
-    std::vector<std::pair<int32_t**, size_t>> place;
-    auto put = [&](const std::vector<int32_t>& v, int32_t** dst) {
-        place.push_back({dst, all.size()});
-        all.insert(all.end(), v.begin(), v.end());
-        all.resize((all.size() + 3) / 4 * 4);  // items are read as int4
-    };
-    for (int heaviest = 0; heaviest < 2; ++heaviest) {
-        for (int f = 0; f < kBatchFamilies; ++f) {
-            if (f == kBatchFamilyGather) {
-                work = tiles[f];
-                b->fam_tiles[f] = (int64_t)work.size();
-                if (heaviest)
-                    std::stable_sort(work.begin(), work.end(), [&](int32_t x, int32_t y) {
-                        return range[2 * (size_t)x + 1] - range[2 * (size_t)x] > range[2 * (size_t)y + 1] - range[2 * (size_t)y];
-                    });
-            } else {
-                b->fam_tiles[f] = lattice_batch_work(tiles[f], range, grid_tiles, slot, split, heaviest != 0, &work);
-            }
-            put(work, heaviest ? &b->d_lpt[f] : &b->d_natural[f]);
-        }
-        b->merged_tiles = lattice_batch_work(both, range, grid_tiles, slot, split, heaviest != 0, &work);
-        put(work, heaviest ? &b->d_lpt_m : &b->d_natural_m);
-    }
-    b->n_cut = (int64_t)cut.size() / 4;
-    put(cut, &b->d_cut);
+    close_run();
     int32_t* d_all = nullptr;
     KIWI_TRY(balloc(b, all.size(), &d_all));
-    for (const auto& e : place) *e.first = d_all + e.second;
+    for (const Place& p : where) {
+        KiwiBatch::Run& r = b->runs[p.run];
+        (p.list ? r.*p.list : (r.*p.lists)[p.family]) = d_all + p.at;
+    }
     KIWI_CUDA(ctx, cudaMemcpyAsync(d_all, all.data(), sizeof(int32_t) * all.size(), cudaMemcpyHostToDevice, ctx->stream));
     KIWI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));  // `all` is local
-    return balloc(b, (size_t)places * 4 * kTileCells, &b->d_sums);
+    return KIWI_OK;
 }
 
 int batch_build(KiwiBatch* b, const KiwiBatchItem* in) {
@@ -400,7 +468,12 @@ int kiwi_batch_create(KiwiCtx* ctx, const KiwiBatchItem* items, int n_items, int
     b->n_items = n_items;
     b->precision = precision;
     b->merge = form == KIWI_FP64;
-    const int rc = batch_build(b, items);
+    int rc = KIWI_OK;
+    try {
+        rc = batch_build(b, items);
+    } catch (const std::bad_alloc&) {
+        rc = set_err(ctx, KIWI_ERR_ALLOC, "batch: out of host memory");
+    }
     if (rc != KIWI_OK) {
         batch_free(b);
         delete b;
@@ -419,9 +492,12 @@ int kiwi_batch_run(KiwiBatch* b, KiwiStats* item_stats, KiwiStats* total) {
     KIWI_TRY(batch_time_once(b, &ms));
     std::vector<DevStats> h(b->n_items);
     KIWI_CUDA(ctx, cudaMemcpy(h.data(), b->d_stats, sizeof(DevStats) * b->n_items, cudaMemcpyDeviceToHost));
-    // mean velocities, one launch per family present, the cut tiles' sums
-    int64_t kernels = b->n_items + (b->n_cut > 0 ? 1 : 0);
-    for (int f = 0; f < kBatchFamilies; ++f) kernels += b->fam_tiles[f] > 0 ? 1 : 0;
+    // mean velocities, per run one launch per family present and the cut tiles' sums
+    int64_t kernels = b->n_items;
+    for (const KiwiBatch::Run& r : b->runs) {
+        kernels += r.n_cut > 0 ? 1 : 0;
+        for (int f = 0; f < kBatchFamilies; ++f) kernels += r.items[f] > 0 ? 1 : 0;
+    }
     (void)launches0;
     KiwiStats sum{};
     for (int i = 0; i < b->n_items; ++i) {
@@ -467,7 +543,7 @@ int kiwi_batch_tune(KiwiBatch* b, int* chosen) {
     float best = 1e30f;
     bool best_lpt = b->lpt, best_merge = b->merge;
     int best_ctas = b->ctas_per_sm;
-    const bool both = families_present(b) > 1 && b->fam_tiles[kBatchFamilyGather] == 0;
+    const bool both = families_present(b) > 1 && b->fam_items[kBatchFamilyGather] == 0;
     for (int merge = both ? 1 : 0; merge >= 0; --merge) {
         for (int lpt = 1; lpt >= 0; --lpt) {
             for (int ctas = 1; ctas <= 2; ++ctas) {

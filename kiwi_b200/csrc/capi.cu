@@ -165,7 +165,7 @@ int sph_to_grid_dev(KiwiCtx* ctx, const DevParticles& P, const CartGeom& g, cons
         KIWI_LAUNCHED(ctx);
     }
     TileLists tl{sorted_vals, range, ntiles, total};
-    // the FP64 form orders its own work (box_work_make)
+    // the FP64 form orders its own work (box_work_next)
     const bool own_order = (precision & KIWI_FORM_MASK) == KIWI_FP64 && (kc.cubic || !(precision & KIWI_FULL_BOX));
     if (n_parts > 1) {
         // this part's tiles: a contiguous run of the tile order holding ~1/n_parts of the entries

@@ -142,16 +142,19 @@ int fp64_measure_peak(KiwiCtx* ctx, double* tflops);
 struct BoxItem {
     int32_t tile, seg, nseg, slot;
 };
-// The work of a box-mass gather over a call's tiles: items (heaviest first), or none when the tiles run as they are;
-// the places of the cut tiles' sums and the cut tiles, whose outputs box_work_finish forms.
+// The work of a box-mass gather over a run of a call's tiles (nearly always all of them): items (heaviest first), or
+// none when the tiles run as they are; the places of the cut tiles' sums and the cut tiles, whose outputs
+// box_work_finish forms.  box_work_next makes the next run's, from tile `done` of the call on; the last run ends with
+// done >= all.
 struct BoxWork {
+    int64_t done = 0, all = 0, run = 0;  // run: tiles per run, 0 all at once
     const BoxItem* items = nullptr;
     int64_t n = 0;
     const BoxItem* cut = nullptr;
     int64_t n_cut = 0;
     double* sums = nullptr;
 };
-int box_work_make(KiwiCtx* ctx, const TileLists& tl, BoxWork* w);
+int box_work_next(KiwiCtx* ctx, const TileLists& tl, BoxWork* w);
 int box_work_finish(KiwiCtx* ctx, const CartGeom& g, const BoxWork& w, const CartOutputs& out);
 int lattice_init_tables(KiwiCtx* ctx);
 int adjoint_init_tables(KiwiCtx* ctx);
@@ -164,11 +167,13 @@ int lattice_mixed_gather(KiwiCtx* ctx, const CartGeom& g, const DevParticles& P,
 int lattice_batch_prepare(KiwiCtx* ctx);
 // A batch's work (four ints per item: tile, segment, the tile's segments, the place of its sums): the items of
 // `tiles` given every tile's range, its grid's tile count and its place (host); split: long lists cut into
-// segments, else whole tiles; heaviest: in descending order of their entries.  Returns their number.
-int lattice_batch_work(const std::vector<int32_t>& tiles, const std::vector<int64_t>& range,
-                       const std::vector<int64_t>& grid_tiles, const std::vector<int32_t>& slot, bool split, bool heaviest,
-                       std::vector<int32_t>* work);
+// segments, else whole tiles; weight: their entries.
+void lattice_batch_work(const std::vector<int32_t>& tiles, const std::vector<int64_t>& range,
+                        const std::vector<int64_t>& grid_tiles, const std::vector<int32_t>& slot, bool split,
+                        std::vector<int32_t>* work, std::vector<int64_t>* weight);
 int64_t lattice_batch_segments(int64_t cnt, int64_t grid_tiles);
+// Segments whose sums a batch holds at a time (16 KB each: 1 GB).
+constexpr int64_t kBatchPlaces = 65536;
 // sums: raw sums of the cut tiles' segments, 4 x kTileCells doubles each; d_cut: the cut tiles' first items.
 int lattice_batch_gather(KiwiCtx* ctx, int family, const BatchItemDev* d_items, const int32_t* d_item_of_tile,
                          const int32_t* d_work, int64_t nwork, const uint32_t* list,

@@ -503,11 +503,14 @@ int fp64_cart_gather(KiwiCtx* ctx, const CartGeom& g, const DevParticles& P, con
         constexpr size_t smem = BoxCaps<1, false, true>::kSmem;
         KIWI_CUDA(ctx, cudaFuncSetAttribute(k_cart_box_tab, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         BoxWork w;
-        KIWI_TRY(box_work_make(ctx, tl, &w));
-        k_cart_box_tab<<<(unsigned)w.n, kBoxThreads, smem, ctx->stream>>>(g, P, k.tab, tl.list, tl.range, tl.map, w.items,
-                                                                          out, w.sums, d_stats);
-        KIWI_LAUNCHED(ctx);
-        return box_work_finish(ctx, g, w, out);
+        do {
+            KIWI_TRY(box_work_next(ctx, tl, &w));
+            k_cart_box_tab<<<(unsigned)w.n, kBoxThreads, smem, ctx->stream>>>(g, P, k.tab, tl.list, tl.range, tl.map,
+                                                                              w.items, out, w.sums, d_stats);
+            KIWI_LAUNCHED(ctx);
+            KIWI_TRY(box_work_finish(ctx, g, w, out));
+        } while (w.done < w.all);
+        return KIWI_OK;
     } else if (k.tabulated) {
         k_cart_gather_tab<<<grid, kThreads, 0, ctx->stream>>>(g, P, k.tab, tl.list, tl.range, tl.map, out, d_stats);
     } else if (!reference_order && (k.cubic || !full_box)) {

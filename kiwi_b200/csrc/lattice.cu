@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(256) k_box_combine(CartGeom g, const BoxItem* 
     box_combine(g, out, it.tile, sums + (int64_t)it.slot * 4 * kTileCells, it.nseg);
 }
 
-// The items of the tiles map[0 .. n) (every tile if null), heaviest first by 64 classes of their entry counts (the
+// The items of the tiles map[first .. first + n) (tiles from `first` on if null), heaviest first by 64 classes of their entry counts (the
 // order among the items, and among the places of their sums, does not affect any result).  counts: items, places
 // of sums, cut tiles, then the classes' sizes and their running starts (64 each).
 constexpr int kBoxClasses = 64;
@@ -89,7 +89,8 @@ __device__ __forceinline__ int box_class(int64_t len, int64_t ntiles) {
 }
 template <bool EMIT>
 __global__ void __launch_bounds__(256) k_box_items(const int64_t* __restrict__ range, int64_t ntiles,
-                                                   const int32_t* __restrict__ map, int64_t n, int* __restrict__ counts,
+                                                   const int32_t* __restrict__ map, int64_t first, int64_t n,
+                                                   int* __restrict__ counts,
                                                    BoxItem* __restrict__ items, BoxItem* __restrict__ cut) {
     __shared__ int s_n[kBoxClasses], s_at[kBoxClasses];
     if (threadIdx.x < kBoxClasses) s_n[threadIdx.x] = 0;
@@ -97,7 +98,7 @@ __global__ void __launch_bounds__(256) k_box_items(const int64_t* __restrict__ r
     const int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     int t = 0, nseg = 0, full = 0, last = 0, at_full = 0, at_last = 0;
     if (w < n) {
-        t = map ? map[w] : (int)w;
+        t = map ? map[first + w] : (int)(first + w);
         const int64_t cnt = range[2 * (int64_t)t + 1] - range[2 * (int64_t)t], len = box_segment(cnt, ntiles);
         nseg = cnt > len ? (int)((cnt + len - 1) / len) : 1;
         full = box_class(len, ntiles);
@@ -257,32 +258,55 @@ static int box_launch_kernel(KiwiCtx* ctx, int64_t blocks, const CartGeom& g, co
     }
 }
 
-int box_work_make(KiwiCtx* ctx, const TileLists& tl, BoxWork* w) {
-    const int64_t n = tl.map ? tl.nmap : tl.ntiles;
-    *w = BoxWork{};
-    w->n = n;
+int box_work_next(KiwiCtx* ctx, const TileLists& tl, BoxWork* w) {
+    w->all = tl.map ? tl.nmap : tl.ntiles;
+    const int64_t first = w->done;
+    int64_t n = w->all - first;
     // no list can be longer than a segment: the tiles as they are
-    if (tl.total <= box_segment(0, tl.ntiles)) return KIWI_OK;
+    if (tl.total <= box_segment(0, tl.ntiles)) {
+        w->n = n;
+        w->done = w->all;
+        return KIWI_OK;
+    }
     constexpr int kCounts = 4 + 2 * kBoxClasses + 2;
+    const int64_t most = box_most(tl.ntiles);
     int* counts = nullptr;
     KIWI_TRY(scratch_t(ctx, S_BOX_COUNTS, kCounts, &counts));
-    KIWI_CUDA(ctx, cudaMemsetAsync(counts, 0, sizeof(int) * kCounts, ctx->stream));
-    const unsigned nb = (unsigned)((n + 255) / 256);
-    k_box_items<false><<<nb, 256, 0, ctx->stream>>>(tl.range, tl.ntiles, tl.map, n, counts, nullptr, nullptr);
-    KIWI_LAUNCHED(ctx);
     int h[3] = {0, 0, 0};
-    KIWI_CUDA(ctx, cudaMemcpyAsync(h, counts, sizeof h, cudaMemcpyDeviceToHost, ctx->stream));
-    KIWI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    // the run: all that is left, or as many tiles as kBoxPlaces hold; half as many as long as their sums cannot be had
+    for (;;) {
+        if (w->run > 0) n = std::min(n, w->run);
+        KIWI_CUDA(ctx, cudaMemsetAsync(counts, 0, sizeof(int) * kCounts, ctx->stream));
+        k_box_items<false><<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(tl.range, tl.ntiles, tl.map, first, n,
+                                                                                counts, nullptr, nullptr);
+        KIWI_LAUNCHED(ctx);
+        KIWI_CUDA(ctx, cudaMemcpyAsync(h, counts, sizeof h, cudaMemcpyDeviceToHost, ctx->stream));
+        KIWI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        if (h[1] > kBoxPlaces && n > kBoxPlaces / most) {
+            w->run = kBoxPlaces / most;
+            continue;
+        }
+        w->sums = nullptr;
+        if (h[1] == 0) break;
+        // (runs take the most that one may need, so that the buffer does not grow from run to run)
+        const size_t places = w->run > 0 ? (size_t)(n * most) : (size_t)h[1];
+        const int rc = scratch_t(ctx, S_BOX_SUMS, places * 4 * kTileCells, &w->sums);
+        if (rc == KIWI_OK) break;
+        if (rc != KIWI_ERR_ALLOC || n <= 1) return rc;
+        ctx->err.clear();
+        w->run = (n + 1) / 2;
+    }
     BoxItem *items = nullptr, *cut = nullptr;
     KIWI_TRY(scratch_t(ctx, S_BOX_ITEMS, (size_t)h[0], &items));
     KIWI_TRY(scratch_t(ctx, S_BOX_CUT, (size_t)(h[2] > 0 ? h[2] : 1), &cut));
-    if (h[1] > 0) KIWI_TRY(scratch_t(ctx, S_BOX_SUMS, (size_t)h[1] * 4 * kTileCells, &w->sums));
-    k_box_items<true><<<nb, 256, 0, ctx->stream>>>(tl.range, tl.ntiles, tl.map, n, counts, items, cut);
+    k_box_items<true><<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(tl.range, tl.ntiles, tl.map, first, n, counts,
+                                                                           items, cut);
     KIWI_LAUNCHED(ctx);
     w->items = items;
     w->n = h[0];
     w->cut = cut;
     w->n_cut = h[2];
+    w->done = first + n;
     return KIWI_OK;
 }
 
@@ -300,27 +324,28 @@ int lattice_cart_gather(KiwiCtx* ctx, const CartGeom& g, const DevParticles& P, 
         return box_launch_kernel<true>(ctx, tl.map ? tl.nmap : tl.ntiles, g, P, k, tl, nullptr, out, nullptr, d_stats,
                                        full_box);
     BoxWork w;
-    KIWI_TRY(box_work_make(ctx, tl, &w));
-    KIWI_TRY(box_launch_kernel<false>(ctx, w.n, g, P, k, tl, w.items, out, w.sums, d_stats, full_box));
-    return box_work_finish(ctx, g, w, out);
+    do {
+        KIWI_TRY(box_work_next(ctx, tl, &w));
+        KIWI_TRY(box_launch_kernel<false>(ctx, w.n, g, P, k, tl, w.items, out, w.sums, d_stats, full_box));
+        KIWI_TRY(box_work_finish(ctx, g, w, out));
+    } while (w.done < w.all);
+    return KIWI_OK;
 }
 
-// The work of a batch's tiles tiles[0 .. n) with their ranges (host): natural order, or heaviest segment first.
-int lattice_batch_work(const std::vector<int32_t>& tiles, const std::vector<int64_t>& range,
-                       const std::vector<int64_t>& grid_tiles, const std::vector<int32_t>& slot, bool split, bool heaviest,
-                       std::vector<int32_t>* work) {
-    std::vector<std::pair<int64_t, BoxItem>> v;
+void lattice_batch_work(const std::vector<int32_t>& tiles, const std::vector<int64_t>& range,
+                        const std::vector<int64_t>& grid_tiles, const std::vector<int32_t>& slot, bool split,
+                        std::vector<int32_t>* work, std::vector<int64_t>* weight) {
+    work->clear();
+    weight->clear();
     for (const int32_t t : tiles) {
         const int64_t cnt = range[2 * (size_t)t + 1] - range[2 * (size_t)t];
         const int64_t len = split ? box_segment(cnt, grid_tiles[(size_t)t]) : cnt;
         const int nseg = cnt > len ? (int)((cnt + len - 1) / len) : 1;
-        for (int s = 0; s < nseg; ++s)
-            v.push_back({nseg > 1 ? std::min(len, cnt - s * len) : cnt, BoxItem{t, s, nseg, nseg > 1 ? slot[(size_t)t] : 0}});
+        for (int s = 0; s < nseg; ++s) {
+            work->insert(work->end(), {t, s, nseg, nseg > 1 ? slot[(size_t)t] : 0});
+            weight->push_back(nseg > 1 ? std::min(len, cnt - s * len) : cnt);
+        }
     }
-    if (heaviest) std::stable_sort(v.begin(), v.end(), [](const auto& a, const auto& b) { return a.first > b.first; });
-    work->clear();
-    for (const auto& e : v) work->insert(work->end(), {e.second.tile, e.second.seg, e.second.nseg, e.second.slot});
-    return (int)v.size();
 }
 
 int64_t lattice_batch_segments(int64_t cnt, int64_t grid_tiles) {
