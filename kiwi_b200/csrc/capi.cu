@@ -112,7 +112,6 @@ int sph_to_grid_dev(KiwiCtx* ctx, const DevParticles& P, const CartGeom& g, cons
         if ((precision & KIWI_FORM_MASK) == KIWI_FP32_MIXED)
             return set_err(ctx, KIWI_ERR_UNSUPPORTED, "the FP32-mixed form is available for the analytic integral only");
         KIWI_TRY(table_ensure(ctx, &kc.tab));
-        if ((precision & KIWI_FORM_MASK) == KIWI_FP64) KIWI_TRY(table_blocks(ctx, &kc.tab));
     }
     const int64_t launches0 = ctx->launches;
     DevStats* d_stats = nullptr;
@@ -208,8 +207,9 @@ int sph_to_grid_dev(KiwiCtx* ctx, const DevParticles& P, const CartGeom& g, cons
         tl.nmap = ntiles;
     }
 
-    KIWI_CUDA(ctx, cudaEventRecord(ctx->ev[0], ctx->stream));
     const int form = precision & KIWI_FORM_MASK;
+    if (kc.tabulated && form == KIWI_FP64) KIWI_TRY(table_blocks(ctx));  // (after the binning's scratch)
+    KIWI_CUDA(ctx, cudaEventRecord(ctx->ev[0], ctx->stream));
     const bool full_box = (precision & KIWI_FULL_BOX) != 0;
     int64_t fp64_tiles = 0;
     if ((precision & KIWI_FP32_GUARANTEE) && form != KIWI_FP32_MIXED)

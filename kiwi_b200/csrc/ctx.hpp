@@ -14,7 +14,9 @@ namespace kiwi_b200 {
 // the sub-grid sizes and split points of its three axes and the values, laid out as the reference does.
 struct TabDev {
     const double* v = nullptr;
-    const double* v4 = nullptr;  // the table in blocks of four neighbours (table_blocks), or null
+    // the table in blocks of four neighbours (table_blocks), or null; the context's own is read at the launch, since a
+    // scratch request that finds no memory gives it back
+    const double* v4 = nullptr;
     int nr01 = 0, nR_01 = 0, nphi1 = 0, nr02 = 0, nR_02 = 0, nphi2 = 0, nr0 = 0, nR_0 = 0, nphi = 0;
     double rl = 0.0, mul = 0.0, cphil = 0.0;
 };
@@ -103,7 +105,15 @@ inline int scratch(KiwiCtx* ctx, int slot, size_t bytes, void** out) {
         }
         size_t want = bytes + bytes / 4;
         cudaError_t e = cudaMalloc(&ctx->slot_ptr[slot], want);
+        if (e != cudaSuccess && ctx->tab.v4) {  // the table's block copy is a convenience: given back first
+            cudaGetLastError();
+            cudaStreamSynchronize(ctx->stream);
+            cudaFree(const_cast<double*>(ctx->tab.v4));
+            ctx->tab.v4 = nullptr;
+            e = cudaMalloc(&ctx->slot_ptr[slot], want);
+        }
         if (e != cudaSuccess) {
+            ctx->slot_ptr[slot] = nullptr;
             cudaGetLastError();
             return set_err(ctx, KIWI_ERR_ALLOC, "cudaMalloc of %zu bytes of scratch failed: %s", want,
                            cudaGetErrorString(e));

@@ -29,9 +29,9 @@ struct KernelChoice {
 
 // tabulated.cu: the context's density table, generating the canonical one if it holds none.
 int table_ensure(KiwiCtx* ctx, TabDev* out);
-// The same with the table also in blocks of four neighbours (four times its memory, 730 MB for the canonical shape,
-// released with it), unless that is over 4 GB or cannot be had.
-int table_blocks(KiwiCtx* ctx, TabDev* out);
+// The context's table also in blocks of four neighbours (four times its memory, 730 MB for the canonical shape; released
+// with it, or when other scratch finds no memory), unless that is over 4 GB or cannot be had.
+int table_blocks(KiwiCtx* ctx);
 void table_free(KiwiCtx* ctx);
 
 // Tile lists built by the binning step: tile t owns list[range[2t] .. range[2t+1]) (particle indices in

@@ -505,7 +505,9 @@ int fp64_cart_gather(KiwiCtx* ctx, const CartGeom& g, const DevParticles& P, con
         BoxWork w;
         do {
             KIWI_TRY(box_work_next(ctx, tl, &w));
-            k_cart_box_tab<<<(unsigned)w.n, kBoxThreads, smem, ctx->stream>>>(g, P, k.tab, tl.list, tl.range, tl.map,
+            TabDev tab = k.tab;
+            tab.v4 = ctx->tab.v4;
+            k_cart_box_tab<<<(unsigned)w.n, kBoxThreads, smem, ctx->stream>>>(g, P, tab, tl.list, tl.range, tl.map,
                                                                               w.items, out, w.sums, d_stats);
             KIWI_LAUNCHED(ctx);
             KIWI_TRY(box_work_finish(ctx, g, w, out));

@@ -202,7 +202,7 @@ int table_ensure(KiwiCtx* ctx, TabDev* out) {
     return KIWI_OK;
 }
 
-int table_blocks(KiwiCtx* ctx, TabDev* out) {
+int table_blocks(KiwiCtx* ctx) {
     const int64_t n = (int64_t)(ctx->tab.nr0 + 1) * (ctx->tab.nR_0 + 1) * (ctx->tab.nphi + 1);
     if (!ctx->tab.v4 && n * (int64_t)sizeof(double4) <= ((int64_t)4 << 30)) {
         double4* d = nullptr;
@@ -214,7 +214,6 @@ int table_blocks(KiwiCtx* ctx, TabDev* out) {
             cudaGetLastError();  // the lookups read the table itself
         }
     }
-    *out = ctx->tab;
     return KIWI_OK;
 }
 
