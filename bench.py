@@ -56,11 +56,13 @@ CELL_ASSEMBLY = 60.0
 # The FP64 box-mass kernel's work items (cubic spline, counted in box_math.cuh; a line counts as two edge tiers, a
 # point as six vertex pyramids): a line beyond the support 5 flops, within it 60 flops + 6 transcendentals for the
 # outer piece alone and 105 + 11 for both; a point within the support 75 + 5, beyond it 12, of which the former are
-# 26 % on the default workload (counted over 3,000 of its particles); a cell ~12 flops.
+# 26 % on the default workload (counted over 3,000 of its particles; the kernel's counter holds both, so that other
+# workloads and kernels have no achieved rate here); a cell ~12 flops.
 BOX_EDGE_OUTER = 2.5
 BOX_EDGE_MIDDLE = 30.0 + TRANS_FLOPS * 3
 BOX_EDGE_INNER = 52.5 + TRANS_FLOPS * 5.5
-BOX_VERTEX_PYRAMID = (0.26 * (75.0 + TRANS_FLOPS * 5) + 0.74 * 12.0) / 6
+BOX_NEAR_SHARE = {"n": 2_000_000, "res": 256, "kernel": "cubic_spline", "share": 0.26}
+BOX_VERTEX_PYRAMID = (BOX_NEAR_SHARE["share"] * (75.0 + TRANS_FLOPS * 5) + (1 - BOX_NEAR_SHARE["share"]) * 12.0) / 6
 BOX_CELL_ASSEMBLY = 12.0
 
 # DRAM bytes (read + write) of one k_cart_box launch on the default workload (2 M particles, 256^3) from
@@ -895,7 +897,7 @@ def main():
         """Per-cell and total-mass error of FP32-form densities g against FP64-form densities r."""
         msk = r >= 1e-6 * r.max()
         rel = ((g[msk] - r[msk]).abs() / r[msk]).double()
-        acc = {"against": "the FP64 form (lattice), same input", "cells_above_1e-6_peak": int(msk.sum()),
+        acc = {"against": "the FP64 form, same input", "cells_above_1e-6_peak": int(msk.sum()),
                "nonfinite_cells": int((~torch.isfinite(g)).sum()),
                "max_rel_cell_err": float(rel.max()), "median_rel_cell_err": float(rel.median()),
                "q99_rel_cell_err": float(torch.quantile(rel[: 1 << 24].float(), 0.99)),
@@ -929,7 +931,7 @@ def main():
             steps32 = args.steps if prec == "fp32_mixed" else min(args.steps, 2)
             for _ in range(min(args.warmup, 2)):
                 kiwi_b200.sph_to_grid_device(dP, bounds, shape, o32, kernel=ki, precision=prec, ctx=ctx)
-            ms32, pairs32 = 0.0, 0
+            ms32, pairs32, work32 = 0.0, 0, 0.0
             for _ in range(steps32):
                 with torch.cuda.stream(stream):
                     flush.zero_()
@@ -942,8 +944,13 @@ def main():
                 e1.synchronize()
                 ms32 += e0.elapsed_time(e1)
                 pairs32 += st32["sphere_pairs"]
+                work32 += (st32["edge_tiers_outer"] * EDGE_OUTER + st32["edge_tiers_middle"] * EDGE_MIDDLE +
+                           st32["edge_tiers_inner"] * EDGE_INNER + st32["vertex_pyramids"] * VERTEX_PYRAMID +
+                           st32["evaluated_pairs"] * CELL_ASSEMBLY)
             acc32 = fp32_accuracy(o32["density"], out["density"], st32, prec)
             v32 = pairs32 / (ms32 * 1e-3)
+            if prec == "fp32_mixed":
+                achieved32 = work32 / (ms32 * 1e-3) / 1e12
             fp32_side[prec] = {"precision": prec, "value": v32 * ws, "unit": "pair-integrals/s", "steps": steps32,
                                "ms_per_step": ms32 / steps32,
                                "ratio_vs_fp64": v32 / (tot_ms and sph_pairs / (tot_ms * 1e-3)),
@@ -1014,18 +1021,19 @@ def main():
             kname = ("k_cart_lattice_f32 (FP32 lattice tiers with rounding bounds; flagged tiles recomputed in FP64)"
                      if args.precision == "fp32_mixed_guaranteed" else
                      "k_cart_lattice_mixed (FP32 lattice tiers, FP64 islands and assembly)" if is32 else
-                     "k_cart_box (FP64 box-mass gather)" if args.kernel == "cubic_spline"
-                     else "k_cart_box (FP64 box-mass gather; work items costed at the cubic spline's rates)")
+                     "k_cart_box (FP64 box-mass gather)")
             eo, em, ei, vp, cell = ((EDGE_OUTER, EDGE_MIDDLE, EDGE_INNER, VERTEX_PYRAMID, CELL_ASSEMBLY) if is32 else
                                     (BOX_EDGE_OUTER, BOX_EDGE_MIDDLE, BOX_EDGE_INNER, BOX_VERTEX_PYRAMID, BOX_CELL_ASSEMBLY))
             work = (items["edge_tiers_outer"] * eo + items["edge_tiers_middle"] * em + items["edge_tiers_inner"] * ei +
                     items["vertex_pyramids"] * vp + evaluated * cell) / args.steps
-            work_per_pair = work / max(evaluated_per_launch, 1)
+            if not is32 and any(getattr(args, k) != BOX_NEAR_SHARE[k] for k in ("n", "res", "kernel")):
+                work = None  # the share of points within the support is not known here
+            work_per_pair = work / max(evaluated_per_launch, 1) if work is not None else None
         else:
             kname = "k_cart_gather (FP64 cell-integral gather, reference evaluation order)"
             work_per_pair = WORK_PER_BBOX_PAIR if args.full_box else WORK_PER_SUPPORT_PAIR
             work = evaluated_per_launch * work_per_pair
-        achieved = work / (g_ms * 1e-3) / 1e12
+        achieved = work / (g_ms * 1e-3) / 1e12 if work is not None else None
         peak = kiwi_b200.measure_fp32_peak(ctx) if is32 else peak_fp64
         # DRAM traffic of the kernel per launch: an ncu capture of this exact workload (one pass,
         # dram__bytes_read.sum + dram__bytes_write.sum), stated with the commit it was captured at; the
@@ -1063,7 +1071,7 @@ def main():
             "roofline": {"bound": "fp32" if is32 else "fp64", "kernel": kname, "work_items_per_launch":
                          {k: v / args.steps for k, v in items.items()},
                          "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
-                         "frac": achieved / peak if peak else None, "traffic": traffic,
+                         "frac": achieved / peak if peak and achieved is not None else None, "traffic": traffic,
                          "traffic_source": traffic_src,
                          "hbm": ({"achieved_gbs": traffic / (g_ms * 1e-3) / 1e9, "peak_gbs": hbm_peak,
                                   "frac": traffic / (g_ms * 1e-3) / 1e9 / hbm_peak, "peak_source": hbm_src}
@@ -1083,12 +1091,10 @@ def main():
         if parity_c1 is not None:
             line["parity_c1"] = parity_c1
         if fp32_side is not None:
-            # the FP32 lattice kernel evaluates the same lattice work items as the FP64 one
             peak32 = kiwi_b200.measure_fp32_peak(ctx)
             side = fp32_side["fp32_mixed"]
-            a32 = work_per_pair * side["value"] / ws / 1e12
-            side["roofline"] = {"bound": "fp32", "kernel": "k_cart_lattice_mixed", "achieved": a32, "peak": peak32,
-                                "unit": "TFLOP/s", "frac": a32 / peak32 if peak32 else None,
+            side["roofline"] = {"bound": "fp32", "kernel": "k_cart_lattice_mixed", "achieved": achieved32, "peak": peak32,
+                                "unit": "TFLOP/s", "frac": achieved32 / peak32 if peak32 else None,
                                 "peak_source": "measured FP32 FMA probe (kiwi_measure_fp32_peak) in this run"}
             line["fp32_mixed"] = side
             line["fp32_mixed_guaranteed"] = fp32_side["fp32_mixed_guaranteed"]
