@@ -1,4 +1,5 @@
-// Forward-mode derivatives for the adjoint: a value with N partial derivatives (Dual4: with respect to the
+// Forward-mode derivatives, by which the host tests check derivatives of the closed forms (the adjoint's are in closed form
+// themselves, box_grad.cuh): a value with N partial derivatives (Dual4: with respect to the
 // particle's x0, y0, z0 and h; Dual3: x0, y0, z0), propagated through every arithmetic operation and libm
 // call by the chain rule.  Instantiating the closed-form face walk (kiwi_math.cuh) with Dual4 gives the exact derivatives
 // of the computed cell integral (branch by branch: region choices, the foot rule and the clamp are

@@ -15,7 +15,6 @@
 #include <math.h>
 #include <stdint.h>
 
-#include <type_traits>
 
 #include "kernel_tables.h"
 
@@ -35,7 +34,7 @@ constexpr double kPi = 3.14159265358979323846;
 
 // Every function of the cubic closed form and of the face walk is written once over the real type T:
 // T = double is the FP64 evaluation (the reference's operations one by one), T = Dual4 (dual.cuh) carries
-// the derivatives with respect to the particle's position and smoothing length for the adjoint.
+// the derivatives with respect to the particle's position and smoothing length, for the host tests.
 template <class T>
 struct CubicWallT {
     bool valid;
@@ -383,13 +382,6 @@ template <class T>
 KIWI_HD T vmin2(const T& a, const T& b) { return a < b ? a : b; }
 
 // Vertex source for the face walk: VX(i), VY(i), VZ(i) give vertex i of the face (n vertices, n >= 3).
-// Whether a face-walk evaluator takes the vertex pyramid's leg along the edge (at_len(t)) instead of its
-// angle (at(phi)).
-template <class E, class = void>
-struct EvalUsesLengths : std::false_type {};
-template <class E>
-struct EvalUsesLengths<E, std::void_t<decltype(E::kLengths)>> : std::integral_constant<bool, E::kLengths> {};
-
 // face_integral_impl of src/kernel_integral.cpp:471-647, including the out_vert reachability rule.
 // T is the type of the particle's coordinates (the face's vertices are plain doubles): double, or Dual4
 // for the derivatives of the face integral with respect to the particle.
@@ -446,28 +438,15 @@ KIWI_HD T face_integral(T x0, T y0, T z0, T support_radius, const Verts& V, int 
                 inside_polygon = false;
             }
         }
-        bool foot_beyond_endpoint, first_wider;
         T I1v = 0.0, I2v = 0.0;
-        if constexpr (EvalUsesLengths<Eval>::value) {
-            // the legs along the edge line from each vertex to the foot: r12 |cos a| and |r23 - r12 cos a|
-            // (the reference's r12 sin(phi1) and r13 sin(phi2)); phi1 >= phi2 iff t1 >= t2
-            const T t1 = r12 * fabs(cosa), t2 = fabs(r23 - r12 * cosa);
-            foot_beyond_endpoint = (t1 >= r23) || (t2 >= r23);
-            first_wider = t1 >= t2;
-            ev.set_edge(R_0);
-            I1v = ev.at_len(t1);
-            I2v = ev.at_len(t2);
-        } else {
-            const T phi1 = (R_0 < r12) ? acos(R_0 / r12) : T(0.0);
-            const T phi2 = (R_0 < r13) ? acos(R_0 / r13) : T(0.0);
-            foot_beyond_endpoint = (r12 * sin(phi1) >= r23) || (r13 * sin(phi2) >= r23);
-            first_wider = phi1 >= phi2;
-            ev.set_edge(R_0);
+        const T phi1 = (R_0 < r12) ? acos(R_0 / r12) : T(0.0);
+        const T phi2 = (R_0 < r13) ? acos(R_0 / r13) : T(0.0);
+        const bool foot_beyond_endpoint = (r12 * sin(phi1) >= r23) || (r13 * sin(phi2) >= r23), first_wider = phi1 >= phi2;
+        ev.set_edge(R_0);
 #pragma unroll 1
-            for (int v = 0; v < 2; ++v) {
-                const T t = ev.at(v == 0 ? phi1 : phi2);
-                if (v == 0) I1v = t; else I2v = t;
-            }
+        for (int v = 0; v < 2; ++v) {
+            const T t = ev.at(v == 0 ? phi1 : phi2);
+            if (v == 0) I1v = t; else I2v = t;
         }
         const T in_plane_dist = foot_beyond_endpoint ? vmin2(r12, r13) : R_0;
         min_edge_dist = vmin2(min_edge_dist, in_plane_dist);

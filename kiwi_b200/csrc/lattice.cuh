@@ -1,4 +1,5 @@
-// Lattice-factorised cell integrals for box cells (cubic spline closed form).
+// Lattice-factorised cell integrals for box cells (cubic spline closed form): the FP32-mixed kernels (lattice_tile.cuh,
+// mixed.cu), and the bookkeeping that the FP64 form's kernels (box_tile.cuh, adjoint.cu) share with them.
 //
 // The reference evaluates each (particle, cell) pair as 6 faces x 4 edges x 2 vertex pyramids
 // (src/kernel_integral.cpp:471-647, src/cartesian_grid.cpp:246-259).  For axis-aligned cells every one of
@@ -17,7 +18,7 @@
 // the same 48 vertex-pyramid terms with the same signs (a face's edge/foot-beyond rule of
 // src/kernel_integral.cpp:613-631 is the 2-D inclusion-exclusion of a cumulative function) -- with
 // every series written in its triangle's or edge's own lengths from a few reciprocals (lattice_edge,
-// lattice_corner, lattice_pyramid) instead of acos(R_0/r12) followed by sincos and a division per ratio.
+// lattice_corner) instead of acos(R_0/r12) followed by sincos and a division per ratio.
 #pragma once
 
 #include "cart_common.cuh"
@@ -25,30 +26,6 @@
 #include "lattice_math.cuh"
 
 namespace kiwi_b200 {
-
-constexpr int kLatECap = 1536;   // edge-tier entries per chunk (one full 8^3 particle box needs 486)
-constexpr int kLatSCap = 4096;   // corner values per chunk (one full 8^3 particle box needs 2187)
-
-// Face-walk evaluator of the plain FP64 Voronoi map (CubicEval's role): the edge tier in the edge's own
-// lengths (lattice_edge) and each vertex pyramid from its triangle's lengths (lattice_pyramid); the face
-// walk hands it the leg t along the edge instead of the angle (kLengths).
-struct LenCubicEval {
-    static constexpr bool kLengths = true;
-    double h = 0.0, ih = 0.0, r0 = 0.0, R_0 = 0.0, D2 = 0.0, D3 = 0.0;
-    __device__ void set_wall(double ar0) { r0 = ar0; }
-    __device__ void set_edge(double R) {
-        R_0 = R;
-        D2 = D3 = 0.0;
-        if (r0 != 0.0 && R != 0.0 && r0 * r0 + R * R <= 4.0 * (h * h)) {
-            const LatticeEdge e = lattice_edge(h, ih, r0, R);
-            D2 = e.D2;
-            D3 = e.D3;
-        }
-    }
-    __device__ double at_len(double t) const {
-        return (r0 == 0.0 || R_0 == 0.0 || t == 0.0) ? 0.0 : lattice_pyramid(h, ih, r0, R_0, t, D2, D3);
-    }
-};
 
 // Position of the smallest j with s_off[j] <= it among the chunk's np particles (s_off ascending).
 static __device__ __forceinline__ int chunk_search(const int* s_off, int np, int it) {

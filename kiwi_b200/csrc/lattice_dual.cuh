@@ -1,4 +1,4 @@
-// Generic-kernel edge records with forward derivatives, for the adjoint's lattice form: the record of
+// Generic-kernel edge records with forward derivatives, for the host tests: the record of
 // lattice_generic_edge_t evaluated in DualN<N>.  The segment boundaries phi_end are only compared with the
 // vertices' angles (a choice taken on values), so they are kept as values; the continuity offsets carry
 // their derivatives.  Layout, kLatGenDualRec(N) doubles: [0] = nseg + 8 x first region, [1..3] = phi_end of

@@ -1,5 +1,5 @@
 // The closed-form maths of the lattice kernels (cubic spline and table-driven generic kernels), written over
-// the real type T (double in the forward kernels, Dual4 in the adjoint) and compiled both for the device and,
+// the real type T (F32 and double in the FP32-mixed kernels, dual numbers in the host tests) and compiled both for the device and,
 // by the test-only check tests/host_math_check.cpp, for the host.  The kernels' bookkeeping (chunk lists,
 // warp votes, lattice offsets) is in lattice.cuh.
 #pragma once
@@ -48,8 +48,8 @@ KIWI_LAT void leg_angles(T a1, T ia1, T a2, T ia2, T& pa, T& pb) {
 // The wall constants of the cubic spline (src/kernel_integral.cpp:222-247) divided by r0^3, as
 // polynomials in r0 / h and h / r0 (the reference forms B_k = r0^3 / 4 (...) and divides by r0^3 at each
 // use).  Powers from one reciprocal of h and one of r0.  The functions below are written over the real
-// type T: double for the forward kernels, Dual4 (dual.cuh) for the adjoint, whose value part is then the
-// forward's bit for bit.
+// type T, also for the forward-mode dual numbers (dual.cuh) by which the host tests check derivatives; a dual number's
+// value part is the double's bit for bit.
 template <class T>
 struct LatticeWall {
     T r0h, r0h2, r0h3, r0h_2, r0h_3;  // (r0/h)^k and (h/r0)^k
@@ -131,52 +131,6 @@ KIWI_LAT_EDGE LatticeEdgeT<T> lattice_edge(T h, T ih, T r0, T R_0) {
                  4. / 15. * w.r0h_3 * I1 + b23 * I0 + D2;
     }
     return {D2, D3};
-}
-
-// One vertex pyramid of the face walk (src/kernel_integral.cpp:356-400) from its right triangle's
-// lengths: legs R_0 (projection -> edge line) and t (along the edge line) in a wall at distance r0,
-// r the distance to the vertex.  The series is lattice_corner's for one pyramid: phi = atan2(t, R_0),
-// tan(phi) = t / R_0, 1 / cos^2(phi) = (R_0^2 + t^2) / R_0^2, u = t / r, 1 - u^2 = (r0^2 + R_0^2) / r^2,
-// u / a = t r0 / (R_0 r).  Beyond 2h the tier is K (-(h/r0)^3 / 4 I1 + B3 / r0^3 phi + D3) with
-// K = (r0/h)^3 / pi, i.e. (-I1 + 4 x^3 b3 phi) / (4 pi) + K D3 with x = r0 / h and x^3 b3 a polynomial in
-// x; for r0 >= 2h (B3 / r0^3 = (h/r0)^3 / 4) it is (phi - I1) / (4 pi) + K D3, the difference of the two
-// arctangents taken as atan(t s^2 R_0 / ((r + r0) (R_0^2 r + t^2 r0))), s^2 = R_0^2 + t^2, which does not
-// cancel.  The ratios come from one reciprocal of r0 r R_0 t and one of r0^2 + R_0^2.
-// ih = 1 / h; r0, R_0, t > 0; (D2, D3) the edge tier of the triangle's edge line.
-template <class T>
-KIWI_LAT T lattice_pyramid(T h, T ih, T r0, T R_0, T t, T D2, T D3) {
-    const T s2 = R_0 * R_0 + t * t;
-    const T r2 = r0 * r0 + s2;
-    const T r = sqrt(r2);
-    const T phi = atan2(t, R_0);
-    if (!(r2 < 4.0 * (h * h))) {
-        const T x = r0 * ih, x2 = x * x, x3 = x2 * x;
-        const T K = x3 * (1.0 / kPi);
-        if (r0 >= 2.0 * h)
-            return 0.25 / kPi * atan(t * s2 * R_0 / ((r + r0) * (R_0 * R_0 * r + t * t * r0))) + K * D3;
-        const T x4 = x2 * x2, x5 = x4 * x, x6 = x3 * x3;
-        const T p = r0 > h ? -4. / 3. * x3 + x4 - 0.3 * x5 + 1. / 30. * x6 - 1. / 15. + 8. / 5. * x
-                                : -2. / 3. * x3 + 0.3 * x5 - 0.1 * x6 + 7. / 5. * x;
-        return 0.25 / kPi * (p * phi - atan(t * r0 / (R_0 * r))) + K * D3;
-    }
-    const T inv = 1.0 / (r0 * r * (R_0 * t));
-    const T ir0 = r * (R_0 * t) * inv, ir = r0 * (R_0 * t) * inv, iR0 = r0 * r * t * inv;
-    const LatticeWall<T> w = lattice_wall(ih, h, ir0, r0);
-    const T K = w.r0h3 * (1.0 / kPi);
-    const T a = R_0 * ir0, a2k = a * a, u = t * ir;
-    const T tanp = t * iR0, sec2 = s2 * iR0 * iR0;
-    const T iomu2 = r2 / (r0 * r0 + R_0 * R_0);
-    const T I0 = phi;
-    const T I_2 = phi + a2k * tanp;
-    const T I_4 = phi + 2 * a2k * tanp + 1. / 3. * a2k * a2k * tanp * (2. + sec2);
-    const T logs = log1p(2.0 * u * (1.0 + u) * iomu2);
-    const T I1 = atan(tanp * r0 * ir);
-    const T I_1 = a / 2. * logs + I1;
-    const T I_3 = I_1 + a * (1. + a2k) / 4. * (2 * u * iomu2 + logs);
-    const T I_5 = I_3 + a * (1. + a2k) * (1. + a2k) / 16. * ((10 * u - 6 * u * u * u) * iomu2 * iomu2 + 3. * logs);
-    if (r2 < h * h) return K * (1. / 6. * I_2 - 3. / 40. * w.r0h2 * I_4 + 1. / 40. * w.r0h3 * I_5 + wall_b1_in(w) * I0);
-    return K * (0.25 * (4. / 3. * I_2 - w.r0h * I_3 + 0.3 * w.r0h2 * I_4 - 1. / 30. * w.r0h3 * I_5 + 1. / 15. * w.r0h_3 * I1) +
-                (r0 > h ? wall_b2_mid(w) : wall_b2_in(w)) * I0 + D2);
 }
 
 // The pyramid pair of one corner value, F(r0, a1, a2) + F(r0, a2, a1): the two right triangles of the
