@@ -21,7 +21,9 @@ the three A sum to pi/2.  Hence, with e1, e2, e3 the elementary symmetric functi
 The first form's terms are of order one and cancel to T <= 1/8; taking each logarithm's leading term into the
 polynomial leaves terms of T's own order (a third of the rounding error).  C, a polynomial in r, e2 and e3, is
 stored in powers of r - c, c the piece's outer end b for the splines and CENTRE b for the Wendland kernels (one
-piece of a high degree): where the cells' masses are smallest its own terms then do not cancel either.
+piece of a high degree), so that its own terms cancel little where the cells' masses are smallest, nor about the
+particle, where T is: with 3/4, cells of 0.02 H about the particle of the Wendland C6 kernel erred by 1.5e-12 of their
+mass, with 3/8 by 1e-14, and the cells at the support's end as before.
 
 A kernel with several pieces is the sum over its breakpoints b of difference kernels W_s - W_{s+1} supported on
 r < b.  Where the point lies beyond b, the difference kernel's mass follows from the directions in which the
@@ -201,7 +203,7 @@ def edge_poly(n, b):
 
 
 # array layouts: exponents of each coefficient
-CENTRE = Q(3,4)
+CENTRE, CONE_CENTRE = Q(3, 8), Q(3, 4)
 # C: powers of r - c for each e2^j e3^l: 13 | e2: 9 | e2^2: 5 | e3: 7 | e2 e3: 3 | e2^3: 1 | e3^2: 1
 C_BLOCKS = [((0, 0), 13), ((1, 0), 9), ((2, 0), 5), ((0, 1), 7), ((1, 1), 3), ((3, 0), 1), ((0, 2), 1)]
 LAY_Q = [(i, 0) for i in range(1, 7)] + [(i, 1) for i in range(5)] + [(i, 2) for i in range(3)] + [(0, 3)]
@@ -392,7 +394,7 @@ def kernel_box(K):
             d[n] = d.get(n, Q(0)) - c
         scs.append(scale({n: c for n, c in d.items() if c}, b))
     top = max(n for p in polys for n in p)
-    cregs = [cone_region(p, b if K.spline else CENTRE * b) for p, b in zip(polys, K.breaks)]
+    cregs = [cone_region(p, b if K.spline else CONE_CENTRE * b) for p, b in zip(polys, K.breaks)]
     cscs = []
     for s, b in enumerate(K.breaks):
         nxt = polys[s + 1] if s + 1 < len(polys) else {}

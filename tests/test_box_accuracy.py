@@ -13,6 +13,7 @@ from test_box_math import KERNELS, SUPPORT, _polygon, quad_oracle  # noqa: F401
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 DP = C.POINTER(C.c_double)
+EPS = 2.0 ** -53
 # largest errors measured (kernel mass 1), over a whole 32^3 grid too: cells 1.1e-15, 3.4e-15, 9.9e-15, 1.4e-15, 7.9e-15, 8.6e-14
 CELL = [7e-15, 2e-14, 6e-14, 9e-15, 5e-14, 5e-13]
 # and faces 1.2e-16, 4.1e-16, 9.5e-16, 2.0e-16, 1.6e-15, 1.2e-14
@@ -64,3 +65,22 @@ def test_faces(bx, quad_oracle, kernel):  # noqa: F811
         want = quad_oracle.face_integral(*p, v, kernel=-1 if kernel == 0 else kernel, h=H / SUPPORT[kernel], support=H)[0]
         worst = max(worst, abs(bx.bx_face(kernel, v.ctypes.data_as(DP), n, p.ctypes.data_as(DP), H) - want))
     assert worst <= FACE[kernel], worst
+
+
+@pytest.mark.parametrize("kernel", range(6), ids=KERNELS)
+def test_cells_about_the_particle(bx, quad_oracle, kernel):  # noqa: F811
+    """Relative to their own mass, cells of 0.02 and 0.05 of the support about the particle, where the box masses are small.
+    Bound: a cell's eight corners hold at most eight times its mass, each with some four roundings."""
+    for cell in (0.02, 0.05):
+        pos, n, lo = (0.31 * cell, 0.77 * cell, 0.45 * cell), 4, -2 * cell
+        P = {k: np.array([v]) for k, v in zip(("x", "y", "z", "vx", "vy", "vz", "m", "h"),
+                                             (*pos, 0.0, 0.0, 0.0, 1.0, 1.0 / SUPPORT[kernel]))}
+        truth = quad_oracle.sph_to_grid(P, (lo, -lo) * 3, (n, n, n), kernel=-1 if kernel == 0 else kernel,
+                                        support_in_h=SUPPORT[kernel])[4][0].reshape(n, n, n).astype(float)
+        off = [(lo + np.arange(n + 1) * (-2 * lo / n) - p) / (SUPPORT[kernel] * P["h"][0]) for p in pos]
+        T = np.zeros((n + 1,) * 3)
+        for i in np.ndindex(T.shape):
+            u = [off[a][i[a]] for a in range(3)]
+            T[i] = np.sign(u).prod() * bx.bx_mass(kernel, 0, (C.c_double * 3)(*np.abs(u)))
+        cells = np.diff(np.diff(np.diff(T, axis=0), axis=1), axis=2)
+        assert np.max(np.abs(cells - truth) / truth) <= 8 * 8 * 4 * EPS
