@@ -304,8 +304,9 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_cart_gather_tab(CartGe
 
 // The tabulated integral over every cell of the particles' bounding boxes, work items as the FP64 form's.  Built
 // here, without FMA contraction, so that every lookup lands on the reference's table entries with its weights.
-// Bound by the lookups' table reads: scattered 32-byte blocks (12 per point), about half of them from DRAM.  With the
-// indices formed per point and eight 8-byte reads per lookup, L1 was bound by its wavefronts at 21.9 ms; now 12.9.
+// Bound by the latency of the lookups' table reads: scattered 32-byte blocks (12 per point), of which 45 % hit L2 and the
+// rest come from DRAM, at half of its rate.  With the indices formed per point and eight 8-byte reads per lookup, L1 was
+// bound by its wavefronts at 21.9 ms; now 12.9.
 __global__ void __launch_bounds__(kBoxThreads, 2) k_cart_box_tab(CartGeom g, DevParticles P, const TabDev tab,
                                                                  const uint32_t* __restrict__ list,
                                                                  const int64_t* __restrict__ range,

@@ -6,11 +6,12 @@
 //      the support radius (face_reachable: the out_vert rule of src/kernel_integral.cpp:636-645 and
 //      src/mapping.cpp:187-193).  It needs no integrals.  Run twice: first it counts each particle's
 //      visited cells, then it writes them (in walk order) at the particle's offset with, per visited
-//      cell, which of its faces lead to a cell the walk processed earlier.
+//      cell, which of its faces lead to a cell the walk processed earlier; or once, through a staging area, where an
+//      earlier map told the totals.  Walks of more than kWalkCap cells run in a launch of their own.
 //  (2) a stable radix sort of the pairs by cell index: every cell's particles stay in ascending order.
-//  (3) k_vor_faces and k_vor_sum (or k_vor_gather, both in one launch): the cell's faces are staged in shared memory, each thread takes
-//      one particle of the cell's list and evaluates compute_cell_integral (src/mapping.cpp:105-206): the
-//      sum over the cell's faces of the face walk, clamped at 0; the values are then added in particle
+//  (3) k_vor_faces and k_vor_sum (or k_vor_gather, both in one launch): the cell's faces are staged in shared
+//      memory, each thread takes one particle of the cell's list and evaluates compute_cell_integral
+//      (src/mapping.cpp:105-206): the sum over the cell's faces, clamped at 0; the values are then added in particle
 //      order -- the reference's single-threaded summation order, no atomics -- and finalised as
 //      src/mapping.cpp:482-502 does.
 // The reference keeps a per-particle cache of face values keyed by the pair of cells (src/mapping.cpp:
@@ -114,8 +115,8 @@ constexpr int kGatherVertCap = 1024;  // vertices staged in shared memory per ce
 // k_vor_faces: a face item packs (pair slot << 7 | face), for cells of at most 128 faces
 constexpr int kFaceItemMaxFaces = 128;
 constexpr int kFaceItemCap = 2048;  // 4 KB of items beside the 24 KB of staged vertices
-// k_vor_faces: CTAs per SM the register allocation leaves room for (4: 128 registers a thread, a few
-// spilled; 8 % faster than 3 CTAs at 166 registers)
+// k_vor_faces: CTAs per SM the register allocation leaves room for: 4 (128 registers a thread, some spilled).  A map of
+// 64 k particles on 64 k cells: 32.3 ms, 33.1 with 3 and 38.7 with 2 (quintic spline 60.3, 60.6, 70.7).
 #ifndef KIWI_VOR_FACES_MIN_BLOCKS
 #define KIWI_VOR_FACES_MIN_BLOCKS 4
 #endif
