@@ -48,6 +48,10 @@ def test_sums_are_bounded(kiwi):
     kiwi.sph_to_grid_device(P, BOUNDS, SHAPE, whole, ctx=ctx)
     assert free - _free() < 400e6
     assert all(torch.equal(whole[k], parts[k]) for k in whole)
+    halves = _new()
+    for p in range(2):  # (two runs each, over a part's own tiles)
+        kiwi.sph_to_grid_device(P, BOUNDS, SHAPE, halves, ctx=ctx, part=p, n_parts=2)
+    assert all(torch.equal(halves[k], parts[k]) for k in halves)
     # a context whose sums hold one part's at the time the memory is taken
     ctx, little = kiwi.Context(0), _new()
     for p in range(8):
